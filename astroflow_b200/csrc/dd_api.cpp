@@ -49,31 +49,19 @@ int64_t round_up(int64_t v, int64_t m) { return (v + m - 1) / m * m; }
 // Bytes of one stage-1 sum: uint16 for 8-bit input in narrow subbands, else the
 // reference's accumulator type (uint32, or uint64 for 32-bit samples).
 int64_t inter_elem(const dd_plan& P) { return P.inter16 ? 2 : (P.nbits == 32 ? 8 : 4); }
-// Stage 1 of 8-bit samples into 32-bit sums widens its 16-bit lanes every 256
-// sources only when a subband holds more than 257 channels (257 x 255 fits).
-// 16-bit samples are always summed into 32-bit lanes (the "wide" variant).
-#ifndef DD_SUM16_WIDE
-#define DD_SUM16_WIDE 1
-#endif
-bool stage1_flush(const dd_plan& P) {
-  return (P.nbits == 8 && !P.inter16 && P.sbw > 257) || (P.nbits == 16 && DD_SUM16_WIDE);
+// Whether stage 1 sums into 32-bit words.
+bool stage1_flush(const dd_plan& P) { return !P.inter16; }
+
+// Kernel variants of the two stages: 8-bit input in subbands of at most 64 channels
+// has 16-bit subband sums, which stage 2 reads with their shifted twin.
+int stage1_kind(const dd_plan& P) {
+  return P.nbits == 16 ? kSumKindU16Wide : P.inter16 ? kSumKindU8Out16 : kSumKindU8Flush;
 }
+int stage2_kind(const dd_plan& P) { return P.inter16 ? kSumKindU16Twin : kSumKindU32; }
+// Byte offset from a subband-sum buffer to its twin (0: no twin).
+int64_t twin_offset(const dd_plan& P) { return P.twin ? P.inter_bytes : 0; }
 
 // ---- frequency table and band (dedispered.cu:1003-1031, cpucal.hpp:85-116)
-// Kernel variant of stage 2: 16-bit subband sums (8-bit input, subbands of at
-// most 64 channels) four per pipeline stage, read from the sums and their
-// shifted twin when stage 1 writes one, else 32-bit sums.
-int stage2_kind(const dd_plan& P) {
-  return P.inter16 ? (P.twin ? kSumKindU16Twin : kSumKindU16Quad) : kSumKindU32;
-}
-#ifndef DD_PAIR_STAGES
-#define DD_PAIR_STAGES 0
-#endif
-// Byte offset from a subband-sum buffer to its twin (0: no twin).
-int64_t twin_offset(const dd_plan& P) {
-  return P.twin ? (DD_PAIR_STAGES ? 2 : 1) * P.inter_bytes : 0;
-}
-
 void build_freq(dd_plan& P) {
   const int n = P.hdr.nchans;
   P.freq.resize(n);
@@ -299,6 +287,41 @@ int window_bytes(int spread, int tile, int elem, int qs = 2) {
   return sum_smem_bytes(static_cast<int>(w), 2, qs) <= 200 * 1024 ? static_cast<int>(w) : 0;
 }
 
+// Stage 1 adds the channels of a subband with the delays of kSumRows nominal DMs per
+// block.  At one output column those delays lie far apart at the low end of the
+// band (5,250 samples for 8 rows of a 4096-channel chunk to DM 3000), so each row is
+// shifted by its smallest delay in the subband (rounded down to 16 samples, which
+// keeps its stores aligned): what is left, a delay's growth inside the subband, is
+// at most a few hundred samples.  Returns the shifted table and fills the skews
+// ([row group][subband][kSumRows], relative to the group's first row) and the reach
+// of the windows.
+std::vector<int32_t> skew_stage1(dd_plan& P, std::vector<int32_t>& skew) {
+  const int64_t ngrp = (P.ndm_nom + kSumRows - 1) / kSumRows;
+  skew.assign(static_cast<size_t>(ngrp * P.nsb * kSumRows), 0);
+  std::vector<int32_t> tab(P.h_delay);
+  P.max_skew1 = P.reach1 = 0;
+  for (int64_t g = 0; g < ngrp; ++g)
+    for (int64_t sb = 0; sb < P.nsb; ++sb) {
+      const int64_t c0 = sb * P.sbw, c1 = std::min<int64_t>(c0 + P.sbw, P.dch);
+      int32_t* sk = skew.data() + (g * P.nsb + sb) * kSumRows;
+      int first = 0, last = 0, reach = 0;
+      for (int64_t r = g * kSumRows; r < std::min((g + 1) * kSumRows, P.ndm_nom); ++r) {
+        int32_t* row = tab.data() + r * P.dch;
+        const int least = *std::min_element(row + c0, row + c1);
+        if (r == g * kSumRows) first = least;
+        last = std::max(last, (least - first) & ~15);  // delays grow with the DM
+        sk[r - g * kSumRows] = last;
+        for (int64_t c = c0; c < c1; ++c) {
+          row[c] -= last;
+          reach = std::max(reach, row[c]);
+        }
+      }
+      P.max_skew1 = std::max<int64_t>(P.max_skew1, last);
+      P.reach1 = std::max<int64_t>(P.reach1, last + reach);
+    }
+  return tab;
+}
+
 void upload_desc(DevBuf& b, const std::vector<SumDesc>& d) {
   b.alloc(sizeof(SumDesc) * d.size());
   DD_CUDA_TRY(cudaMemcpy(b.p, d.data(), sizeof(SumDesc) * d.size(), cudaMemcpyHostToDevice));
@@ -322,31 +345,26 @@ void upload(DevBuf& b, const void* h, size_t bytes) {
 // (reallocated, zeroed).  Results do not depend on the tiling.
 void set_tiling(dd_plan& P, int64_t budget) {
   const int64_t kT = tile_samples();
-  // Subband sums: 32-bit words (uint64 for 32-bit samples; uint16 in builds with
-  // DD_INTER32=0).  Tile length L plus the stage-2 halo (max_res) should fill
-  // whole stage-1 block tiles T1: L = n*T1 - R with R the halo rounded to the
-  // base tile; n grows while one tile of subband sums stays within the budget and
-  // the tile is not longer than the chunk.
+  // The fewest tiles whose subband sums (tile and stage-2 halo) stay within the
+  // budget, all of the same length.
   const int64_t per_col = P.ndm_nom * P.nsb * inter_elem(P) * (P.twin ? 2 : 1);
-  const int64_t T1 = P.win1 ? sum_variant_tile(P.elem, stage1_flush(P)) : kT;
-  const int64_t R = round_up(std::max<int64_t>(P.max_res, 1), kT);
-  int64_t n = 1;
-  while (n * T1 - R < kT) ++n;
-  while (((n + 1) * T1 - R) * per_col <= budget && (n * T1 - R) < P.nout) ++n;
-  const int64_t L = std::max<int64_t>(kT, n * T1 - R);
+  const int64_t most = std::max<int64_t>(kT, budget / per_col - P.max_res);
+  const int64_t ntiles = (P.nout + most - 1) / most;
+  const int64_t L = round_up((P.nout + ntiles - 1) / ntiles, 64);
   P.tile = L;
   P.inter_budget = budget;
   // Stage-2 blocks past the tile's last column read up to one block tile beyond it
   // (their columns are not stored).
   const int64_t T2 = P.win2 ? sum_kind_tile(stage2_kind(P)) : kT;
   P.tile_pitch = round_up(round_up(L + P.max_res, kT) + T2 + 64, 64);
-  const int64_t ntiles = (P.nbin + L - 1) / L;
-  P.xpitch = round_up(ntiles * L + round_up(L + P.max_res, 8192) + P.max_delay + 8192, 64);
+  // Stage-1 windows end at most one block tile (below 8192) past their last column
+  // and its reach.
+  P.xpitch = round_up(std::max(P.nbin, P.nout + P.max_res + std::max<int64_t>(P.reach1, P.max_delay)) + 8192 + 64, 64);
   P.d_x.alloc(static_cast<size_t>(P.dch * P.xpitch) * P.elem);
   DD_CUDA_TRY(cudaMemsetAsync(P.d_x.p, 0, P.d_x.bytes, cudaStreamLegacy));
   P.inter_bytes = P.ndm_nom * P.nsb * P.tile_pitch * inter_elem(P);
   // (+256: the twin's staged windows may start one 16-byte block past the sums')
-  P.d_inter.alloc(static_cast<size_t>((DD_PAIR_STAGES ? 2 : 1) * (P.twin ? 2 : 1) * P.inter_bytes) + 256);
+  P.d_inter.alloc(static_cast<size_t>((P.twin ? 2 : 1) * P.inter_bytes) + 256);
   DD_CUDA_TRY(cudaMemsetAsync(P.d_inter.p, 0, P.d_inter.bytes, cudaStreamLegacy));
   DD_CUDA_TRY(cudaStreamSynchronize(cudaStreamLegacy));
 }
@@ -407,26 +425,24 @@ void create_subband(dd_plan& P) {
   for (int v : P.h_res) { P.max_res = std::max(P.max_res, v); minr = std::min(minr, v); }
   if (mind < 0 || minr < 0)
     throw invalid("negative dispersion delays (DM below zero or band order) are not supported");
-#ifndef DD_INTER32
-#define DD_INTER32 0
-#endif
-  P.inter16 = (P.nbits == 8 && P.sbw <= 64 && !DD_INTER32) ? 1 : 0;
+  P.inter16 = (P.nbits == 8 && P.sbw <= 64) ? 1 : 0;
   if (P.nbits <= 16) {
-    const int T1 = sum_variant_tile(P.elem, stage1_flush(P));
-    P.win1 = window_bytes(table_spread(P.h_delay, P.ndm_nom, P.dch, kSumRows, 0), T1, P.elem);
-  }
-  // the twin needs the staged stage 1 (which writes it) and the staged stage 2
-  P.twin = (P.inter16 && P.win1 && DD_SUM16_TWIN) ? 1 : 0;
-  if (P.nbits <= 16) {
-    // stage-2 sources: the stage-1 sums (uint16 or uint32)
-    const int e2 = static_cast<int>(inter_elem(P));
-    const int T2 = sum_kind_tile(stage2_kind(P));
-    P.win2 = window_bytes(table_spread(P.h_res, P.dm_steps, P.nsb, kSumRows, P.ndm0), T2, e2,
+    std::vector<int32_t> skew;
+    const std::vector<int32_t> tab = skew_stage1(P, skew);
+    P.win1 = window_bytes(table_spread(tab, P.ndm_nom, P.dch, kSumRows, 0),
+                          sum_kind_tile(stage1_kind(P)), P.elem);
+    P.win2 = window_bytes(table_spread(P.h_res, P.dm_steps, P.nsb, kSumRows, P.ndm0),
+                          sum_kind_tile(stage2_kind(P)), static_cast<int>(inter_elem(P)),
                           sum_kind_qs(stage2_kind(P)));
+    // 16-bit sums: the staged stage 2 reads the twin that the staged stage 1 writes
+    P.twin = (P.inter16 && P.win1 && P.win2) ? 1 : 0;
+    if (P.inter16 && !P.twin) P.win2 = 0;
+    if (P.win1) {
+      upload_desc(P.d_desc1, build_sum_desc(tab, P.ndm_nom, P.dch, 0));
+      upload(P.d_skew1, skew.data(), sizeof(int32_t) * skew.size());
+    }
+    if (P.win2) upload_desc(P.d_desc2, build_sum_desc(P.h_res, P.dm_steps, P.nsb, P.ndm0));
   }
-  if (!P.win2) P.twin = 0;
-  if (P.win1) upload_desc(P.d_desc1, build_sum_desc(P.h_delay, P.ndm_nom, P.dch, 0));
-  if (P.win2) upload_desc(P.d_desc2, build_sum_desc(P.h_res, P.dm_steps, P.nsb, P.ndm0));
   set_tiling(P, int64_t(DD_INTER_MB) << 20);
   if (ds > 1 || callsite_zdm_active(P))
     P.d_binned.alloc(static_cast<size_t>(P.nbin * P.hdr.nchans) * P.elem);
@@ -444,7 +460,7 @@ void create_subband(dd_plan& P) {
 void set_brute_window(dd_plan& P) {
   P.winb = 0;
   if (P.p.time_downsample == 1 && P.nbits <= 16) {
-    const int T = sum_variant_tile(P.elem, P.nbits == 8 || P.nbits == 16);
+    const int T = sum_kind_tile(P.nbits == 8 ? kSumKindU8Flush : kSumKindU16Wide);
     P.winb = window_bytes(table_spread(P.h_delay, P.dm_steps, P.nc, kSumRows, 0), T, P.elem);
   }
   if (P.winb) upload_desc(P.d_descb, build_sum_desc(P.h_delay, P.dm_steps, P.nc, 0));
@@ -607,7 +623,7 @@ void run_rfi_and_prep(dd_plan& P, const void* input, uint8_t* masks_out, uint32_
 
 // Staged-sum launches of one subband time tile starting at t0 (stage 1: the
 // prepared input into the tile of subband sums; stage 2: the tile into the output).
-SumLaunch stage1_launch(const dd_plan& P, int64_t t0, int buf = 0) {
+SumLaunch stage1_launch(const dd_plan& P, int64_t t0) {
   SumLaunch L{};
   L.mode = SumLaunch::kStage1;
   L.src = static_cast<const char*>(P.d_x.p);
@@ -618,32 +634,31 @@ SumLaunch stage1_launch(const dd_plan& P, int64_t t0, int buf = 0) {
   L.nsrc_total = P.dch;
   L.nrows_total = P.ndm_nom;
   L.group = P.sbw;
-  L.rows_per_block = kSumRows;
   L.nsb_out = P.nsb;
-  L.out = static_cast<char*>(P.d_inter.p) + buf * P.inter_bytes;
+  L.out = static_cast<char*>(P.d_inter.p);
   L.out_pitch = P.tile_pitch * inter_elem(P);
   L.out_col0 = 0;
   L.out_elem = static_cast<int>(inter_elem(P));
-  L.ncols = P.tile + P.max_res;
+  L.ncols = std::min<int64_t>(P.tile, P.nout - t0) + P.max_res;
+  L.skew = P.d_skew1.as<int32_t>();
+  L.max_skew = P.max_skew1;
   L.win_bytes = P.win1;
   L.src_bytes = P.elem;
   L.flush = stage1_flush(P) ? 1 : 0;
-  L.lane_per = 1;
   L.grid_y = static_cast<unsigned>((P.ndm_nom + kSumRows - 1) / kSumRows);
   L.grid_z = static_cast<unsigned>(P.nsb);
   L.desc = P.d_desc1.as<SumDesc>();
   L.desc_pitch = P.dch;
   L.stages = P.stages_override ? P.stages_override : sum_kind_stages(sum_kind(L), P.win1);
   L.err = P.d_err.as<int>();
-  L.one = 1;
   L.twin_off = twin_offset(P);
   return L;
 }
 
-SumLaunch stage2_launch(const dd_plan& P, int64_t t0, void* output, int buf = 0) {
+SumLaunch stage2_launch(const dd_plan& P, int64_t t0, void* output) {
   SumLaunch L{};
   L.mode = SumLaunch::kStage2;
-  L.src = static_cast<const char*>(P.d_inter.p) + buf * P.inter_bytes;
+  L.src = static_cast<const char*>(P.d_inter.p);
   L.src_pitch = P.tile_pitch * inter_elem(P);
   L.off = P.d_res.as<int32_t>();
   L.off_pitch = P.nsb;
@@ -651,7 +666,6 @@ SumLaunch stage2_launch(const dd_plan& P, int64_t t0, void* output, int buf = 0)
   L.nsrc_total = P.nsb;
   L.nrows_total = P.dm_steps;
   L.group = P.ndm0;
-  L.rows_per_block = kSumRows;
   L.out = static_cast<char*>(output);
   L.out_pitch = P.nout * 4;
   L.out_col0 = t0;
@@ -660,14 +674,12 @@ SumLaunch stage2_launch(const dd_plan& P, int64_t t0, void* output, int buf = 0)
   L.win_bytes = P.win2;
   L.src_bytes = static_cast<int>(inter_elem(P));
   L.flush = 0;
-  L.lane_per = P.inter16 ? 65535 / (255 * P.sbw) : 1;  // >= 4 for subbands of <= 64 channels
   L.grid_y = static_cast<unsigned>(P.ndm_nom * ((P.ndm0 + kSumRows - 1) / kSumRows));
   L.grid_z = 1;
   L.desc = P.d_desc2.as<SumDesc>();
   L.desc_pitch = P.nsb;
   L.stages = P.stages_override ? P.stages_override : sum_kind_stages(stage2_kind(P), P.win2);
   L.err = P.d_err.as<int>();
-  L.one = 1;
   L.twin_off = twin_offset(P);
   return L;
 }
@@ -689,32 +701,6 @@ void run_subband(dd_plan& P, const void* input, void* output, uint8_t* masks_out
   run_rfi_and_prep(P, input, masks_out, bounds_out, prepped, st);
   if (pf) pf->prep.emplace_back(a, pf->mark());
   if (before_sums) before_sums();
-  // With DD_PAIR_STAGES, stage 1 of tile k+1 shares a launch with stage 2 of tile
-  // k (alternating subband-sum buffers).  Measured on B200 at the headline size it
-  // is no faster than running the stages one after another (148.6 vs 145.8 ms per
-  // step), so the default build keeps them apart.
-  if (DD_PAIR_STAGES && !pf && P.win1 && P.win2 && P.nout > P.tile) {
-    const int64_t ntiles = (P.nout + P.tile - 1) / P.tile;
-    launch_sum(stage1_launch(P, 0, 0), st);
-    bool paired = true;
-    for (int64_t k = 1; k <= ntiles; ++k) {
-      const int64_t tprev = (k - 1) * P.tile;
-      if (before_out) before_out(tprev, std::min<int64_t>(P.tile, P.nout - tprev));
-      const SumLaunch s2 = stage2_launch(P, tprev, output, static_cast<int>((k - 1) & 1));
-      if (k < ntiles) {
-        const SumLaunch s1 = stage1_launch(P, k * P.tile, static_cast<int>(k & 1));
-        if (!(paired = launch_sum_pair(s1, s2, st))) {
-          launch_sum(s2, st);
-          launch_sum(s1, st);
-        }
-      } else {
-        launch_sum(s2, st);
-      }
-      if (after_tile) after_tile(tprev, std::min<int64_t>(P.tile, P.nout - tprev));
-    }
-    (void)paired;
-    return;
-  }
   for (int64_t t0 = 0; t0 < P.nout; t0 += P.tile) {
     cudaEvent_t b1 = pf ? pf->mark() : nullptr;
     if (P.win1) {
@@ -730,7 +716,7 @@ void run_subband(dd_plan& P, const void* input, void* output, uint8_t* masks_out
       s1.ndm_nom = P.ndm_nom;
       s1.sbw = P.sbw;
       s1.t0 = t0;
-      s1.ncols = P.tile + P.max_res;
+      s1.ncols = std::min<int64_t>(P.tile, P.nout - t0) + P.max_res;
       s1.inter = P.d_inter.p;
       s1.tile_pitch = P.tile_pitch;
       s1.inter16 = P.inter16;
@@ -775,7 +761,6 @@ SumLaunch brute_launch(const dd_plan& P, void* output) {
   L.base = 0;
   L.nsrc_total = P.nc;
   L.nrows_total = P.dm_steps;
-  L.rows_per_block = kSumRows;
   L.out = static_cast<char*>(output);
   L.out_pitch = P.out_cols * 4;
   L.out_col0 = 0;
@@ -784,14 +769,12 @@ SumLaunch brute_launch(const dd_plan& P, void* output) {
   L.win_bytes = P.winb;
   L.src_bytes = P.elem;
   L.flush = (P.nbits == 8 || P.nbits == 16) ? 1 : 0;  // 8-bit: widened lanes; 16-bit: 32-bit sums
-  L.lane_per = 1;
   L.grid_y = static_cast<unsigned>((P.dm_steps + kSumRows - 1) / kSumRows);
   L.grid_z = 1;
   L.desc = P.d_descb.as<SumDesc>();
   L.desc_pitch = P.nc;
   L.stages = sum_kind_stages(sum_kind(L), P.winb);
   L.err = P.d_err.as<int>();
-  L.one = 1;
   return L;
 }
 
@@ -864,7 +847,7 @@ void check_device_error(dd_plan& P, cudaStream_t st) {
 int64_t workspace_of(const dd_plan& P) {
   const DevBuf* bufs[] = {&P.d_delay, &P.d_res, &P.d_lags, &P.d_bad_keep, &P.d_win, &P.d_seg_t0,
                           &P.d_binned, &P.d_bin_lut, &P.d_x, &P.d_inter, &P.d_stats, &P.d_iqrm_scratch,
-                          &P.d_masks, &P.d_segmask, &P.d_zdm, &P.d_desc1, &P.d_desc2,
+                          &P.d_masks, &P.d_segmask, &P.d_zdm, &P.d_skew1, &P.d_desc1, &P.d_desc2,
                           &P.d_descb, &P.d_err};
   int64_t t = 0;
   for (auto* b : bufs) t += static_cast<int64_t>(b->bytes);

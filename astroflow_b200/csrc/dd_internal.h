@@ -82,6 +82,8 @@ struct dd_plan {
   int64_t tile_pitch = 0;    // row pitch of the inter tile (elements)
   int64_t xpitch = 0;        // row pitch of the channel-major prepared input (elements)
   int win1 = 0, win2 = 0;    // staged window bytes of the shared-memory sums (0: not used)
+  int64_t max_skew1 = 0;     // largest row skew of stage 1
+  int64_t reach1 = 0;        // largest offset a stage-1 window reads past its column
 
   // brute-force geometry (CPU path semantics)
   int64_t nc = 0;            // channels summed, [cs, ce)
@@ -116,7 +118,7 @@ struct dd_plan {
   bool host_pending = false;          // host_done marks copies a later run must wait for
   std::vector<cudaEvent_t> host_tile_copied;  // per time tile: its output copy of the last run
   int64_t host_tile = 0;                      // the time tile those copies were made with
-  dd::DevBuf d_inter;    // stage-1 tile (two buffers in a DD_PAIR_STAGES build)
+  dd::DevBuf d_inter;    // stage-1 tile, then its twin
   dd::DevBuf d_bin_lut;  // full-bin values of the time binning (8/16-bit samples, ds > 1)
   int64_t inter_bytes = 0; // bytes of one buffer
   int64_t inter_budget = 0; // subband-sum bytes per time tile the tiling was set for
@@ -126,6 +128,7 @@ struct dd_plan {
   dd::DevBuf d_masks;    // IQRM window masks [nwin][nchans]
   dd::DevBuf d_segmask;  // [nseg][nchans]
   dd::DevBuf d_zdm;      // per-sample zero-DM offsets [nbin]
+  dd::DevBuf d_skew1;                    // row skews of stage 1 (SumLaunch::skew)
   dd::DevBuf d_desc1, d_desc2, d_descb;  // staging descriptors: stage 1, stage 2, brute force
   dd::DevBuf d_err;      // device error word of the staged sums (0: no error)
   double adds = 0;
@@ -268,21 +271,11 @@ inline void allow_dynamic_smem(K kernel, size_t dynamic_smem) {
 }
 
 // ---- shared-memory staged sums (dd_sumsmem.cu) ----
-constexpr int kSumRows = 8;  // output rows per block
-// Groups of warps the block's rows are split over: each group covers the whole
-// tile for kSumRows/ROWSPLIT rows (fewer accumulators per thread, more words per
-// lane).  Measured at the headline size (ms, stage 1 / stage 2): one group, 5
-// words per lane 77.0 / 53.9; two groups, 5 words 80.0 / 51.4; two groups, 9
-// words 77.6 / 50.9; two groups, 7 words 82.1 / 52.1.  The quad kernel (stage 2)
-// takes two groups of 9 words, the 8-bit kernels one group of 5.
-#ifndef DD_SUM_ROWSPLIT
-#define DD_SUM_ROWSPLIT 1
-#endif
-#ifndef DD_SUM16Q_ROWSPLIT
-#define DD_SUM16Q_ROWSPLIT 2
-#endif
-constexpr int kSumRowsPT = kSumRows / DD_SUM_ROWSPLIT;
-constexpr int kSumRowsPTQ = kSumRows / DD_SUM16Q_ROWSPLIT;
+// Output rows per block.  A staged window serves all of them, so the traffic from L2
+// into shared memory falls with their number; rows are split over warp groups that
+// each cover the whole tile (kSumRowsPT* rows per thread).
+constexpr int kSumRows = 16;
+constexpr int kSumRowsPT8 = 8, kSumRowsPTW = 8, kSumRowsPT32 = 8, kSumRowsPTT = 4;
 // Staging descriptor of one (row group, source) pair of a staged sum: the
 // smallest offset of the group's rows for that source, the spread of their
 // offsets, and each row's offset relative to the smallest.  Built on the host
@@ -293,7 +286,7 @@ struct SumDesc {
   uint16_t rel[kSumRows];
   int32_t pad[2];
 };
-static_assert(sizeof(SumDesc) == 32, "SumDesc is 32 bytes");
+static_assert(sizeof(SumDesc) == 48, "bulk copies move whole 16-byte units");
 struct SumLaunch {
   enum Mode { kStage1 = 0, kStage2 = 1, kBrute = 2 };
   int mode;
@@ -305,7 +298,6 @@ struct SumLaunch {
   int64_t nsrc_total;      // stage 1: channels of the band; stage 2: subbands; brute: channels
   int64_t nrows_total;     // stage 1: nominal DMs; stage 2 and brute: DM trials
   int group;               // stage 1: subband width; stage 2: fine DMs per nominal DM
-  int rows_per_block;      // kSumRows
   int64_t nsb_out;         // stage 1: subbands (inter rows are (j, sb))
   char* out;               // byte address of output row 0, column 0
   int64_t out_pitch;       // bytes between output rows (stage 1: between (j, sb) rows)
@@ -314,14 +306,17 @@ struct SumLaunch {
   int64_t ncols;           // columns of the launch
   int win_bytes;           // bytes of one staged source window
   int src_bytes;           // 1 or 2
-  int flush;               // 8-bit sources: add the lanes into the output every 256 sources
-  int lane_per;            // 16-bit sources: sources per 16-bit lane before widening
+  int flush;               // 8- and 16-bit sources into 32-bit sums
   unsigned grid_y, grid_z;
   const SumDesc* desc;     // [grid_y][desc_pitch] staging descriptors
   int64_t desc_pitch;      // descriptors per row group (= columns of the offset table)
+  // Stage 1: row r of group y and subband sb computes column u - skew of its row at
+  // position u of the launch, skew[(y * nsb_out + sb) * kSumRows + r] (see
+  // skew_stage1); the launch spans ncols + max_skew positions.
+  const int32_t* skew;
+  int64_t max_skew;
   int stages;              // staged source pairs in flight (2..4)
   int* err;                // device error word: set when a bounded wait gives up
-  unsigned one;            // 1 (a multiplier the compiler cannot fold)
   // 16-bit subband sums with a one-sample-shifted twin (0: none): the twin of the
   // element at byte address a sits at a + twin_off and holds the element before
   // it, twin[i] = sums[i - 1].  Stage 1 writes both; stage 2 reads a source whose
@@ -339,7 +334,7 @@ constexpr int kSumMaxStages = DD_SUM_MAX_STAGES;  // staged source pairs in flig
 void launch_sum(const SumLaunch& L, cudaStream_t st);
 int sum_tile_samples(int src_bytes, int nw);
 // Shared memory of a staged sum with `stages` pairs in flight.
-// qs: source windows per pipeline stage (2, or 4 for the quad kernel).
+// qs: source windows per pipeline stage.
 size_t sum_smem_bytes(int win_bytes, int stages, int qs = 2);
 // Pairs in flight that fit the shared memory of two blocks per SM (at least 2),
 // next to `extra` bytes the kernel needs besides its ring (cap_kb: the shared
@@ -356,21 +351,11 @@ std::vector<SumDesc> build_sum_desc(const std::vector<int32_t>& tab, int64_t nro
 // Device error codes of the staged sums.
 constexpr int kErrWaitFull = 1;   // a consumer gave up waiting for a staged window
 constexpr int kErrWaitEmpty = 2;  // the producer gave up waiting for a free stage
-// Tile (samples per block) of the kernel launch_sum picks for these sources.
-// Words per lane of the staged sums (tile = 8 warps x 32 lanes x words x samples
-// per word): 16-bit sources, 8-bit sources, 8-bit sources widened to 32 bits.
-#ifndef DD_SUM16_NW
-#define DD_SUM16_NW 4
-#endif
+// Words per lane of the staged sums (an odd number of consecutive words for 8- and
+// 16-bit samples, interleaved words for the others) and blocks per SM they are
+// compiled for (register budget).
 #ifndef DD_SUM8_NW
 #define DD_SUM8_NW 5
-#endif
-#ifndef DD_SUM8F_NW
-#define DD_SUM8F_NW 5
-#endif
-// Blocks per SM the staged-sum kernels are compiled for (register budget).
-#ifndef DD_SUM16_MINB
-#define DD_SUM16_MINB 2
 #endif
 #ifndef DD_SUM8_MINB
 #define DD_SUM8_MINB 2
@@ -381,19 +366,8 @@ constexpr int kErrWaitEmpty = 2;  // the producer gave up waiting for a free sta
 #ifndef DD_SUM32_MINB
 #define DD_SUM32_MINB 2
 #endif
-constexpr int kSum32NW = DD_SUM32_NW;  // words per lane of the 32-bit staged sum
 #ifndef DD_SUM16W_NW
 #define DD_SUM16W_NW 5
-#endif
-// Warp groups the block's rows are split over in the 16-bit-into-32-bit kernel,
-// blocks per SM it is built for and the shared memory (KB) it stays within.  Two
-// warp groups of four rows at three blocks per SM take stage 1 of the
-// 8192-channel 16-bit case on 2^18 samples (DM 0:0.25:500) from 29.5 to 24.5 ms
-// but leave the full configuration (2^21 samples, three ranges) unchanged (first
-// range 194.8 against 195.6 ms), so one group at two blocks per SM stays the
-// default.
-#ifndef DD_SUM16W_ROWSPLIT
-#define DD_SUM16W_ROWSPLIT 1
 #endif
 #ifndef DD_SUM16W_MINB
 #define DD_SUM16W_MINB 2
@@ -401,70 +375,34 @@ constexpr int kSum32NW = DD_SUM32_NW;  // words per lane of the 32-bit staged su
 #ifndef DD_SUM16W_SMEM_KB
 #define DD_SUM16W_SMEM_KB 100
 #endif
-constexpr int kSumRowsPTW = kSumRows / DD_SUM16W_ROWSPLIT;
-// Words per lane of the 16-bit quad stage-2 kernel (odd: conflict-free consecutive words).
-#ifndef DD_SUM16Q_NW
-#define DD_SUM16Q_NW 9
-#endif
-constexpr int kSum16QNW = DD_SUM16Q_NW;
-// Stage 2 on 16-bit sums with a shifted twin (k_sum_u16t): words per lane (lanes
-// own interleaved words, so any count is conflict-free) and warp groups the
-// block's rows are split over.
 #ifndef DD_SUM16T_NW
 #define DD_SUM16T_NW 6
 #endif
-#ifndef DD_SUM16T_ROWSPLIT
-#define DD_SUM16T_ROWSPLIT 2
-#endif
-constexpr int kSum16TNW = DD_SUM16T_NW;
-constexpr int kSumRowsPTT = kSumRows / DD_SUM16T_ROWSPLIT;
-// Stage 2 of 8-bit input reads a twin of the subband sums (1) or aligns odd
-// offsets with byte permutes (0, the quad kernel).  Measured at the headline
-// size (ms, stage 1 / stage 2 / step): quad 69.3 / 46.8 / 120.6; twin with the
-// stage-1 twin stored lane by lane 81.2 / 36.6 / 122.1; twin stored in 16-byte
-// chunks through shared memory 71.1 / 36.6 / 112.0.
-#ifndef DD_SUM16_TWIN
-#define DD_SUM16_TWIN 1
-#endif
-// flush: 8-bit lanes added into the output every 256 sources; 16-bit sources summed into
-// 32-bit lanes (the k_sum_u16w variant).
-inline int sum_variant_tile(int src_bytes, bool flush) {
-  return src_bytes == 4   ? sum_tile_samples(4, kSum32NW)
-         : src_bytes == 2 ? (flush ? sum_tile_samples(2, DD_SUM16W_NW) / DD_SUM16W_ROWSPLIT
-                                   : sum_tile_samples(2, DD_SUM16_NW))
-                          : sum_tile_samples(1, flush ? DD_SUM8F_NW : DD_SUM8_NW) / DD_SUM_ROWSPLIT;
-}
-// Tile (samples per block) of a kernel variant (SumKind below).
-inline int sum_kind_tile(int kind);
-// Kernel variant of a staged sum: 8-bit sources into 16-bit sums, 8-bit sources
-// widened to 32 bits (many sources), 8-bit, 16-bit and 32-bit sources.
-enum SumKind { kSumKindU8Out16 = 0, kSumKindU8Flush = 1, kSumKindU8 = 2, kSumKindU16 = 3,
-               kSumKindU32 = 4, kSumKindU16Wide = 5, kSumKindU16Quad = 6, kSumKindU16Twin = 7 };
-constexpr int kSumKinds = 8;
+constexpr int kSum32NW = DD_SUM32_NW, kSum16TNW = DD_SUM16T_NW;
+// Kernel variant of a staged sum: 8-bit sources into 16-bit sums, 8-bit sources into
+// 32-bit sums, 32-bit sources, 16-bit sources into 32-bit sums, and 16-bit subband
+// sums with their one-sample-shifted twin (stage 2 of 8-bit input).
+enum SumKind { kSumKindU8Out16 = 0, kSumKindU8Flush = 1, kSumKindU32 = 2, kSumKindU16Wide = 3,
+               kSumKindU16Twin = 4 };
+constexpr int kSumKinds = 5;
 int sum_kind(const SumLaunch& L);
+// Tile (samples per block) of a kernel variant.
 inline int sum_kind_tile(int kind) {
   switch (kind) {
-    case kSumKindU8Out16: case kSumKindU8: return sum_tile_samples(1, DD_SUM8_NW) / DD_SUM_ROWSPLIT;
-    case kSumKindU8Flush: return sum_tile_samples(1, DD_SUM8F_NW) / DD_SUM_ROWSPLIT;
-    case kSumKindU16: return sum_tile_samples(2, DD_SUM16_NW);
-    case kSumKindU16Wide: return sum_tile_samples(2, DD_SUM16W_NW) / DD_SUM16W_ROWSPLIT;
-    case kSumKindU16Quad: return sum_tile_samples(2, kSum16QNW) / DD_SUM16Q_ROWSPLIT;
-    case kSumKindU16Twin: return sum_tile_samples(2, kSum16TNW) / DD_SUM16T_ROWSPLIT;
-    default: return sum_tile_samples(4, kSum32NW);
+    case kSumKindU8Out16: case kSumKindU8Flush:
+      return sum_tile_samples(1, DD_SUM8_NW) * kSumRowsPT8 / kSumRows;
+    case kSumKindU16Wide: return sum_tile_samples(2, DD_SUM16W_NW) * kSumRowsPTW / kSumRows;
+    case kSumKindU16Twin: return sum_tile_samples(2, kSum16TNW) * kSumRowsPTT / kSumRows;
+    default: return sum_tile_samples(4, kSum32NW) * kSumRowsPT32 / kSumRows;
   }
 }
-// Source windows per pipeline stage of a kernel variant: 4 for kSumKindU16Quad, 8
-// for kSumKindU16Twin (four sources, each with its twin), else 2.
-inline int sum_kind_qs(int kind) {
-  return kind == kSumKindU16Quad ? 4 : kind == kSumKindU16Twin ? 8 : 2;
-}
+// Source windows per pipeline stage of a kernel variant: 8 for kSumKindU16Twin (four
+// sources, each with its twin), else 2.
+inline int sum_kind_qs(int kind) { return kind == kSumKindU16Twin ? 8 : 2; }
 // Shared memory of a launch (its variant's windows per stage, plus the variant's
 // staging past the ring, sum_kind_extra_smem).
 size_t sum_launch_smem(const SumLaunch& L);
 size_t sum_kind_extra_smem(int kind);
-// Stage 1 of one tile and stage 2 of another in one launch (false: no paired
-// kernel for these variants; nothing launched).
-bool launch_sum_pair(const SumLaunch& L1, const SumLaunch& L2, cudaStream_t st);
 unsigned sum_grid_x(const SumLaunch& L);
 // One group of a batched (persistent) launch: all blocks of one staged sum.
 struct SumBatchGroup {
