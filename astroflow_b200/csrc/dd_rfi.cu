@@ -109,7 +109,47 @@ __global__ void k_time_binning_lut(const T* __restrict__ in, T* __restrict__ out
 }
 
 // ---------------------------------------------------------------- IQRM sums
-// Block: 256 consecutive channels of [cs, cs+csub); grid.y: time chunks.
+// Calls f(a, b, w) for the runs [a, b) of samples of [lo, hi) that the same windows
+// cover, so that overlapping windows (5 s every 2.5 s) share one read of the chunk; w
+// is the first window that ends after a (starts and ends both grow along the list).
+template <typename F>
+__device__ __forceinline__ void for_window_runs(const uint32_t* __restrict__ win, int nwin,
+                                                int64_t lo, int64_t hi, F&& f) {
+  int first = 0, last = nwin;
+  while (first < last) {
+    const int mid = (first + last) >> 1;
+    if (static_cast<int64_t>(win[2 * mid + 1]) > lo) last = mid; else first = mid + 1;
+  }
+  for (int64_t a = lo; a < hi;) {
+    while (first < nwin && static_cast<int64_t>(win[2 * first + 1]) <= a) ++first;
+    int64_t b = hi;
+    bool covered = false;
+    for (int w = first; w < nwin; ++w) {
+      const int64_t t0 = win[2 * w], t1 = win[2 * w + 1];
+      if (t1 < b) b = t1;
+      if (t0 > a) {
+        if (t0 < b) b = t0;
+        break;
+      }
+      covered = true;
+    }
+    if (covered) f(a, b, first);
+    a = b;
+  }
+}
+// Adds one channel's sums of the run that starts at sample a to the windows covering
+// it, from window w on.
+__device__ __forceinline__ void add_window_sums(const uint32_t* __restrict__ win, int nwin, int w, int64_t a,
+                                                int64_t csub, int64_t i, unsigned long long s,
+                                                unsigned long long q,
+                                                unsigned long long* __restrict__ sums) {
+  for (; w < nwin && static_cast<int64_t>(win[2 * w]) <= a; ++w) {
+    atomicAdd(&sums[(static_cast<int64_t>(w) * 2) * csub + i], s);
+    atomicAdd(&sums[(static_cast<int64_t>(w) * 2 + 1) * csub + i], q);
+  }
+}
+
+// One channel per thread; grid.y: chunks of samples.
 template <typename T>
 __global__ void k_iqrm_stats(const T* __restrict__ x, int64_t nsamp, int64_t nchans, int64_t cs,
                              int64_t csub, const uint32_t* __restrict__ win, int nwin,
@@ -119,57 +159,102 @@ __global__ void k_iqrm_stats(const T* __restrict__ x, int64_t nsamp, int64_t nch
   const int64_t c = cs + i;
   const int64_t lo = static_cast<int64_t>(blockIdx.y) * chunk;
   const int64_t hi = lo + chunk < nsamp ? lo + chunk : nsamp;
-  for (int w = 0; w < nwin; ++w) {
-    int64_t a = win[2 * w] > lo ? win[2 * w] : lo;
-    int64_t b = win[2 * w + 1] < hi ? win[2 * w + 1] : hi;
-    if (a >= b) continue;
+  for_window_runs(win, nwin, lo, hi, [&](int64_t a, int64_t b, int w) {
     unsigned long long s = 0, s2 = 0;
     for (int64_t t = a; t < b; ++t) {
       unsigned long long v = x[t * nchans + c];
       s += v;
       s2 += v * v;
     }
-    atomicAdd(&sums[(static_cast<int64_t>(w) * 2) * csub + i], s);
-    atomicAdd(&sums[(static_cast<int64_t>(w) * 2 + 1) * csub + i], s2);
-  }
+    add_window_sums(win, nwin, w, a, csub, i, s, s2, sums);
+  });
 }
 
-// 8-bit samples, four channels per thread (one aligned 32-bit load per row, a
-// warp reading 128 contiguous bytes): thread k covers channels (cs & ~3) + 4k ..
-// + 3; per window and time chunk it keeps 32-bit partial sums (a chunk of at
-// most 1024 rows: 1024 x 255^2 < 2^32) and adds them to the 64-bit sums of the
-// channels inside [cs, cs+csub).  Needs nchans % 4 == 0 and an aligned input.
-__global__ void k_iqrm_stats_u8w(const uint8_t* __restrict__ x, int64_t nsamp, int64_t nchans,
-                                 int64_t cs, int64_t csub, const uint32_t* __restrict__ win,
-                                 int nwin, int64_t chunk, unsigned long long* __restrict__ sums) {
+// 8-bit samples, four channels per thread: thread k covers channels (cs & ~3) + 4k
+// .. + 3, one 32-bit word per row.  The words of four rows are transposed by byte
+// permutes into one word per channel, whose sum and sum of squares are one dot
+// product each: one operation per sample where taking the bytes apart took three.
+// A chunk holds at most 1024 rows, so that the 32-bit partial sums cannot overflow
+// (1024 x 255^2 < 2^32).  Needs nchans % 4 == 0 and an aligned input.  Bound by the
+// reads (2,048 channels x 75,001 samples in two overlapping windows: 59 us, 298 us
+// with one read per window, byte-wise sums and 1024-row chunks only).
+__global__ void __launch_bounds__(128) k_iqrm_stats_u8w(
+    const uint8_t* __restrict__ x, int64_t nsamp, int64_t nchans, int64_t cs, int64_t csub,
+    const uint32_t* __restrict__ win, int nwin, int64_t chunk, unsigned long long* __restrict__ sums) {
   const int64_t c4 = (cs & ~int64_t(3)) + 4 * (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x);
   if (c4 >= cs + csub) return;
   const int64_t lo = static_cast<int64_t>(blockIdx.y) * chunk;
   const int64_t hi = lo + chunk < nsamp ? lo + chunk : nsamp;
-  for (int w = 0; w < nwin; ++w) {
-    const int64_t a = win[2 * w] > lo ? win[2 * w] : lo;
-    const int64_t b = win[2 * w + 1] < hi ? win[2 * w + 1] : hi;
-    if (a >= b) continue;
+  for_window_runs(win, nwin, lo, hi, [&](int64_t a, int64_t b, int w) {
     uint32_t s[4] = {0u, 0u, 0u, 0u}, q[4] = {0u, 0u, 0u, 0u};
-#pragma unroll 8
-    for (int64_t t = a; t < b; ++t) {  // unrolled: eight rows' loads in flight
-      const uint32_t v = __ldg(reinterpret_cast<const uint32_t*>(x + t * nchans + c4));
+    auto add4 = [&](uint32_t v0, uint32_t v1, uint32_t v2, uint32_t v3) {
+      const uint32_t lo01 = __byte_perm(v0, v1, 0x5140), hi01 = __byte_perm(v0, v1, 0x7362);
+      const uint32_t lo23 = __byte_perm(v2, v3, 0x5140), hi23 = __byte_perm(v2, v3, 0x7362);
+      const uint32_t o[4] = {__byte_perm(lo01, lo23, 0x5410), __byte_perm(lo01, lo23, 0x7632),
+                             __byte_perm(hi01, hi23, 0x5410), __byte_perm(hi01, hi23, 0x7632)};
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
-        const uint32_t e = (v >> (8 * k)) & 0xffu;
-        s[k] += e;
-        q[k] += e * e;
+        s[k] = __dp4a(o[k], 0x01010101u, s[k]);
+        q[k] = __dp4a(o[k], o[k], q[k]);
       }
+    };
+    const uint8_t* p = x + a * nchans + c4;
+    auto row = [&](int64_t r) { return __ldg(reinterpret_cast<const uint32_t*>(p + r * nchans)); };
+    const int64_t n = b - a;
+    int64_t r = 0;
+    for (; r + 16 <= n; r += 16) {  // sixteen rows' loads in flight
+      uint32_t v[16];
+#pragma unroll
+      for (int k = 0; k < 16; ++k) v[k] = row(r + k);
+#pragma unroll
+      for (int k = 0; k < 16; k += 4) add4(v[k], v[k + 1], v[k + 2], v[k + 3]);
     }
+    for (; r < n; ++r) add4(row(r), 0u, 0u, 0u);
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       const int64_t ch = c4 + k;
-      if (ch < cs || ch >= cs + csub) continue;
-      const int64_t i = ch - cs;
-      atomicAdd(&sums[(static_cast<int64_t>(w) * 2) * csub + i], static_cast<unsigned long long>(s[k]));
-      atomicAdd(&sums[(static_cast<int64_t>(w) * 2 + 1) * csub + i], static_cast<unsigned long long>(q[k]));
+      if (ch >= cs && ch < cs + csub) add_window_sums(win, nwin, w, a, csub, ch - cs, s[k], q[k], sums);
     }
-  }
+  });
+}
+
+// 16-bit samples, two channels per thread (one 32-bit word per row): 32-bit sums and
+// 64-bit sums of squares per chunk.  Needs nchans % 2 == 0 and an aligned input.
+__global__ void __launch_bounds__(128) k_iqrm_stats_u16w(
+    const uint16_t* __restrict__ x, int64_t nsamp, int64_t nchans, int64_t cs, int64_t csub,
+    const uint32_t* __restrict__ win, int nwin, int64_t chunk, unsigned long long* __restrict__ sums) {
+  const int64_t c2 = (cs & ~int64_t(1)) + 2 * (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x);
+  if (c2 >= cs + csub) return;
+  const int64_t lo = static_cast<int64_t>(blockIdx.y) * chunk;
+  const int64_t hi = lo + chunk < nsamp ? lo + chunk : nsamp;
+  for_window_runs(win, nwin, lo, hi, [&](int64_t a, int64_t b, int w) {
+    uint32_t s[2] = {0u, 0u};
+    unsigned long long q[2] = {0u, 0u};
+    const uint16_t* p = x + a * nchans + c2;
+    auto add = [&](uint32_t v) {
+      const uint32_t l = v & 0xffffu, h = v >> 16;
+      s[0] += l;
+      s[1] += h;
+      q[0] += static_cast<unsigned long long>(l) * l;
+      q[1] += static_cast<unsigned long long>(h) * h;
+    };
+    auto row = [&](int64_t r) { return __ldg(reinterpret_cast<const uint32_t*>(p + r * nchans)); };
+    const int64_t n = b - a;
+    int64_t r = 0;
+    for (; r + 16 <= n; r += 16) {
+      uint32_t v[16];
+#pragma unroll
+      for (int k = 0; k < 16; ++k) v[k] = row(r + k);
+#pragma unroll
+      for (int k = 0; k < 16; ++k) add(v[k]);
+    }
+    for (; r < n; ++r) add(row(r));
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const int64_t ch = c2 + k;
+      if (ch >= cs && ch < cs + csub) add_window_sums(win, nwin, w, a, csub, ch - cs, s[k], q[k], sums);
+    }
+  });
 }
 
 __device__ __forceinline__ int iqrm_target(int lag, int i, int csub) {
@@ -178,126 +263,179 @@ __device__ __forceinline__ int iqrm_target(int lag, int i, int csub) {
 }
 
 // Percentile of iqrm.cu:299-306 (host code there): pos = q*(n-1) in double,
-// linear interpolation with the float difference promoted to double.
-__device__ __forceinline__ float pct_sorted(const float* v, int n, float q) {
-  if (n == 1) return v[0];
-  double pos = __dmul_rn(static_cast<double>(q), static_cast<double>(n - 1));
-  int lo = static_cast<int>(floor(pos));
-  int hi = static_cast<int>(ceil(pos));
-  double w = __dsub_rn(pos, static_cast<double>(lo));
-  float dlt = __fsub_rn(v[hi], v[lo]);
-  return static_cast<float>(__dadd_rn(static_cast<double>(v[lo]), __dmul_rn(static_cast<double>(dlt), w)));
+// linear interpolation with the float difference promoted to double, between the
+// order statistics at floor(pos) and ceil(pos).
+__device__ __forceinline__ double pct_pos(int n, float q) {
+  return __dmul_rn(static_cast<double>(q), static_cast<double>(n - 1));
+}
+__device__ __forceinline__ float pct_value(double pos, float lo, float hi) {
+  const double w = __dsub_rn(pos, floor(pos));
+  const float dlt = __fsub_rn(hi, lo);
+  return static_cast<float>(__dadd_rn(static_cast<double>(lo), __dmul_rn(static_cast<double>(dlt), w)));
+}
+// Floats as unsigned words of the same order, and back.
+__device__ __forceinline__ uint32_t order_key(float v) {
+  const uint32_t u = __float_as_uint(v);
+  return (u & 0x80000000u) ? ~u : u | 0x80000000u;
+}
+__device__ __forceinline__ float key_value(uint32_t k) {
+  return __uint_as_float((k & 0x80000000u) ? k ^ 0x80000000u : ~k);
 }
 
-// One block per window.  Scratch per window: x, d (float), recv, cast (int),
-// flags (nlags x csub bytes).  Dynamic shared memory: the sort buffer.
-__global__ void k_iqrm_decide(const unsigned long long* __restrict__ sums,
-                              const uint32_t* __restrict__ win, int64_t nchans, int64_t cs,
-                              int csub, int mode, float nsigma, const int32_t* __restrict__ lags,
-                              int nlags, int variant, float* __restrict__ xs,
-                              float* __restrict__ ds_, int* __restrict__ recv,
-                              int* __restrict__ cast_, uint8_t* __restrict__ flags,
-                              int sort_n, uint8_t* __restrict__ masks) {
-  extern __shared__ float srt[];
-  __shared__ float s_med, s_thr;
-  __shared__ int s_skip;
-  const int w = blockIdx.x;
+// Statistic per channel of every window, make_stat_from_sums (iqrm.cu:72-91); clears
+// the vote counters and the masks.  grid: windows x channels.
+__global__ void k_iqrm_stat(const unsigned long long* __restrict__ sums,
+                            const uint32_t* __restrict__ win, int64_t nchans, int64_t csub,
+                            int mode, int variant, float* __restrict__ xs, int* __restrict__ recv,
+                            int* __restrict__ cast_, uint8_t* __restrict__ masks) {
+  const int64_t w = blockIdx.x;
+  const int64_t i = static_cast<int64_t>(blockIdx.y) * blockDim.x + threadIdx.x;
+  if (i < nchans) masks[w * nchans + i] = 0;
   const unsigned W = win[2 * w + 1] - win[2 * w];
-  float* x = xs + static_cast<int64_t>(w) * csub;
-  float* d = ds_ + static_cast<int64_t>(w) * csub;
+  if (i >= csub || W == 0) return;
+  const unsigned long long* s1 = sums + w * 2 * csub;
+  const unsigned long long* s2 = s1 + csub;
+  float x;
+  const double mean = __ddiv_rn(static_cast<double>(s1[i]), static_cast<double>(W));
+  if (mode == 0) {
+    x = static_cast<float>(mean);
+  } else {
+    const double e2 = __ddiv_rn(static_cast<double>(s2[i]), static_cast<double>(W));
+    double var = (variant & 8) ? __fma_rn(-mean, mean, e2) : __dsub_rn(e2, __dmul_rn(mean, mean));
+    if (var < 0.0) var = 0.0;
+    x = static_cast<float>(sqrt(var));
+  }
+  xs[w * csub + i] = x;
+  recv[w * csub + i] = 0;
+  cast_[w * csub + i] = 0;
+}
+
+// One block per (window, lag): the lagged differences, their quartiles and the votes
+// of this lag.  The six order statistics the percentiles need come from a bisection
+// over the 32 bits of the differences' order keys: per bit, the block counts the keys
+// below each of the three candidates (warp sums by one reduction instruction, one
+// barrier).  Bound by the latency of those 32 rounds (30 us for 4,096 channels, the
+// whole decision 42 us); one block per window that sorted every lag's differences in
+// turn took 364 us for 8 lags of 4,096 channels and 597 us for 26 lags of 2,048.
+// Dynamic shared memory: the csub keys.
+constexpr int kLagThreads = 512;
+__global__ void __launch_bounds__(kLagThreads) k_iqrm_lag(
+    const uint32_t* __restrict__ win, int csub, float nsigma, const int32_t* __restrict__ lags,
+    int nlags, int variant, const float* __restrict__ xs, int* __restrict__ recv,
+    int* __restrict__ cast_, uint8_t* __restrict__ flags) {
+  extern __shared__ uint32_t keys[];
+  constexpr int kWarpsL = kLagThreads / 32;
+  __shared__ uint32_t part[2][3][kWarpsL];
+  const int l = blockIdx.y, w = blockIdx.x;
+  if (win[2 * w + 1] == win[2 * w]) return;
+  const int lag = lags[l];
+  const float* x = xs + static_cast<int64_t>(w) * csub;
+  uint8_t* fl = flags + (static_cast<int64_t>(w) * nlags + l) * csub;
   int* rc = recv + static_cast<int64_t>(w) * csub;
   int* cc = cast_ + static_cast<int64_t>(w) * csub;
-  uint8_t* fl = flags + static_cast<int64_t>(w) * nlags * csub;
-  uint8_t* mask = masks + static_cast<int64_t>(w) * nchans;
-  const unsigned long long* s1 = sums + (static_cast<int64_t>(w) * 2) * csub;
-  const unsigned long long* s2 = s1 + csub;
-  for (int c = threadIdx.x; c < nchans; c += blockDim.x) mask[c] = 0;
-  if (W == 0 || csub == 0) return;
-  // Statistic per channel, make_stat_from_sums (iqrm.cu:72-91).
-  for (int i = threadIdx.x; i < csub; i += blockDim.x) {
-    double mean = __ddiv_rn(static_cast<double>(s1[i]), static_cast<double>(W));
-    if (mode == 0) {
-      x[i] = static_cast<float>(mean);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  // Lagged difference with edge clipping, make_diff_with_clipping (iqrm.cu:94-117).
+  for (int k = threadIdx.x; k < csub; k += kLagThreads) {
+    float v;
+    if (lag < 0) {
+      const int cut = csub + lag;
+      v = k < cut ? __fsub_rn(x[k], x[k - lag]) : __fsub_rn(x[cut], x[csub - 1]);
     } else {
-      double e2 = __ddiv_rn(static_cast<double>(s2[i]), static_cast<double>(W));
-      double var = (variant & 8) ? __fma_rn(-mean, mean, e2) : __dsub_rn(e2, __dmul_rn(mean, mean));
-      if (var < 0.0) var = 0.0;
-      x[i] = static_cast<float>(sqrt(var));
+      v = k < lag ? __fsub_rn(x[lag], x[0]) : __fsub_rn(x[k], x[k - lag]);
     }
-    rc[i] = 0;
-    cc[i] = 0;
+    keys[k] = order_key(v);
   }
   __syncthreads();
-  for (int l = 0; l < nlags; ++l) {
-    const int lag = lags[l];
-    // Lagged difference with edge clipping, make_diff_with_clipping (iqrm.cu:94-117).
-    for (int k = threadIdx.x; k < sort_n; k += blockDim.x) {
-      float v = FLT_MAX;
-      if (k < csub) {
-        if (lag < 0) {
-          int cut = csub + lag;
-          v = k < cut ? __fsub_rn(x[k], x[k - lag]) : __fsub_rn(x[cut], x[csub - 1]);
-        } else {
-          v = k < lag ? __fsub_rn(x[lag], x[0]) : __fsub_rn(x[k], x[k - lag]);
-        }
-        d[k] = v;
-        fl[static_cast<int64_t>(l) * csub + k] = 0;
-      }
-      srt[k] = k < csub ? v : __int_as_float(0x7f800000);  // +inf pads past the end
+  // block sums of three counts; two buffers, so that one barrier per call suffices
+  int buf = 0;
+  auto block_sums = [&](uint32_t (&c)[3]) {
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      const uint32_t t = __reduce_add_sync(0xffffffffu, c[j]);
+      if (lane == 0) part[buf][j][warp] = t;
     }
     __syncthreads();
-    // Bitonic sort of sort_n (power of two) floats, ascending.
-    for (int size = 2; size <= sort_n; size <<= 1) {
-      for (int stride = size >> 1; stride > 0; stride >>= 1) {
-        for (int k = threadIdx.x; k < sort_n; k += blockDim.x) {
-          int p = k ^ stride;
-          if (p > k) {
-            float a = srt[k], b = srt[p];
-            bool up = (k & size) == 0;
-            if ((a > b) == up) { srt[k] = b; srt[p] = a; }
-          }
-        }
-        __syncthreads();
-      }
+#pragma unroll
+    for (int j = 0; j < 3; ++j)
+      c[j] = __reduce_add_sync(0xffffffffu, lane < kWarpsL ? part[buf][j][lane] : 0u);
+    buf ^= 1;
+  };
+  const double pos[3] = {pct_pos(csub, 0.25f), pct_pos(csub, 0.50f), pct_pos(csub, 0.75f)};
+  uint32_t rank[3], key[3] = {0u, 0u, 0u};
+#pragma unroll
+  for (int j = 0; j < 3; ++j) rank[j] = static_cast<uint32_t>(floor(pos[j]));
+  for (int bit = 31; bit >= 0; --bit) {
+    // the largest t with at most rank keys below it is the key of that rank
+    uint32_t c[3] = {0u, 0u, 0u};
+    const uint32_t t0 = key[0] | (1u << bit), t1 = key[1] | (1u << bit), t2 = key[2] | (1u << bit);
+    for (int k = threadIdx.x; k < csub; k += kLagThreads) {
+      const uint32_t v = keys[k];
+      c[0] += v < t0;
+      c[1] += v < t1;
+      c[2] += v < t2;
     }
-    if (threadIdx.x == 0) {
-      float q1 = pct_sorted(srt, csub, 0.25f);
-      float med = pct_sorted(srt, csub, 0.50f);
-      float q3 = pct_sorted(srt, csub, 0.75f);
-      float s;
-      if (variant & 4) s = fabsf(__fmul_rn(__fsub_rn(q3, q1), __frcp_rn(1.349f)));
-      else s = fabsf(__fdiv_rn(__fsub_rn(q3, q1), 1.349f));
-      bool skip = !(s > 0.f) || !isfinite(s);
-      s_skip = skip;
-      s_med = med;
-      s_thr = __fmul_rn(nsigma, s);
-    }
-    __syncthreads();
-    if (!s_skip) {
-      // flag_and_count_kernel (iqrm.cu:120-151).
-      const float med = s_med, thr = s_thr;
-      for (int i = threadIdx.x; i < csub; i += blockDim.x) {
-        float val = __fsub_rn(d[i], med);
-        if (val > thr) {
-          fl[static_cast<int64_t>(l) * csub + i] = 1;
-          atomicAdd(&rc[i], 1);
-          atomicAdd(&cc[iqrm_target(lag, i, csub)], 1);
-        }
-      }
-    }
-    __syncthreads();
+    block_sums(c);
+    if (c[0] <= rank[0]) key[0] = t0;
+    if (c[1] <= rank[1]) key[1] = t1;
+    if (c[2] <= rank[2]) key[2] = t2;
   }
-  // merge_lags_to_mask_kernel (iqrm.cu:154-185).
-  for (int i = threadIdx.x; i < csub; i += blockDim.x) {
-    int ri = rc[i];
-    uint8_t m = 0;
-    if (ri > 0) {
-      for (int l = 0; l < nlags; ++l) {
-        if (!fl[static_cast<int64_t>(l) * csub + i]) continue;
-        if (cc[iqrm_target(lags[l], i, csub)] < ri) { m = 1; break; }
-      }
+  // the next order statistic: the same key again, or the least one above it
+  uint32_t c[3] = {0u, 0u, 0u}, up[3] = {~0u, ~0u, ~0u};
+  for (int k = threadIdx.x; k < csub; k += kLagThreads) {
+    const uint32_t v = keys[k];
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      if (v <= key[j]) ++c[j];
+      else up[j] = min(up[j], v);
     }
-    mask[cs + i] = m;
+  }
+  block_sums(c);
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    const uint32_t t = __reduce_min_sync(0xffffffffu, up[j]);
+    if (lane == 0) part[buf][j][warp] = t;
+  }
+  __syncthreads();
+  float pct[3];
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    const uint32_t above = __reduce_min_sync(0xffffffffu, lane < kWarpsL ? part[buf][j][lane] : ~0u);
+    const bool next = ceil(pos[j]) > floor(pos[j]) && c[j] < rank[j] + 2u;
+    pct[j] = pct_value(pos[j], key_value(key[j]), key_value(next ? above : key[j]));
+  }
+  float s;
+  if (variant & 4) s = fabsf(__fmul_rn(__fsub_rn(pct[2], pct[0]), __frcp_rn(1.349f)));
+  else s = fabsf(__fdiv_rn(__fsub_rn(pct[2], pct[0]), 1.349f));
+  const bool skip = !(s > 0.f) || !isfinite(s);
+  // flag_and_count_kernel (iqrm.cu:120-151).
+  const float med = pct[1], thr = __fmul_rn(nsigma, s);
+  for (int i = threadIdx.x; i < csub; i += kLagThreads) {
+    const bool hit = !skip && __fsub_rn(key_value(keys[i]), med) > thr;
+    fl[i] = hit ? 1 : 0;
+    if (hit) {
+      atomicAdd(&rc[i], 1);
+      atomicAdd(&cc[iqrm_target(lag, i, csub)], 1);
+    }
+  }
+}
+
+// merge_lags_to_mask_kernel (iqrm.cu:154-185).  grid: windows x channels.
+__global__ void k_iqrm_merge(const uint32_t* __restrict__ win, int64_t nchans, int64_t cs, int csub,
+                             const int32_t* __restrict__ lags, int nlags,
+                             const int* __restrict__ recv, const int* __restrict__ cast_,
+                             const uint8_t* __restrict__ flags, uint8_t* __restrict__ masks) {
+  const int w = blockIdx.x;
+  const int i = blockIdx.y * blockDim.x + threadIdx.x;
+  if (i >= csub || win[2 * w + 1] == win[2 * w]) return;
+  const int ri = recv[static_cast<int64_t>(w) * csub + i];
+  if (ri <= 0) return;
+  const int* cc = cast_ + static_cast<int64_t>(w) * csub;
+  for (int l = 0; l < nlags; ++l) {
+    if (!flags[(static_cast<int64_t>(w) * nlags + l) * csub + i]) continue;
+    if (cc[iqrm_target(lags[l], i, csub)] < ri) {
+      masks[static_cast<int64_t>(w) * nchans + cs + i] = 1;
+      return;
+    }
   }
 }
 
@@ -662,21 +800,28 @@ void launch_iqrm_stats(const void* x, int nbits, int64_t nsamp, int64_t nchans, 
                        int64_t csub, const uint32_t* d_win, int nwin, unsigned long long* d_sums,
                        cudaStream_t st) {
   DD_CUDA_TRY(cudaMemsetAsync(d_sums, 0, sizeof(unsigned long long) * 2 * csub * nwin, st));
-  const int64_t chunk = 1024;
-  dim3 grid(static_cast<unsigned>((csub + 255) / 256), static_cast<unsigned>((nsamp + chunk - 1) / chunk));
-  if (nbits == 8 && nchans % 4 == 0 && reinterpret_cast<uintptr_t>(x) % 4 == 0) {
-    const int64_t words = (csub + (cs & 3) + 3) / 4;
-    dim3 g4(static_cast<unsigned>((words + 255) / 256), grid.y);
-    k_iqrm_stats_u8w<<<g4, 256, 0, st>>>(static_cast<const uint8_t*>(x), nsamp, nchans, cs, csub,
-                                         d_win, nwin, chunk, d_sums);
-    DD_LAUNCHED();
-    return;
-  }
-  switch (nbits) {
-    case 8: k_iqrm_stats<uint8_t><<<grid, 256, 0, st>>>(static_cast<const uint8_t*>(x), nsamp, nchans, cs, csub, d_win, nwin, chunk, d_sums); break;
-    case 16: k_iqrm_stats<uint16_t><<<grid, 256, 0, st>>>(static_cast<const uint16_t*>(x), nsamp, nchans, cs, csub, d_win, nwin, chunk, d_sums); break;
-    default: k_iqrm_stats<uint32_t><<<grid, 256, 0, st>>>(static_cast<const uint32_t*>(x), nsamp, nchans, cs, csub, d_win, nwin, chunk, d_sums); break;
-  }
+  // chunks of at most 1024 samples (32-bit partial sums), fewer where the grid would
+  // hold less than eight blocks per SM: a thread reads its channels row by row, so the
+  // bytes in flight grow with the blocks
+  const int threads = nbits == 32 ? 256 : 128;
+  const bool u8w = nbits == 8 && nchans % 4 == 0 && reinterpret_cast<uintptr_t>(x) % 4 == 0;
+  const bool u16w = nbits == 16 && nchans % 2 == 0 && reinterpret_cast<uintptr_t>(x) % 4 == 0;
+  const int64_t per = u8w ? 4 : u16w ? 2 : 1;
+  const int64_t cols = (csub + (cs % per) + per - 1) / per;
+  const int64_t gx = (cols + threads - 1) / threads;
+  int64_t chunk = 1024;
+  while (chunk > 64 && gx * ((nsamp + chunk - 1) / chunk) < 148 * 8) chunk /= 2;
+  const dim3 grid(static_cast<unsigned>(gx), static_cast<unsigned>((nsamp + chunk - 1) / chunk));
+  if (u8w)
+    k_iqrm_stats_u8w<<<grid, threads, 0, st>>>(static_cast<const uint8_t*>(x), nsamp, nchans, cs, csub, d_win, nwin, chunk, d_sums);
+  else if (u16w)
+    k_iqrm_stats_u16w<<<grid, threads, 0, st>>>(static_cast<const uint16_t*>(x), nsamp, nchans, cs, csub, d_win, nwin, chunk, d_sums);
+  else if (nbits == 8)
+    k_iqrm_stats<uint8_t><<<grid, threads, 0, st>>>(static_cast<const uint8_t*>(x), nsamp, nchans, cs, csub, d_win, nwin, chunk, d_sums);
+  else if (nbits == 16)
+    k_iqrm_stats<uint16_t><<<grid, threads, 0, st>>>(static_cast<const uint16_t*>(x), nsamp, nchans, cs, csub, d_win, nwin, chunk, d_sums);
+  else
+    k_iqrm_stats<uint32_t><<<grid, threads, 0, st>>>(static_cast<const uint32_t*>(x), nsamp, nchans, cs, csub, d_win, nwin, chunk, d_sums);
   DD_LAUNCHED();
 }
 
@@ -684,9 +829,9 @@ size_t iqrm_scratch_bytes(int nwin, int64_t csub, int nlags) {
   return static_cast<size_t>(nwin) * csub * (4 + 4 + 4 + 4 + nlags) + 256;
 }
 
-// k_iqrm_decide sorts one window's csub statistics in shared memory (the next
-// power of two of csub floats); reject band widths whose sort buffer exceeds the
-// current device's opt-in shared memory per block.
+// k_iqrm_lag holds one window's csub differences in shared memory; band widths are
+// limited to those whose next power of two of floats fits the current device's opt-in
+// shared memory per block.
 void check_iqrm_channels(int64_t csub) {
   int64_t sort_n = 1;
   while (sort_n < csub) sort_n <<= 1;
@@ -709,20 +854,24 @@ void launch_iqrm_decide(const unsigned long long* d_sums, int nwin, const uint32
                         int64_t nchans, int64_t cs, int64_t csub, int mode, float nsigma,
                         const int32_t* d_lags, int nlags, int variant, void* scratch,
                         uint8_t* d_masks, cudaStream_t st) {
+  // scratch (iqrm_scratch_bytes): statistics, an unused row, vote counters, flags
   char* p = static_cast<char*>(scratch);
-  float* xs = reinterpret_cast<float*>(p); p += sizeof(float) * nwin * csub;
-  float* ds_ = reinterpret_cast<float*>(p); p += sizeof(float) * nwin * csub;
+  float* xs = reinterpret_cast<float*>(p); p += 2 * sizeof(float) * nwin * csub;
   int* recv = reinterpret_cast<int*>(p); p += sizeof(int) * nwin * csub;
   int* cast_ = reinterpret_cast<int*>(p); p += sizeof(int) * nwin * csub;
   uint8_t* flags = reinterpret_cast<uint8_t*>(p);
   check_iqrm_channels(csub);
-  int sort_n = 1;
-  while (sort_n < csub) sort_n <<= 1;
-  const size_t smem = sizeof(float) * sort_n;
-  allow_dynamic_smem(k_iqrm_decide, smem);
-  k_iqrm_decide<<<nwin, 1024, smem, st>>>(d_sums, d_win, nchans, cs, static_cast<int>(csub), mode,
-                                          nsigma, d_lags, nlags, variant, xs, ds_, recv, cast_,
-                                          flags, sort_n, d_masks);
+  const int n = static_cast<int>(csub);
+  const dim3 all(static_cast<unsigned>(nwin), static_cast<unsigned>((nchans + 255) / 256));
+  k_iqrm_stat<<<all, 256, 0, st>>>(d_sums, d_win, nchans, csub, mode, variant, xs, recv, cast_, d_masks);
+  DD_LAUNCHED();
+  const size_t smem = sizeof(uint32_t) * csub;
+  allow_dynamic_smem(k_iqrm_lag, smem);
+  k_iqrm_lag<<<dim3(static_cast<unsigned>(nwin), static_cast<unsigned>(nlags)), kLagThreads, smem, st>>>(
+      d_win, n, nsigma, d_lags, nlags, variant, xs, recv, cast_, flags);
+  DD_LAUNCHED();
+  const dim3 band(static_cast<unsigned>(nwin), static_cast<unsigned>((csub + 255) / 256));
+  k_iqrm_merge<<<band, 256, 0, st>>>(d_win, nchans, cs, n, d_lags, nlags, recv, cast_, flags, d_masks);
   DD_LAUNCHED();
 }
 

@@ -1,0 +1,54 @@
+"""IQRM masks on the GPU against the oracle's restatement, bit for bit, where the
+word-wise sums, the window runs and the order statistics can go wrong: bands of one to a
+few thousand channels that start off a word, sample counts around the sixteen-row
+blocks and the chunk length, overlapping windows, and flat bands whose differences tie."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+from astroflow_b200.dedisp import IqrmParams, iqrm_masks_noalloc  # noqa: E402
+from oracle import oracle as O  # noqa: E402
+
+TSAMP = 1e-3
+
+
+def to_dev(x):
+    signed = {1: np.uint8, 2: np.int16, 4: np.int32}[x.dtype.itemsize]
+    t = torch.from_numpy(x.view(signed)).cuda()
+    return t.view({1: torch.uint8, 2: torch.uint16, 4: torch.uint32}[x.dtype.itemsize])
+
+
+@pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("nbits,nchans,cs,ce,nsamp,win,flat", [
+    (8, 8, 0, 2, 17, 0.0, False),
+    (8, 64, 3, 62, 1023, 0.3, False),
+    (8, 512, 1, 510, 1025, 0.5, False),
+    (8, 2048, 0, 2047, 4099, 1.0, False),
+    (8, 258, 5, 257, 2500, 0.7, False),
+    (8, 256, 0, 256, 1040, 0.4, True),
+    (16, 130, 1, 129, 3001, 0.6, False),
+    (16, 4097, 0, 4096, 515, 0.0, False),
+    (32, 100, 7, 93, 1500, 0.25, False),
+])
+def test_masks_equal_oracle(nbits, nchans, cs, ce, nsamp, win, flat, mode):
+    rng = np.random.default_rng(nchans * 7 + nsamp)
+    dt = {8: np.uint8, 16: np.uint16, 32: np.uint32}[nbits]
+    mid, sd = {8: (128, 20), 16: (32768, 2000), 32: (1e6, 6e4)}[nbits]
+    x = rng.normal(mid, sd, (nsamp, nchans))
+    if flat:  # whole blocks of channels equal: differences tie at zero
+        x[:] = mid
+        x[:, ::7] += rng.normal(0, sd, (nsamp, len(range(0, nchans, 7))))
+    for c in rng.choice(nchans, max(1, nchans // 16), replace=False):
+        x[:, c] += 4 * sd * np.sin(np.arange(nsamp) * 0.37) + 2 * sd
+    x = np.clip(np.rint(x), 0, 2.0 ** nbits - 1).astype(dt)
+    iq = IqrmParams(mode=mode, radius_frac=0.1, nsigma=3.0, geofactor=1.5, win_sec=win,
+                    hop_sec=win / 2, include_tail=True)
+    t0, t1, want = O.iqrm_masks(x.copy(), nchans, cs, ce, TSAMP, iq)
+    masks = torch.full((len(t0) + 1, nchans), 9, dtype=torch.uint8, device="cuda")
+    bounds = torch.zeros((len(t0) + 1, 2), dtype=torch.int32, device="cuda")
+    n = iqrm_masks_noalloc(to_dev(x), nchans, cs, ce, TSAMP, iq, masks, bounds)
+    assert n == len(t0)
+    assert np.array_equal(masks[:n].cpu().numpy(), want)
+    assert np.array_equal(bounds[:n].cpu().numpy(), np.stack([t0, t1], 1).astype(np.int32))
