@@ -46,20 +46,47 @@ Error invalid(const char* fmt, double a = 0, double b = 0, double c = 0, double 
 
 int64_t round_up(int64_t v, int64_t m) { return (v + m - 1) / m * m; }
 
-// Bytes of one stage-1 sum: uint16 for 8-bit input in narrow subbands, else the
-// reference's accumulator type (uint32, or uint64 for 32-bit samples).
-int64_t inter_elem(const dd_plan& P) { return P.inter16 ? 2 : (P.nbits == 32 ? 8 : 4); }
-// Whether stage 1 sums into 32-bit words.
-bool stage1_flush(const dd_plan& P) { return !P.inter16; }
+// Bytes of one stage-1 sum (of one word of a plane, when folded): uint16 for 8-bit
+// input in narrow subbands, else the reference's accumulator type (uint32, or uint64
+// for 32-bit samples).
+int64_t inter_elem(const dd_plan& P) {
+  return P.fold > 1 ? 4 : P.inter16 ? 2 : (P.nbits == 32 ? 8 : 4);
+}
+// Bytes of one element of the prepared input.
+int64_t x_elem(const dd_plan& P) { return P.fold > 1 ? 4 : P.elem; }
 
 // Kernel variants of the two stages: 8-bit input in subbands of at most 64 channels
-// has 16-bit subband sums, which stage 2 reads with their shifted twin.
+// has 16-bit subband sums (packed planes when folded, else with a twin).
 int stage1_kind(const dd_plan& P) {
+  if (P.fold > 1) return P.nbits == 16 ? kSumKindFold16 : P.inter16 ? kSumKindFold8 : kSumKindFold8W;
   return P.nbits == 16 ? kSumKindU16Wide : P.inter16 ? kSumKindU8Out16 : kSumKindU8Flush;
 }
-int stage2_kind(const dd_plan& P) { return P.inter16 ? kSumKindU16Twin : kSumKindU32; }
+int stage2_kind(const dd_plan& P) {
+  return !P.inter16 ? kSumKindPlane32 : P.fold > 1 ? kSumKindPlane16 : kSumKindU16Twin;
+}
+int brute_kind(const dd_plan& P) {
+  if (P.fold > 1) return P.nbits == 16 ? kSumKindFold16 : kSumKindFold8W;
+  return P.nbits == 16 ? kSumKindU16Wide : kSumKindU8Flush;
+}
+// Samples per folded word, or 1 where the fold does not pay.  A folded word holds the
+// samples of the segments at one position, so all positions up to a segment and the
+// largest delay are written, up to four times the chunk: that costs the layout kernel
+// bytes, and each addition gains what the shifts and second loads of unfolded samples
+// take.  Measured on 4096 channels, 2^17 samples to DM 3000 (1.6 GB extra; folded /
+// time order, ms): 9.6 additions per extra byte (601 trials) 4.08 / 3.13, 24 (1501
+// trials) 3.85 / 4.03, 95 (6001 trials) 9.10 / 12.0; 8192 channels of 16 bits, 2001
+// trials 20.0 / 29.5; brute force over 1024 channels 5.60 / 8.69.
+int choose_fold(const dd_plan& P, int64_t ncols, int64_t nchan, int64_t reach, double adds) {
+  if (P.nbits > 16) return 1;
+  const int fold = P.nbits == 8 ? 4 : 2;
+  const int64_t words = std::min<int64_t>(P.nbin, (ncols + fold - 1) / fold + reach);
+  const double extra = static_cast<double>(nchan) * (4.0 * words - static_cast<double>(P.nbin) * P.elem);
+  return adds > 16.0 * extra ? fold : 1;
+}
 // Byte offset from a subband-sum buffer to its twin (0: no twin).
 int64_t twin_offset(const dd_plan& P) { return P.twin ? P.inter_bytes : 0; }
+// Bytes between the planes of subband sums.
+int64_t plane_bytes(const dd_plan& P) { return P.ndm_nom * P.nsb * P.tile_pitch * inter_elem(P); }
 
 // ---- frequency table and band (dedispered.cu:1003-1031, cpucal.hpp:85-116)
 void build_freq(dd_plan& P) {
@@ -345,12 +372,15 @@ void upload(DevBuf& b, const void* h, size_t bytes) {
 // (reallocated, zeroed).  Results do not depend on the tiling.
 void set_tiling(dd_plan& P, int64_t budget) {
   const int64_t kT = tile_samples();
+  const int copies = P.twin ? 2 : P.planes;
+  P.seg = P.fold > 1 ? round_up((P.nout + P.fold - 1) / P.fold, 8) : P.nout;
   // The fewest tiles whose subband sums (tile and stage-2 halo) stay within the
-  // budget, all of the same length.
-  const int64_t per_col = P.ndm_nom * P.nsb * inter_elem(P) * (P.twin ? 2 : 1);
-  const int64_t most = std::max<int64_t>(kT, budget / per_col - P.max_res);
-  const int64_t ntiles = (P.nout + most - 1) / most;
-  const int64_t L = round_up((P.nout + ntiles - 1) / ntiles, 64);
+  // budget, all of the same length; chunks of 2^16 columns have two at least, so that
+  // the host path can copy one tile's columns out while the next is summed.
+  const int64_t per_col = P.ndm_nom * P.nsb * inter_elem(P) * copies;
+  const int64_t most = std::max<int64_t>(P.fold > 1 ? 1024 : kT, budget / per_col - P.max_res);
+  const int64_t ntiles = std::max<int64_t>((P.seg + most - 1) / most, P.nout >= 65536 ? 2 : 1);
+  const int64_t L = round_up((P.seg + ntiles - 1) / ntiles, 64);
   P.tile = L;
   P.inter_budget = budget;
   // Stage-2 blocks past the tile's last column read up to one block tile beyond it
@@ -359,12 +389,13 @@ void set_tiling(dd_plan& P, int64_t budget) {
   P.tile_pitch = round_up(round_up(L + P.max_res, kT) + T2 + 64, 64);
   // Stage-1 windows end at most one block tile (below 8192) past their last column
   // and its reach.
-  P.xpitch = round_up(std::max(P.nbin, P.nout + P.max_res + std::max<int64_t>(P.reach1, P.max_delay)) + 8192 + 64, 64);
-  P.d_x.alloc(static_cast<size_t>(P.dch * P.xpitch) * P.elem);
+  const int64_t last = P.seg + P.max_res + std::max<int64_t>(P.reach1, P.max_delay);
+  P.xpitch = round_up((P.fold > 1 ? last : std::max(P.nbin, last)) + 8192 + 64, 64);
+  P.d_x.alloc(static_cast<size_t>(P.dch * P.xpitch) * x_elem(P));
   DD_CUDA_TRY(cudaMemsetAsync(P.d_x.p, 0, P.d_x.bytes, cudaStreamLegacy));
-  P.inter_bytes = P.ndm_nom * P.nsb * P.tile_pitch * inter_elem(P);
+  P.inter_bytes = plane_bytes(P);
   // (+256: the twin's staged windows may start one 16-byte block past the sums')
-  P.d_inter.alloc(static_cast<size_t>((P.twin ? 2 : 1) * P.inter_bytes) + 256);
+  P.d_inter.alloc(static_cast<size_t>(copies * P.inter_bytes) + 256);
   DD_CUDA_TRY(cudaMemsetAsync(P.d_inter.p, 0, P.d_inter.bytes, cudaStreamLegacy));
   DD_CUDA_TRY(cudaStreamSynchronize(cudaStreamLegacy));
 }
@@ -426,17 +457,28 @@ void create_subband(dd_plan& P) {
   if (mind < 0 || minr < 0)
     throw invalid("negative dispersion delays (DM below zero or band order) are not supported");
   P.inter16 = (P.nbits == 8 && P.sbw <= 64) ? 1 : 0;
+  P.adds = static_cast<double>(P.ndm_nom) * P.dch * P.nout +
+           static_cast<double>(P.dm_steps) * P.nsb * P.nout;
   if (P.nbits <= 16) {
     std::vector<int32_t> skew;
     const std::vector<int32_t> tab = skew_stage1(P, skew);
-    P.win1 = window_bytes(table_spread(tab, P.ndm_nom, P.dch, kSumRows, 0),
-                          sum_kind_tile(stage1_kind(P)), P.elem);
-    P.win2 = window_bytes(table_spread(P.h_res, P.dm_steps, P.nsb, kSumRows, P.ndm0),
-                          sum_kind_tile(stage2_kind(P)), static_cast<int>(inter_elem(P)),
-                          sum_kind_qs(stage2_kind(P)));
-    // 16-bit sums: the staged stage 2 reads the twin that the staged stage 1 writes
-    P.twin = (P.inter16 && P.win1 && P.win2) ? 1 : 0;
-    if (P.inter16 && !P.twin) P.win2 = 0;
+    const int spread1 = table_spread(tab, P.ndm_nom, P.dch, kSumRows, 0);
+    const int spread2 = table_spread(P.h_res, P.dm_steps, P.nsb, kSumRows, P.ndm0);
+    auto set_windows = [&](int fold) {
+      P.fold = fold;
+      P.planes = fold == 1 ? 1 : P.inter16 ? 2 : fold;
+      const int k1 = stage1_kind(P), k2 = stage2_kind(P);
+      P.win1 = window_bytes(spread1, sum_kind_tile(k1), sum_kind_elem(k1), sum_kind_qs(k1));
+      P.win2 = window_bytes(spread2, sum_kind_tile(k2), sum_kind_elem(k2), sum_kind_qs(k2));
+    };
+    set_windows(choose_fold(P, P.nout, P.dch, P.max_res + P.reach1, P.adds));
+    if (P.fold > 1 && !(P.win1 && P.win2)) set_windows(1);  // the direct kernels read time order
+    if (P.fold == 1 && P.inter16) {
+      // 16-bit sums in time order: the staged stage 2 reads the twin that the staged
+      // stage 1 writes
+      P.twin = (P.win1 && P.win2) ? 1 : 0;
+      if (!P.twin) P.win2 = 0;
+    }
     if (P.win1) {
       upload_desc(P.d_desc1, build_sum_desc(tab, P.ndm_nom, P.dch, 0));
       upload(P.d_skew1, skew.data(), sizeof(int32_t) * skew.size());
@@ -451,19 +493,35 @@ void create_subband(dd_plan& P) {
     launch_binning_lut(P.d_bin_lut.p, P.nbits, ds, cudaStreamLegacy);
     DD_CUDA_TRY(cudaStreamSynchronize(cudaStreamLegacy));
   }
-  P.adds = static_cast<double>(P.ndm_nom) * P.dch * P.nout +
-           static_cast<double>(P.dm_steps) * P.nsb * P.nout;
 }
 
-// The staged-window sums serve 8- and 16-bit samples without downsampling (one
-// source row per channel); other cases use the direct kernels.
+// Layout and staging of the brute-force sums.  The staged-window sums serve 8- and
+// 16-bit samples without downsampling (one source row per channel); other cases use the
+// direct kernels on the phase rows.  Allocates the prepared input when its layout
+// changes.
 void set_brute_window(dd_plan& P) {
+  const bool had = P.d_x.bytes != 0;
+  const int fold0 = P.fold;
   P.winb = 0;
+  P.fold = 1;
   if (P.p.time_downsample == 1 && P.nbits <= 16) {
-    const int T = sum_kind_tile(P.nbits == 8 ? kSumKindU8Flush : kSumKindU16Wide);
-    P.winb = window_bytes(table_spread(P.h_delay, P.dm_steps, P.nc, kSumRows, 0), T, P.elem);
+    const int spread = table_spread(P.h_delay, P.dm_steps, P.nc, kSumRows, 0);
+    auto set_window = [&](int fold) {
+      P.fold = fold;
+      const int k = brute_kind(P);
+      P.winb = window_bytes(spread, sum_kind_tile(k), sum_kind_elem(k), sum_kind_qs(k));
+    };
+    set_window(choose_fold(P, P.out_cols, P.nc, P.max_delay, P.adds));
+    if (P.fold > 1 && !P.winb) set_window(1);
   }
   if (P.winb) upload_desc(P.d_descb, build_sum_desc(P.h_delay, P.dm_steps, P.nc, 0));
+  if (had && P.fold == fold0) return;
+  P.seg = P.fold > 1 ? round_up((P.out_cols + P.fold - 1) / P.fold, 8) : P.out_cols;
+  // (a folded row holds a segment, the padding of phase_len past the chunk and a tile)
+  P.xpitch = P.fold > 1 ? round_up(P.seg + P.phase_len - P.nin + 2048 + 64, 64) : P.phase_len;
+  const int64_t rows = P.nc * P.p.time_downsample;
+  P.d_x.alloc(static_cast<size_t>(rows * P.xpitch) * x_elem(P));
+  DD_CUDA_TRY(cudaMemset(P.d_x.p, 0, P.d_x.bytes));
 }
 
 void create_brute(dd_plan& P) {
@@ -496,13 +554,11 @@ void create_brute(dd_plan& P) {
   if (mind < 0) throw invalid("negative dispersion delays are not supported");
   const int64_t kT = tile_samples();
   P.phase_len = round_up((P.nin + ds - 1) / ds + P.max_delay / ds + round_up(P.cols0, kT) + kT + 64, 64);
-  P.d_x.alloc(static_cast<size_t>(P.nc * ds * P.phase_len) * P.elem);
-  DD_CUDA_TRY(cudaMemset(P.d_x.p, 0, P.d_x.bytes));
+  P.adds = static_cast<double>(P.dm_steps) * P.nc * P.out_cols;
   P.d_delay.alloc(sizeof(int32_t) * P.h_delay.size());
   DD_CUDA_TRY(cudaMemcpy(P.d_delay.p, P.h_delay.data(), sizeof(int32_t) * P.h_delay.size(),
                          cudaMemcpyHostToDevice));
   set_brute_window(P);
-  P.adds = static_cast<double>(P.dm_steps) * P.nc * P.out_cols;
 }
 
 void create_rfi(dd_plan& P) {
@@ -617,6 +673,9 @@ void run_rfi_and_prep(dd_plan& P, const void* input, uint8_t* masks_out, uint32_
   a.c1 = P.ce + 1;
   a.ds = 1;
   a.pitch = P.xpitch;
+  a.fold = P.fold;
+  a.seg = P.seg;
+  a.nwords = std::min(P.nbin, P.xpitch);
   a.full_out = prepped;
   launch_prep(a, st);
 }
@@ -626,8 +685,9 @@ void run_rfi_and_prep(dd_plan& P, const void* input, uint8_t* masks_out, uint32_
 SumLaunch stage1_launch(const dd_plan& P, int64_t t0) {
   SumLaunch L{};
   L.mode = SumLaunch::kStage1;
+  L.kind = stage1_kind(P);
   L.src = static_cast<const char*>(P.d_x.p);
-  L.src_pitch = P.xpitch * P.elem;
+  L.src_pitch = P.xpitch * x_elem(P);
   L.off = P.d_delay.as<int32_t>();
   L.off_pitch = P.dch;
   L.base = t0;
@@ -639,12 +699,11 @@ SumLaunch stage1_launch(const dd_plan& P, int64_t t0) {
   L.out_pitch = P.tile_pitch * inter_elem(P);
   L.out_col0 = 0;
   L.out_elem = static_cast<int>(inter_elem(P));
-  L.ncols = std::min<int64_t>(P.tile, P.nout - t0) + P.max_res;
+  L.ncols = std::min<int64_t>(P.tile, P.seg - t0) + P.max_res;
+  L.seg_stride = plane_bytes(P);
   L.skew = P.d_skew1.as<int32_t>();
   L.max_skew = P.max_skew1;
   L.win_bytes = P.win1;
-  L.src_bytes = P.elem;
-  L.flush = stage1_flush(P) ? 1 : 0;
   L.grid_y = static_cast<unsigned>((P.ndm_nom + kSumRows - 1) / kSumRows);
   L.grid_z = static_cast<unsigned>(P.nsb);
   L.desc = P.d_desc1.as<SumDesc>();
@@ -658,6 +717,7 @@ SumLaunch stage1_launch(const dd_plan& P, int64_t t0) {
 SumLaunch stage2_launch(const dd_plan& P, int64_t t0, void* output) {
   SumLaunch L{};
   L.mode = SumLaunch::kStage2;
+  L.kind = stage2_kind(P);
   L.src = static_cast<const char*>(P.d_inter.p);
   L.src_pitch = P.tile_pitch * inter_elem(P);
   L.off = P.d_res.as<int32_t>();
@@ -670,12 +730,13 @@ SumLaunch stage2_launch(const dd_plan& P, int64_t t0, void* output) {
   L.out_pitch = P.nout * 4;
   L.out_col0 = t0;
   L.out_elem = 4;
-  L.ncols = std::min<int64_t>(P.tile, P.nout - t0);
+  L.ncols = std::min<int64_t>(P.tile, P.seg - t0);
+  L.seg = P.seg;
+  L.nout = P.nout;
+  L.plane_bytes = plane_bytes(P);
   L.win_bytes = P.win2;
-  L.src_bytes = static_cast<int>(inter_elem(P));
-  L.flush = 0;
   L.grid_y = static_cast<unsigned>(P.ndm_nom * ((P.ndm0 + kSumRows - 1) / kSumRows));
-  L.grid_z = 1;
+  L.grid_z = static_cast<unsigned>(P.planes);
   L.desc = P.d_desc2.as<SumDesc>();
   L.desc_pitch = P.nsb;
   L.stages = P.stages_override ? P.stages_override : sum_kind_stages(stage2_kind(P), P.win2);
@@ -685,13 +746,13 @@ SumLaunch stage2_launch(const dd_plan& P, int64_t t0, void* output) {
 }
 
 // after_tile(t0, cols): called once the work producing output columns
-// [t0, t0 + cols) of every DM row has been queued on the stream.
+// [t0, t0 + cols) of every segment (the whole row when the plan is not folded) of every
+// DM row has been queued on the stream.
 using TileHook = std::function<void(int64_t, int64_t)>;
 
 // before_sums: called once the RFI stages and the layout are queued, before the
 // first sum that writes `output`.
-// before_out(t0, cols): called before the first launch that writes output
-// columns [t0, t0 + cols) of the DM rows.
+// before_out(t0, cols): called before the first launch that writes those columns.
 void run_subband(dd_plan& P, const void* input, void* output, uint8_t* masks_out,
                  uint32_t* bounds_out, void* prepped, cudaStream_t st, Prof* pf = nullptr,
                  const TileHook& after_tile = TileHook(),
@@ -701,7 +762,7 @@ void run_subband(dd_plan& P, const void* input, void* output, uint8_t* masks_out
   run_rfi_and_prep(P, input, masks_out, bounds_out, prepped, st);
   if (pf) pf->prep.emplace_back(a, pf->mark());
   if (before_sums) before_sums();
-  for (int64_t t0 = 0; t0 < P.nout; t0 += P.tile) {
+  for (int64_t t0 = 0; t0 < P.seg; t0 += P.tile) {
     cudaEvent_t b1 = pf ? pf->mark() : nullptr;
     if (P.win1) {
       launch_sum(stage1_launch(P, t0), st);
@@ -716,14 +777,14 @@ void run_subband(dd_plan& P, const void* input, void* output, uint8_t* masks_out
       s1.ndm_nom = P.ndm_nom;
       s1.sbw = P.sbw;
       s1.t0 = t0;
-      s1.ncols = std::min<int64_t>(P.tile, P.nout - t0) + P.max_res;
+      s1.ncols = std::min<int64_t>(P.tile, P.seg - t0) + P.max_res;
       s1.inter = P.d_inter.p;
       s1.tile_pitch = P.tile_pitch;
       s1.inter16 = P.inter16;
       launch_stage1(s1, st);
     }
     if (pf) pf->s1.emplace_back(b1, pf->mark());
-    if (before_out) before_out(t0, std::min<int64_t>(P.tile, P.nout - t0));
+    if (before_out) before_out(t0, std::min<int64_t>(P.tile, P.seg - t0));
     cudaEvent_t b2 = pf ? pf->mark() : nullptr;
     if (P.win2) {
       launch_sum(stage2_launch(P, t0, output), st);
@@ -746,7 +807,7 @@ void run_subband(dd_plan& P, const void* input, void* output, uint8_t* masks_out
       launch_stage2(s2, st);
     }
     if (pf) pf->s2.emplace_back(b2, pf->mark());
-    if (after_tile) after_tile(t0, std::min<int64_t>(P.tile, P.nout - t0));
+    if (after_tile) after_tile(t0, std::min<int64_t>(P.tile, P.seg - t0));
   }
 }
 
@@ -754,8 +815,9 @@ void run_subband(dd_plan& P, const void* input, void* output, uint8_t* masks_out
 SumLaunch brute_launch(const dd_plan& P, void* output) {
   SumLaunch L{};
   L.mode = SumLaunch::kBrute;
+  L.kind = brute_kind(P);
   L.src = static_cast<const char*>(P.d_x.p);
-  L.src_pitch = P.phase_len * P.elem;
+  L.src_pitch = P.xpitch * x_elem(P);
   L.off = P.d_delay.as<int32_t>();
   L.off_pitch = P.nc;
   L.base = 0;
@@ -765,10 +827,11 @@ SumLaunch brute_launch(const dd_plan& P, void* output) {
   L.out_pitch = P.out_cols * 4;
   L.out_col0 = 0;
   L.out_elem = 4;
-  L.ncols = P.out_cols;
+  L.ncols = P.seg;
+  L.seg = P.seg;
+  L.seg_stride = P.seg * 4;
+  L.nout = P.out_cols;
   L.win_bytes = P.winb;
-  L.src_bytes = P.elem;
-  L.flush = (P.nbits == 8 || P.nbits == 16) ? 1 : 0;  // 8-bit: widened lanes; 16-bit: 32-bit sums
   L.grid_y = static_cast<unsigned>((P.dm_steps + kSumRows - 1) / kSumRows);
   L.grid_z = 1;
   L.desc = P.d_descb.as<SumDesc>();
@@ -788,7 +851,10 @@ void run_brute_prep(dd_plan& P, const void* input, void* prepped, cudaStream_t s
   a.c0 = P.cs;
   a.c1 = P.ce;
   a.ds = P.p.time_downsample;
-  a.pitch = P.phase_len;
+  a.pitch = P.xpitch;
+  a.fold = P.fold;
+  a.seg = P.seg;
+  a.nwords = std::min(P.nin, P.xpitch);
   a.full_out = prepped;
   launch_prep(a, st);
 }
@@ -1045,7 +1111,7 @@ int dd_plan_get_info(const dd_plan* P, dd_plan_info* info) {
     o.delay_rows = P->p.algorithm == DD_ALGO_BRUTE ? P->dm_steps : P->ndm_nom;
     o.delay_cols = P->p.algorithm == DD_ALGO_BRUTE ? P->nc : P->dch;
     o.table_mismatch_fp64 = P->table_mismatch_fp64;
-    o.tile_samples = P->tile;
+    o.tile_samples = P->tile * P->fold;
     o.subband_sum_copies = P->p.algorithm == DD_ALGO_SUBBAND ? (P->twin ? 2 : 1) : 0;
     o.adds_per_run = P->adds;
     *info = o;
@@ -1152,7 +1218,7 @@ int dd_plan_autotune(dd_plan* P, const void* input, void* output, int32_t reps, 
     rep.default_ms = time_shape();
     rep.best_ms = rep.default_ms;
     rep.best_budget_bytes = budget0;
-    rep.best_tile_samples = P->tile;
+    rep.best_tile_samples = P->tile * P->fold;
     rep.best_stages = stages0;
     rep.candidates = 1;
     std::vector<int64_t> tiles_seen;
@@ -1174,7 +1240,7 @@ int dd_plan_autotune(dd_plan* P, const void* input, void* output, int32_t reps, 
         if (ms < rep.best_ms) {
           rep.best_ms = ms;
           rep.best_budget_bytes = budget;
-          rep.best_tile_samples = P->tile;
+          rep.best_tile_samples = P->tile * P->fold;
           rep.best_stages = S;
         }
       }
@@ -1287,7 +1353,7 @@ void enqueue_host_run(dd_plan& P, const void* h_input, void* h_output, cudaStrea
       for (cudaEvent_t ev : copied) cudaEventDestroy(ev);
     };
     const bool same_tiling = P.host_pending && P.host_tile == P.tile &&
-                             P.host_tile_copied.size() == static_cast<size_t>((P.nout + P.tile - 1) / P.tile);
+                             P.host_tile_copied.size() == static_cast<size_t>((P.seg + P.tile - 1) / P.tile);
     try {
       run_subband(P, P.d_host_in.p, d_out, nullptr, nullptr, nullptr, st, nullptr,
                   [&](int64_t t0, int64_t n) {
@@ -1299,10 +1365,14 @@ void enqueue_host_run(dd_plan& P, const void* h_input, void* h_output, cudaStrea
                     DD_CUDA_TRY(cudaEventRecord(ev, st));
                     DD_CUDA_TRY(cudaStreamWaitEvent(P.copy_stream, ev, 0));
                     const size_t pitch = static_cast<size_t>(cols) * oelem;
-                    DD_CUDA_TRY(cudaMemcpy2DAsync(static_cast<char*>(h_output) + t0 * oelem, pitch,
-                                                  d_out + t0 * oelem, pitch, n * oelem,
-                                                  static_cast<size_t>(P.dm_steps),
-                                                  cudaMemcpyDeviceToHost, P.copy_stream));
+                    for (int64_t s0 = 0; s0 < P.nout; s0 += P.seg) {
+                      const int64_t nc = std::min(n, std::min(P.seg, P.nout - s0) - t0);
+                      if (nc <= 0) continue;
+                      DD_CUDA_TRY(cudaMemcpy2DAsync(static_cast<char*>(h_output) + (s0 + t0) * oelem, pitch,
+                                                    d_out + (s0 + t0) * oelem, pitch, nc * oelem,
+                                                    static_cast<size_t>(P.dm_steps),
+                                                    cudaMemcpyDeviceToHost, P.copy_stream));
+                    }
                     DD_CUDA_TRY(cudaEventRecord(done, P.copy_stream));
                   },
                   [&]() {
@@ -1460,7 +1530,7 @@ void build_groups(dd_batch& B, void* const* outputs) {
   int64_t max_tiles = 1;
   for (int p = 0; p < n; ++p)
     if (!B.own[p] && B.plans[p]->p.algorithm == DD_ALGO_SUBBAND)
-      max_tiles = std::max<int64_t>(max_tiles, (B.plans[p]->nout + B.plans[p]->tile - 1) / B.plans[p]->tile);
+      max_tiles = std::max<int64_t>(max_tiles, (B.plans[p]->seg + B.plans[p]->tile - 1) / B.plans[p]->tile);
   // The sums of one stage of every plan, tile by tile: stage[k][0] = stage 1 of tile
   // k, stage[k][1] = stage 2 of tile k (and the brute-force sums at k = 0).
   std::vector<std::vector<std::pair<int, SumLaunch>>> stage(2 * max_tiles);
@@ -1472,7 +1542,7 @@ void build_groups(dd_batch& B, void* const* outputs) {
         if (k == 0) stage[1].emplace_back(p, brute_launch(P, outputs[p]));
         continue;
       }
-      if (k * P.tile >= P.nout) continue;
+      if (k * P.tile >= P.seg) continue;
       stage[2 * k].emplace_back(p, stage1_launch(P, k * P.tile));
       stage[2 * k + 1].emplace_back(p, stage2_launch(P, k * P.tile, outputs[p]));
     }

@@ -77,6 +77,12 @@ struct dd_plan {
   int sbw = 32, ndm0 = 32;
   int max_delay = 0, max_res = 0;
   int inter16 = 0;           // stage-1 sums stored as uint16 (8-bit input, narrow subbands)
+  // Folded layout (dd_sumsmem.cu): samples per word (4 or 2; 1: not folded), output
+  // columns per segment (all of them when not folded), planes of subband sums.  The
+  // time tiles, and x and subband-sum pitches of a folded plan count words.
+  int fold = 1;
+  int64_t seg = 0;
+  int planes = 1;
   int twin = 0;              // stage 1 also writes the one-sample-shifted twin of its uint16 sums
   int64_t tile = 0;          // time tile of the stage-1 -> stage-2 pipeline
   int64_t tile_pitch = 0;    // row pitch of the inter tile (elements)
@@ -208,6 +214,10 @@ struct PrepArgs {
   int64_t c0, c1;          // channels [c0, c1)
   int ds;
   int64_t pitch;           // elements per output row
+  // folded layout (fold 4 or 2): out[(c - c0)][s] = the samples s, s + seg, ... of the
+  // channel in one 32-bit word, words [0, nwords)
+  int fold;
+  int64_t seg, nwords;
   void* full_out;          // optional [nsamp][nchans] copy after all stages
 };
 void launch_prep(const PrepArgs& a, cudaStream_t st);
@@ -275,7 +285,7 @@ inline void allow_dynamic_smem(K kernel, size_t dynamic_smem) {
 // into shared memory falls with their number; rows are split over warp groups that
 // each cover the whole tile (kSumRowsPT* rows per thread).
 constexpr int kSumRows = 16;
-constexpr int kSumRowsPT8 = 8, kSumRowsPTW = 8, kSumRowsPT32 = 8, kSumRowsPTT = 4;
+constexpr int kSumRowsPT8 = 8, kSumRowsPTW = 8, kSumRowsPTT = 4;
 // Staging descriptor of one (row group, source) pair of a staged sum: the
 // smallest offset of the group's rows for that source, the spread of their
 // offsets, and each row's offset relative to the smallest.  Built on the host
@@ -290,6 +300,7 @@ static_assert(sizeof(SumDesc) == 48, "bulk copies move whole 16-byte units");
 struct SumLaunch {
   enum Mode { kStage1 = 0, kStage2 = 1, kBrute = 2 };
   int mode;
+  int kind;                // SumKind
   const char* src;         // byte address of source row 0
   int64_t src_pitch;       // bytes between source rows
   const int32_t* off;      // per-row, per-source offsets (elements)
@@ -305,8 +316,10 @@ struct SumLaunch {
   int out_elem;            // bytes per output element
   int64_t ncols;           // columns of the launch
   int win_bytes;           // bytes of one staged source window
-  int src_bytes;           // 1 or 2
-  int flush;               // 8- and 16-bit sources into 32-bit sums
+  // Folded sums: bytes between the segments' (or packed planes') outputs of stage 1
+  // and brute force; bytes between the planes stage 2 reads; columns per segment and
+  // of the chunk where the sums go to the output (seg 0: into planes).
+  int64_t seg_stride, plane_bytes, seg, nout;
   unsigned grid_y, grid_z;
   const SumDesc* desc;     // [grid_y][desc_pitch] staging descriptors
   int64_t desc_pitch;      // descriptors per row group (= columns of the offset table)
@@ -360,45 +373,102 @@ constexpr int kErrWaitEmpty = 2;  // the producer gave up waiting for a free sta
 #ifndef DD_SUM8_MINB
 #define DD_SUM8_MINB 2
 #endif
-#ifndef DD_SUM32_NW
-#define DD_SUM32_NW 8
-#endif
-#ifndef DD_SUM32_MINB
-#define DD_SUM32_MINB 2
-#endif
 #ifndef DD_SUM16W_NW
 #define DD_SUM16W_NW 5
 #endif
 #ifndef DD_SUM16W_MINB
 #define DD_SUM16W_MINB 2
 #endif
-#ifndef DD_SUM16W_SMEM_KB
-#define DD_SUM16W_SMEM_KB 100
-#endif
 #ifndef DD_SUM16T_NW
 #define DD_SUM16T_NW 6
 #endif
-constexpr int kSum32NW = DD_SUM32_NW, kSum16TNW = DD_SUM16T_NW;
-// Kernel variant of a staged sum: 8-bit sources into 16-bit sums, 8-bit sources into
-// 32-bit sums, 32-bit sources, 16-bit sources into 32-bit sums, and 16-bit subband
-// sums with their one-sample-shifted twin (stage 2 of 8-bit input).
-enum SumKind { kSumKindU8Out16 = 0, kSumKindU8Flush = 1, kSumKindU32 = 2, kSumKindU16Wide = 3,
-               kSumKindU16Twin = 4 };
-constexpr int kSumKinds = 5;
+constexpr int kSum16TNW = DD_SUM16T_NW;
+// Folded sums: rows per thread, words per lane and blocks per SM.  Few rows of many
+// words: a row of a stage costs one load of its offsets and four addresses whatever its
+// words.  Measured (4096 channels, 2^17 samples, 6001 trials, stage 1 / stage 2, ms; and
+// brute force, 1024 channels, 1001 trials): rows x words 8 x 5 4.83 / 3.61, 5.81;
+// 4 x 10 4.52 / 3.46, 5.40; 2 x 20 4.44 / 3.41, 5.54; 2 x 12 at three blocks per SM
+// 4.86 / 3.49, 7.04.  16-bit samples (8192 channels, 2001 trials): 8 x 5 and 8 x 8
+// 10.2 / 8.11, 2 x 20 and 2 x 32 9.36 / 7.81.
+#ifndef DD_FOLD8_RB
+#define DD_FOLD8_RB 2
+#endif
+#ifndef DD_FOLD8_NW
+#define DD_FOLD8_NW 20
+#endif
+#ifndef DD_FOLD8W_RB
+#define DD_FOLD8W_RB 4
+#endif
+#ifndef DD_FOLD8W_NW
+#define DD_FOLD8W_NW 10
+#endif
+#ifndef DD_FOLD8_MINB
+#define DD_FOLD8_MINB 2
+#endif
+#ifndef DD_FOLD16_RB
+#define DD_FOLD16_RB 2
+#endif
+#ifndef DD_FOLD16_NW
+#define DD_FOLD16_NW 20
+#endif
+#ifndef DD_FOLD16_MINB
+#define DD_FOLD16_MINB 2
+#endif
+#ifndef DD_PLANE16_RB
+#define DD_PLANE16_RB 2
+#endif
+#ifndef DD_PLANE16_NW
+#define DD_PLANE16_NW 20
+#endif
+#ifndef DD_PLANE16_MINB
+#define DD_PLANE16_MINB 2
+#endif
+#ifndef DD_PLANE32_RB
+#define DD_PLANE32_RB 2
+#endif
+#ifndef DD_PLANE32_NW
+#define DD_PLANE32_NW 32
+#endif
+#ifndef DD_PLANE32_MINB
+#define DD_PLANE32_MINB 2
+#endif
+constexpr int kFold8RB = DD_FOLD8_RB, kFold8NW = DD_FOLD8_NW;
+constexpr int kFold8WRB = DD_FOLD8W_RB, kFold8WNW = DD_FOLD8W_NW;
+constexpr int kFold16RB = DD_FOLD16_RB, kFold16NW = DD_FOLD16_NW;
+constexpr int kPlane16RB = DD_PLANE16_RB, kPlane16NW = DD_PLANE16_NW;
+constexpr int kPlane32RB = DD_PLANE32_RB, kPlane32NW = DD_PLANE32_NW;
+// Kernel variants of the staged sums.  Samples in time order: 8-bit into 16-bit sums
+// (U8Out16) or 32-bit sums (U8Flush), 16-bit into 32-bit sums (U16Wide), 16-bit subband
+// sums with their one-sample-shifted twin (U16Twin).  Folded samples: 8-bit into
+// packed 16-bit planes (Fold8) or 32-bit sums (Fold8W), 16-bit into 32-bit sums
+// (Fold16), and stage 2 of packed planes (Plane16).  Stage 2 of 32-bit sums, folded or
+// not (Plane32).
+enum SumKind { kSumKindU8Out16, kSumKindU8Flush, kSumKindU16Wide, kSumKindU16Twin, kSumKindFold8,
+               kSumKindFold8W, kSumKindFold16, kSumKindPlane16, kSumKindPlane32, kSumKinds };
 int sum_kind(const SumLaunch& L);
-// Tile (samples per block) of a kernel variant.
+// Tile of a kernel variant: samples per block, or words for the folded sums and Plane32.
 inline int sum_kind_tile(int kind) {
+  const auto words = [](int rb, int nw) { return sum_tile_samples(4, nw) * rb / kSumRows; };
   switch (kind) {
     case kSumKindU8Out16: case kSumKindU8Flush:
       return sum_tile_samples(1, DD_SUM8_NW) * kSumRowsPT8 / kSumRows;
     case kSumKindU16Wide: return sum_tile_samples(2, DD_SUM16W_NW) * kSumRowsPTW / kSumRows;
     case kSumKindU16Twin: return sum_tile_samples(2, kSum16TNW) * kSumRowsPTT / kSumRows;
-    default: return sum_tile_samples(4, kSum32NW) * kSumRowsPT32 / kSumRows;
+    case kSumKindFold8: return words(kFold8RB, kFold8NW);
+    case kSumKindFold8W: return words(kFold8WRB, kFold8WNW);
+    case kSumKindFold16: return words(kFold16RB, kFold16NW);
+    case kSumKindPlane16: return words(kPlane16RB, kPlane16NW);
+    default: return words(kPlane32RB, kPlane32NW);
   }
 }
-// Source windows per pipeline stage of a kernel variant: 8 for kSumKindU16Twin (four
-// sources, each with its twin), else 2.
-inline int sum_kind_qs(int kind) { return kind == kSumKindU16Twin ? 8 : 2; }
+// Source windows per pipeline stage of a kernel variant.
+inline int sum_kind_qs(int kind) {
+  return kind == kSumKindU16Twin ? 8 : kind >= kSumKindFold8 ? 4 : 2;
+}
+// Bytes of a source element: samples, 16-bit sums or words.
+inline int sum_kind_elem(int kind) {
+  return kind == kSumKindU8Out16 || kind == kSumKindU8Flush ? 1 : kind >= kSumKindFold8 ? 4 : 2;
+}
 // Shared memory of a launch (its variant's windows per stage, plus the variant's
 // staging past the ring, sum_kind_extra_smem).
 size_t sum_launch_smem(const SumLaunch& L);

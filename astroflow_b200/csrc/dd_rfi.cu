@@ -513,6 +513,23 @@ __device__ __forceinline__ T zdm_float_sub(T v, float mean) {
   return static_cast<T>(r);
 }
 
+// The value of sample t of channel c after the RFI stages.
+template <typename T>
+__device__ __forceinline__ T prepared_value(const PrepArgs& a, const T* x, int64_t t, int64_t c) {
+  T v = x[t * a.nchans + c];
+  if (a.segmask) {
+    const int s = find_seg(a.seg_t0, a.nseg, t);
+    if (a.segmask[static_cast<int64_t>(s) * a.nchans + c]) v = 0;
+  }
+  if (a.zdm_off && c >= a.zdm_cs && c < a.zdm_ce) {
+    const uint32_t m = a.zdm_off[t];
+    v = static_cast<T>(static_cast<uint32_t>(v) > m ? static_cast<uint32_t>(v) - m : 0u);
+  }
+  if (a.zdm_mean && c >= a.zdm_cs && c < a.zdm_ce) v = zdm_float_sub<T>(v, a.zdm_mean[t]);
+  if (a.keep && !a.keep[c]) v = 0;
+  return v;
+}
+
 // Fused RFI application and transpose to the channel-major layout.
 // Tile: 64 samples x 64 channels, 256 threads.
 template <typename T>
@@ -528,17 +545,7 @@ __global__ void k_prep(PrepArgs a) {
     const int64_t t = tb + r;
     T v = 0;
     if (t < a.nsamp && c < a.c1) {
-      v = x[t * a.nchans + c];
-      if (a.segmask) {
-        const int s = find_seg(a.seg_t0, a.nseg, t);
-        if (a.segmask[static_cast<int64_t>(s) * a.nchans + c]) v = 0;
-      }
-      if (a.zdm_off && c >= a.zdm_cs && c < a.zdm_ce) {
-        const uint32_t m = a.zdm_off[t];
-        v = static_cast<T>(static_cast<uint32_t>(v) > m ? static_cast<uint32_t>(v) - m : 0u);
-      }
-      if (a.zdm_mean && c >= a.zdm_cs && c < a.zdm_ce) v = zdm_float_sub<T>(v, a.zdm_mean[t]);
-      if (a.keep && !a.keep[c]) v = 0;
+      v = prepared_value<T>(a, x, t, c);
     }
     tile[r][tx] = v;
   }
@@ -725,6 +732,157 @@ __global__ void __launch_bounds__(256) k_prep_u16(PrepArgs a) {
   }
 }
 
+// Folded layout, any channel count and alignment: word s of channel c holds the
+// samples s + f * seg, f = 0 .. F-1 (F = 4 of 8 bits, 2 of 16).  Tile: 64 words x 64
+// channels, 256 threads.
+template <typename T>
+__global__ void __launch_bounds__(256) k_prep_fold(PrepArgs a) {
+  constexpr int F = 4 / sizeof(T);
+  __shared__ uint32_t tile[64][65];  // [channel][word]
+  const T* x = static_cast<const T*>(a.x);
+  const int64_t sb = static_cast<int64_t>(blockIdx.x) * 64;
+  const int64_t cb = a.c0 + static_cast<int64_t>(blockIdx.y) * 64;
+  const int tx = threadIdx.x & 63, ty = threadIdx.x >> 6;
+  const int64_t c = cb + tx;
+  for (int r = ty; r < 64; r += 4) {
+    uint32_t w = 0;
+    if (c < a.c1)
+#pragma unroll
+      for (int f = 0; f < F; ++f) {
+        const int64_t t = sb + r + f * a.seg;
+        if (t < a.nsamp) w |= static_cast<uint32_t>(prepared_value<T>(a, x, t, c)) << (8 * sizeof(T) * f);
+      }
+    tile[tx][r] = w;
+  }
+  __syncthreads();
+  uint32_t* out = static_cast<uint32_t*>(a.out);
+  for (int r = ty; r < 64; r += 4)
+    if (cb + r < a.c1 && sb + tx < a.nwords) out[(cb + r - a.c0) * a.pitch + sb + tx] = tile[r][tx];
+}
+
+// The same with word loads: four channels per load (4 or 8 bytes), the RFI stages
+// word-wise as in k_prep_u8 / k_prep_u16, and the samples of the segments put together
+// by byte permutes, so that shared memory is written and read once per output word.
+// Needs nchans % 4 == 0 and an aligned input; channel words are read from c0 & ~3.
+template <typename T>
+__global__ void __launch_bounds__(256) k_prep_fold_w(PrepArgs a) {
+  constexpr int F = 4 / sizeof(T);   // samples per word
+  constexpr int V = sizeof(T);       // 32-bit words per four channels
+  __shared__ uint32_t tile[64][65];  // [channel][word]
+  const T* x = static_cast<const T*>(a.x);
+  const int64_t sb = static_cast<int64_t>(blockIdx.x) * 64;
+  const int64_t cb = (a.c0 & ~int64_t(3)) + static_cast<int64_t>(blockIdx.y) * 64;
+  const int w = threadIdx.x & 15, r0 = threadIdx.x >> 4;
+  const int64_t c = cb + 4 * w;
+  const bool cvalid = c < a.nchans;
+  uint32_t drop[V], inrange[V];  // per lane: bad channel / zero-DM applies
+#pragma unroll
+  for (int v = 0; v < V; ++v) drop[v] = inrange[v] = 0;
+  if (cvalid) {
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+      const int64_t ch = c + b;
+      const uint32_t lane = V == 1 ? 0xffu << (8 * b) : 0xffffu << (16 * (b & 1));
+      if (a.keep && !a.keep[ch]) drop[V == 1 ? 0 : b >> 1] |= lane;
+      if (a.zdm_off && ch >= a.zdm_cs && ch < a.zdm_ce) inrange[V == 1 ? 0 : b >> 1] |= lane;
+    }
+  }
+  // the IQRM mask of this thread's channels in the tile's rows of each segment: rows of
+  // one tile lie in one IQRM segment but for the tiles at its ends
+  uint32_t keep4[F];
+  bool one[F];
+#pragma unroll
+  for (int f = 0; f < F; ++f) {
+    keep4[f] = ~0u;
+    one[f] = true;
+    if (a.segmask && cvalid) {
+      const int64_t t = sb + f * a.seg;
+      const int s0 = find_seg(a.seg_t0, a.nseg, t);
+      one[f] = s0 + 1 >= a.nseg || static_cast<int64_t>(a.seg_t0[s0 + 1]) > t + 63;
+      if (one[f])
+        keep4[f] = ~__vcmpne4(*reinterpret_cast<const uint32_t*>(
+                                  a.segmask + static_cast<int64_t>(s0) * a.nchans + c), 0u);
+    }
+  }
+  uint32_t in[4][F][V];
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+#pragma unroll
+    for (int f = 0; f < F; ++f) {
+      const int64_t t = sb + r0 + 16 * k + f * a.seg;
+#pragma unroll
+      for (int v = 0; v < V; ++v) in[k][f][v] = 0;
+      if (cvalid && t < a.nsamp) {
+        const T* p = x + t * a.nchans + c;
+        if constexpr (V == 1) {
+          in[k][f][0] = __ldg(reinterpret_cast<const uint32_t*>(p));
+        } else {
+          const uint2 u = __ldg(reinterpret_cast<const uint2*>(p));
+          in[k][f][0] = u.x;
+          in[k][f][V - 1] = u.y;
+        }
+      }
+    }
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+#pragma unroll
+    for (int f = 0; f < F; ++f) {
+      const int64_t t = sb + r0 + 16 * k + f * a.seg;
+      if (!cvalid || t >= a.nsamp) continue;
+      uint32_t m4 = keep4[f];
+      if (a.segmask && !one[f])
+        m4 = ~__vcmpne4(*reinterpret_cast<const uint32_t*>(
+                            a.segmask + static_cast<int64_t>(find_seg(a.seg_t0, a.nseg, t)) * a.nchans + c), 0u);
+      if constexpr (V == 1) {
+        uint32_t v = in[k][f][0] & m4;
+        if (a.zdm_off) {
+          const uint32_t m = min(a.zdm_off[t], 255u) * 0x01010101u;
+          v = (__vsubus4(v, m) & inrange[0]) | (v & ~inrange[0]);
+        }
+        in[k][f][0] = v & ~drop[0];
+      } else {
+        uint32_t u0 = in[k][f][0] & __byte_perm(m4, 0u, 0x1100);
+        uint32_t u1 = in[k][f][V - 1] & __byte_perm(m4, 0u, 0x3322);
+        if (a.zdm_off) {
+          const uint32_t m = min(a.zdm_off[t], 65535u) * 0x00010001u;
+          u0 = (__vsubus2(u0, m) & inrange[0]) | (u0 & ~inrange[0]);
+          u1 = (__vsubus2(u1, m) & inrange[V - 1]) | (u1 & ~inrange[V - 1]);
+        }
+        in[k][f][0] = u0 & ~drop[0];
+        in[k][f][V - 1] = u1 & ~drop[V - 1];
+      }
+    }
+    uint32_t o[4];
+    if constexpr (V == 1) {
+      const uint32_t v0 = in[k][0][0], v1 = in[k][1][0], v2 = in[k][F - 2][0], v3 = in[k][F - 1][0];
+      const uint32_t lo01 = __byte_perm(v0, v1, 0x5140), hi01 = __byte_perm(v0, v1, 0x7362);
+      const uint32_t lo23 = __byte_perm(v2, v3, 0x5140), hi23 = __byte_perm(v2, v3, 0x7362);
+      o[0] = __byte_perm(lo01, lo23, 0x5410);
+      o[1] = __byte_perm(lo01, lo23, 0x7632);
+      o[2] = __byte_perm(hi01, hi23, 0x5410);
+      o[3] = __byte_perm(hi01, hi23, 0x7632);
+    } else {
+      o[0] = __byte_perm(in[k][0][0], in[k][1][0], 0x5410);
+      o[1] = __byte_perm(in[k][0][0], in[k][1][0], 0x7632);
+      o[2] = __byte_perm(in[k][0][V - 1], in[k][1][V - 1], 0x5410);
+      o[3] = __byte_perm(in[k][0][V - 1], in[k][1][V - 1], 0x7632);
+    }
+#pragma unroll
+    for (int b = 0; b < 4; ++b) tile[4 * w + b][r0 + 16 * k] = o[b];
+  }
+  __syncthreads();
+  uint32_t* out = static_cast<uint32_t*>(a.out);
+  const int lane = threadIdx.x & 31;
+  for (int r = threadIdx.x >> 5; r < 64; r += 8) {
+    const int64_t cc = cb + r;
+    if (cc < a.c0 || cc >= a.c1) continue;
+    uint32_t* dst = out + (cc - a.c0) * a.pitch + sb;
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      if (sb + lane + 32 * h < a.nwords) dst[lane + 32 * h] = tile[r][lane + 32 * h];
+  }
+}
+
 // Full-layout copy of the prepared input (parity checks only): all channels.
 template <typename T>
 __global__ void k_prep_full(PrepArgs a) {
@@ -733,18 +891,7 @@ __global__ void k_prep_full(PrepArgs a) {
   const int64_t c = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (c >= a.nchans) return;
   for (int64_t t = blockIdx.y; t < a.nsamp; t += gridDim.y) {
-  T v = x[t * a.nchans + c];
-  if (a.segmask) {
-    const int s = find_seg(a.seg_t0, a.nseg, t);
-    if (a.segmask[static_cast<int64_t>(s) * a.nchans + c]) v = 0;
-  }
-  if (a.zdm_off && c >= a.zdm_cs && c < a.zdm_ce) {
-    const uint32_t m = a.zdm_off[t];
-    v = static_cast<T>(static_cast<uint32_t>(v) > m ? static_cast<uint32_t>(v) - m : 0u);
-  }
-  if (a.zdm_mean && c >= a.zdm_cs && c < a.zdm_ce) v = zdm_float_sub<T>(v, a.zdm_mean[t]);
-  if (a.keep && !a.keep[c]) v = 0;
-  out[t * a.nchans + c] = v;
+    out[t * a.nchans + c] = prepared_value<T>(a, x, t, c);
   }
 }
 
@@ -909,7 +1056,16 @@ void launch_zdm_offsets(const void* x, int nbits, int64_t nsamp, int64_t nchans,
 
 void launch_prep(const PrepArgs& a, cudaStream_t st) {
   // the word-wise kernels apply integer zero-DM offsets only
-  if (a.out && !a.zdm_mean && a.nbits == 8 && a.ds == 1 && a.nchans % 4 == 0 && a.pitch % 4 == 0 &&
+  if (a.out && a.fold > 1) {
+    const bool wide = !a.zdm_mean && a.nchans % 4 == 0 && reinterpret_cast<uintptr_t>(a.x) % (a.nbits / 2) == 0;
+    const int64_t cw0 = wide ? a.c0 & ~int64_t(3) : a.c0;
+    const dim3 grid(static_cast<unsigned>((a.nwords + 63) / 64), static_cast<unsigned>((a.c1 - cw0 + 63) / 64));
+    if (a.nbits == 8 && wide) k_prep_fold_w<uint8_t><<<grid, 256, 0, st>>>(a);
+    else if (a.nbits == 8) k_prep_fold<uint8_t><<<grid, 256, 0, st>>>(a);
+    else if (wide) k_prep_fold_w<uint16_t><<<grid, 256, 0, st>>>(a);
+    else k_prep_fold<uint16_t><<<grid, 256, 0, st>>>(a);
+    DD_LAUNCHED();
+  } else if (a.out && !a.zdm_mean && a.nbits == 8 && a.ds == 1 && a.nchans % 4 == 0 && a.pitch % 4 == 0 &&
       reinterpret_cast<uintptr_t>(a.x) % 4 == 0 && reinterpret_cast<uintptr_t>(a.out) % 4 == 0) {
     const int64_t cw0 = a.c0 & ~int64_t(3);
     const int64_t span = 64 * kPrepU8Subtiles;

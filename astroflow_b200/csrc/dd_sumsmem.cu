@@ -134,7 +134,7 @@ struct Geo {
   int64_t src_pitch;   // bytes between consecutive sources
   const SumDesc* desc; // descriptor of source 0 for this block's row group
   int64_t base;        // element index added to every offset
-  int nsrc, nrows;     // nrows 0: nothing to do
+  int nsrc, nrows;     // nrows <= 0: nothing to do
   char* out;           // row 0, launch column 0 (byte address)
   int64_t out_pitch;   // bytes between output rows
   const int32_t* skew; // per row, or nullptr
@@ -165,8 +165,6 @@ __device__ __forceinline__ Geo make_geo(const SumLaunch& L, int T, uint3 blk) {
       g.out = L.out + (j0 * L.nsb_out + sb) * L.out_pitch + L.out_col0 * L.out_elem;
       g.out_pitch = L.nsb_out * L.out_pitch;
       g.skew = L.skew + (static_cast<int64_t>(blk.y) * L.nsb_out + sb) * kSumRows;
-      // the last row has the largest skew
-      if (g.col >= g.ncols + __ldg(g.skew + g.nrows - 1)) g.nrows = 0;
       break;
     }
     case SumLaunch::kStage2: {
@@ -175,7 +173,7 @@ __device__ __forceinline__ Geo make_geo(const SumLaunch& L, int T, uint3 blk) {
       const int64_t j = blk.y / per_nom;
       const int64_t m0 = j * L.group + static_cast<int64_t>(blk.y % per_nom) * kSumRows;
       const int64_t mend = min((j + 1) * L.group, L.nrows_total);
-      g.src = L.src + j * L.nsrc_total * L.src_pitch;
+      g.src = L.src + blk.z * L.plane_bytes + j * L.nsrc_total * L.src_pitch;
       g.desc = drow;
       g.nsrc = static_cast<int>(L.nsrc_total);
       g.nrows = static_cast<int>(max(static_cast<int64_t>(0), min(static_cast<int64_t>(kSumRows), mend - m0)));
@@ -317,9 +315,44 @@ __device__ __forceinline__ void produce_twin(const Geo& g, Pipe& P, uint32_t* sw
     }
 }
 
+// The same for sources of 32-bit words (folded samples and their sums), four per
+// stage: every offset is a whole word, so a row's offset needs no shift.
+__device__ __forceinline__ void produce_words(const Geo& g, Pipe& P, uint32_t* sw, int ww, int zero_q,
+                                              int tile_words, const GroupDesc<4>& d, int q, int s, int lane) {
+  const int i = lane >> 4, r = lane & 15;
+  uint32_t nbytes[2] = {0, 0};
+  const char* gsrc[2] = {nullptr, nullptr};
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int k = i + 2 * h;  // source of the stage
+    const int src = 4 * q + k;
+    int idx = zero_q;
+    if (src < g.nsrc) {
+      const int64_t e0 = g.base + d.lo[h];
+      const int64_t a0 = e0 & ~int64_t(3);
+      idx = (4 * s + k) * ww + static_cast<int>(e0 - a0) + d.rel[h];
+      if (r == 0) {
+        nbytes[h] = static_cast<uint32_t>((e0 + d.span[h] + tile_words - a0 + 3) & ~int64_t(3)) * 4u;
+        gsrc[h] = g.src + static_cast<int64_t>(src) * g.src_pitch + 4 * a0;
+      }
+    }
+    P.row[s][r][k] = idx;
+  }
+  uint32_t total = nbytes[0] + nbytes[1];
+  total += __shfl_xor_sync(0xffffffffu, total, 16);
+  __syncwarp();
+  if (lane == 0) mbar_arrive_expect_tx(&P.full[s], total);
+  __syncwarp();
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+    if (nbytes[h]) bulk_copy(sw + (4 * s + i + 2 * h) * ww, gsrc[h], nbytes[h], &P.full[s]);
+}
+
 // Pipeline driver shared by the kernels: calls body(stage, cur) for every group of
-// QS sources once their windows are in shared memory (TWIN: each source is staged
-// with its shifted twin, see produce_twin; QS is 4).  The warps take turns at
+// QS sources once their windows are in shared memory, and setup() once the first
+// windows are on their way; false when the block has nothing to store (kModeTwin: each source is staged
+// with its shifted twin, see produce_twin; kModeWords: see produce_words; QS is 4 for
+// both; `tile` is in bytes, for kModeWords in words).  The warps take turns at
 // staging: warp q % kWarps stages group q, D groups before they are summed, and has
 // loaded the group's descriptors kWarps groups earlier, so that no warp carries the
 // staging beside its sums and none waits for a descriptor.  D leaves a stage of slack
@@ -328,11 +361,11 @@ __device__ __forceinline__ void produce_twin(const Geo& g, Pipe& P, uint32_t* sw
 // 1, 3.8 in stage 2): 4096 channels of 8 bits, 2^20 samples, 6001 trials took 66.2 +
 // 40.1 ms (stages 1 and 2) that way and 56.6 + 32.8 ms with turns; brute force over
 // 1024 channels, 2^17 samples, 1001 trials 10.8 and 8.5 ms.
-constexpr int kModePlain = 0, kModeTwin = 1;
-template <int SB, int QS = 2, int MODE = kModePlain, typename Body>
-__device__ __forceinline__ void run_pipeline(const SumLaunch& L, const Geo& g, Pipe& P,
-                                             uint32_t* sw, int tile_bytes, Body&& body) {
-  static_assert(QS == (MODE == kModeTwin ? 4 : 2), "pairs of sources, or four with their twins");
+constexpr int kModePlain = 0, kModeTwin = 1, kModeWords = 2;
+template <int SB, int QS = 2, int MODE = kModePlain, typename Setup, typename Body>
+__device__ __forceinline__ bool run_pipeline(const SumLaunch& L, const Geo& g, Pipe& P,
+                                             uint32_t* sw, int tile, Setup&& setup, Body&& body) {
+  static_assert(QS == (MODE == kModePlain ? 2 : 4), "sources per stage");
   static_assert(kMaxStages <= kWarps, "each warp stages at most one group before the loop");
   constexpr int kWinPerSrc = MODE == kModeTwin ? 2 : 1;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -343,6 +376,8 @@ __device__ __forceinline__ void run_pipeline(const SumLaunch& L, const Geo& g, P
   const int ngroups = (g.nsrc + QS - 1) / QS;
   GroupDesc<QS> desc;
   desc.load(g, warp, lane);
+  // stage 1: blocks past the last column of every row (the last row has the largest skew)
+  if (g.skew && g.col >= g.ncols + __ldg(g.skew + g.nrows - 1)) return false;
   if (threadIdx.x == 0) {
     for (int s = 0; s < S; ++s) {
       mbar_init(&P.full[s], 1);
@@ -354,19 +389,23 @@ __device__ __forceinline__ void run_pipeline(const SumLaunch& L, const Geo& g, P
   // order earlier generic accesses to the windows (a previous task of a persistent
   // block) before the bulk copies that refill them
   asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-  for (int i = threadIdx.x; i < ww; i += kThreads) sw[zero_q + i] = 0u;
+  if (g.nsrc % QS)  // a source is missing in the last group
+    for (int i = threadIdx.x; i < ww; i += kThreads) sw[zero_q + i] = 0u;
   __syncthreads();
   volatile int* failed = &P.failed;
   int next = warp;  // the next group this warp stages
   auto stage_next = [&](int s) {
     if constexpr (MODE == kModeTwin)
-      produce_twin(g, P, sw, ww, zero_q, tile_bytes, L.twin_off, desc, next, s, lane);
+      produce_twin(g, P, sw, ww, zero_q, tile, L.twin_off, desc, next, s, lane);
+    else if constexpr (MODE == kModeWords)
+      produce_words(g, P, sw, ww, zero_q, tile, desc, next, s, lane);
     else
-      produce<SB>(g, P, sw, ww, zero_q, tile_bytes, desc, next, s, lane);
+      produce<SB>(g, P, sw, ww, zero_q, tile, desc, next, s, lane);
     next += kWarps;
     desc.load(g, next, lane);
   };
   if (next < min(D, ngroups)) stage_next(next);
+  setup();
   int s_cur = 0, p = 0;
   uint32_t ph_cur = 0;
   for (; p < ngroups; ++p) {
@@ -411,18 +450,22 @@ __device__ __forceinline__ void run_pipeline(const SumLaunch& L, const Geo& g, P
       asm volatile("mbarrier.inval.shared::cta.b64 [%0];\n" ::"r"(smem_addr(&P.empty[st])) : "memory");
     }
   }
+  return !P.failed;
 }
 
-// Rows of this thread's warp group that have columns in the block, as a bit mask:
-// skews move rows in and out of the first and last blocks of a launch, and the last
-// row group may hold fewer rows.
+// A block's rows are dealt to its warp groups in turn (group i has rows i, i + groups,
+// ...), so that blocks in which some rows have no columns still keep every warp busy.
+// Rows of this thread's warp group that have columns in the block, as a bit mask: skews
+// move rows in and out of the first and last blocks of a launch, and the last row group
+// may hold fewer rows.
 template <int RB, int T>
 __device__ __forceinline__ uint32_t active_rows(const Geo& g, int rbase) {
+  constexpr int kGroups = kSumRows / RB;
   uint32_t act = 0;
 #pragma unroll
   for (int r = 0; r < RB; ++r)
-    if (rbase + r < g.nrows) {
-      const int64_t c = row_col(g, rbase + r);
+    if (rbase + kGroups * r < g.nrows) {
+      const int64_t c = row_col(g, rbase + kGroups * r);
       if (c < g.ncols && c + T > 0) act |= 1u << r;
     }
   return act;
@@ -453,9 +496,9 @@ __device__ __forceinline__ void sum_u8(const SumLaunch& L, uint3 blk, uint32_t* 
   const Geo g = make_geo(L, T, blk);
   if (g.nrows <= 0) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int rbase = (warp / kWarpsPerTile) * RB, wt = warp % kWarpsPerTile;
+  const int rbase = warp / kWarpsPerTile, wt = warp % kWarpsPerTile;
   const int wbase = wt * 32 * NW + lane * NW;
-  const uint32_t act = active_rows<RB, T>(g, rbase);
+  uint32_t act = 0;
   constexpr int kSeg = 32 * NW * 4;  // samples of a warp's segment
   uint32_t p01[RB][NW], p23[RB][NW];  // field sums of samples (4w, 4w+1) and (4w+2, 4w+3)
 #pragma unroll
@@ -478,8 +521,8 @@ __device__ __forceinline__ void sum_u8(const SumLaunch& L, uint3 blk, uint32_t* 
         p01[r][k] = p23[r][k] = 0;
       }
       __syncwarp();
-      const int64_t c0 = row_col(g, rbase + r) + static_cast<int64_t>(wt) * kSeg;  // multiple of 4
-      uint32_t* out = reinterpret_cast<uint32_t*>(g.out + (rbase + r) * g.out_pitch) + c0;
+      const int64_t c0 = row_col(g, rbase + kGroups * r) + static_cast<int64_t>(wt) * kSeg;  // multiple of 4
+      uint32_t* out = reinterpret_cast<uint32_t*>(g.out + (rbase + kGroups * r) * g.out_pitch) + c0;
       for (int e = 4 * lane; e < kSeg; e += 128) {
         uint4 v = *reinterpret_cast<const uint4*>(st + e);
         if (c0 + e < 0) continue;
@@ -500,9 +543,9 @@ __device__ __forceinline__ void sum_u8(const SumLaunch& L, uint3 blk, uint32_t* 
   };
   int since = 0;       // sources summed in the fields since the last flush
   bool stored = false; // the output holds partial sums of an earlier flush
-  run_pipeline<1>(L, g, P, sw, T, [&](int s, const uint32_t* win) {
+  const bool ok = run_pipeline<1>(L, g, P, sw, T, [&] { act = active_rows<RB, T>(g, rbase); }, [&](int s, const uint32_t* win) {
     for_rows<RB>(act, [&](int r) {
-      const int4 rw = row_info(P, s, rbase + r);
+      const int4 rw = row_info(P, s, rbase + kGroups * r);
       const uint32_t* w0 = win + rw.x + wbase;
       const uint32_t* w1 = win + rw.z + wbase;
       uint32_t va[NW + 1], vb[NW + 1];
@@ -525,7 +568,7 @@ __device__ __forceinline__ void sum_u8(const SumLaunch& L, uint3 blk, uint32_t* 
       }
     }
   });
-  if (P.failed) return;
+  if (!ok) return;
   if constexpr (!OUT16) {
     if (since > 0 || !stored) flush(stored);
     return;
@@ -546,8 +589,8 @@ __device__ __forceinline__ void sum_u8(const SumLaunch& L, uint3 blk, uint32_t* 
       *reinterpret_cast<uint2*>(st + 4 * (lane * NW + k)) =
           make_uint2(dot_pack(p01[r][k]), dot_pack(p23[r][k]));
     __syncwarp();
-    const int64_t c0 = row_col(g, rbase + r) + static_cast<int64_t>(wt) * kSeg;  // multiple of 8
-    char* row = g.out + (rbase + r) * g.out_pitch;
+    const int64_t c0 = row_col(g, rbase + kGroups * r) + static_cast<int64_t>(wt) * kSeg;  // multiple of 8
+    char* row = g.out + (rbase + kGroups * r) * g.out_pitch;
     uint16_t* out = reinterpret_cast<uint16_t*>(row) + c0;
     uint16_t* tw = L.twin_off ? reinterpret_cast<uint16_t*>(row + L.twin_off) + c0 : nullptr;
     for (int e = 8 * lane; e < kSeg; e += 256) {
@@ -597,17 +640,17 @@ __device__ __forceinline__ void sum_u16_wide(const SumLaunch& L, uint3 blk, uint
   const Geo g = make_geo(L, T, blk);
   if (g.nrows <= 0) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int rbase = (warp / kWarpsPerTile) * RB, wt = warp % kWarpsPerTile;
+  const int rbase = warp / kWarpsPerTile, wt = warp % kWarpsPerTile;
   const int wbase = wt * 32 * NW + lane * NW;  // consecutive words, as in sum_u8
-  const uint32_t act = active_rows<RB, T>(g, rbase);
+  uint32_t act = 0;
   uint32_t lo32[RB][NW], hi32[RB][NW];
 #pragma unroll
   for (int r = 0; r < RB; ++r)
 #pragma unroll
     for (int k = 0; k < NW; ++k) lo32[r][k] = hi32[r][k] = 0;
-  run_pipeline<2>(L, g, P, sw, 2 * T, [&](int s, const uint32_t* win) {
+  const bool ok = run_pipeline<2>(L, g, P, sw, 2 * T, [&] { act = active_rows<RB, T>(g, rbase); }, [&](int s, const uint32_t* win) {
     for_rows<RB>(act, [&](int r) {
-      const int4 rw = row_info(P, s, rbase + r);
+      const int4 rw = row_info(P, s, rbase + kGroups * r);
       const uint32_t* w0 = win + rw.x + wbase;
       const uint32_t* w1 = win + rw.z + wbase;
       uint32_t va[NW + 1], vb[NW + 1];
@@ -630,12 +673,12 @@ __device__ __forceinline__ void sum_u16_wide(const SumLaunch& L, uint3 blk, uint
   for (int r = 0; r < RB; ++r)
 #pragma unroll
     for (int k = 0; k < NW; ++k) lo32[r][k] -= hi32[r][k] << 16;
-  if (P.failed) return;
+  if (!ok) return;
 #pragma unroll
   for (int r = 0; r < RB; ++r) {
     if (!(act >> r & 1u)) continue;
-    const int64_t c0 = row_col(g, rbase + r);
-    uint32_t* row = reinterpret_cast<uint32_t*>(g.out + (rbase + r) * g.out_pitch);
+    const int64_t c0 = row_col(g, rbase + kGroups * r);
+    uint32_t* row = reinterpret_cast<uint32_t*>(g.out + (rbase + kGroups * r) * g.out_pitch);
 #pragma unroll
     for (int k = 0; k < NW; ++k) {
       const int64_t c = c0 + static_cast<int64_t>(wbase + k) * 2;  // even
@@ -651,44 +694,264 @@ __device__ __forceinline__ void sum_u16_wide(const SumLaunch& L, uint3 blk, uint
   }
 }
 
-// ------------------------------------------------------------------ 32-bit samples
-// Sources of 32-bit words (stage-1 sums stored as uint32): every sample is a whole
-// word, so no shifts; sums wrap modulo 2^32 like the reference's uint32 accumulators.
-template <int RB, int NW>
-__device__ __forceinline__ void sum_u32(const SumLaunch& L, uint3 blk, uint32_t* sw, Pipe& P) {
+// ------------------------------------------------------------------ folded samples
+// A folded chunk holds in word s the samples s, s + H, s + 2H, s + 3H of a channel
+// (8-bit samples, H a quarter of the output columns) or s, s + H (16-bit samples, H
+// half of them): one word position stands for a column in each of those segments.  A
+// delay moves all of them alike, so every row of every source reads whole aligned
+// words whatever its delay: no shift, no neighbouring word.  Per word of four 8-bit
+// samples that is one shared load and two dot products.  The subband sums keep the
+// fold (segments 0, 1 and 2, 3 as two planes of packed 16-bit pairs, or one plane of
+// 32-bit sums per segment), so stage 2 reads aligned words too and needs no twin.
+// Lanes own interleaved words (lane l: l, l + 32, ...): a warp's loads and stores are
+// 32 consecutive words.  Bound: shared loads and dot products both allow 128 sample
+// additions per cycle and SM (3.7e13 per second); stage 1 runs 2.4e13 (first and last
+// blocks of a time tile, whose rows are partly idle, cost it most: 2.7e13 with 8 GiB
+// tiles), stage 2 (two bytes per addition: 64 per cycle) 1.5e13, its load pipe 85 %
+// busy.  Against samples in time order: 4096 channels, 2^20 samples, 6001 trials 56.6 +
+// 32.8 -> 34.4 + 27.3 ms.
+
+// Columns of segment f that are stored, in launch columns: below ncols, and for sums
+// into the output (L.seg > 0) inside the segment and the chunk.
+__device__ __forceinline__ int64_t seg_cols(const SumLaunch& L, int f) {
+  if (!L.seg) return L.ncols;
+  return min(L.ncols, min(L.seg, L.nout - f * L.seg) - L.out_col0);
+}
+
+// Folded 8-bit samples into packed 16-bit planes (PACK) or 32-bit sums per segment.
+template <int RB, int NW, bool PACK>
+__device__ __forceinline__ void sum_fold8(const SumLaunch& L, uint3 blk, uint32_t* sw, Pipe& P) {
   constexpr int kGroups = kSumRows / RB;  // warp groups sharing the rows, as in sum_u8
   constexpr int kWarpsPerTile = kWarps / kGroups;
   constexpr int T = kWarpsPerTile * 32 * NW;
   const Geo g = make_geo(L, T, blk);
   if (g.nrows <= 0) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int rbase = (warp / kWarpsPerTile) * RB;
+  const int rbase = warp / kWarpsPerTile;
   const int wbase = (warp % kWarpsPerTile) * 32 * NW + lane;
-  const uint32_t act = active_rows<RB, T>(g, rbase);
+  uint32_t act = 0;
+  uint32_t p01[RB][NW], p23[RB][NW];  // field sums of segments 0, 1 and 2, 3
+#pragma unroll
+  for (int r = 0; r < RB; ++r)
+#pragma unroll
+    for (int k = 0; k < NW; ++k) p01[r][k] = p23[r][k] = 0;
+  // 32-bit outputs: adds the fields to what an earlier flush stored when `add`, and
+  // clears them.  The block owns its outputs; the additions are reductions in L2, which
+  // the warp does not wait for (128 consecutive bytes each).
+  auto flush = [&](bool add) {
+#pragma unroll
+    for (int r = 0; r < RB; ++r) {
+      if (!(act >> r & 1u)) continue;
+      const int64_t c0 = row_col(g, rbase + kGroups * r) + wbase;
+      char* row = g.out + (rbase + kGroups * r) * g.out_pitch;
+#pragma unroll
+      for (int f = 0; f < 4; ++f) {
+        uint32_t* out = reinterpret_cast<uint32_t*>(row + f * L.seg_stride) + c0;
+        const int64_t lim = seg_cols(L, f) - c0;
+#pragma unroll
+        for (int k = 0; k < NW; ++k) {
+          const uint32_t p = f < 2 ? p01[r][k] : p23[r][k];
+          const uint32_t v = (f & 1) ? p >> 15 : p & 0x7fffu;
+          if (32 * k >= lim || c0 + 32 * k < 0) continue;
+          if (add) atomicAdd(out + 32 * k, v);
+          else out[32 * k] = v;
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < NW; ++k) p01[r][k] = p23[r][k] = 0;
+    }
+  };
+  int since = 0;
+  bool stored = false;
+  const bool ok = run_pipeline<4, 4, kModeWords>(L, g, P, sw, T, [&] { act = active_rows<RB, T>(g, rbase); }, [&](int s, const uint32_t* win) {
+    for_rows<RB>(act, [&](int r) {
+      const int4 a = row_info(P, s, rbase + kGroups * r);
+      const uint32_t* w0 = win + a.x + wbase;
+      const uint32_t* w1 = win + a.y + wbase;
+      const uint32_t* w2 = win + a.z + wbase;
+      const uint32_t* w3 = win + a.w + wbase;
+#pragma unroll
+      for (int k = 0; k < NW; ++k) {
+        const uint32_t v0 = w0[32 * k], v1 = w1[32 * k], v2 = w2[32 * k], v3 = w3[32 * k];
+        p01[r][k] = dot_lo(v3, dot_lo(v2, dot_lo(v1, dot_lo(v0, p01[r][k]))));
+        p23[r][k] = dot_hi(v3, dot_hi(v2, dot_hi(v1, dot_hi(v0, p23[r][k]))));
+      }
+    });
+    if constexpr (!PACK) {  // (packed sums hold at most 64 sources)
+      since += 4;
+      if (since >= kDotSources) {
+        flush(stored);
+        stored = true;
+        since = 0;
+      }
+    }
+  });
+  if (!ok) return;
+  if constexpr (!PACK) {
+    if (since > 0 || !stored) flush(stored);
+    return;
+  }
+#pragma unroll
+  for (int r = 0; r < RB; ++r) {
+    if (!(act >> r & 1u)) continue;
+    const int64_t c0 = row_col(g, rbase + kGroups * r) + wbase;
+    char* row = g.out + (rbase + kGroups * r) * g.out_pitch;
+    uint32_t* o0 = reinterpret_cast<uint32_t*>(row) + c0;
+    uint32_t* o1 = reinterpret_cast<uint32_t*>(row + L.seg_stride) + c0;
+#pragma unroll
+    for (int k = 0; k < NW; ++k)
+      if (c0 + 32 * k >= 0 && c0 + 32 * k < g.ncols) {
+        o0[32 * k] = dot_pack(p01[r][k]);
+        o1[32 * k] = dot_pack(p23[r][k]);
+      }
+  }
+}
+
+// Folded 16-bit samples into 32-bit sums per segment: words are summed whole
+// (wrapping) beside their high halves; the low samples' sums are whole - (high << 16)
+// (at most 65537 sources of 65535 each: no wrap of the low sums).
+template <int RB, int NW>
+__device__ __forceinline__ void sum_fold16(const SumLaunch& L, uint3 blk, uint32_t* sw, Pipe& P) {
+  constexpr int kGroups = kSumRows / RB;
+  constexpr int kWarpsPerTile = kWarps / kGroups;
+  constexpr int T = kWarpsPerTile * 32 * NW;
+  const Geo g = make_geo(L, T, blk);
+  if (g.nrows <= 0) return;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rbase = warp / kWarpsPerTile;
+  const int wbase = (warp % kWarpsPerTile) * 32 * NW + lane;
+  uint32_t act = 0;
+  uint32_t all[RB][NW], hi[RB][NW];
+#pragma unroll
+  for (int r = 0; r < RB; ++r)
+#pragma unroll
+    for (int k = 0; k < NW; ++k) all[r][k] = hi[r][k] = 0;
+  const bool ok = run_pipeline<4, 4, kModeWords>(L, g, P, sw, T, [&] { act = active_rows<RB, T>(g, rbase); }, [&](int s, const uint32_t* win) {
+    for_rows<RB>(act, [&](int r) {
+      const int4 a = row_info(P, s, rbase + kGroups * r);
+      const uint32_t* w0 = win + a.x + wbase;
+      const uint32_t* w1 = win + a.y + wbase;
+      const uint32_t* w2 = win + a.z + wbase;
+      const uint32_t* w3 = win + a.w + wbase;
+#pragma unroll
+      for (int k = 0; k < NW; ++k) {
+        const uint32_t v0 = w0[32 * k], v1 = w1[32 * k], v2 = w2[32 * k], v3 = w3[32 * k];
+        all[r][k] += v0 + v1;
+        all[r][k] += v2 + v3;
+        hi[r][k] = high_add(v3, high_add(v2, high_add(v1, high_add(v0, hi[r][k]))));
+      }
+    });
+  });
+  if (!ok) return;
+  const int64_t lim0 = seg_cols(L, 0), lim1 = seg_cols(L, 1);
+#pragma unroll
+  for (int r = 0; r < RB; ++r) {
+    if (!(act >> r & 1u)) continue;
+    const int64_t c0 = row_col(g, rbase + kGroups * r) + wbase;
+    char* row = g.out + (rbase + kGroups * r) * g.out_pitch;
+    uint32_t* o0 = reinterpret_cast<uint32_t*>(row) + c0;
+    uint32_t* o1 = reinterpret_cast<uint32_t*>(row + L.seg_stride) + c0;
+#pragma unroll
+    for (int k = 0; k < NW; ++k) {
+      const int64_t c = c0 + 32 * k;
+      if (c < 0) continue;
+      if (c < lim0) o0[32 * k] = all[r][k] - (hi[r][k] << 16);
+      if (c < lim1) o1[32 * k] = hi[r][k];
+    }
+  }
+}
+
+// Stage 2 of packed 16-bit planes: grid z = plane p, holding segments 2p (low halves)
+// and 2p + 1.  Four words (each half <= 64 x 255) are added before the halves part.
+template <int RB, int NW>
+__device__ __forceinline__ void sum_plane16(const SumLaunch& L, uint3 blk, uint32_t* sw, Pipe& P) {
+  constexpr int kGroups = kSumRows / RB;
+  constexpr int kWarpsPerTile = kWarps / kGroups;
+  constexpr int T = kWarpsPerTile * 32 * NW;
+  const Geo g = make_geo(L, T, blk);
+  if (g.nrows <= 0) return;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rbase = warp / kWarpsPerTile;
+  const int wbase = (warp % kWarpsPerTile) * 32 * NW + lane;
+  uint32_t act = 0;
+  uint32_t all[RB][NW], hi[RB][NW];
+#pragma unroll
+  for (int r = 0; r < RB; ++r)
+#pragma unroll
+    for (int k = 0; k < NW; ++k) all[r][k] = hi[r][k] = 0;
+  const bool ok = run_pipeline<4, 4, kModeWords>(L, g, P, sw, T, [&] { act = active_rows<RB, T>(g, rbase); }, [&](int s, const uint32_t* win) {
+    for_rows<RB>(act, [&](int r) {
+      const int4 a = row_info(P, s, rbase + kGroups * r);
+      const uint32_t* w0 = win + a.x + wbase;
+      const uint32_t* w1 = win + a.y + wbase;
+      const uint32_t* w2 = win + a.z + wbase;
+      const uint32_t* w3 = win + a.w + wbase;
+#pragma unroll
+      for (int k = 0; k < NW; ++k) {
+        const uint32_t q = (w0[32 * k] + w1[32 * k] + w2[32 * k]) + w3[32 * k];
+        all[r][k] += q;
+        hi[r][k] = high_add(q, hi[r][k]);
+      }
+    });
+  });
+  if (!ok) return;
+  const int f = 2 * static_cast<int>(blk.z);
+  const int64_t c0 = g.col + wbase, lim0 = seg_cols(L, f) - c0, lim1 = seg_cols(L, f + 1) - c0;
+#pragma unroll
+  for (int r = 0; r < RB; ++r) {
+    if (!(act >> r & 1u)) continue;
+    uint32_t* o0 = reinterpret_cast<uint32_t*>(g.out + (rbase + kGroups * r) * g.out_pitch) + f * L.seg + c0;
+    uint32_t* o1 = o0 + L.seg;
+#pragma unroll
+    for (int k = 0; k < NW; ++k) {
+      if (32 * k < lim0) o0[32 * k] = all[r][k] - (hi[r][k] << 16);
+      if (32 * k < lim1) o1[32 * k] = hi[r][k];
+    }
+  }
+}
+
+// Stage 2 of 32-bit subband sums (grid z = plane = segment; one plane when the sums
+// are not folded).  Sums wrap modulo 2^32 like the reference's uint32 accumulators.
+template <int RB, int NW>
+__device__ __forceinline__ void sum_plane32(const SumLaunch& L, uint3 blk, uint32_t* sw, Pipe& P) {
+  constexpr int kGroups = kSumRows / RB;
+  constexpr int kWarpsPerTile = kWarps / kGroups;
+  constexpr int T = kWarpsPerTile * 32 * NW;
+  const Geo g = make_geo(L, T, blk);
+  if (g.nrows <= 0) return;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rbase = warp / kWarpsPerTile;
+  const int wbase = (warp % kWarpsPerTile) * 32 * NW + lane;
+  uint32_t act = 0;
   uint32_t acc[RB][NW];
 #pragma unroll
   for (int r = 0; r < RB; ++r)
 #pragma unroll
     for (int k = 0; k < NW; ++k) acc[r][k] = 0;
-  run_pipeline<4>(L, g, P, sw, 4 * T, [&](int s, const uint32_t* win) {
+  const bool ok = run_pipeline<4, 4, kModeWords>(L, g, P, sw, T, [&] { act = active_rows<RB, T>(g, rbase); }, [&](int s, const uint32_t* win) {
     for_rows<RB>(act, [&](int r) {
-      const int4 rw = row_info(P, s, rbase + r);
-      const uint32_t* w0 = win + rw.x + wbase;
-      const uint32_t* w1 = win + rw.z + wbase;
+      const int4 a = row_info(P, s, rbase + kGroups * r);
+      const uint32_t* w0 = win + a.x + wbase;
+      const uint32_t* w1 = win + a.y + wbase;
+      const uint32_t* w2 = win + a.z + wbase;
+      const uint32_t* w3 = win + a.w + wbase;
 #pragma unroll
-      for (int k = 0; k < NW; ++k) acc[r][k] += w0[32 * k] + w1[32 * k];
+      for (int k = 0; k < NW; ++k) {
+        acc[r][k] += w0[32 * k] + w1[32 * k];
+        acc[r][k] += w2[32 * k] + w3[32 * k];
+      }
     });
   });
-  if (P.failed) return;
+  if (!ok) return;
+  const int f = static_cast<int>(blk.z);
+  const int64_t c0 = g.col + wbase, lim = seg_cols(L, f) - c0;
 #pragma unroll
   for (int r = 0; r < RB; ++r) {
     if (!(act >> r & 1u)) continue;
-    uint32_t* row = reinterpret_cast<uint32_t*>(g.out + (rbase + r) * g.out_pitch) + g.col;
+    uint32_t* out = reinterpret_cast<uint32_t*>(g.out + (rbase + kGroups * r) * g.out_pitch) + f * L.seg + c0;
 #pragma unroll
-    for (int k = 0; k < NW; ++k) {
-      const int64_t t = wbase + 32 * k;
-      if (g.col + t < g.ncols) row[t] = acc[r][k];
-    }
+    for (int k = 0; k < NW; ++k)
+      if (32 * k < lim) out[32 * k] = acc[r][k];
   }
 }
 
@@ -715,17 +978,17 @@ __device__ __forceinline__ void sum_u16_twin(const SumLaunch& L, uint3 blk, uint
   const Geo g = make_geo(L, T, blk);
   if (g.nrows <= 0) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int rbase = (warp / kWarpsPerTile) * RB;
+  const int rbase = warp / kWarpsPerTile;
   const int wbase = (warp % kWarpsPerTile) * 32 * NW + lane;
-  const uint32_t act = active_rows<RB, T>(g, rbase);
+  uint32_t act = 0;
   uint32_t lo[RB][NW], hi[RB][NW];
 #pragma unroll
   for (int r = 0; r < RB; ++r)
 #pragma unroll
     for (int k = 0; k < NW; ++k) lo[r][k] = hi[r][k] = 0;
-  run_pipeline<2, 4, kModeTwin>(L, g, P, sw, 2 * T, [&](int s, const uint32_t* win) {
+  const bool ok = run_pipeline<2, 4, kModeTwin>(L, g, P, sw, 2 * T, [&] { act = active_rows<RB, T>(g, rbase); }, [&](int s, const uint32_t* win) {
     for_rows<RB>(act, [&](int r) {
-      const int4 a = row_info(P, s, rbase + r);
+      const int4 a = row_info(P, s, rbase + kGroups * r);
       const uint32_t* w0 = win + a.x + wbase;
       const uint32_t* w1 = win + a.y + wbase;
       const uint32_t* w2 = win + a.z + wbase;
@@ -738,11 +1001,11 @@ __device__ __forceinline__ void sum_u16_twin(const SumLaunch& L, uint3 blk, uint
       }
     });
   });
-  if (P.failed) return;
+  if (!ok) return;
 #pragma unroll
   for (int r = 0; r < RB; ++r) {
     if (!(act >> r & 1u)) continue;
-    uint32_t* row = reinterpret_cast<uint32_t*>(g.out + (rbase + r) * g.out_pitch) + g.col;
+    uint32_t* row = reinterpret_cast<uint32_t*>(g.out + (rbase + kGroups * r) * g.out_pitch) + g.col;
 #pragma unroll
     for (int k = 0; k < NW; ++k) {
       const int64_t t = static_cast<int64_t>(wbase + 32 * k) * 2;
@@ -777,11 +1040,29 @@ __global__ void __launch_bounds__(kThreads, DD_SUM16T_MINB) k_sum_u16t(SumLaunch
   __shared__ Pipe P;
   sum_u16_twin<RB, NW>(L, blockIdx, sw, P);
 }
-template <int RB, int NW>
-__global__ void __launch_bounds__(kThreads, DD_SUM32_MINB) k_sum_u32(SumLaunch L) {
+template <int RB, int NW, bool PACK>
+__global__ void __launch_bounds__(kThreads, DD_FOLD8_MINB) k_sum_fold8(SumLaunch L) {
   extern __shared__ __align__(128) uint32_t sw[];
   __shared__ Pipe P;
-  sum_u32<RB, NW>(L, blockIdx, sw, P);
+  sum_fold8<RB, NW, PACK>(L, blockIdx, sw, P);
+}
+template <int RB, int NW>
+__global__ void __launch_bounds__(kThreads, DD_FOLD16_MINB) k_sum_fold16(SumLaunch L) {
+  extern __shared__ __align__(128) uint32_t sw[];
+  __shared__ Pipe P;
+  sum_fold16<RB, NW>(L, blockIdx, sw, P);
+}
+template <int RB, int NW>
+__global__ void __launch_bounds__(kThreads, DD_PLANE16_MINB) k_sum_plane16(SumLaunch L) {
+  extern __shared__ __align__(128) uint32_t sw[];
+  __shared__ Pipe P;
+  sum_plane16<RB, NW>(L, blockIdx, sw, P);
+}
+template <int RB, int NW>
+__global__ void __launch_bounds__(kThreads, DD_PLANE32_MINB) k_sum_plane32(SumLaunch L) {
+  extern __shared__ __align__(128) uint32_t sw[];
+  __shared__ Pipe P;
+  sum_plane32<RB, NW>(L, blockIdx, sw, P);
 }
 
 // ------------------------------------------------------------------ batched launches
@@ -818,7 +1099,11 @@ __device__ __forceinline__ void run_one(const SumLaunch& L, uint3 blk, uint32_t*
   else if constexpr (KIND == kSumKindU8Flush) sum_u8<kSumRowsPT8, DD_SUM8_NW, false>(L, blk, sw, P);
   else if constexpr (KIND == kSumKindU16Wide) sum_u16_wide<kSumRowsPTW, DD_SUM16W_NW>(L, blk, sw, P);
   else if constexpr (KIND == kSumKindU16Twin) sum_u16_twin<kSumRowsPTT, kSum16TNW>(L, blk, sw, P);
-  else sum_u32<kSumRowsPT32, kSum32NW>(L, blk, sw, P);
+  else if constexpr (KIND == kSumKindFold8) sum_fold8<kFold8RB, kFold8NW, true>(L, blk, sw, P);
+  else if constexpr (KIND == kSumKindFold8W) sum_fold8<kFold8WRB, kFold8WNW, false>(L, blk, sw, P);
+  else if constexpr (KIND == kSumKindFold16) sum_fold16<kFold16RB, kFold16NW>(L, blk, sw, P);
+  else if constexpr (KIND == kSumKindPlane16) sum_plane16<kPlane16RB, kPlane16NW>(L, blk, sw, P);
+  else sum_plane32<kPlane32RB, kPlane32NW>(L, blk, sw, P);
 }
 
 // Grouped launch: one grid over the blocks of several staged sums of the same
@@ -851,7 +1136,11 @@ __device__ __forceinline__ void run_kind(int kind, const SumLaunch& L, uint3 blk
     case kSumKindU8Flush: run_one<kSumKindU8Flush>(L, blk, sw, P); break;
     case kSumKindU16Wide: run_one<kSumKindU16Wide>(L, blk, sw, P); break;
     case kSumKindU16Twin: run_one<kSumKindU16Twin>(L, blk, sw, P); break;
-    default: run_one<kSumKindU32>(L, blk, sw, P); break;
+    case kSumKindFold8: run_one<kSumKindFold8>(L, blk, sw, P); break;
+    case kSumKindFold8W: run_one<kSumKindFold8W>(L, blk, sw, P); break;
+    case kSumKindFold16: run_one<kSumKindFold16>(L, blk, sw, P); break;
+    case kSumKindPlane16: run_one<kSumKindPlane16>(L, blk, sw, P); break;
+    default: run_one<kSumKindPlane32>(L, blk, sw, P); break;
   }
 }
 
@@ -954,9 +1243,7 @@ int sum_stages(int win_bytes, int qs, size_t extra, int cap_kb) {
 
 int sum_kind_stages(int kind, int win_bytes) {
   return sum_stages(win_bytes, sum_kind_qs(kind), sum_kind_extra_smem(kind),
-                    kind == kSumKindU16Twin   ? DD_SUM16T_SMEM_KB
-                    : kind == kSumKindU16Wide ? DD_SUM16W_SMEM_KB
-                                              : DD_SUM_SMEM_KB);
+                    kind == kSumKindU16Twin ? DD_SUM16T_SMEM_KB : DD_SUM_SMEM_KB);
 }
 
 std::vector<SumDesc> build_sum_desc(const std::vector<int32_t>& tab, int64_t nrows,
@@ -1000,18 +1287,15 @@ void launch_sum(const SumLaunch& L, cudaStream_t st) {
     case kSumKindU8Flush: launch_k(k_sum_u8<kSumRowsPT8, DD_SUM8_NW, false>, grid, smem, L, st); break;
     case kSumKindU16Wide: launch_k(k_sum_u16w<kSumRowsPTW, DD_SUM16W_NW>, grid, smem, L, st); break;
     case kSumKindU16Twin: launch_k(k_sum_u16t<kSumRowsPTT, kSum16TNW>, grid, smem, L, st); break;
-    default: launch_k(k_sum_u32<kSumRowsPT32, kSum32NW>, grid, smem, L, st); break;
+    case kSumKindFold8: launch_k(k_sum_fold8<kFold8RB, kFold8NW, true>, grid, smem, L, st); break;
+    case kSumKindFold8W: launch_k(k_sum_fold8<kFold8WRB, kFold8WNW, false>, grid, smem, L, st); break;
+    case kSumKindFold16: launch_k(k_sum_fold16<kFold16RB, kFold16NW>, grid, smem, L, st); break;
+    case kSumKindPlane16: launch_k(k_sum_plane16<kPlane16RB, kPlane16NW>, grid, smem, L, st); break;
+    default: launch_k(k_sum_plane32<kPlane32RB, kPlane32NW>, grid, smem, L, st); break;
   }
 }
 
-int sum_kind(const SumLaunch& L) {
-  if (L.src_bytes == 1) {
-    if (L.out_elem == 2) return kSumKindU8Out16;
-    return kSumKindU8Flush;
-  }
-  if (L.src_bytes == 2) return L.flush ? kSumKindU16Wide : kSumKindU16Twin;
-  return kSumKindU32;
-}
+int sum_kind(const SumLaunch& L) { return L.kind; }
 unsigned sum_grid_x(const SumLaunch& L) {
   const int T = sum_kind_tile(sum_kind(L));
   return static_cast<unsigned>((L.ncols + L.max_skew + T - 1) / T);
@@ -1048,7 +1332,11 @@ void launch_sum_grouped(const SumBatchGroup* d_groups, int ngroups, long long to
     case kSumKindU8Flush: launch_grouped_k<kSumKindU8Flush>(d_groups, ngroups, total, smem, st); break;
     case kSumKindU16Wide: launch_grouped_k<kSumKindU16Wide>(d_groups, ngroups, total, smem, st); break;
     case kSumKindU16Twin: launch_grouped_k<kSumKindU16Twin>(d_groups, ngroups, total, smem, st); break;
-    default: launch_grouped_k<kSumKindU32>(d_groups, ngroups, total, smem, st); break;
+    case kSumKindFold8: launch_grouped_k<kSumKindFold8>(d_groups, ngroups, total, smem, st); break;
+    case kSumKindFold8W: launch_grouped_k<kSumKindFold8W>(d_groups, ngroups, total, smem, st); break;
+    case kSumKindFold16: launch_grouped_k<kSumKindFold16>(d_groups, ngroups, total, smem, st); break;
+    case kSumKindPlane16: launch_grouped_k<kSumKindPlane16>(d_groups, ngroups, total, smem, st); break;
+    default: launch_grouped_k<kSumKindPlane32>(d_groups, ngroups, total, smem, st); break;
   }
 }
 

@@ -1,0 +1,121 @@
+"""Dedispersion sums against the oracle where the layouts and staged kernels can go wrong:
+column counts around the folded segments and block tiles, rows around the row groups,
+subbands around the field and packing limits at full-scale samples, channel counts off
+the load words, band starts, RFI stages per folded segment, and plans whose delays are
+too long for the fold (time-order kernels).  Sums are whole numbers: equality."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+from astroflow_b200.dedisp import Batch, IqrmParams, Plan, RfiParams  # noqa: E402
+from oracle import oracle as O  # noqa: E402
+
+F32 = np.float32
+
+
+def to_np(t):
+    return t.view(torch.int32).cpu().numpy().view(np.uint32)
+
+
+def dev(x):
+    return torch.from_numpy(x.view(np.int16) if x.dtype == np.uint16 else x).cuda().view(
+        torch.uint16 if x.dtype == np.uint16 else torch.uint8)
+
+
+def data(n, nchans, nbits, full=False):
+    rng = np.random.default_rng(n * 31 + nchans)
+    dt = np.uint8 if nbits == 8 else np.uint16
+    top = 2 ** nbits - 1
+    x = rng.integers(0, top + 1, size=(n, nchans)).astype(dt)
+    if full:
+        x[rng.random((n, nchans)) < 0.97] = top
+    return x
+
+
+def subband(n, nchans, nbits, hi, step, ds, width, band, zdm, iqrm, tsamp=64e-6, full=False):
+    x = data(n, nchans, nbits, full)
+    foff = float(F32(300.0 / nchans))
+    hdr = dict(tsamp=float(F32(tsamp)), fch1=1150.0, foff=foff, nbits=nbits, nchans=nchans, ndata=n)
+    freq = O.freq_table_header(hdr["fch1"], hdr["foff"], nchans)
+    f0, f1 = freq[0] + band * (freq[-1] - freq[0]), freq[-1]
+    fs, fe = float(F32(f0)), float(F32(f1))
+    iq = IqrmParams(mode=1, radius_frac=0.1, nsigma=3.0, win_sec=n * tsamp * 0.4, hop_sec=n * tsamp * 0.2)
+    plan = Plan(hdr, 0.0, hi, fs, fe, step, ds, algorithm="subband", subband_width=width,
+                zero_dm_mode="range" if zdm else "callsite",
+                rfi=RfiParams(use_zero_dm=zdm, use_iqrm=iqrm, iqrm=iq, use_mask=True), bad_channels=[1, nchans // 2])
+    ref = x.copy()
+    if ds > 1:
+        ref = O.time_binning(ref, nchans, ds)
+    cs, ce = plan.info["chan_start"], plan.info["chan_end"]
+    if iqrm:
+        t0, t1, masks = O.iqrm_masks(ref, nchans, cs, ce, float(F32(F32(tsamp) * F32(ds))), iq)
+        O.apply_window_masks(ref, nchans, t0, t1, masks)
+    if zdm:
+        O.zero_dm_range_exact(ref, nchans, cs, ce)
+    O.mark_channels(ref, nchans, [1, nchans // 2])
+    op = O.subband_plan(freq, n, 0.0, hi, fs, fe, step, ds, sb_width=width)
+    d1, r2 = plan.tables()
+    return plan, x, O.subband_sums(ref, nchans, op, d1, r2)
+
+
+@pytest.mark.parametrize("n,nchans,nbits,hi,step,ds,width,band,zdm,iqrm", [
+    (2560, 64, 8, 100.0, 0.5, 1, 32, 0.0, False, False),     # one tile of every segment
+    (2561, 64, 8, 100.0, 0.5, 1, 32, 0.0, False, False),
+    (2527, 64, 8, 500.0, 0.5, 1, 16, 0.0, True, True),
+    (5, 64, 8, 20.0, 0.5, 1, 32, 0.0, False, False),         # fewer columns than segments
+    (37, 64, 16, 20.0, 0.5, 1, 32, 0.0, False, False),
+    (10243, 97, 8, 260.0, 0.5, 1, 33, 0.1, True, True),      # channels off the load words
+    (4099, 130, 16, 260.0, 0.5, 1, 64, 0.1, True, True),
+    (4096, 256, 8, 100.0, 0.3, 1, 64, 0.0, False, True),
+    (3001, 260, 8, 100.0, 0.3, 1, 65, 0.0, False, False),    # 32-bit subband sums
+    (3000, 384, 8, 60.0, 0.3, 1, 128, 0.0, True, False),
+    (3000, 400, 8, 60.0, 0.3, 1, 129, 0.0, False, False),    # fields moved out inside a subband
+    (2900, 600, 8, 60.0, 0.3, 1, 300, 0.0, False, False),
+    (2900, 320, 16, 60.0, 0.3, 1, 160, 0.0, False, False),
+    (9001, 128, 8, 300.0, 0.5, 2, 32, 0.2, True, True),      # binned
+    (8003, 128, 16, 300.0, 0.5, 4, 32, 0.0, False, True),
+    (3000, 64, 8, 3000.0, 200.0, 1, 32, 0.0, True, True),    # delays beyond the chunk, few rows
+    (3000, 64, 16, 3000.0, 100.0, 1, 32, 0.0, False, False),
+    (70000, 64, 8, 400.0, 2.0, 1, 16, 0.0, False, False),    # several tiles
+])
+@pytest.mark.parametrize("full", [False, True])
+def test_subband_equals_oracle(n, nchans, nbits, hi, step, ds, width, band, zdm, iqrm, full):
+    plan, x, want = subband(n, nchans, nbits, hi, step, ds, width, band, zdm, iqrm, full=full)
+    out = to_np(plan.run(dev(x)))
+    assert out.shape == want.shape and np.array_equal(out, want)
+    host = plan.run_host(x)
+    assert np.array_equal(host, want)
+
+
+@pytest.mark.parametrize("n,nc,nbits,hi,step", [
+    (2560, 65, 8, 100.0, 0.5), (2561, 129, 8, 300.0, 1.0), (2559, 258, 8, 64.0, 4.0),
+    (1000, 300, 16, 100.0, 0.5), (1283, 33, 16, 15.0, 1.0), (9, 130, 8, 20.0, 1.0),
+    (700, 64, 8, 3000.0, 300.0),
+])
+def test_brute_force_equals_oracle(n, nc, nbits, hi, step):
+    x = data(n, nc, nbits, full=True)
+    tsamp, foff = 1e-4, 300.0 / nc
+    freq = O.freq_table_fil(1150.0, foff, nc)
+    fs, fe = float(F32(freq[0])), float(F32(freq[-1]))
+    hdr = dict(tsamp=tsamp, fch1=1150.0, foff=foff, nbits=nbits, nchans=nc, ndata=n)
+    ts = n * tsamp * 0.49
+    plan = Plan(hdr, 0.0, hi, fs, fe, step, 1, ts, algorithm="brute", freq_mode="fil")
+    want = np.concatenate(O.bruteforce_cpu(x, nc, freq, tsamp, 0.0, hi, fs, fe, step, 1, ts,
+                                           delay=plan.tables()[0]), axis=1)
+    assert np.array_equal(to_np(plan.run(dev(x))), want)
+
+
+@pytest.mark.parametrize("persistent", [False, True])
+def test_batch_of_all_layouts_equals_oracle(persistent):
+    specs = [(3001, 260, 8, 100.0, 0.3, 1, 65, 0.0, False, False),
+             (2561, 64, 8, 100.0, 0.5, 1, 32, 0.0, True, True),
+             (3000, 64, 8, 3000.0, 200.0, 1, 32, 0.0, False, False),
+             (4099, 130, 16, 260.0, 0.5, 1, 64, 0.1, False, False)]
+    got = [subband(*s) for s in specs]
+    batch = Batch([g[0] for g in got], persistent=persistent)
+    outs = batch.run([dev(g[1]) for g in got])
+    batch.status()
+    for o, (_, _, want) in zip(outs, got):
+        assert np.array_equal(to_np(o), want)
