@@ -65,6 +65,7 @@ int stage2_kind(const dd_plan& P) {
   return !P.inter16 ? kSumKindPlane32 : P.fold > 1 ? kSumKindPlane16 : kSumKindU16Twin;
 }
 int brute_kind(const dd_plan& P) {
+  if (P.p.time_downsample > 1) return P.nbits == 16 ? kSumKindU16Phase : kSumKindU8Phase;
   if (P.fold > 1) return P.nbits == 16 ? kSumKindFold16 : kSumKindFold8W;
   return P.nbits == 16 ? kSumKindU16Wide : kSumKindU8Flush;
 }
@@ -495,10 +496,42 @@ void create_subband(dd_plan& P) {
   }
 }
 
+// Staging of downsampled brute-force sums (8- and 16-bit samples, up to 16 phases).
+// Column t of the slice that starts at sample S reads sample S + t * ds + delay: phase
+// (p + delay) % ds, element S / ds + (p + delay) / ds + t of that phase row, p = S % ds.
+// One descriptor table per pattern p the slices have.  All slices run in one launch; the
+// direct kernel, launch by slice, took 16.6 ms for 1000 channels, 61441 samples, 501
+// trials.
+void set_phase_window(dd_plan& P) {
+  const int ds = P.p.time_downsample;
+  if (ds > 16 || P.nbits > 16 || P.nslices > 65535) return;
+  const int k = brute_kind(P), patterns = P.phases_merge ? 1 : ds;
+  const int64_t n = P.dm_steps * P.nc;
+  std::vector<SumDesc> all;
+  std::vector<int32_t> off(static_cast<size_t>(n));
+  int spread = 0;
+  for (int p = 0; p < patterns; ++p) {
+    for (int64_t i = 0; i < n; ++i) off[i] = (p + P.h_delay[i]) / ds;
+    spread = std::max(spread, table_spread(off, P.dm_steps, P.nc, kSumRows, 0));
+    std::vector<SumDesc> d = build_sum_desc(off, P.dm_steps, P.nc, 0);
+    for (int64_t m = 0; m < P.dm_steps; ++m)
+      for (int64_t c = 0; c < P.nc; ++c)
+        d[(m / kSumRows) * P.nc + c].phase[(m % kSumRows) >> 3] |=
+            static_cast<uint32_t>((p + P.h_delay[m * P.nc + c]) % ds) << (4 * (m & 7));
+    P.pattern_descs = static_cast<int64_t>(d.size());
+    all.insert(all.end(), d.begin(), d.end());
+  }
+  const int64_t sub = round_up(static_cast<int64_t>(spread + sum_kind_tile(k)) * P.elem + 40, 16);
+  if (sum_smem_bytes(static_cast<int>(std::min<int64_t>(sub * ds, 1 << 24)), 2) + sum_kind_extra_smem(k) > 200 * 1024) return;
+  P.subb = static_cast<int>(sub);
+  P.winb = P.subb * ds;
+  upload_desc(P.d_descb, all);
+}
+
 // Layout and staging of the brute-force sums.  The staged-window sums serve 8- and
-// 16-bit samples without downsampling (one source row per channel); other cases use the
-// direct kernels on the phase rows.  Allocates the prepared input when its layout
-// changes.
+// 16-bit samples (without downsampling one source row per channel, else its phase
+// rows); other cases use the direct kernels on the phase rows.  Allocates the prepared
+// input when its layout changes.
 void set_brute_window(dd_plan& P) {
   const bool had = P.d_x.bytes != 0;
   const int fold0 = P.fold;
@@ -514,13 +547,15 @@ void set_brute_window(dd_plan& P) {
     set_window(choose_fold(P, P.out_cols, P.nc, P.max_delay, P.adds));
     if (P.fold > 1 && !P.winb) set_window(1);
   }
-  if (P.winb) upload_desc(P.d_descb, build_sum_desc(P.h_delay, P.dm_steps, P.nc, 0));
+  if (P.p.time_downsample > 1) set_phase_window(P);
+  else if (P.winb) upload_desc(P.d_descb, build_sum_desc(P.h_delay, P.dm_steps, P.nc, 0));
   if (had && P.fold == fold0) return;
   P.seg = P.fold > 1 ? round_up((P.out_cols + P.fold - 1) / P.fold, 8) : P.out_cols;
   // (a folded row holds a segment, the padding of phase_len past the chunk and a tile)
   P.xpitch = P.fold > 1 ? round_up(P.seg + P.phase_len - P.nin + 2048 + 64, 64) : P.phase_len;
   const int64_t rows = P.nc * P.p.time_downsample;
-  P.d_x.alloc(static_cast<size_t>(rows * P.xpitch) * x_elem(P));
+  // (+8192 elements: staged windows may end a block tile past the last row)
+  P.d_x.alloc(static_cast<size_t>(rows * P.xpitch + 8192) * x_elem(P));
   DD_CUDA_TRY(cudaMemset(P.d_x.p, 0, P.d_x.bytes));
 }
 
@@ -832,8 +867,18 @@ SumLaunch brute_launch(const dd_plan& P, void* output) {
   L.seg_stride = P.seg * 4;
   L.nout = P.out_cols;
   L.win_bytes = P.winb;
+  if (P.p.time_downsample > 1) {
+    L.ds = P.p.time_downsample;
+    L.sub_bytes = P.subb;
+    L.phase_pitch = P.phase_len * P.elem;
+    L.src_pitch = L.ds * L.phase_pitch;
+    L.sps = P.sps;
+    L.nin = P.nin;
+    L.desc_pattern = P.pattern_descs;
+    if (!P.phases_merge) L.ncols = P.cols0;  // per slice; merged, the chunk is one slice
+  }
   L.grid_y = static_cast<unsigned>((P.dm_steps + kSumRows - 1) / kSumRows);
-  L.grid_z = 1;
+  L.grid_z = L.ds > 1 && !P.phases_merge ? static_cast<unsigned>(P.nslices) : 1;
   L.desc = P.d_descb.as<SumDesc>();
   L.desc_pitch = P.nc;
   L.stages = sum_kind_stages(sum_kind(L), P.winb);
@@ -1502,6 +1547,7 @@ bool batched_plan(const dd_plan& P, bool persistent) {
   const bool brute = P.p.algorithm == DD_ALGO_BRUTE;
   if (brute ? !P.winb : (!P.win1 || !P.win2)) return false;
   if (!persistent) return true;
+  if (brute && P.p.time_downsample > 1) return false;  // no phase-row kernel in k_sum_batch
   return brute ? sum_launch_smem(brute_launch(P, nullptr)) <= kBatchSmemCap
                : sum_launch_smem(stage1_launch(P, 0)) <= kBatchSmemCap &&
                      sum_launch_smem(stage2_launch(P, 0, nullptr)) <= kBatchSmemCap;

@@ -101,6 +101,8 @@ struct dd_plan {
   int64_t phase_len = 0;     // padded length of one phase row of the brute-force layout
   bool phases_merge = true;  // slices share one phase pattern (sps % ds == 0)
   int winb = 0;              // staged window bytes of the brute-force sums (0: not used)
+  int subb = 0;              // ... of one phase row of a window (downsampled)
+  int64_t pattern_descs = 0; // descriptors per slice pattern (downsampled)
 
   // tables (host copies)
   std::vector<int32_t> h_delay;  // [ndm_nom][dch] (subband) or [dm_steps][nc] (brute)
@@ -294,7 +296,7 @@ struct SumDesc {
   int32_t lo;
   int32_t span;
   uint16_t rel[kSumRows];
-  int32_t pad[2];
+  uint32_t phase[2];  // downsampled brute force: four bits per row, its delay's phase
 };
 static_assert(sizeof(SumDesc) == 48, "bulk copies move whole 16-byte units");
 struct SumLaunch {
@@ -328,6 +330,12 @@ struct SumLaunch {
   // skew_stage1); the launch spans ncols + max_skew positions.
   const int32_t* skew;
   int64_t max_skew;
+  // Downsampled brute force (ds > 1): grid z = slice of sps samples of the chunk's nin;
+  // a source is ds phase rows (samples ph, ph + ds, ... of the channel) phase_pitch bytes
+  // apart, staged in parts of sub_bytes; desc has a table of desc_pattern descriptors for
+  // every first sample of a slice modulo ds.
+  int ds, sub_bytes;
+  int64_t sps, nin, phase_pitch, desc_pattern;
   int stages;              // staged source pairs in flight (2..4)
   int* err;                // device error word: set when a bounded wait gives up
   // 16-bit subband sums with a one-sample-shifted twin (0: none): the twin of the
@@ -439,20 +447,22 @@ constexpr int kPlane16RB = DD_PLANE16_RB, kPlane16NW = DD_PLANE16_NW;
 constexpr int kPlane32RB = DD_PLANE32_RB, kPlane32NW = DD_PLANE32_NW;
 // Kernel variants of the staged sums.  Samples in time order: 8-bit into 16-bit sums
 // (U8Out16) or 32-bit sums (U8Flush), 16-bit into 32-bit sums (U16Wide), 16-bit subband
-// sums with their one-sample-shifted twin (U16Twin).  Folded samples: 8-bit into
+// sums with their one-sample-shifted twin (U16Twin), and the phase rows of downsampled
+// brute force (U8Phase, U16Phase).  Folded samples: 8-bit into
 // packed 16-bit planes (Fold8) or 32-bit sums (Fold8W), 16-bit into 32-bit sums
 // (Fold16), and stage 2 of packed planes (Plane16).  Stage 2 of 32-bit sums, folded or
 // not (Plane32).
-enum SumKind { kSumKindU8Out16, kSumKindU8Flush, kSumKindU16Wide, kSumKindU16Twin, kSumKindFold8,
+enum SumKind { kSumKindU8Out16, kSumKindU8Flush, kSumKindU16Wide, kSumKindU16Twin,
+               kSumKindU8Phase, kSumKindU16Phase, kSumKindFold8,
                kSumKindFold8W, kSumKindFold16, kSumKindPlane16, kSumKindPlane32, kSumKinds };
 int sum_kind(const SumLaunch& L);
 // Tile of a kernel variant: samples per block, or words for the folded sums and Plane32.
 inline int sum_kind_tile(int kind) {
   const auto words = [](int rb, int nw) { return sum_tile_samples(4, nw) * rb / kSumRows; };
   switch (kind) {
-    case kSumKindU8Out16: case kSumKindU8Flush:
+    case kSumKindU8Out16: case kSumKindU8Flush: case kSumKindU8Phase:
       return sum_tile_samples(1, DD_SUM8_NW) * kSumRowsPT8 / kSumRows;
-    case kSumKindU16Wide: return sum_tile_samples(2, DD_SUM16W_NW) * kSumRowsPTW / kSumRows;
+    case kSumKindU16Wide: case kSumKindU16Phase: return sum_tile_samples(2, DD_SUM16W_NW) * kSumRowsPTW / kSumRows;
     case kSumKindU16Twin: return sum_tile_samples(2, kSum16TNW) * kSumRowsPTT / kSumRows;
     case kSumKindFold8: return words(kFold8RB, kFold8NW);
     case kSumKindFold8W: return words(kFold8WRB, kFold8WNW);
@@ -467,7 +477,8 @@ inline int sum_kind_qs(int kind) {
 }
 // Bytes of a source element: samples, 16-bit sums or words.
 inline int sum_kind_elem(int kind) {
-  return kind == kSumKindU8Out16 || kind == kSumKindU8Flush ? 1 : kind >= kSumKindFold8 ? 4 : 2;
+  return kind == kSumKindU8Out16 || kind == kSumKindU8Flush || kind == kSumKindU8Phase ? 1
+         : kind >= kSumKindFold8                                                         ? 4 : 2;
 }
 // Shared memory of a launch (its variant's windows per stage, plus the variant's
 // staging past the ring, sum_kind_extra_smem).

@@ -145,6 +145,7 @@ __device__ __forceinline__ int64_t row_col(const Geo& g, int r) {
   return g.col - (g.skew ? __ldg(g.skew + r) : 0);
 }
 
+template <bool PHASES = false>
 __device__ __forceinline__ Geo make_geo(const SumLaunch& L, int T, uint3 blk) {
   Geo g;
   const int64_t tile = blk.x;
@@ -189,6 +190,16 @@ __device__ __forceinline__ Geo make_geo(const SumLaunch& L, int T, uint3 blk) {
       g.nrows = static_cast<int>(min(static_cast<int64_t>(kSumRows), L.nrows_total - m0));
       g.out = L.out + m0 * L.out_pitch + L.out_col0 * L.out_elem;
       g.out_pitch = L.out_pitch;
+      if constexpr (PHASES) {
+        // slice blk.z: column t is sample start + t * ds of every channel's delayed row
+        const int64_t start = static_cast<int64_t>(blk.z) * L.sps;
+        g.desc += (start % L.ds) * L.desc_pattern;
+        g.base = start / L.ds + g.col;
+        g.src_pitch = L.src_pitch;
+        g.ncols = min(L.ncols, (L.nin - start + L.ds - 1) / L.ds);
+        g.out += static_cast<int64_t>(blk.z) * L.ncols * L.out_elem;
+        return g;
+      }
       break;
     }
   }
@@ -232,6 +243,12 @@ struct GroupDesc {
       }
     }
   }
+  // the phase rows (downsampled brute force) of the lane's sources
+  __device__ __forceinline__ int phase(const Geo& g, int q, int lane) const {
+    const int src = QS * q + (lane >> 4);
+    if (src >= g.nsrc) return 0;
+    return (__ldg(&g.desc[src].phase[(lane >> 3) & 1]) >> (4 * (lane & 7))) & 15;
+  }
 };
 
 // Stages source pair q in stage s, by all lanes of one warp: lane 16i + r writes row
@@ -262,6 +279,39 @@ __device__ __forceinline__ void produce(const Geo& g, Pipe& P, uint32_t* sw, int
   if (lane == 0) mbar_arrive_expect_tx(&P.full[s], total);
   __syncwarp();
   if (nbytes) bulk_copy(sw + (2 * s + i) * ww, gsrc, nbytes, &P.full[s]);
+}
+
+// The same for downsampled brute force: a source is its channel's ds phase rows (L.ds),
+// each staged from the same element on into its own part of the window, and row r reads
+// the phase that its delay falls on.
+template <int SB>
+__device__ __forceinline__ void produce_phases(const SumLaunch& L, const Geo& g, Pipe& P, uint32_t* sw,
+                                               int ww, int zero_q, int tile_bytes, const GroupDesc<2>& d,
+                                               int phase, int q, int s, int lane) {
+  const int i = lane >> 4, r = lane & 15;
+  const int src = 2 * q + i;
+  uint32_t nbytes = 0;
+  const char* gsrc = nullptr;
+  int2 rw = make_int2(zero_q, 0);
+  if (src < g.nsrc) {
+    const int64_t firstb = (g.base + d.lo[0]) * SB;
+    const int64_t a0 = firstb & ~int64_t(15);
+    const int ob = static_cast<int>(firstb - a0) + d.rel[0] * SB;
+    rw = make_int2((2 * s + i) * ww + phase * (L.sub_bytes >> 2) + (ob >> 2), (ob & 3) * 8);
+    if (r == 0) {
+      const int64_t last = firstb + static_cast<int64_t>(d.span[0]) * SB + tile_bytes + 8;
+      nbytes = static_cast<uint32_t>((last - a0 + 15) & ~int64_t(15));
+      gsrc = g.src + static_cast<int64_t>(src) * g.src_pitch + a0;
+    }
+  }
+  *reinterpret_cast<int2*>(&P.row[s][r][2 * i]) = rw;
+  const uint32_t total = (nbytes + __shfl_xor_sync(0xffffffffu, nbytes, 16)) * static_cast<uint32_t>(L.ds);
+  __syncwarp();
+  if (lane == 0) mbar_arrive_expect_tx(&P.full[s], total);
+  __syncwarp();
+  if (nbytes)
+    for (int ph = 0; ph < L.ds; ++ph)
+      bulk_copy(sw + (2 * s + i) * ww + ph * (L.sub_bytes >> 2), gsrc + ph * L.phase_pitch, nbytes, &P.full[s]);
 }
 
 // The same for the twin-window sums (16-bit sources with a one-sample-shifted twin,
@@ -361,11 +411,11 @@ __device__ __forceinline__ void produce_words(const Geo& g, Pipe& P, uint32_t* s
 // 1, 3.8 in stage 2): 4096 channels of 8 bits, 2^20 samples, 6001 trials took 66.2 +
 // 40.1 ms (stages 1 and 2) that way and 56.6 + 32.8 ms with turns; brute force over
 // 1024 channels, 2^17 samples, 1001 trials 10.8 and 8.5 ms.
-constexpr int kModePlain = 0, kModeTwin = 1, kModeWords = 2;
+constexpr int kModePlain = 0, kModeTwin = 1, kModeWords = 2, kModePhase = 3;
 template <int SB, int QS = 2, int MODE = kModePlain, typename Setup, typename Body>
 __device__ __forceinline__ bool run_pipeline(const SumLaunch& L, const Geo& g, Pipe& P,
                                              uint32_t* sw, int tile, Setup&& setup, Body&& body) {
-  static_assert(QS == (MODE == kModePlain ? 2 : 4), "sources per stage");
+  static_assert(QS == (MODE == kModePlain || MODE == kModePhase ? 2 : 4), "sources per stage");
   static_assert(kMaxStages <= kWarps, "each warp stages at most one group before the loop");
   constexpr int kWinPerSrc = MODE == kModeTwin ? 2 : 1;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -394,15 +444,20 @@ __device__ __forceinline__ bool run_pipeline(const SumLaunch& L, const Geo& g, P
   __syncthreads();
   volatile int* failed = &P.failed;
   int next = warp;  // the next group this warp stages
+  int phase = 0;
+  if constexpr (MODE == kModePhase) phase = desc.phase(g, next, lane);
   auto stage_next = [&](int s) {
     if constexpr (MODE == kModeTwin)
       produce_twin(g, P, sw, ww, zero_q, tile, L.twin_off, desc, next, s, lane);
     else if constexpr (MODE == kModeWords)
       produce_words(g, P, sw, ww, zero_q, tile, desc, next, s, lane);
+    else if constexpr (MODE == kModePhase)
+      produce_phases<SB>(L, g, P, sw, ww, zero_q, tile, desc, phase, next, s, lane);
     else
       produce<SB>(g, P, sw, ww, zero_q, tile, desc, next, s, lane);
     next += kWarps;
     desc.load(g, next, lane);
+    if constexpr (MODE == kModePhase) phase = desc.phase(g, next, lane);
   };
   if (next < min(D, ngroups)) stage_next(next);
   setup();
@@ -485,7 +540,7 @@ __device__ __forceinline__ void for_rows(uint32_t act, F&& f) {
 }
 
 // ------------------------------------------------------------------ 8-bit samples
-template <int RB, int NW, bool OUT16>
+template <int RB, int NW, bool OUT16, int MODE = kModePlain>
 __device__ __forceinline__ void sum_u8(const SumLaunch& L, uint3 blk, uint32_t* sw, Pipe& P) {
   static_assert(NW & 1, "an odd number of consecutive words per lane: conflict-free loads");
   // RB rows per thread: the block's kSumRows rows are split over kSumRows/RB
@@ -493,7 +548,7 @@ __device__ __forceinline__ void sum_u8(const SumLaunch& L, uint3 blk, uint32_t* 
   constexpr int kGroups = kSumRows / RB;
   constexpr int kWarpsPerTile = kWarps / kGroups;
   constexpr int T = kWarpsPerTile * 32 * NW * 4;
-  const Geo g = make_geo(L, T, blk);
+  const Geo g = make_geo<MODE == kModePhase>(L, T, blk);
   if (g.nrows <= 0) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rbase = warp / kWarpsPerTile, wt = warp % kWarpsPerTile;
@@ -543,7 +598,7 @@ __device__ __forceinline__ void sum_u8(const SumLaunch& L, uint3 blk, uint32_t* 
   };
   int since = 0;       // sources summed in the fields since the last flush
   bool stored = false; // the output holds partial sums of an earlier flush
-  const bool ok = run_pipeline<1>(L, g, P, sw, T, [&] { act = active_rows<RB, T>(g, rbase); }, [&](int s, const uint32_t* win) {
+  const bool ok = run_pipeline<1, 2, MODE>(L, g, P, sw, T, [&] { act = active_rows<RB, T>(g, rbase); }, [&](int s, const uint32_t* win) {
     for_rows<RB>(act, [&](int r) {
       const int4 rw = row_info(P, s, rbase + kGroups * r);
       const uint32_t* w0 = win + rw.x + wbase;
@@ -630,14 +685,14 @@ __device__ __forceinline__ void sum_u8(const SumLaunch& L, uint3 blk, uint32_t* 
 // (two sources per three-input add); the low samples' sums come out at the end
 // as whole - (high << 16).  Three integer-pipe operations per word and source,
 // where taking the halves apart by masks and offset-dependent selects took five.
-template <int RB, int NW>
+template <int RB, int NW, int MODE = kModePlain>
 __device__ __forceinline__ void sum_u16_wide(const SumLaunch& L, uint3 blk, uint32_t* sw, Pipe& P) {
   // RB rows per thread: the block's rows are split over kSumRows/RB warp groups,
   // each covering the whole tile for its RB rows (as in sum_u8)
   constexpr int kGroups = kSumRows / RB;
   constexpr int kWarpsPerTile = kWarps / kGroups;
   constexpr int T = kWarpsPerTile * 32 * NW * 2;
-  const Geo g = make_geo(L, T, blk);
+  const Geo g = make_geo<MODE == kModePhase>(L, T, blk);
   if (g.nrows <= 0) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rbase = warp / kWarpsPerTile, wt = warp % kWarpsPerTile;
@@ -648,7 +703,7 @@ __device__ __forceinline__ void sum_u16_wide(const SumLaunch& L, uint3 blk, uint
   for (int r = 0; r < RB; ++r)
 #pragma unroll
     for (int k = 0; k < NW; ++k) lo32[r][k] = hi32[r][k] = 0;
-  const bool ok = run_pipeline<2>(L, g, P, sw, 2 * T, [&] { act = active_rows<RB, T>(g, rbase); }, [&](int s, const uint32_t* win) {
+  const bool ok = run_pipeline<2, 2, MODE>(L, g, P, sw, 2 * T, [&] { act = active_rows<RB, T>(g, rbase); }, [&](int s, const uint32_t* win) {
     for_rows<RB>(act, [&](int r) {
       const int4 rw = row_info(P, s, rbase + kGroups * r);
       const uint32_t* w0 = win + rw.x + wbase;
@@ -1022,17 +1077,17 @@ __device__ __forceinline__ void sum_u16_twin(const SumLaunch& L, uint3 blk, uint
   }
 }
 
-template <int RB, int NW, bool OUT16>
+template <int RB, int NW, bool OUT16, int MODE = kModePlain>
 __global__ void __launch_bounds__(kThreads, DD_SUM8_MINB) k_sum_u8(SumLaunch L) {
   extern __shared__ __align__(128) uint32_t sw[];
   __shared__ Pipe P;
-  sum_u8<RB, NW, OUT16>(L, blockIdx, sw, P);
+  sum_u8<RB, NW, OUT16, MODE>(L, blockIdx, sw, P);
 }
-template <int RB, int NW>
+template <int RB, int NW, int MODE = kModePlain>
 __global__ void __launch_bounds__(kThreads, DD_SUM16W_MINB) k_sum_u16w(SumLaunch L) {
   extern __shared__ __align__(128) uint32_t sw[];
   __shared__ Pipe P;
-  sum_u16_wide<RB, NW>(L, blockIdx, sw, P);
+  sum_u16_wide<RB, NW, MODE>(L, blockIdx, sw, P);
 }
 template <int RB, int NW>
 __global__ void __launch_bounds__(kThreads, DD_SUM16T_MINB) k_sum_u16t(SumLaunch L) {
@@ -1099,6 +1154,8 @@ __device__ __forceinline__ void run_one(const SumLaunch& L, uint3 blk, uint32_t*
   else if constexpr (KIND == kSumKindU8Flush) sum_u8<kSumRowsPT8, DD_SUM8_NW, false>(L, blk, sw, P);
   else if constexpr (KIND == kSumKindU16Wide) sum_u16_wide<kSumRowsPTW, DD_SUM16W_NW>(L, blk, sw, P);
   else if constexpr (KIND == kSumKindU16Twin) sum_u16_twin<kSumRowsPTT, kSum16TNW>(L, blk, sw, P);
+  else if constexpr (KIND == kSumKindU8Phase) sum_u8<kSumRowsPT8, DD_SUM8_NW, false, kModePhase>(L, blk, sw, P);
+  else if constexpr (KIND == kSumKindU16Phase) sum_u16_wide<kSumRowsPTW, DD_SUM16W_NW, kModePhase>(L, blk, sw, P);
   else if constexpr (KIND == kSumKindFold8) sum_fold8<kFold8RB, kFold8NW, true>(L, blk, sw, P);
   else if constexpr (KIND == kSumKindFold8W) sum_fold8<kFold8WRB, kFold8WNW, false>(L, blk, sw, P);
   else if constexpr (KIND == kSumKindFold16) sum_fold16<kFold16RB, kFold16NW>(L, blk, sw, P);
@@ -1218,7 +1275,7 @@ size_t sum_smem_bytes(int win_bytes, int stages, int qs) {
 size_t sum_kind_extra_smem(int kind) {
   // the flush staging of the 8-bit kernel with 32-bit outputs: one segment of
   // 32-bit sums per warp
-  return kind == kSumKindU8Flush ? static_cast<size_t>(kWarps) * 32 * DD_SUM8_NW * 4 * sizeof(uint32_t) : 0;
+  return kind == kSumKindU8Flush || kind == kSumKindU8Phase ? static_cast<size_t>(kWarps) * 32 * DD_SUM8_NW * 4 * sizeof(uint32_t) : 0;
 }
 
 size_t sum_launch_smem(const SumLaunch& L) {
@@ -1287,6 +1344,8 @@ void launch_sum(const SumLaunch& L, cudaStream_t st) {
     case kSumKindU8Flush: launch_k(k_sum_u8<kSumRowsPT8, DD_SUM8_NW, false>, grid, smem, L, st); break;
     case kSumKindU16Wide: launch_k(k_sum_u16w<kSumRowsPTW, DD_SUM16W_NW>, grid, smem, L, st); break;
     case kSumKindU16Twin: launch_k(k_sum_u16t<kSumRowsPTT, kSum16TNW>, grid, smem, L, st); break;
+    case kSumKindU8Phase: launch_k(k_sum_u8<kSumRowsPT8, DD_SUM8_NW, false, kModePhase>, grid, smem, L, st); break;
+    case kSumKindU16Phase: launch_k(k_sum_u16w<kSumRowsPTW, DD_SUM16W_NW, kModePhase>, grid, smem, L, st); break;
     case kSumKindFold8: launch_k(k_sum_fold8<kFold8RB, kFold8NW, true>, grid, smem, L, st); break;
     case kSumKindFold8W: launch_k(k_sum_fold8<kFold8WRB, kFold8WNW, false>, grid, smem, L, st); break;
     case kSumKindFold16: launch_k(k_sum_fold16<kFold16RB, kFold16NW>, grid, smem, L, st); break;
@@ -1332,6 +1391,8 @@ void launch_sum_grouped(const SumBatchGroup* d_groups, int ngroups, long long to
     case kSumKindU8Flush: launch_grouped_k<kSumKindU8Flush>(d_groups, ngroups, total, smem, st); break;
     case kSumKindU16Wide: launch_grouped_k<kSumKindU16Wide>(d_groups, ngroups, total, smem, st); break;
     case kSumKindU16Twin: launch_grouped_k<kSumKindU16Twin>(d_groups, ngroups, total, smem, st); break;
+    case kSumKindU8Phase: launch_grouped_k<kSumKindU8Phase>(d_groups, ngroups, total, smem, st); break;
+    case kSumKindU16Phase: launch_grouped_k<kSumKindU16Phase>(d_groups, ngroups, total, smem, st); break;
     case kSumKindFold8: launch_grouped_k<kSumKindFold8>(d_groups, ngroups, total, smem, st); break;
     case kSumKindFold8W: launch_grouped_k<kSumKindFold8W>(d_groups, ngroups, total, smem, st); break;
     case kSumKindFold16: launch_grouped_k<kSumKindFold16>(d_groups, ngroups, total, smem, st); break;

@@ -107,6 +107,25 @@ def test_brute_force_equals_oracle(n, nc, nbits, hi, step):
     assert np.array_equal(to_np(plan.run(dev(x))), want)
 
 
+@pytest.mark.parametrize("n,nc,nbits,hi,step,ds,frac", [
+    (6001, 65, 8, 100.0, 1.0, 2, 0.1667), (5121, 130, 8, 300.0, 2.0, 3, 0.21),
+    (5120, 64, 8, 300.0, 1.0, 2, 0.25), (4000, 33, 16, 200.0, 1.0, 4, 0.3),
+    (4001, 130, 16, 200.0, 5.0, 2, 0.49), (9001, 40, 8, 100.0, 3.0, 8, 0.5),
+    (6000, 40, 8, 100.0, 3.0, 16, 0.4), (6000, 40, 8, 100.0, 3.0, 17, 0.4),
+])
+def test_downsampled_brute_force_equals_oracle(n, nc, nbits, hi, step, ds, frac):
+    x = data(n, nc, nbits, full=True)
+    tsamp, foff = 1e-4, 300.0 / nc
+    freq = O.freq_table_fil(1150.0, foff, nc)
+    fs, fe = float(F32(freq[0])), float(F32(freq[-1]))
+    hdr = dict(tsamp=tsamp, fch1=1150.0, foff=foff, nbits=nbits, nchans=nc, ndata=n)
+    ts = n * tsamp * frac
+    plan = Plan(hdr, 0.0, hi, fs, fe, step, ds, ts, algorithm="brute", freq_mode="fil")
+    want = np.concatenate(O.bruteforce_cpu(x, nc, freq, tsamp, 0.0, hi, fs, fe, step, ds, ts,
+                                           delay=plan.tables()[0]), axis=1)
+    assert np.array_equal(to_np(plan.run(dev(x))), want)
+
+
 @pytest.mark.parametrize("persistent", [False, True])
 def test_batch_of_all_layouts_equals_oracle(persistent):
     specs = [(3001, 260, 8, 100.0, 0.3, 1, 65, 0.0, False, False),
