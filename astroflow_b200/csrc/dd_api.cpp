@@ -156,14 +156,18 @@ int64_t brute_table(const double* freq, int64_t cs, int64_t ce, int64_t ref_ch, 
   volatile float ref2 = ref * ref;
   const float inv_ref2 = 1.0f / ref2;
   int64_t mism = 0;
+  std::vector<double> disp(static_cast<size_t>(nc));
+  for (int64_t c = 0; c < nc; ++c) {
+    const double f = freq[cs + c], r = freq[ref_ch];
+    disp[c] = 1.0 / (f * f) - 1.0 / (r * r);
+  }
   for (int64_t s = 0; s < dm_steps; ++s) {
     volatile float idx = static_cast<float>(static_cast<size_t>(s));
     volatile float prod = idx * dm_step;
     volatile float dm = dm_low + prod;
     for (int64_t c = 0; c < nc; ++c) {
       const double dm64 = static_cast<double>(dm_low) + static_cast<double>(s) * dm_step;
-      const double f = freq[cs + c], r = freq[ref_ch];
-      const double e = 4148.808 * dm64 * (1.0 / (f * f) - 1.0 / (r * r)) / tsamp;
+      const double e = 4148.808 * dm64 * disp[c] / tsamp;
       const int v64 = static_cast<int>(std::floor(e + 0.5));
       int32_t& out = table[s * nc + c];
       if (mode == DD_TABLE_IEEE) {
@@ -284,29 +288,6 @@ struct Prof {
   }
 };
 
-// Largest spread (max - min) of a table's offsets over groups of `rows` consecutive
-// rows, per column; rows are grouped within blocks of `group` rows (0: no blocks).
-int table_spread(const std::vector<int32_t>& tab, int64_t nrows, int64_t ncols, int rows,
-                 int64_t group) {
-  int spread = 0;
-  const int64_t blk = group > 0 ? group : nrows;
-  for (int64_t b0 = 0; b0 < nrows; b0 += blk) {
-    const int64_t b1 = std::min(nrows, b0 + blk);
-    for (int64_t r0 = b0; r0 < b1; r0 += rows) {
-      const int64_t r1 = std::min(b1, r0 + rows);
-      for (int64_t c = 0; c < ncols; ++c) {
-        int lo = tab[r0 * ncols + c], hi = lo;
-        for (int64_t r = r0 + 1; r < r1; ++r) {
-          lo = std::min(lo, tab[r * ncols + c]);
-          hi = std::max(hi, tab[r * ncols + c]);
-        }
-        spread = std::max(spread, hi - lo);
-      }
-    }
-  }
-  return spread;
-}
-
 // Bytes of one staged window: the tile plus the rows' spread, 16-byte alignment
 // slack and the funnel shift's extra word; 0 when the four windows of a block
 // would not fit comfortably in shared memory.
@@ -327,7 +308,7 @@ std::vector<int32_t> skew_stage1(dd_plan& P, std::vector<int32_t>& skew) {
   const int64_t ngrp = (P.ndm_nom + kSumRows - 1) / kSumRows;
   skew.assign(static_cast<size_t>(ngrp * P.nsb * kSumRows), 0);
   std::vector<int32_t> tab(P.h_delay);
-  P.max_skew1 = P.reach1 = 0;
+  P.max_skew1 = P.reach1 = P.max_off1 = 0;
   for (int64_t g = 0; g < ngrp; ++g)
     for (int64_t sb = 0; sb < P.nsb; ++sb) {
       const int64_t c0 = sb * P.sbw, c1 = std::min<int64_t>(c0 + P.sbw, P.dch);
@@ -346,6 +327,7 @@ std::vector<int32_t> skew_stage1(dd_plan& P, std::vector<int32_t>& skew) {
       }
       P.max_skew1 = std::max<int64_t>(P.max_skew1, last);
       P.reach1 = std::max<int64_t>(P.reach1, last + reach);
+      P.max_off1 = std::max<int64_t>(P.max_off1, reach);
     }
   return tab;
 }
@@ -388,10 +370,12 @@ void set_tiling(dd_plan& P, int64_t budget) {
   // (their columns are not stored).
   const int64_t T2 = P.win2 ? sum_kind_tile(stage2_kind(P)) : kT;
   P.tile_pitch = round_up(round_up(L + P.max_res, kT) + T2 + 64, 64);
-  // Stage-1 windows end at most one block tile (below 8192) past their last column
-  // and its reach.
+  // Stage-1 windows start before the chunk's end (later ones are skipped) and end a
+  // block tile and their spread past their first element; the direct kernels read up to
+  // the largest delay past a tile's last column.
   const int64_t last = P.seg + P.max_res + std::max<int64_t>(P.reach1, P.max_delay);
-  P.xpitch = round_up((P.fold > 1 ? last : std::max(P.nbin, last)) + 8192 + 64, 64);
+  P.xpitch = P.win1 ? round_up((P.fold > 1 ? std::min(P.nbin, last) : P.nbin) + sum_kind_tile(stage1_kind(P)) + P.spread1 + 64, 64)
+                    : round_up(std::max(P.nbin, last) + 8192 + 64, 64);
   P.d_x.alloc(static_cast<size_t>(P.dch * P.xpitch) * x_elem(P));
   DD_CUDA_TRY(cudaMemsetAsync(P.d_x.p, 0, P.d_x.bytes, cudaStreamLegacy));
   P.inter_bytes = plane_bytes(P);
@@ -426,11 +410,15 @@ void create_subband(dd_plan& P) {
   // FP64 comparison table for the coarse delays (and replacement in FP64 mode).
   int64_t mism = 0;
   const double tsamp = P.tsamp, r = P.freq[P.ce];
+  std::vector<double> disp(static_cast<size_t>(P.dch));
+  for (int64_t c = 0; c < P.dch; ++c) {
+    const double f = P.freq[P.cs + c];
+    disp[c] = 1.0 / (f * f) - 1.0 / (r * r);
+  }
   for (int64_t j = 0; j < P.ndm_nom; ++j) {
     const double dm = static_cast<double>(P.p.dm_low) + static_cast<double>(j) * P.ndm0 * P.p.dm_step;
     for (int64_t c = 0; c < P.dch; ++c) {
-      const double f = P.freq[P.cs + c];
-      const int v = static_cast<int>(std::floor(4148.808 * dm * (1.0 / (f * f) - 1.0 / (r * r)) / tsamp + 0.5)) / ds;
+      const int v = static_cast<int>(std::floor(4148.808 * dm * disp[c] / tsamp + 0.5)) / ds;
       mism += (v != P.h_delay[j * P.dch + c]);
       if (P.p.table_mode == DD_TABLE_FP64) P.h_delay[j * P.dch + c] = v;
     }
@@ -463,8 +451,10 @@ void create_subband(dd_plan& P) {
   if (P.nbits <= 16) {
     std::vector<int32_t> skew;
     const std::vector<int32_t> tab = skew_stage1(P, skew);
-    const int spread1 = table_spread(tab, P.ndm_nom, P.dch, kSumRows, 0);
-    const int spread2 = table_spread(P.h_res, P.dm_steps, P.nsb, kSumRows, P.ndm0);
+    int spread1 = 0, spread2 = 0;
+    const std::vector<SumDesc> desc1 = build_sum_desc(tab, P.ndm_nom, P.dch, 0, &spread1);
+    const std::vector<SumDesc> desc2 = build_sum_desc(P.h_res, P.dm_steps, P.nsb, P.ndm0, &spread2);
+    P.spread1 = spread1;
     auto set_windows = [&](int fold) {
       P.fold = fold;
       P.planes = fold == 1 ? 1 : P.inter16 ? 2 : fold;
@@ -481,10 +471,10 @@ void create_subband(dd_plan& P) {
       if (!P.twin) P.win2 = 0;
     }
     if (P.win1) {
-      upload_desc(P.d_desc1, build_sum_desc(tab, P.ndm_nom, P.dch, 0));
+      upload_desc(P.d_desc1, desc1);
       upload(P.d_skew1, skew.data(), sizeof(int32_t) * skew.size());
     }
-    if (P.win2) upload_desc(P.d_desc2, build_sum_desc(P.h_res, P.dm_steps, P.nsb, P.ndm0));
+    if (P.win2) upload_desc(P.d_desc2, desc2);
   }
   set_tiling(P, int64_t(DD_INTER_MB) << 20);
   if (ds > 1 || callsite_zdm_active(P))
@@ -510,14 +500,18 @@ void set_phase_window(dd_plan& P) {
   std::vector<SumDesc> all;
   std::vector<int32_t> off(static_cast<size_t>(n));
   int spread = 0;
+  const uint32_t uds = static_cast<uint32_t>(ds);
   for (int p = 0; p < patterns; ++p) {
-    for (int64_t i = 0; i < n; ++i) off[i] = (p + P.h_delay[i]) / ds;
-    spread = std::max(spread, table_spread(off, P.dm_steps, P.nc, kSumRows, 0));
-    std::vector<SumDesc> d = build_sum_desc(off, P.dm_steps, P.nc, 0);
-    for (int64_t m = 0; m < P.dm_steps; ++m)
+    for (int64_t i = 0; i < n; ++i) off[i] = static_cast<int32_t>(static_cast<uint32_t>(p + P.h_delay[i]) / uds);
+    int sp = 0;
+    std::vector<SumDesc> d = build_sum_desc(off, P.dm_steps, P.nc, 0, &sp);
+    spread = std::max(spread, sp);
+    for (int64_t m = 0; m < P.dm_steps; ++m) {
+      SumDesc* row = d.data() + (m / kSumRows) * P.nc;
+      const int half = (m % kSumRows) >> 3, shift = 4 * (m & 7);
       for (int64_t c = 0; c < P.nc; ++c)
-        d[(m / kSumRows) * P.nc + c].phase[(m % kSumRows) >> 3] |=
-            static_cast<uint32_t>((p + P.h_delay[m * P.nc + c]) % ds) << (4 * (m & 7));
+        row[c].phase[half] |= static_cast<uint32_t>(p + P.h_delay[m * P.nc + c] - off[m * P.nc + c] * ds) << shift;
+    }
     P.pattern_descs = static_cast<int64_t>(d.size());
     all.insert(all.end(), d.begin(), d.end());
   }
@@ -535,10 +529,13 @@ void set_phase_window(dd_plan& P) {
 void set_brute_window(dd_plan& P) {
   const bool had = P.d_x.bytes != 0;
   const int fold0 = P.fold;
+  int spread = 0;
   P.winb = 0;
   P.fold = 1;
-  if (P.p.time_downsample == 1 && P.nbits <= 16) {
-    const int spread = table_spread(P.h_delay, P.dm_steps, P.nc, kSumRows, 0);
+  if (P.p.time_downsample > 1) {
+    set_phase_window(P);
+  } else if (P.nbits <= 16) {
+    const std::vector<SumDesc> desc = build_sum_desc(P.h_delay, P.dm_steps, P.nc, 0, &spread);
     auto set_window = [&](int fold) {
       P.fold = fold;
       const int k = brute_kind(P);
@@ -546,16 +543,18 @@ void set_brute_window(dd_plan& P) {
     };
     set_window(choose_fold(P, P.out_cols, P.nc, P.max_delay, P.adds));
     if (P.fold > 1 && !P.winb) set_window(1);
+    if (P.winb) upload_desc(P.d_descb, desc);
   }
-  if (P.p.time_downsample > 1) set_phase_window(P);
-  else if (P.winb) upload_desc(P.d_descb, build_sum_desc(P.h_delay, P.dm_steps, P.nc, 0));
-  if (had && P.fold == fold0) return;
   P.seg = P.fold > 1 ? round_up((P.out_cols + P.fold - 1) / P.fold, 8) : P.out_cols;
-  // (a folded row holds a segment, the padding of phase_len past the chunk and a tile)
-  P.xpitch = P.fold > 1 ? round_up(P.seg + P.phase_len - P.nin + 2048 + 64, 64) : P.phase_len;
-  const int64_t rows = P.nc * P.p.time_downsample;
-  // (+8192 elements: staged windows may end a block tile past the last row)
-  P.d_x.alloc(static_cast<size_t>(rows * P.xpitch + 8192) * x_elem(P));
+  // folded windows start before the chunk's end and inside a segment and the padding of
+  // phase_len, and end a block tile and their spread later
+  const int64_t pitch =
+      P.fold > 1 ? round_up(std::min(P.nin, P.seg + P.phase_len - P.nin) + sum_kind_tile(brute_kind(P)) + spread + 64, 64)
+                 : P.phase_len;
+  if (had && P.fold == fold0 && pitch == P.xpitch) return;
+  P.xpitch = pitch;
+  // (+8192 elements: windows in time order may end a block tile past the last row)
+  P.d_x.alloc(static_cast<size_t>(P.nc * P.p.time_downsample * P.xpitch + 8192) * x_elem(P));
   DD_CUDA_TRY(cudaMemset(P.d_x.p, 0, P.d_x.bytes));
 }
 
@@ -726,6 +725,8 @@ SumLaunch stage1_launch(const dd_plan& P, int64_t t0) {
   L.off = P.d_delay.as<int32_t>();
   L.off_pitch = P.dch;
   L.base = t0;
+  L.valid = P.nbin;
+  L.max_off = P.max_off1;
   L.nsrc_total = P.dch;
   L.nrows_total = P.ndm_nom;
   L.group = P.sbw;
@@ -758,6 +759,7 @@ SumLaunch stage2_launch(const dd_plan& P, int64_t t0, void* output) {
   L.off = P.d_res.as<int32_t>();
   L.off_pitch = P.nsb;
   L.base = 0;
+  L.valid = INT64_MAX;
   L.nsrc_total = P.nsb;
   L.nrows_total = P.dm_steps;
   L.group = P.ndm0;
@@ -856,6 +858,8 @@ SumLaunch brute_launch(const dd_plan& P, void* output) {
   L.off = P.d_delay.as<int32_t>();
   L.off_pitch = P.nc;
   L.base = 0;
+  L.valid = (P.nin + P.p.time_downsample - 1) / P.p.time_downsample;
+  L.max_off = P.max_delay / P.p.time_downsample + 1;
   L.nsrc_total = P.nc;
   L.nrows_total = P.dm_steps;
   L.out = static_cast<char*>(output);

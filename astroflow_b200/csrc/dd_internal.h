@@ -90,6 +90,8 @@ struct dd_plan {
   int win1 = 0, win2 = 0;    // staged window bytes of the shared-memory sums (0: not used)
   int64_t max_skew1 = 0;     // largest row skew of stage 1
   int64_t reach1 = 0;        // largest offset a stage-1 window reads past its column
+  int64_t spread1 = 0;       // largest spread of a stage-1 window
+  int64_t max_off1 = 0;      // largest skewed stage-1 offset
 
   // brute-force geometry (CPU path semantics)
   int64_t nc = 0;            // channels summed, [cs, ce)
@@ -308,6 +310,8 @@ struct SumLaunch {
   const int32_t* off;      // per-row, per-source offsets (elements)
   int64_t off_pitch;       // entries between consecutive rows of `off`
   int64_t base;            // element index added to every offset
+  int64_t valid;           // source elements from here on are zero: windows starting there are skipped
+  int64_t max_off;         // largest offset of any row and source
   int64_t nsrc_total;      // stage 1: channels of the band; stage 2: subbands; brute: channels
   int64_t nrows_total;     // stage 1: nominal DMs; stage 2 and brute: DM trials
   int group;               // stage 1: subband width; stage 2: fine DMs per nominal DM
@@ -366,9 +370,10 @@ int sum_stages(int win_bytes, int qs = 2, size_t extra = 0, int cap_kb = 0);
 int sum_kind_stages(int kind, int win_bytes);
 // Descriptors of a [nrows][ncols] offset table for row groups of kSumRows rows,
 // grouped within blocks of `group` rows (0: one block), in the launch's
-// blockIdx.y order.  Fails if a group's spread exceeds 65535.
+// blockIdx.y order, and the largest spread of a group's offsets (a window that holds
+// more than 65535 never fits shared memory, window_bytes).
 std::vector<SumDesc> build_sum_desc(const std::vector<int32_t>& tab, int64_t nrows,
-                                    int64_t ncols, int64_t group);
+                                    int64_t ncols, int64_t group, int* spread);
 // Device error codes of the staged sums.
 constexpr int kErrWaitFull = 1;   // a consumer gave up waiting for a staged window
 constexpr int kErrWaitEmpty = 2;  // the producer gave up waiting for a free stage

@@ -135,6 +135,7 @@ struct Geo {
   const SumDesc* desc; // descriptor of source 0 for this block's row group
   int64_t base;        // element index added to every offset
   int nsrc, nrows;     // nrows <= 0: nothing to do
+  int64_t valid;       // source elements: from here on they are zero (past the chunk)
   char* out;           // row 0, launch column 0 (byte address)
   int64_t out_pitch;   // bytes between output rows
   const int32_t* skew; // per row, or nullptr
@@ -152,6 +153,7 @@ __device__ __forceinline__ Geo make_geo(const SumLaunch& L, int T, uint3 blk) {
   g.col = tile * T;
   g.ncols = L.ncols;
   g.skew = nullptr;
+  g.valid = L.valid;
   const SumDesc* drow = L.desc + static_cast<int64_t>(blk.y) * L.desc_pitch;
   switch (L.mode) {
     case SumLaunch::kStage1: {
@@ -216,6 +218,7 @@ struct __align__(16) Pipe {
   // per row: word index and shift (bits) of sample 0 in the window of source i of
   // the stage at [2i], [2i+1]; twin windows (four sources): word indices only
   int row[kMaxStages][kSumRows][4];
+  uint32_t first[kWarps];      // first source with samples of the chunk, by warp
   int failed;
 };
 __device__ __forceinline__ int4 row_info(const Pipe& P, int s, int r) {
@@ -262,7 +265,7 @@ __device__ __forceinline__ void produce(const Geo& g, Pipe& P, uint32_t* sw, int
   uint32_t nbytes = 0;
   const char* gsrc = nullptr;
   int2 rw = make_int2(zero_q, 0);
-  if (src < g.nsrc) {
+  if (src < g.nsrc && g.base + d.lo[0] < g.valid) {
     const int64_t firstb = (g.base + d.lo[0]) * SB;
     const int64_t a0 = firstb & ~int64_t(15);
     const int ob = static_cast<int>(firstb - a0) + d.rel[0] * SB;
@@ -293,7 +296,7 @@ __device__ __forceinline__ void produce_phases(const SumLaunch& L, const Geo& g,
   uint32_t nbytes = 0;
   const char* gsrc = nullptr;
   int2 rw = make_int2(zero_q, 0);
-  if (src < g.nsrc) {
+  if (src < g.nsrc && g.base + d.lo[0] < g.valid) {
     const int64_t firstb = (g.base + d.lo[0]) * SB;
     const int64_t a0 = firstb & ~int64_t(15);
     const int ob = static_cast<int>(firstb - a0) + d.rel[0] * SB;
@@ -377,8 +380,8 @@ __device__ __forceinline__ void produce_words(const Geo& g, Pipe& P, uint32_t* s
     const int k = i + 2 * h;  // source of the stage
     const int src = 4 * q + k;
     int idx = zero_q;
-    if (src < g.nsrc) {
-      const int64_t e0 = g.base + d.lo[h];
+    const int64_t e0 = g.base + d.lo[h];
+    if (src < g.nsrc && e0 < g.valid) {
       const int64_t a0 = e0 & ~int64_t(3);
       idx = (4 * s + k) * ww + static_cast<int>(e0 - a0) + d.rel[h];
       if (r == 0) {
@@ -398,9 +401,29 @@ __device__ __forceinline__ void produce_words(const Geo& g, Pipe& P, uint32_t* s
     if (nbytes[h]) bulk_copy(sw + (4 * s + i + 2 * h) * ww, gsrc[h], nbytes[h], &P.full[s]);
 }
 
+// Delays past the chunk's end leave a block's first sources (the lowest frequencies)
+// without samples: takes them off the block's sources, in whole groups of QS, so that
+// they are neither staged nor summed.  Only blocks that reach past the end look.
+template <int QS>
+__device__ __forceinline__ void skip_empty_sources(const SumLaunch& L, Geo& g, Pipe& P) {
+  if (g.base + L.max_off < g.valid) return;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  uint32_t first = static_cast<uint32_t>(g.nsrc);
+  for (int i = threadIdx.x; i < g.nsrc && i < static_cast<int>(first); i += kThreads)
+    if (g.base + __ldg(&g.desc[i].lo) < g.valid) first = i;
+  first = __reduce_min_sync(0xffffffffu, first);
+  if (lane == 0) P.first[warp] = first;
+  __syncthreads();
+  first = __reduce_min_sync(0xffffffffu, P.first[lane & (kWarps - 1)]);
+  const int skip = static_cast<int>(first) / QS * QS;
+  g.src += skip * g.src_pitch;
+  g.desc += skip;
+  g.nsrc -= skip;
+}
+
 // Pipeline driver shared by the kernels: calls body(stage, cur) for every group of
 // QS sources once their windows are in shared memory, and setup() once the first
-// windows are on their way; false when the block has nothing to store (kModeTwin: each source is staged
+// windows are on their way (SKIP: sources may lie past the chunk's end); false when the block has nothing to store (kModeTwin: each source is staged
 // with its shifted twin, see produce_twin; kModeWords: see produce_words; QS is 4 for
 // both; `tile` is in bytes, for kModeWords in words).  The warps take turns at
 // staging: warp q % kWarps stages group q, D groups before they are summed, and has
@@ -412,8 +435,8 @@ __device__ __forceinline__ void produce_words(const Geo& g, Pipe& P, uint32_t* s
 // 40.1 ms (stages 1 and 2) that way and 56.6 + 32.8 ms with turns; brute force over
 // 1024 channels, 2^17 samples, 1001 trials 10.8 and 8.5 ms.
 constexpr int kModePlain = 0, kModeTwin = 1, kModeWords = 2, kModePhase = 3;
-template <int SB, int QS = 2, int MODE = kModePlain, typename Setup, typename Body>
-__device__ __forceinline__ bool run_pipeline(const SumLaunch& L, const Geo& g, Pipe& P,
+template <int SB, int QS, int MODE, bool SKIP, typename Setup, typename Body>
+__device__ __forceinline__ bool run_pipeline(const SumLaunch& L, Geo& g, Pipe& P,
                                              uint32_t* sw, int tile, Setup&& setup, Body&& body) {
   static_assert(QS == (MODE == kModePlain || MODE == kModePhase ? 2 : 4), "sources per stage");
   static_assert(kMaxStages <= kWarps, "each warp stages at most one group before the loop");
@@ -423,6 +446,7 @@ __device__ __forceinline__ bool run_pipeline(const SumLaunch& L, const Geo& g, P
   const int S = L.stages;
   const int D = max(1, S - 2);
   const int zero_q = kWinPerSrc * QS * S * ww;
+  if constexpr (SKIP) skip_empty_sources<QS>(L, g, P);
   const int ngroups = (g.nsrc + QS - 1) / QS;
   GroupDesc<QS> desc;
   desc.load(g, warp, lane);
@@ -439,7 +463,7 @@ __device__ __forceinline__ bool run_pipeline(const SumLaunch& L, const Geo& g, P
   // order earlier generic accesses to the windows (a previous task of a persistent
   // block) before the bulk copies that refill them
   asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-  if (g.nsrc % QS)  // a source is missing in the last group
+  if (SKIP || g.nsrc % QS)  // a source may be missing, or past the chunk
     for (int i = threadIdx.x; i < ww; i += kThreads) sw[zero_q + i] = 0u;
   __syncthreads();
   volatile int* failed = &P.failed;
@@ -548,7 +572,7 @@ __device__ __forceinline__ void sum_u8(const SumLaunch& L, uint3 blk, uint32_t* 
   constexpr int kGroups = kSumRows / RB;
   constexpr int kWarpsPerTile = kWarps / kGroups;
   constexpr int T = kWarpsPerTile * 32 * NW * 4;
-  const Geo g = make_geo<MODE == kModePhase>(L, T, blk);
+  Geo g = make_geo<MODE == kModePhase>(L, T, blk);
   if (g.nrows <= 0) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rbase = warp / kWarpsPerTile, wt = warp % kWarpsPerTile;
@@ -598,7 +622,7 @@ __device__ __forceinline__ void sum_u8(const SumLaunch& L, uint3 blk, uint32_t* 
   };
   int since = 0;       // sources summed in the fields since the last flush
   bool stored = false; // the output holds partial sums of an earlier flush
-  const bool ok = run_pipeline<1, 2, MODE>(L, g, P, sw, T, [&] { act = active_rows<RB, T>(g, rbase); }, [&](int s, const uint32_t* win) {
+  const bool ok = run_pipeline<1, 2, MODE, true>(L, g, P, sw, T, [&] { act = active_rows<RB, T>(g, rbase); }, [&](int s, const uint32_t* win) {
     for_rows<RB>(act, [&](int r) {
       const int4 rw = row_info(P, s, rbase + kGroups * r);
       const uint32_t* w0 = win + rw.x + wbase;
@@ -692,7 +716,7 @@ __device__ __forceinline__ void sum_u16_wide(const SumLaunch& L, uint3 blk, uint
   constexpr int kGroups = kSumRows / RB;
   constexpr int kWarpsPerTile = kWarps / kGroups;
   constexpr int T = kWarpsPerTile * 32 * NW * 2;
-  const Geo g = make_geo<MODE == kModePhase>(L, T, blk);
+  Geo g = make_geo<MODE == kModePhase>(L, T, blk);
   if (g.nrows <= 0) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rbase = warp / kWarpsPerTile, wt = warp % kWarpsPerTile;
@@ -703,7 +727,7 @@ __device__ __forceinline__ void sum_u16_wide(const SumLaunch& L, uint3 blk, uint
   for (int r = 0; r < RB; ++r)
 #pragma unroll
     for (int k = 0; k < NW; ++k) lo32[r][k] = hi32[r][k] = 0;
-  const bool ok = run_pipeline<2, 2, MODE>(L, g, P, sw, 2 * T, [&] { act = active_rows<RB, T>(g, rbase); }, [&](int s, const uint32_t* win) {
+  const bool ok = run_pipeline<2, 2, MODE, true>(L, g, P, sw, 2 * T, [&] { act = active_rows<RB, T>(g, rbase); }, [&](int s, const uint32_t* win) {
     for_rows<RB>(act, [&](int r) {
       const int4 rw = row_info(P, s, rbase + kGroups * r);
       const uint32_t* w0 = win + rw.x + wbase;
@@ -779,7 +803,7 @@ __device__ __forceinline__ void sum_fold8(const SumLaunch& L, uint3 blk, uint32_
   constexpr int kGroups = kSumRows / RB;  // warp groups sharing the rows, as in sum_u8
   constexpr int kWarpsPerTile = kWarps / kGroups;
   constexpr int T = kWarpsPerTile * 32 * NW;
-  const Geo g = make_geo(L, T, blk);
+  Geo g = make_geo(L, T, blk);
   if (g.nrows <= 0) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rbase = warp / kWarpsPerTile;
@@ -818,7 +842,7 @@ __device__ __forceinline__ void sum_fold8(const SumLaunch& L, uint3 blk, uint32_
   };
   int since = 0;
   bool stored = false;
-  const bool ok = run_pipeline<4, 4, kModeWords>(L, g, P, sw, T, [&] { act = active_rows<RB, T>(g, rbase); }, [&](int s, const uint32_t* win) {
+  const bool ok = run_pipeline<4, 4, kModeWords, true>(L, g, P, sw, T, [&] { act = active_rows<RB, T>(g, rbase); }, [&](int s, const uint32_t* win) {
     for_rows<RB>(act, [&](int r) {
       const int4 a = row_info(P, s, rbase + kGroups * r);
       const uint32_t* w0 = win + a.x + wbase;
@@ -870,7 +894,7 @@ __device__ __forceinline__ void sum_fold16(const SumLaunch& L, uint3 blk, uint32
   constexpr int kGroups = kSumRows / RB;
   constexpr int kWarpsPerTile = kWarps / kGroups;
   constexpr int T = kWarpsPerTile * 32 * NW;
-  const Geo g = make_geo(L, T, blk);
+  Geo g = make_geo(L, T, blk);
   if (g.nrows <= 0) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rbase = warp / kWarpsPerTile;
@@ -881,7 +905,7 @@ __device__ __forceinline__ void sum_fold16(const SumLaunch& L, uint3 blk, uint32
   for (int r = 0; r < RB; ++r)
 #pragma unroll
     for (int k = 0; k < NW; ++k) all[r][k] = hi[r][k] = 0;
-  const bool ok = run_pipeline<4, 4, kModeWords>(L, g, P, sw, T, [&] { act = active_rows<RB, T>(g, rbase); }, [&](int s, const uint32_t* win) {
+  const bool ok = run_pipeline<4, 4, kModeWords, true>(L, g, P, sw, T, [&] { act = active_rows<RB, T>(g, rbase); }, [&](int s, const uint32_t* win) {
     for_rows<RB>(act, [&](int r) {
       const int4 a = row_info(P, s, rbase + kGroups * r);
       const uint32_t* w0 = win + a.x + wbase;
@@ -923,7 +947,7 @@ __device__ __forceinline__ void sum_plane16(const SumLaunch& L, uint3 blk, uint3
   constexpr int kGroups = kSumRows / RB;
   constexpr int kWarpsPerTile = kWarps / kGroups;
   constexpr int T = kWarpsPerTile * 32 * NW;
-  const Geo g = make_geo(L, T, blk);
+  Geo g = make_geo(L, T, blk);
   if (g.nrows <= 0) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rbase = warp / kWarpsPerTile;
@@ -934,7 +958,7 @@ __device__ __forceinline__ void sum_plane16(const SumLaunch& L, uint3 blk, uint3
   for (int r = 0; r < RB; ++r)
 #pragma unroll
     for (int k = 0; k < NW; ++k) all[r][k] = hi[r][k] = 0;
-  const bool ok = run_pipeline<4, 4, kModeWords>(L, g, P, sw, T, [&] { act = active_rows<RB, T>(g, rbase); }, [&](int s, const uint32_t* win) {
+  const bool ok = run_pipeline<4, 4, kModeWords, false>(L, g, P, sw, T, [&] { act = active_rows<RB, T>(g, rbase); }, [&](int s, const uint32_t* win) {
     for_rows<RB>(act, [&](int r) {
       const int4 a = row_info(P, s, rbase + kGroups * r);
       const uint32_t* w0 = win + a.x + wbase;
@@ -972,7 +996,7 @@ __device__ __forceinline__ void sum_plane32(const SumLaunch& L, uint3 blk, uint3
   constexpr int kGroups = kSumRows / RB;
   constexpr int kWarpsPerTile = kWarps / kGroups;
   constexpr int T = kWarpsPerTile * 32 * NW;
-  const Geo g = make_geo(L, T, blk);
+  Geo g = make_geo(L, T, blk);
   if (g.nrows <= 0) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rbase = warp / kWarpsPerTile;
@@ -983,7 +1007,7 @@ __device__ __forceinline__ void sum_plane32(const SumLaunch& L, uint3 blk, uint3
   for (int r = 0; r < RB; ++r)
 #pragma unroll
     for (int k = 0; k < NW; ++k) acc[r][k] = 0;
-  const bool ok = run_pipeline<4, 4, kModeWords>(L, g, P, sw, T, [&] { act = active_rows<RB, T>(g, rbase); }, [&](int s, const uint32_t* win) {
+  const bool ok = run_pipeline<4, 4, kModeWords, false>(L, g, P, sw, T, [&] { act = active_rows<RB, T>(g, rbase); }, [&](int s, const uint32_t* win) {
     for_rows<RB>(act, [&](int r) {
       const int4 a = row_info(P, s, rbase + kGroups * r);
       const uint32_t* w0 = win + a.x + wbase;
@@ -1030,7 +1054,7 @@ __device__ __forceinline__ void sum_u16_twin(const SumLaunch& L, uint3 blk, uint
   constexpr int kGroups = kSumRows / RB;  // warp groups sharing the rows, as in sum_u8
   constexpr int kWarpsPerTile = kWarps / kGroups;
   constexpr int T = kWarpsPerTile * 32 * NW * 2;
-  const Geo g = make_geo(L, T, blk);
+  Geo g = make_geo(L, T, blk);
   if (g.nrows <= 0) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rbase = warp / kWarpsPerTile;
@@ -1041,7 +1065,7 @@ __device__ __forceinline__ void sum_u16_twin(const SumLaunch& L, uint3 blk, uint
   for (int r = 0; r < RB; ++r)
 #pragma unroll
     for (int k = 0; k < NW; ++k) lo[r][k] = hi[r][k] = 0;
-  const bool ok = run_pipeline<2, 4, kModeTwin>(L, g, P, sw, 2 * T, [&] { act = active_rows<RB, T>(g, rbase); }, [&](int s, const uint32_t* win) {
+  const bool ok = run_pipeline<2, 4, kModeTwin, false>(L, g, P, sw, 2 * T, [&] { act = active_rows<RB, T>(g, rbase); }, [&](int s, const uint32_t* win) {
     for_rows<RB>(act, [&](int r) {
       const int4 a = row_info(P, s, rbase + kGroups * r);
       const uint32_t* w0 = win + a.x + wbase;
@@ -1304,11 +1328,12 @@ int sum_kind_stages(int kind, int win_bytes) {
 }
 
 std::vector<SumDesc> build_sum_desc(const std::vector<int32_t>& tab, int64_t nrows,
-                                    int64_t ncols, int64_t group) {
+                                    int64_t ncols, int64_t group, int* spread) {
   const int64_t blk = group > 0 ? group : nrows;
   const int64_t per = (blk + kSumRows - 1) / kSumRows;  // row groups per block of rows
   const int64_t nblk = (nrows + blk - 1) / blk;
   std::vector<SumDesc> d(static_cast<size_t>(nblk * per * ncols));
+  int32_t most = 0;
   for (int64_t b = 0; b < nblk; ++b) {
     const int64_t b0 = b * blk, b1 = std::min(nrows, b0 + blk);
     for (int64_t gi = 0; gi < per; ++gi) {
@@ -1324,13 +1349,14 @@ std::vector<SumDesc> build_sum_desc(const std::vector<int32_t>& tab, int64_t nro
         }
       for (int64_t c = 0; c < ncols; ++c) {
         row[c].span -= row[c].lo;
-        if (row[c].span > 65535) throw Error{DD_ERR_RUNTIME, "staged-sum offsets spread too far"};
+        most = std::max(most, row[c].span);
       }
       for (int64_t r = r0; r < r1; ++r)
         for (int64_t c = 0; c < ncols; ++c)
           row[c].rel[r - r0] = static_cast<uint16_t>(tab[r * ncols + c] - row[c].lo);
     }
   }
+  *spread = most;
   return d;
 }
 
