@@ -530,14 +530,24 @@ __device__ __forceinline__ T prepared_value(const PrepArgs& a, const T* x, int64
   return v;
 }
 
+// Tile of a layout kernel's block: the grid is one-dimensional with the channel groups
+// fastest, so that the blocks running at a time read whole rows of the chunk.
+__device__ __forceinline__ int64_t prep_tile(const PrepArgs& a, int64_t c0, int64_t* group) {
+  const unsigned groups = (static_cast<unsigned>(a.c1 - c0) + 63u) / 64u;  // 32-bit division
+  const unsigned t = blockIdx.x / groups;
+  *group = blockIdx.x - t * groups;
+  return t;
+}
+
 // Fused RFI application and transpose to the channel-major layout.
 // Tile: 64 samples x 64 channels, 256 threads.
 template <typename T>
 __global__ void k_prep(PrepArgs a) {
   __shared__ T tile[64][65];
   const T* x = static_cast<const T*>(a.x);
-  const int64_t tb = static_cast<int64_t>(blockIdx.x) * 64;
-  const int64_t cb = a.c0 + static_cast<int64_t>(blockIdx.y) * 64;
+  int64_t group;
+  const int64_t tb = prep_tile(a, a.c0, &group) * 64;
+  const int64_t cb = a.c0 + group * 64;
   const int tx = threadIdx.x & 63;   // channel within tile (read phase)
   const int ty = threadIdx.x >> 6;   // 0..3
   const int64_t c = cb + tx;
@@ -564,174 +574,6 @@ __global__ void k_prep(PrepArgs a) {
   }
 }
 
-// 8-bit samples without downsampling (the subband layout), as k_prep but four
-// channels per load and four samples per store: a block takes kPrepU8Subtiles
-// consecutive tiles of 64 samples x 64 channels, one after another; for each it
-// applies the masks and the zero-DM offset to whole words with byte-wise SIMD
-// operations and transposes 4x4 byte blocks in registers.  Needs
-// nchans % 4 == 0 (aligned word loads); channel words are read from c0 & ~3 and
-// channels outside [c0, c1) are not stored.
-constexpr int kPrepU8Subtiles = 4;
-__global__ void __launch_bounds__(256) k_prep_u8(PrepArgs a) {
-  __shared__ uint32_t tile[64][17];  // [sample][channel word], padded
-  const uint8_t* x = static_cast<const uint8_t*>(a.x);
-  const int64_t cb = (a.c0 & ~int64_t(3)) + static_cast<int64_t>(blockIdx.y) * 64;
-  const int w = threadIdx.x & 15;  // channel word of the tile (load phase)
-  const int64_t c = cb + 4 * w;
-  const bool cvalid = c < a.nchans;
-  uint32_t drop = 0, inrange = 0;  // per byte: bad channel / zero-DM applies
-  if (cvalid) {
-#pragma unroll
-    for (int b = 0; b < 4; ++b) {
-      const int64_t ch = c + b;
-      if (a.keep && !a.keep[ch]) drop |= 0xffu << (8 * b);
-      if (a.zdm_off && ch >= a.zdm_cs && ch < a.zdm_ce) inrange |= 0xffu << (8 * b);
-    }
-  }
-  const int i = threadIdx.x & 15;  // store phase: samples 4i .. 4i+3
-  const int j = threadIdx.x >> 4;  // channel word j: channels 4j .. 4j+3
-  const int r0 = threadIdx.x >> 4;  // load phase: rows r0, r0 + 16, r0 + 32, r0 + 48
-  uint8_t* out = static_cast<uint8_t*>(a.out);
-  const int64_t tile0 = static_cast<int64_t>(blockIdx.x) * kPrepU8Subtiles * 64;
-  // this thread's source word in row tile0 + r0, and the stride of 16 rows
-  const uint8_t* src = x + (tile0 + r0) * a.nchans + c;
-  const int64_t step16 = 16 * a.nchans;
-  // this thread's four output rows (channels 4j .. 4j+3) at sample tile0 + 4i
-  uint8_t* dst[4];
-#pragma unroll
-  for (int b = 0; b < 4; ++b) {
-    const int64_t cc = cb + 4 * j + b;
-    dst[b] = (out && cc >= a.c0 && cc < a.c1) ? out + (cc - a.c0) * a.pitch + tile0 + 4 * i : nullptr;
-  }
-  // the raw words of sub-tile `sub` (loads only; masks applied when staged)
-  auto fetch = [&](int sub, uint32_t (&v)[4]) {
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const int64_t t = tile0 + sub * 64 + r0 + 16 * k;
-      v[k] = (cvalid && t < a.nsamp)
-                 ? __ldg(reinterpret_cast<const uint32_t*>(src + (4 * sub + k) * step16))
-                 : 0u;
-    }
-  };
-  uint32_t cur[4], nxt[4];
-  fetch(0, cur);
-  int seg = -1;          // IQRM segment whose mask word is cached in seg_keep
-  uint32_t seg_keep = ~0u;
-  for (int sub = 0; sub < kPrepU8Subtiles; ++sub) {
-    const int64_t tb = tile0 + sub * 64;
-    if (tb >= a.nsamp) break;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const int r = r0 + 16 * k;
-      const int64_t t = tb + r;
-      uint32_t v = cur[k];
-      if (cvalid && t < a.nsamp) {
-        if (a.segmask) {
-          const int sg = find_seg(a.seg_t0, a.nseg, t);
-          if (sg != seg) {  // segments span many rows: the mask word changes rarely
-            seg = sg;
-            seg_keep = ~__vcmpne4(*reinterpret_cast<const uint32_t*>(
-                                      a.segmask + static_cast<int64_t>(sg) * a.nchans + c),
-                                  0u);
-          }
-          v &= seg_keep;
-        }
-        if (a.zdm_off) {
-          const uint32_t m = min(a.zdm_off[t], 255u) * 0x01010101u;
-          v = (__vsubus4(v, m) & inrange) | (v & ~inrange);
-        }
-        v &= ~drop;
-      }
-      tile[r][w] = v;
-    }
-    __syncthreads();
-    if (sub + 1 < kPrepU8Subtiles) fetch(sub + 1, nxt);  // in flight during the stores
-    if (out) {
-      const uint32_t q0 = tile[4 * i][j], q1 = tile[4 * i + 1][j];
-      const uint32_t q2 = tile[4 * i + 2][j], q3 = tile[4 * i + 3][j];
-      const uint32_t lo01 = __byte_perm(q0, q1, 0x5140), hi01 = __byte_perm(q0, q1, 0x7362);
-      const uint32_t lo23 = __byte_perm(q2, q3, 0x5140), hi23 = __byte_perm(q2, q3, 0x7362);
-      const uint32_t o[4] = {__byte_perm(lo01, lo23, 0x5410), __byte_perm(lo01, lo23, 0x7632),
-                             __byte_perm(hi01, hi23, 0x5410), __byte_perm(hi01, hi23, 0x7632)};
-#pragma unroll
-      for (int b = 0; b < 4; ++b)
-        if (dst[b]) *reinterpret_cast<uint32_t*>(dst[b] + sub * 64) = o[b];
-    }
-    __syncthreads();  // the tile is refilled by the next sub-tile
-#pragma unroll
-    for (int k = 0; k < 4; ++k) cur[k] = nxt[k];
-  }
-}
-
-// 16-bit samples without downsampling, as k_prep_u8 with 16-bit lanes: a block
-// takes 64 samples x 64 channels, loads four channels per 8-byte word pair,
-// applies the masks and the zero-DM offset lane-wise, and transposes 4x4 blocks
-// of 16-bit samples in registers into 8-byte stores of four samples per
-// channel.  Needs nchans % 4 == 0; channel words are read from c0 & ~3 and
-// channels outside [c0, c1) are not stored.
-__global__ void __launch_bounds__(256) k_prep_u16(PrepArgs a) {
-  __shared__ uint2 tile[64][17];  // [sample][four-channel group], padded
-  const uint16_t* x = static_cast<const uint16_t*>(a.x);
-  const int64_t tb = static_cast<int64_t>(blockIdx.x) * 64;
-  const int64_t cb = (a.c0 & ~int64_t(3)) + static_cast<int64_t>(blockIdx.y) * 64;
-  {
-    const int w = threadIdx.x & 15;  // four-channel group of the tile
-    const int64_t c = cb + 4 * w;
-    const bool cvalid = c < a.nchans;
-    uint2 drop = make_uint2(0, 0), inrange = make_uint2(0, 0);  // per 16-bit lane
-    if (cvalid) {
-#pragma unroll
-      for (int b = 0; b < 4; ++b) {
-        const int64_t ch = c + b;
-        const uint32_t lane = 0xffffu << (16 * (b & 1));
-        if (a.keep && !a.keep[ch]) (b < 2 ? drop.x : drop.y) |= lane;
-        if (a.zdm_off && ch >= a.zdm_cs && ch < a.zdm_ce) (b < 2 ? inrange.x : inrange.y) |= lane;
-      }
-    }
-    for (int r = threadIdx.x >> 4; r < 64; r += 16) {
-      const int64_t t = tb + r;
-      uint2 v = make_uint2(0, 0);
-      if (cvalid && t < a.nsamp) {
-        v = *reinterpret_cast<const uint2*>(x + t * a.nchans + c);
-        if (a.segmask) {
-          const int sg = find_seg(a.seg_t0, a.nseg, t);
-          const uint32_t k = __vcmpne4(*reinterpret_cast<const uint32_t*>(
-                                           a.segmask + static_cast<int64_t>(sg) * a.nchans + c),
-                                       0u);
-          v.x &= ~__byte_perm(k, 0u, 0x1100);
-          v.y &= ~__byte_perm(k, 0u, 0x3322);
-        }
-        if (a.zdm_off) {
-          const uint32_t m = min(a.zdm_off[t], 65535u) * 0x00010001u;
-          v.x = (__vsubus2(v.x, m) & inrange.x) | (v.x & ~inrange.x);
-          v.y = (__vsubus2(v.y, m) & inrange.y) | (v.y & ~inrange.y);
-        }
-        v.x &= ~drop.x;
-        v.y &= ~drop.y;
-      }
-      tile[r][w] = v;
-    }
-  }
-  __syncthreads();
-  if (!a.out) return;
-  const int i = threadIdx.x & 15;  // samples 4i .. 4i+3
-  const int j = threadIdx.x >> 4;  // channels 4j .. 4j+3
-  const uint2 q0 = tile[4 * i][j], q1 = tile[4 * i + 1][j];
-  const uint2 q2 = tile[4 * i + 2][j], q3 = tile[4 * i + 3][j];
-  const uint2 o[4] = {
-      make_uint2(__byte_perm(q0.x, q1.x, 0x5410), __byte_perm(q2.x, q3.x, 0x5410)),
-      make_uint2(__byte_perm(q0.x, q1.x, 0x7632), __byte_perm(q2.x, q3.x, 0x7632)),
-      make_uint2(__byte_perm(q0.y, q1.y, 0x5410), __byte_perm(q2.y, q3.y, 0x5410)),
-      make_uint2(__byte_perm(q0.y, q1.y, 0x7632), __byte_perm(q2.y, q3.y, 0x7632))};
-  uint16_t* out = static_cast<uint16_t*>(a.out);
-#pragma unroll
-  for (int b = 0; b < 4; ++b) {
-    const int64_t cc = cb + 4 * j + b;
-    if (cc >= a.c0 && cc < a.c1)
-      *reinterpret_cast<uint2*>(out + (cc - a.c0) * a.pitch + tb + 4 * i) = o[b];
-  }
-}
-
 // Folded layout, any channel count and alignment: word s of channel c holds the
 // samples s + f * seg, f = 0 .. F-1 (F = 4 of 8 bits, 2 of 16).  Tile: 64 words x 64
 // channels, 256 threads.
@@ -740,8 +582,9 @@ __global__ void __launch_bounds__(256) k_prep_fold(PrepArgs a) {
   constexpr int F = 4 / sizeof(T);
   __shared__ uint32_t tile[64][65];  // [channel][word]
   const T* x = static_cast<const T*>(a.x);
-  const int64_t sb = static_cast<int64_t>(blockIdx.x) * 64;
-  const int64_t cb = a.c0 + static_cast<int64_t>(blockIdx.y) * 64;
+  int64_t group;
+  const int64_t sb = prep_tile(a, a.c0, &group) * 64;
+  const int64_t cb = a.c0 + group * 64;
   const int tx = threadIdx.x & 63, ty = threadIdx.x >> 6;
   const int64_t c = cb + tx;
   for (int r = ty; r < 64; r += 4) {
@@ -760,64 +603,88 @@ __global__ void __launch_bounds__(256) k_prep_fold(PrepArgs a) {
     if (cb + r < a.c1 && sb + tx < a.nwords) out[(cb + r - a.c0) * a.pitch + sb + tx] = tile[r][tx];
 }
 
-// The same with word loads: four channels per load (4 or 8 bytes), the RFI stages
-// word-wise as in k_prep_u8 / k_prep_u16, and the samples of the segments put together
-// by byte permutes, so that shared memory is written and read once per output word.
-// Needs nchans % 4 == 0 and an aligned input; channel words are read from c0 & ~3.
-template <typename T>
-__global__ void __launch_bounds__(256) k_prep_fold_w(PrepArgs a) {
+// Both layouts without downsampling, with word loads: output word i of channel c holds
+// the samples t = WS * i + fs * f, f = 0 .. F-1, of the channel (F = 4 of 8 bits, 2 of
+// 16): WS 1 and fs seg fold the chunk, WS F and fs 1 keep its order.  A thread loads four
+// channels (4 or 8 bytes) of the F samples of four words, applies the masks and the
+// zero-DM offset to whole words, puts the samples of each channel together by byte
+// permutes, and the block stores 64 words of 64 channels through shared memory, which
+// each output word passes once.  Needs nchans % 4 == 0 and an aligned input; channel
+// words are read from c0 & ~3.  Bound by issue (80 % busy) beside the memory: row
+// pointers and counts are set up once per thread, the tile comes from one 32-bit
+// division, and nothing is 64-bit per load.  4096 channels x 151,000 samples in time
+// order 257 us (4.8 TB/s; 480 us with four loads in flight per thread and 64-bit rows),
+// 131,072 samples folded 905 us (3.9 TB/s).
+struct PrepWords {
+  int64_t fs, nwords, pitch;  // nwords: words to store per channel; pitch in words
+};
+template <typename T, int WS>
+__global__ void __launch_bounds__(256, 6) k_prep_w(PrepArgs a, PrepWords q) {
   constexpr int F = 4 / sizeof(T);   // samples per word
   constexpr int V = sizeof(T);       // 32-bit words per four channels
   __shared__ uint32_t tile[64][65];  // [channel][word]
-  const T* x = static_cast<const T*>(a.x);
-  const int64_t sb = static_cast<int64_t>(blockIdx.x) * 64;
-  const int64_t cb = (a.c0 & ~int64_t(3)) + static_cast<int64_t>(blockIdx.y) * 64;
+  int64_t group;
+  const int64_t sb = prep_tile(a, a.c0 & ~int64_t(3), &group) * 64;
+  const int64_t cb = (a.c0 & ~int64_t(3)) + group * 64;
   const int w = threadIdx.x & 15, r0 = threadIdx.x >> 4;
   const int64_t c = cb + 4 * w;
   const bool cvalid = c < a.nchans;
-  uint32_t drop[V], inrange[V];  // per lane: bad channel / zero-DM applies
+  uint32_t keep[V], inrange[V];  // per lane: not a bad channel / zero-DM applies
 #pragma unroll
-  for (int v = 0; v < V; ++v) drop[v] = inrange[v] = 0;
-  if (cvalid) {
+  for (int v = 0; v < V; ++v) {
+    keep[v] = ~0u;
+    inrange[v] = 0;
+  }
+  if (cvalid && (a.keep || a.zdm_off)) {
 #pragma unroll
     for (int b = 0; b < 4; ++b) {
       const int64_t ch = c + b;
       const uint32_t lane = V == 1 ? 0xffu << (8 * b) : 0xffffu << (16 * (b & 1));
-      if (a.keep && !a.keep[ch]) drop[V == 1 ? 0 : b >> 1] |= lane;
+      if (a.keep && !a.keep[ch]) keep[V == 1 ? 0 : b >> 1] &= ~lane;
       if (a.zdm_off && ch >= a.zdm_cs && ch < a.zdm_ce) inrange[V == 1 ? 0 : b >> 1] |= lane;
     }
   }
-  // the IQRM mask of this thread's channels in the tile's rows of each segment: rows of
-  // one tile lie in one IQRM segment but for the tiles at its ends
-  uint32_t keep4[F];
-  bool one[F];
+  // this thread's words of the tile are r0 + 16k: of each sample slot f the first row,
+  // how many of the tile's words have a sample, and the mask of the IQRM segment that
+  // holds the tile's rows (mixed: they span several)
+  const T* src[F];
+  int have[F];
+  uint32_t mask[F][V];
+  bool mixed = false;
 #pragma unroll
   for (int f = 0; f < F; ++f) {
-    keep4[f] = ~0u;
-    one[f] = true;
-    if (a.segmask && cvalid) {
-      const int64_t t = sb + f * a.seg;
-      const int s0 = find_seg(a.seg_t0, a.nseg, t);
-      one[f] = s0 + 1 >= a.nseg || static_cast<int64_t>(a.seg_t0[s0 + 1]) > t + 63;
-      if (one[f])
-        keep4[f] = ~__vcmpne4(*reinterpret_cast<const uint32_t*>(
-                                  a.segmask + static_cast<int64_t>(s0) * a.nchans + c), 0u);
+    const int64_t t0 = WS * sb + q.fs * f;
+    src[f] = static_cast<const T*>(a.x) + (t0 + WS * r0) * a.nchans + c;
+    const int64_t left = a.nsamp - t0;  // words i with WS * i < left
+    have[f] = !cvalid || left <= 0 ? 0 : left >= WS * 64 ? 64 : (static_cast<int>(left) + WS - 1) / WS;
+#pragma unroll
+    for (int v = 0; v < V; ++v) mask[f][v] = keep[v];
+    if (a.segmask && have[f]) {
+      const int sg = find_seg(a.seg_t0, a.nseg, t0);
+      mixed |= sg + 1 < a.nseg && static_cast<int64_t>(a.seg_t0[sg + 1]) <= t0 + WS * 63;
+      const uint32_t m4 = ~__vcmpne4(*reinterpret_cast<const uint32_t*>(
+                                         a.segmask + static_cast<int64_t>(sg) * a.nchans + c), 0u);
+      if constexpr (V == 1) {
+        mask[f][0] &= m4;
+      } else {
+        mask[f][0] &= __byte_perm(m4, 0u, 0x1100);
+        mask[f][V - 1] &= __byte_perm(m4, 0u, 0x3322);
+      }
     }
   }
+  const int64_t step = 16 * WS * a.nchans;
   uint32_t in[4][F][V];
 #pragma unroll
   for (int k = 0; k < 4; ++k)
 #pragma unroll
     for (int f = 0; f < F; ++f) {
-      const int64_t t = sb + r0 + 16 * k + f * a.seg;
 #pragma unroll
       for (int v = 0; v < V; ++v) in[k][f][v] = 0;
-      if (cvalid && t < a.nsamp) {
-        const T* p = x + t * a.nchans + c;
+      if (r0 + 16 * k < have[f]) {
         if constexpr (V == 1) {
-          in[k][f][0] = __ldg(reinterpret_cast<const uint32_t*>(p));
+          in[k][f][0] = __ldg(reinterpret_cast<const uint32_t*>(src[f] + k * step));
         } else {
-          const uint2 u = __ldg(reinterpret_cast<const uint2*>(p));
+          const uint2 u = __ldg(reinterpret_cast<const uint2*>(src[f] + k * step));
           in[k][f][0] = u.x;
           in[k][f][V - 1] = u.y;
         }
@@ -827,29 +694,29 @@ __global__ void __launch_bounds__(256) k_prep_fold_w(PrepArgs a) {
   for (int k = 0; k < 4; ++k) {
 #pragma unroll
     for (int f = 0; f < F; ++f) {
-      const int64_t t = sb + r0 + 16 * k + f * a.seg;
-      if (!cvalid || t >= a.nsamp) continue;
-      uint32_t m4 = keep4[f];
-      if (a.segmask && !one[f])
-        m4 = ~__vcmpne4(*reinterpret_cast<const uint32_t*>(
-                            a.segmask + static_cast<int64_t>(find_seg(a.seg_t0, a.nseg, t)) * a.nchans + c), 0u);
-      if constexpr (V == 1) {
-        uint32_t v = in[k][f][0] & m4;
-        if (a.zdm_off) {
-          const uint32_t m = min(a.zdm_off[t], 255u) * 0x01010101u;
-          v = (__vsubus4(v, m) & inrange[0]) | (v & ~inrange[0]);
+      if (mixed && r0 + 16 * k < have[f]) {  // rows of several IQRM segments: one by one
+        const int64_t t = WS * (sb + r0 + 16 * k) + q.fs * f;
+        const uint32_t m4 = ~__vcmpne4(*reinterpret_cast<const uint32_t*>(
+                                           a.segmask + static_cast<int64_t>(find_seg(a.seg_t0, a.nseg, t)) * a.nchans + c), 0u);
+        if constexpr (V == 1) {
+          in[k][f][0] &= m4 & keep[0];
+        } else {
+          in[k][f][0] &= __byte_perm(m4, 0u, 0x1100) & keep[0];
+          in[k][f][V - 1] &= __byte_perm(m4, 0u, 0x3322) & keep[V - 1];
         }
-        in[k][f][0] = v & ~drop[0];
       } else {
-        uint32_t u0 = in[k][f][0] & __byte_perm(m4, 0u, 0x1100);
-        uint32_t u1 = in[k][f][V - 1] & __byte_perm(m4, 0u, 0x3322);
-        if (a.zdm_off) {
-          const uint32_t m = min(a.zdm_off[t], 65535u) * 0x00010001u;
-          u0 = (__vsubus2(u0, m) & inrange[0]) | (u0 & ~inrange[0]);
-          u1 = (__vsubus2(u1, m) & inrange[V - 1]) | (u1 & ~inrange[V - 1]);
+#pragma unroll
+        for (int v = 0; v < V; ++v) in[k][f][v] &= mask[f][v];
+      }
+      if (a.zdm_off && r0 + 16 * k < have[f]) {
+        const uint32_t off = a.zdm_off[WS * (sb + r0 + 16 * k) + q.fs * f];
+#pragma unroll
+        for (int v = 0; v < V; ++v) {
+          const uint32_t u = in[k][f][v];
+          const uint32_t d = V == 1 ? __vsubus4(u, min(off, 255u) * 0x01010101u)
+                                    : __vsubus2(u, min(off, 65535u) * 0x00010001u);
+          in[k][f][v] = (d & inrange[v]) | (u & ~inrange[v]);
         }
-        in[k][f][0] = u0 & ~drop[0];
-        in[k][f][V - 1] = u1 & ~drop[V - 1];
       }
     }
     uint32_t o[4];
@@ -871,15 +738,16 @@ __global__ void __launch_bounds__(256) k_prep_fold_w(PrepArgs a) {
     for (int b = 0; b < 4; ++b) tile[4 * w + b][r0 + 16 * k] = o[b];
   }
   __syncthreads();
-  uint32_t* out = static_cast<uint32_t*>(a.out);
-  const int lane = threadIdx.x & 31;
-  for (int r = threadIdx.x >> 5; r < 64; r += 8) {
-    const int64_t cc = cb + r;
-    if (cc < a.c0 || cc >= a.c1) continue;
-    uint32_t* dst = out + (cc - a.c0) * a.pitch + sb;
+  const int lane = threadIdx.x & 31, row = threadIdx.x >> 5;
+  const int64_t words = q.nwords - sb;
+  const int64_t pitch = q.pitch;
+  uint32_t* dst = static_cast<uint32_t*>(a.out) + (cb + row - a.c0) * pitch + sb + lane;
 #pragma unroll
-    for (int h = 0; h < 2; ++h)
-      if (sb + lane + 32 * h < a.nwords) dst[lane + 32 * h] = tile[r][lane + 32 * h];
+  for (int r = 0; r < 64; r += 8, dst += 8 * pitch) {
+    const int64_t cc = cb + row + r;
+    if (cc < a.c0 || cc >= a.c1) continue;
+    if (lane < words) dst[0] = tile[row + r][lane];
+    if (lane + 32 < words) dst[32] = tile[row + r][lane + 32];
   }
 }
 
@@ -1055,31 +923,30 @@ void launch_zdm_offsets(const void* x, int nbits, int64_t nsamp, int64_t nchans,
 }
 
 void launch_prep(const PrepArgs& a, cudaStream_t st) {
-  // the word-wise kernels apply integer zero-DM offsets only
-  if (a.out && a.fold > 1) {
-    const bool wide = !a.zdm_mean && a.nchans % 4 == 0 && reinterpret_cast<uintptr_t>(a.x) % (a.nbits / 2) == 0;
-    const int64_t cw0 = wide ? a.c0 & ~int64_t(3) : a.c0;
-    const dim3 grid(static_cast<unsigned>((a.nwords + 63) / 64), static_cast<unsigned>((a.c1 - cw0 + 63) / 64));
-    if (a.nbits == 8 && wide) k_prep_fold_w<uint8_t><<<grid, 256, 0, st>>>(a);
-    else if (a.nbits == 8) k_prep_fold<uint8_t><<<grid, 256, 0, st>>>(a);
-    else if (wide) k_prep_fold_w<uint16_t><<<grid, 256, 0, st>>>(a);
+  const auto blocks = [&](int64_t tiles, int64_t c0) {
+    const int64_t n = tiles * ((a.c1 - c0 + 63) / 64);
+    if (n >= (int64_t(1) << 31)) throw Error{DD_ERR_INVALID, "chunk too large for the layout kernel"};
+    return static_cast<unsigned>(n);
+  };
+  // the word-wise kernel applies integer zero-DM offsets only
+  const int F = a.nbits == 8 ? 4 : 2;
+  const bool wide = a.out && a.nbits <= 16 && !a.zdm_mean && a.nchans % 4 == 0 &&
+                    reinterpret_cast<uintptr_t>(a.x) % (a.nbits / 2) == 0;
+  if (wide && (a.fold > 1 || (a.ds == 1 && a.pitch % F == 0 && reinterpret_cast<uintptr_t>(a.out) % 4 == 0))) {
+    const PrepWords q = a.fold > 1 ? PrepWords{a.seg, a.nwords, a.pitch} : PrepWords{1, (a.nsamp + F - 1) / F, a.pitch / F};
+    const unsigned grid = blocks((q.nwords + 63) / 64, a.c0 & ~int64_t(3));
+    if (a.nbits == 8 && a.fold > 1) k_prep_w<uint8_t, 1><<<grid, 256, 0, st>>>(a, q);
+    else if (a.nbits == 8) k_prep_w<uint8_t, 4><<<grid, 256, 0, st>>>(a, q);
+    else if (a.fold > 1) k_prep_w<uint16_t, 1><<<grid, 256, 0, st>>>(a, q);
+    else k_prep_w<uint16_t, 2><<<grid, 256, 0, st>>>(a, q);
+    DD_LAUNCHED();
+  } else if (a.out && a.fold > 1) {
+    const unsigned grid = blocks((a.nwords + 63) / 64, a.c0);
+    if (a.nbits == 8) k_prep_fold<uint8_t><<<grid, 256, 0, st>>>(a);
     else k_prep_fold<uint16_t><<<grid, 256, 0, st>>>(a);
     DD_LAUNCHED();
-  } else if (a.out && !a.zdm_mean && a.nbits == 8 && a.ds == 1 && a.nchans % 4 == 0 && a.pitch % 4 == 0 &&
-      reinterpret_cast<uintptr_t>(a.x) % 4 == 0 && reinterpret_cast<uintptr_t>(a.out) % 4 == 0) {
-    const int64_t cw0 = a.c0 & ~int64_t(3);
-    const int64_t span = 64 * kPrepU8Subtiles;
-    dim3 grid(static_cast<unsigned>((a.nsamp + span - 1) / span), static_cast<unsigned>((a.c1 - cw0 + 63) / 64));
-    k_prep_u8<<<grid, 256, 0, st>>>(a);
-    DD_LAUNCHED();
-  } else if (a.out && !a.zdm_mean && a.nbits == 16 && a.ds == 1 && a.nchans % 4 == 0 && a.pitch % 4 == 0 &&
-             reinterpret_cast<uintptr_t>(a.x) % 8 == 0 && reinterpret_cast<uintptr_t>(a.out) % 8 == 0) {
-    const int64_t cw0 = a.c0 & ~int64_t(3);
-    dim3 grid(static_cast<unsigned>((a.nsamp + 63) / 64), static_cast<unsigned>((a.c1 - cw0 + 63) / 64));
-    k_prep_u16<<<grid, 256, 0, st>>>(a);
-    DD_LAUNCHED();
   } else if (a.out) {
-    dim3 grid(static_cast<unsigned>((a.nsamp + 63) / 64), static_cast<unsigned>((a.c1 - a.c0 + 63) / 64));
+    const unsigned grid = blocks((a.nsamp + 63) / 64, a.c0);
     switch (a.nbits) {
       case 8: k_prep<uint8_t><<<grid, 256, 0, st>>>(a); break;
       case 16: k_prep<uint16_t><<<grid, 256, 0, st>>>(a); break;
