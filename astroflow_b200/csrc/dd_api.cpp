@@ -52,19 +52,24 @@ int64_t round_up(int64_t v, int64_t m) { return (v + m - 1) / m * m; }
 int64_t inter_elem(const dd_plan& P) {
   return P.fold > 1 ? 4 : P.inter16 ? 2 : (P.nbits == 32 ? 8 : 4);
 }
+// Bytes of one output sum.
+int out_elem(const dd_plan& P) { return P.nbits == 32 ? 8 : 4; }
 // Bytes of one element of the prepared input.
 int64_t x_elem(const dd_plan& P) { return P.fold > 1 ? 4 : P.elem; }
 
 // Kernel variants of the two stages: 8-bit input in subbands of at most 64 channels
 // has 16-bit subband sums (packed planes when folded, else with a twin).
 int stage1_kind(const dd_plan& P) {
+  if (P.nbits == 32) return kSumKindWord64;
   if (P.fold > 1) return P.nbits == 16 ? kSumKindFold16 : P.inter16 ? kSumKindFold8 : kSumKindFold8W;
   return P.nbits == 16 ? kSumKindU16Wide : P.inter16 ? kSumKindU8Out16 : kSumKindU8Flush;
 }
 int stage2_kind(const dd_plan& P) {
+  if (P.nbits == 32) return kSumKindPlane64;
   return !P.inter16 ? kSumKindPlane32 : P.fold > 1 ? kSumKindPlane16 : kSumKindU16Twin;
 }
 int brute_kind(const dd_plan& P) {
+  if (P.nbits == 32) return kSumKindWord64;
   if (P.p.time_downsample > 1) return P.nbits == 16 ? kSumKindU16Phase : kSumKindU8Phase;
   if (P.fold > 1) return P.nbits == 16 ? kSumKindFold16 : kSumKindFold8W;
   return P.nbits == 16 ? kSumKindU16Wide : kSumKindU8Flush;
@@ -448,7 +453,7 @@ void create_subband(dd_plan& P) {
   P.inter16 = (P.nbits == 8 && P.sbw <= 64) ? 1 : 0;
   P.adds = static_cast<double>(P.ndm_nom) * P.dch * P.nout +
            static_cast<double>(P.dm_steps) * P.nsb * P.nout;
-  if (P.nbits <= 16) {
+  {
     std::vector<int32_t> skew;
     const std::vector<int32_t> tab = skew_stage1(P, skew);
     int spread1 = 0, spread2 = 0;
@@ -534,7 +539,7 @@ void set_brute_window(dd_plan& P) {
   P.fold = 1;
   if (P.p.time_downsample > 1) {
     set_phase_window(P);
-  } else if (P.nbits <= 16) {
+  } else {
     const std::vector<SumDesc> desc = build_sum_desc(P.h_delay, P.dm_steps, P.nc, 0, &spread);
     auto set_window = [&](int fold) {
       P.fold = fold;
@@ -764,9 +769,9 @@ SumLaunch stage2_launch(const dd_plan& P, int64_t t0, void* output) {
   L.nrows_total = P.dm_steps;
   L.group = P.ndm0;
   L.out = static_cast<char*>(output);
-  L.out_pitch = P.nout * 4;
+  L.out_pitch = P.nout * out_elem(P);
   L.out_col0 = t0;
-  L.out_elem = 4;
+  L.out_elem = out_elem(P);
   L.ncols = std::min<int64_t>(P.tile, P.seg - t0);
   L.seg = P.seg;
   L.nout = P.nout;
@@ -863,9 +868,9 @@ SumLaunch brute_launch(const dd_plan& P, void* output) {
   L.nsrc_total = P.nc;
   L.nrows_total = P.dm_steps;
   L.out = static_cast<char*>(output);
-  L.out_pitch = P.out_cols * 4;
+  L.out_pitch = P.out_cols * out_elem(P);
   L.out_col0 = 0;
-  L.out_elem = 4;
+  L.out_elem = out_elem(P);
   L.ncols = P.seg;
   L.seg = P.seg;
   L.seg_stride = P.seg * 4;
@@ -1236,7 +1241,7 @@ int dd_plan_autotune(dd_plan* P, const void* input, void* output, int32_t reps, 
   if (!P || !input || !output || !report) { set_error("NULL argument"); return DD_ERR_INVALID; }
   return guarded([&] {
     DeviceGuard g(P->device);
-    if (P->p.algorithm != DD_ALGO_SUBBAND || !P->win1 || !P->win2)
+    if (P->p.algorithm != DD_ALGO_SUBBAND || P->nbits > 16 || !P->win1 || !P->win2)
       throw Error{DD_ERR_UNSUPPORTED, "autotuning covers the staged subband path"};
     if (reps < 1) throw Error{DD_ERR_INVALID, "reps must be >= 1"};
     cudaStream_t st = static_cast<cudaStream_t>(stream);

@@ -449,6 +449,7 @@ constexpr int kFold8RB = DD_FOLD8_RB, kFold8NW = DD_FOLD8_NW;
 constexpr int kFold8WRB = DD_FOLD8W_RB, kFold8WNW = DD_FOLD8W_NW;
 constexpr int kFold16RB = DD_FOLD16_RB, kFold16NW = DD_FOLD16_NW;
 constexpr int kPlane16RB = DD_PLANE16_RB, kPlane16NW = DD_PLANE16_NW;
+constexpr int kTo64RB = 2, kTo64NW = 16;
 constexpr int kPlane32RB = DD_PLANE32_RB, kPlane32NW = DD_PLANE32_NW;
 // Kernel variants of the staged sums.  Samples in time order: 8-bit into 16-bit sums
 // (U8Out16) or 32-bit sums (U8Flush), 16-bit into 32-bit sums (U16Wide), 16-bit subband
@@ -456,10 +457,12 @@ constexpr int kPlane32RB = DD_PLANE32_RB, kPlane32NW = DD_PLANE32_NW;
 // brute force (U8Phase, U16Phase).  Folded samples: 8-bit into
 // packed 16-bit planes (Fold8) or 32-bit sums (Fold8W), 16-bit into 32-bit sums
 // (Fold16), and stage 2 of packed planes (Plane16).  Stage 2 of 32-bit sums, folded or
-// not (Plane32).
+// not (Plane32).  32-bit samples into 64-bit sums and stage 2 of those (Word64, Plane64;
+// not in batched launches).
 enum SumKind { kSumKindU8Out16, kSumKindU8Flush, kSumKindU16Wide, kSumKindU16Twin,
                kSumKindU8Phase, kSumKindU16Phase, kSumKindFold8,
-               kSumKindFold8W, kSumKindFold16, kSumKindPlane16, kSumKindPlane32, kSumKinds };
+               kSumKindFold8W, kSumKindFold16, kSumKindPlane16, kSumKindPlane32, kSumKindWord64,
+               kSumKindPlane64, kSumKinds };
 int sum_kind(const SumLaunch& L);
 // Tile of a kernel variant: samples per block, or words for the folded sums and Plane32.
 inline int sum_kind_tile(int kind) {
@@ -473,6 +476,7 @@ inline int sum_kind_tile(int kind) {
     case kSumKindFold8W: return words(kFold8WRB, kFold8WNW);
     case kSumKindFold16: return words(kFold16RB, kFold16NW);
     case kSumKindPlane16: return words(kPlane16RB, kPlane16NW);
+    case kSumKindWord64: case kSumKindPlane64: return words(kTo64RB, kTo64NW);
     default: return words(kPlane32RB, kPlane32NW);
   }
 }
@@ -483,6 +487,7 @@ inline int sum_kind_qs(int kind) {
 // Bytes of a source element: samples, 16-bit sums or words.
 inline int sum_kind_elem(int kind) {
   return kind == kSumKindU8Out16 || kind == kSumKindU8Flush || kind == kSumKindU8Phase ? 1
+         : kind == kSumKindPlane64                                                       ? 8
          : kind >= kSumKindFold8                                                         ? 4 : 2;
 }
 // Shared memory of a launch (its variant's windows per stage, plus the variant's

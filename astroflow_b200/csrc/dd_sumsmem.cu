@@ -369,9 +369,11 @@ __device__ __forceinline__ void produce_twin(const Geo& g, Pipe& P, uint32_t* sw
 }
 
 // The same for sources of 32-bit words (folded samples and their sums), four per
-// stage: every offset is a whole word, so a row's offset needs no shift.
+// stage: every offset is a whole word, so a row's offset needs no shift.  EW words per
+// element: 1, or 2 for 64-bit sums (offsets and tile in elements).
+template <int EW>
 __device__ __forceinline__ void produce_words(const Geo& g, Pipe& P, uint32_t* sw, int ww, int zero_q,
-                                              int tile_words, const GroupDesc<4>& d, int q, int s, int lane) {
+                                              int tile, const GroupDesc<4>& d, int q, int s, int lane) {
   const int i = lane >> 4, r = lane & 15;
   uint32_t nbytes[2] = {0, 0};
   const char* gsrc[2] = {nullptr, nullptr};
@@ -382,11 +384,12 @@ __device__ __forceinline__ void produce_words(const Geo& g, Pipe& P, uint32_t* s
     int idx = zero_q;
     const int64_t e0 = g.base + d.lo[h];
     if (src < g.nsrc && e0 < g.valid) {
-      const int64_t a0 = e0 & ~int64_t(3);
-      idx = (4 * s + k) * ww + static_cast<int>(e0 - a0) + d.rel[h];
+      constexpr int kAlign = 4 / EW - 1;  // elements of a 16-byte unit, less one
+      const int64_t a0 = e0 & ~int64_t(kAlign);
+      idx = (4 * s + k) * ww + EW * (static_cast<int>(e0 - a0) + d.rel[h]);
       if (r == 0) {
-        nbytes[h] = static_cast<uint32_t>((e0 + d.span[h] + tile_words - a0 + 3) & ~int64_t(3)) * 4u;
-        gsrc[h] = g.src + static_cast<int64_t>(src) * g.src_pitch + 4 * a0;
+        nbytes[h] = static_cast<uint32_t>((e0 + d.span[h] + tile - a0 + kAlign) & ~int64_t(kAlign)) * 4u * EW;
+        gsrc[h] = g.src + static_cast<int64_t>(src) * g.src_pitch + 4 * EW * a0;
       }
     }
     P.row[s][r][k] = idx;
@@ -425,7 +428,8 @@ __device__ __forceinline__ void skip_empty_sources(const SumLaunch& L, Geo& g, P
 // QS sources once their windows are in shared memory, and setup() once the first
 // windows are on their way (SKIP: sources may lie past the chunk's end); false when the block has nothing to store (kModeTwin: each source is staged
 // with its shifted twin, see produce_twin; kModeWords: see produce_words; QS is 4 for
-// both; `tile` is in bytes, for kModeWords in words).  The warps take turns at
+// both; kModeDwords: the same for 64-bit elements; `tile` is in bytes, for words and
+// dwords in elements).  The warps take turns at
 // staging: warp q % kWarps stages group q, D groups before they are summed, and has
 // loaded the group's descriptors kWarps groups earlier, so that no warp carries the
 // staging beside its sums and none waits for a descriptor.  D leaves a stage of slack
@@ -434,7 +438,7 @@ __device__ __forceinline__ void skip_empty_sources(const SumLaunch& L, Geo& g, P
 // 1, 3.8 in stage 2): 4096 channels of 8 bits, 2^20 samples, 6001 trials took 66.2 +
 // 40.1 ms (stages 1 and 2) that way and 56.6 + 32.8 ms with turns; brute force over
 // 1024 channels, 2^17 samples, 1001 trials 10.8 and 8.5 ms.
-constexpr int kModePlain = 0, kModeTwin = 1, kModeWords = 2, kModePhase = 3;
+constexpr int kModePlain = 0, kModeTwin = 1, kModeWords = 2, kModePhase = 3, kModeDwords = 4;
 template <int SB, int QS, int MODE, bool SKIP, typename Setup, typename Body>
 __device__ __forceinline__ bool run_pipeline(const SumLaunch& L, Geo& g, Pipe& P,
                                              uint32_t* sw, int tile, Setup&& setup, Body&& body) {
@@ -473,8 +477,8 @@ __device__ __forceinline__ bool run_pipeline(const SumLaunch& L, Geo& g, Pipe& P
   auto stage_next = [&](int s) {
     if constexpr (MODE == kModeTwin)
       produce_twin(g, P, sw, ww, zero_q, tile, L.twin_off, desc, next, s, lane);
-    else if constexpr (MODE == kModeWords)
-      produce_words(g, P, sw, ww, zero_q, tile, desc, next, s, lane);
+    else if constexpr (MODE == kModeWords || MODE == kModeDwords)
+      produce_words<MODE == kModeDwords ? 2 : 1>(g, P, sw, ww, zero_q, tile, desc, next, s, lane);
     else if constexpr (MODE == kModePhase)
       produce_phases<SB>(L, g, P, sw, ww, zero_q, tile, desc, phase, next, s, lane);
     else
@@ -1034,6 +1038,59 @@ __device__ __forceinline__ void sum_plane32(const SumLaunch& L, uint3 blk, uint3
   }
 }
 
+// ------------------------------------------------------------------ 32-bit samples
+// Stage 1 and brute force of 32-bit samples into 64-bit sums (the reference's output type
+// for them), and stage 2 of those: words and dwords in time order, lanes own interleaved
+// elements.  Bound by the shared loads (4 or 8 bytes per addition).  1024 channels, 2^15
+// samples, 501 trials, whole run: 1784 us with direct loads of every row, 391 us staged.
+template <int RB, int NW, bool WIDE>
+__device__ __forceinline__ void sum_to64(const SumLaunch& L, uint3 blk, uint32_t* sw, Pipe& P) {
+  constexpr int kGroups = kSumRows / RB;
+  constexpr int kWarpsPerTile = kWarps / kGroups;
+  constexpr int T = kWarpsPerTile * 32 * NW;
+  Geo g = make_geo(L, T, blk);
+  if (g.nrows <= 0) return;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rbase = warp / kWarpsPerTile;
+  const int wbase = (warp % kWarpsPerTile) * 32 * NW + lane;
+  uint32_t act = 0;
+  unsigned long long acc[RB][NW];
+#pragma unroll
+  for (int r = 0; r < RB; ++r)
+#pragma unroll
+    for (int k = 0; k < NW; ++k) acc[r][k] = 0;
+  const bool ok = run_pipeline<4, 4, WIDE ? kModeDwords : kModeWords, !WIDE>(
+      L, g, P, sw, T, [&] { act = active_rows<RB, T>(g, rbase); }, [&](int s, const uint32_t* win) {
+    for_rows<RB>(act, [&](int r) {
+      const int4 a = row_info(P, s, rbase + kGroups * r);
+      const int at[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        if constexpr (WIDE) {
+          const unsigned long long* w = reinterpret_cast<const unsigned long long*>(win + at[i]) + wbase;
+#pragma unroll
+          for (int k = 0; k < NW; ++k) acc[r][k] += w[32 * k];
+        } else {
+          const uint32_t* w = win + at[i] + wbase;
+#pragma unroll
+          for (int k = 0; k < NW; ++k) acc[r][k] += w[32 * k];
+        }
+      }
+    });
+  });
+  if (!ok) return;
+#pragma unroll
+  for (int r = 0; r < RB; ++r) {
+    if (!(act >> r & 1u)) continue;
+    const int64_t c0 = row_col(g, rbase + kGroups * r) + wbase;
+    unsigned long long* out =
+        reinterpret_cast<unsigned long long*>(g.out + (rbase + kGroups * r) * g.out_pitch) + c0;
+#pragma unroll
+    for (int k = 0; k < NW; ++k)
+      if (c0 + 32 * k >= 0 && c0 + 32 * k < g.ncols) out[32 * k] = acc[r][k];
+  }
+}
+
 // ------------------------------------------------------------------ 16-bit sums with a shifted twin
 // Stage 2 of 8-bit input when stage 1 also wrote the one-sample-shifted twin of
 // its sums (SumLaunch::twin_off): a row whose offset for a source is odd reads
@@ -1136,6 +1193,12 @@ __global__ void __launch_bounds__(kThreads, DD_PLANE16_MINB) k_sum_plane16(SumLa
   extern __shared__ __align__(128) uint32_t sw[];
   __shared__ Pipe P;
   sum_plane16<RB, NW>(L, blockIdx, sw, P);
+}
+template <int RB, int NW, bool WIDE>
+__global__ void __launch_bounds__(kThreads, 2) k_sum_to64(SumLaunch L) {
+  extern __shared__ __align__(128) uint32_t sw[];
+  __shared__ Pipe P;
+  sum_to64<RB, NW, WIDE>(L, blockIdx, sw, P);
 }
 template <int RB, int NW>
 __global__ void __launch_bounds__(kThreads, DD_PLANE32_MINB) k_sum_plane32(SumLaunch L) {
@@ -1372,6 +1435,8 @@ void launch_sum(const SumLaunch& L, cudaStream_t st) {
     case kSumKindU16Twin: launch_k(k_sum_u16t<kSumRowsPTT, kSum16TNW>, grid, smem, L, st); break;
     case kSumKindU8Phase: launch_k(k_sum_u8<kSumRowsPT8, DD_SUM8_NW, false, kModePhase>, grid, smem, L, st); break;
     case kSumKindU16Phase: launch_k(k_sum_u16w<kSumRowsPTW, DD_SUM16W_NW, kModePhase>, grid, smem, L, st); break;
+    case kSumKindWord64: launch_k(k_sum_to64<kTo64RB, kTo64NW, false>, grid, smem, L, st); break;
+    case kSumKindPlane64: launch_k(k_sum_to64<kTo64RB, kTo64NW, true>, grid, smem, L, st); break;
     case kSumKindFold8: launch_k(k_sum_fold8<kFold8RB, kFold8NW, true>, grid, smem, L, st); break;
     case kSumKindFold8W: launch_k(k_sum_fold8<kFold8WRB, kFold8WNW, false>, grid, smem, L, st); break;
     case kSumKindFold16: launch_k(k_sum_fold16<kFold16RB, kFold16NW>, grid, smem, L, st); break;

@@ -138,3 +138,34 @@ def test_batch_of_all_layouts_equals_oracle(persistent):
     batch.status()
     for o, (_, _, want) in zip(outs, got):
         assert np.array_equal(to_np(o), want)
+
+
+@pytest.mark.parametrize("n,nchans,hi,step,ds,width", [
+    (511, 37, 100.0, 0.5, 1, 16), (513, 64, 300.0, 0.5, 1, 9), (2049, 130, 60.0, 0.3, 1, 64),
+    (1027, 64, 3000.0, 100.0, 1, 32), (3001, 40, 200.0, 1.0, 2, 8), (70001, 16, 100.0, 4.0, 1, 8),
+])
+def test_32bit_sums_equal_oracle(n, nchans, hi, step, ds, width):
+    rng = np.random.default_rng(n)
+    x = rng.integers(0, 2 ** 32, size=(n, nchans), dtype=np.uint64).astype(np.uint32)
+    x[rng.random(x.shape) < 0.9] = 2 ** 32 - 1
+    xd = torch.from_numpy(x.view(np.int32)).cuda().view(torch.uint32)
+    foff = float(F32(300.0 / nchans))
+    hdr = dict(tsamp=float(F32(64e-6)), fch1=1150.0, foff=foff, nbits=32, nchans=nchans, ndata=n)
+    freq = O.freq_table_header(hdr["fch1"], hdr["foff"], nchans)
+    fs, fe = float(F32(freq[0])), float(F32(freq[-1]))
+    plan = Plan(hdr, 0.0, hi, fs, fe, step, ds, algorithm="subband", subband_width=width)
+    ref = O.time_binning(x.copy(), nchans, ds) if ds > 1 else x
+    op = O.subband_plan(freq, n, 0.0, hi, fs, fe, step, ds, sb_width=width)
+    want = O.subband_sums(ref, nchans, op, *plan.tables())
+    got = plan.run(xd).view(torch.int64).cpu().numpy().view(np.uint64)
+    assert np.array_equal(got, want)
+    if ds > 1:
+        return
+    filfreq = O.freq_table_fil(1150.0, 300.0 / nchans, nchans)
+    bs, be = float(F32(filfreq[0])), float(F32(filfreq[-1]))
+    ts = n * 64e-6 * 0.49
+    bp = Plan(dict(hdr, tsamp=64e-6, foff=300.0 / nchans), 0.0, hi, bs, be, step, 1, ts,
+              algorithm="brute", freq_mode="fil")
+    bw = np.concatenate(O.bruteforce_cpu(x, nchans, filfreq, 64e-6, 0.0, hi, bs, be, step, 1, ts,
+                                         delay=bp.tables()[0]), axis=1)
+    assert np.array_equal(bp.run(xd).view(torch.int64).cpu().numpy().view(np.uint64), bw)
