@@ -61,17 +61,24 @@ int64_t x_elem(const dd_plan& P) { return P.fold > 1 ? 4 : P.elem; }
 // has 16-bit subband sums (packed planes when folded, else with a twin).
 int stage1_kind(const dd_plan& P) {
   if (P.nbits == 32) return kSumKindWord64;
-  if (P.fold > 1) return P.nbits == 16 ? kSumKindFold16 : P.inter16 ? kSumKindFold8 : kSumKindFold8W;
+  if (P.fold > 1) {
+    const int k = P.nbits == 16 ? kSumKindFold16 : P.inter16 ? kSumKindFold8 : kSumKindFold8W;
+    return P.small1 ? sum_kind_small(k) : k;
+  }
   return P.nbits == 16 ? kSumKindU16Wide : P.inter16 ? kSumKindU8Out16 : kSumKindU8Flush;
 }
 int stage2_kind(const dd_plan& P) {
   if (P.nbits == 32) return kSumKindPlane64;
-  return !P.inter16 ? kSumKindPlane32 : P.fold > 1 ? kSumKindPlane16 : kSumKindU16Twin;
+  const int k = !P.inter16 ? kSumKindPlane32 : P.fold > 1 ? kSumKindPlane16 : kSumKindU16Twin;
+  return P.small2 ? sum_kind_small(k) : k;
 }
 int brute_kind(const dd_plan& P) {
   if (P.nbits == 32) return kSumKindWord64;
   if (P.p.time_downsample > 1) return P.nbits == 16 ? kSumKindU16Phase : kSumKindU8Phase;
-  if (P.fold > 1) return P.nbits == 16 ? kSumKindFold16 : kSumKindFold8W;
+  if (P.fold > 1) {
+    const int k = P.nbits == 16 ? kSumKindFold16 : kSumKindFold8W;
+    return P.smallb ? sum_kind_small(k) : k;
+  }
   return P.nbits == 16 ? kSumKindU16Wide : kSumKindU8Flush;
 }
 // Samples per folded word, or 1 where the fold does not pay.  A folded word holds the
@@ -463,6 +470,13 @@ void create_subband(dd_plan& P) {
     auto set_windows = [&](int fold) {
       P.fold = fold;
       P.planes = fold == 1 ? 1 : P.inter16 ? 2 : fold;
+      // blocks of one time tile with whole tiles of words
+      P.small1 = P.small2 = false;
+      const int64_t cols = (P.nout + fold - 1) / fold / (P.nout >= 65536 ? 2 : 1);
+      const auto blocks = [&](int kind, int64_t c) { return (c + sum_kind_tile(kind) - 1) / sum_kind_tile(kind); };
+      const int64_t groups1 = (P.ndm_nom + kSumRows - 1) / kSumRows, groups2 = P.ndm_nom * ((P.ndm0 + kSumRows - 1) / kSumRows);
+      P.small1 = blocks(stage1_kind(P), cols + P.max_res + P.max_skew1 / 2) * groups1 * P.nsb < kSumSmallBlocks;
+      P.small2 = blocks(stage2_kind(P), cols) * groups2 * P.planes < kSumSmallBlocks;
       const int k1 = stage1_kind(P), k2 = stage2_kind(P);
       P.win1 = window_bytes(spread1, sum_kind_tile(k1), sum_kind_elem(k1), sum_kind_qs(k1));
       P.win2 = window_bytes(spread2, sum_kind_tile(k2), sum_kind_elem(k2), sum_kind_qs(k2));
@@ -543,6 +557,9 @@ void set_brute_window(dd_plan& P) {
     const std::vector<SumDesc> desc = build_sum_desc(P.h_delay, P.dm_steps, P.nc, 0, &spread);
     auto set_window = [&](int fold) {
       P.fold = fold;
+      P.smallb = false;
+      const int64_t cols = (P.out_cols + fold - 1) / fold, tile = sum_kind_tile(brute_kind(P));
+      P.smallb = (cols + tile - 1) / tile * ((P.dm_steps + kSumRows - 1) / kSumRows) < kSumSmallBlocks;
       const int k = brute_kind(P);
       P.winb = window_bytes(spread, sum_kind_tile(k), sum_kind_elem(k), sum_kind_qs(k));
     };
@@ -1851,8 +1868,10 @@ struct dd_stream {
   int device = 0;
   int64_t chunk = 0, tail = 0, buf_len = 0;  // input samples
   int64_t row_bytes = 0;                     // bytes per input sample (all channels)
-  dd::DevBuf buf[2];
-  int cur = 0;
+  // [samples][channels], 2 * buf_len samples: the tail of the next push starts at sample
+  // pos and its chunk follows; at the end of the buffer the tail is copied to the front.
+  dd::DevBuf buf;
+  int64_t pos = 0;
   int64_t pushed = 0;
 };
 
@@ -1884,10 +1903,8 @@ int dd_stream_open(const dd_header* header, const dd_plan_params* params, const 
     dd_header h = *header;
     h.ndata = S->buf_len;
     S->plan = make_plan(&h, params, rfi, bad_channels, n_bad, device, S->chunk / ds);
-    for (int b = 0; b < 2; ++b) {
-      S->buf[b].alloc(static_cast<size_t>(S->buf_len * S->row_bytes));
-      DD_CUDA_TRY(cudaMemsetAsync(S->buf[b].p, 0, S->buf[b].bytes, cudaStreamLegacy));
-    }
+    S->buf.alloc(static_cast<size_t>(2 * S->buf_len * S->row_bytes));
+    DD_CUDA_TRY(cudaMemsetAsync(S->buf.p, 0, S->buf.bytes, cudaStreamLegacy));
     DD_CUDA_TRY(cudaStreamSynchronize(cudaStreamLegacy));
   });
   if (rc != DD_OK) {
@@ -1907,18 +1924,22 @@ int dd_stream_push(dd_stream* S, const void* chunk, void* output, void* stream) 
   return guarded([&] {
     DeviceGuard g(S->device);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    char* cur = static_cast<char*>(S->buf[S->cur].p);
-    char* nxt = static_cast<char*>(S->buf[S->cur ^ 1].p);
+    char* buf = static_cast<char*>(S->buf.p);
+    if (S->pos + S->buf_len > 2 * S->buf_len) {
+      // the tail moves to the front once in tail/chunk + 2 pushes (pos > buf_len: the two
+      // places do not overlap); copied on every push it took a tenth of a 0.5 s chunk's time
+      if (S->tail)
+        DD_CUDA_TRY(cudaMemcpyAsync(buf, buf + S->pos * S->row_bytes,
+                                    static_cast<size_t>(S->tail * S->row_bytes),
+                                    cudaMemcpyDeviceToDevice, st));
+      S->pos = 0;
+    }
+    char* cur = buf + S->pos * S->row_bytes;
     DD_CUDA_TRY(cudaMemcpyAsync(cur + S->tail * S->row_bytes, chunk,
                                 static_cast<size_t>(S->chunk * S->row_bytes),
                                 cudaMemcpyDeviceToDevice, st));
     run_subband(*S->plan, cur, output, nullptr, nullptr, nullptr, st);
-    // the next buffer starts with this buffer's last `tail` samples
-    if (S->tail)
-      DD_CUDA_TRY(cudaMemcpyAsync(nxt, cur + S->chunk * S->row_bytes,
-                                  static_cast<size_t>(S->tail * S->row_bytes),
-                                  cudaMemcpyDeviceToDevice, st));
-    S->cur ^= 1;
+    S->pos += S->chunk;
     S->pushed += S->chunk;
   });
 }
@@ -1931,7 +1952,7 @@ int dd_stream_get_info(const dd_stream* S, dd_stream_info* info) {
   o.chunk_samples = S->chunk;
   o.tail_samples = S->tail;
   o.pushed_samples = S->pushed;
-  o.workspace_bytes = workspace_of(*S->plan) + static_cast<int64_t>(S->buf[0].bytes + S->buf[1].bytes);
+  o.workspace_bytes = workspace_of(*S->plan) + static_cast<int64_t>(S->buf.bytes);
   o.adds_per_push = S->plan->adds;
   *info = o;
   return DD_OK;

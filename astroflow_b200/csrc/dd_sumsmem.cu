@@ -1247,6 +1247,11 @@ __device__ __forceinline__ void run_one(const SumLaunch& L, uint3 blk, uint32_t*
   else if constexpr (KIND == kSumKindFold8W) sum_fold8<kFold8WRB, kFold8WNW, false>(L, blk, sw, P);
   else if constexpr (KIND == kSumKindFold16) sum_fold16<kFold16RB, kFold16NW>(L, blk, sw, P);
   else if constexpr (KIND == kSumKindPlane16) sum_plane16<kPlane16RB, kPlane16NW>(L, blk, sw, P);
+  else if constexpr (KIND == kSumKindFold8S) sum_fold8<kFold8RB, kFold8NW / 2, true>(L, blk, sw, P);
+  else if constexpr (KIND == kSumKindFold8WS) sum_fold8<kFold8WRB, kFold8WNW / 2, false>(L, blk, sw, P);
+  else if constexpr (KIND == kSumKindFold16S) sum_fold16<kFold16RB, kFold16NW / 2>(L, blk, sw, P);
+  else if constexpr (KIND == kSumKindPlane16S) sum_plane16<kPlane16RB, kPlane16NW / 2>(L, blk, sw, P);
+  else if constexpr (KIND == kSumKindPlane32S) sum_plane32<kPlane32RB, kPlane32NW / 2>(L, blk, sw, P);
   else sum_plane32<kPlane32RB, kPlane32NW>(L, blk, sw, P);
 }
 
@@ -1284,6 +1289,11 @@ __device__ __forceinline__ void run_kind(int kind, const SumLaunch& L, uint3 blk
     case kSumKindFold8W: run_one<kSumKindFold8W>(L, blk, sw, P); break;
     case kSumKindFold16: run_one<kSumKindFold16>(L, blk, sw, P); break;
     case kSumKindPlane16: run_one<kSumKindPlane16>(L, blk, sw, P); break;
+    case kSumKindFold8S: run_one<kSumKindFold8S>(L, blk, sw, P); break;
+    case kSumKindFold8WS: run_one<kSumKindFold8WS>(L, blk, sw, P); break;
+    case kSumKindFold16S: run_one<kSumKindFold16S>(L, blk, sw, P); break;
+    case kSumKindPlane16S: run_one<kSumKindPlane16S>(L, blk, sw, P); break;
+    case kSumKindPlane32S: run_one<kSumKindPlane32S>(L, blk, sw, P); break;
     default: run_one<kSumKindPlane32>(L, blk, sw, P); break;
   }
 }
@@ -1441,6 +1451,11 @@ void launch_sum(const SumLaunch& L, cudaStream_t st) {
     case kSumKindFold8W: launch_k(k_sum_fold8<kFold8WRB, kFold8WNW, false>, grid, smem, L, st); break;
     case kSumKindFold16: launch_k(k_sum_fold16<kFold16RB, kFold16NW>, grid, smem, L, st); break;
     case kSumKindPlane16: launch_k(k_sum_plane16<kPlane16RB, kPlane16NW>, grid, smem, L, st); break;
+    case kSumKindFold8S: launch_k(k_sum_fold8<kFold8RB, kFold8NW / 2, true>, grid, smem, L, st); break;
+    case kSumKindFold8WS: launch_k(k_sum_fold8<kFold8WRB, kFold8WNW / 2, false>, grid, smem, L, st); break;
+    case kSumKindFold16S: launch_k(k_sum_fold16<kFold16RB, kFold16NW / 2>, grid, smem, L, st); break;
+    case kSumKindPlane16S: launch_k(k_sum_plane16<kPlane16RB, kPlane16NW / 2>, grid, smem, L, st); break;
+    case kSumKindPlane32S: launch_k(k_sum_plane32<kPlane32RB, kPlane32NW / 2>, grid, smem, L, st); break;
     default: launch_k(k_sum_plane32<kPlane32RB, kPlane32NW>, grid, smem, L, st); break;
   }
 }
@@ -1488,6 +1503,11 @@ void launch_sum_grouped(const SumBatchGroup* d_groups, int ngroups, long long to
     case kSumKindFold8W: launch_grouped_k<kSumKindFold8W>(d_groups, ngroups, total, smem, st); break;
     case kSumKindFold16: launch_grouped_k<kSumKindFold16>(d_groups, ngroups, total, smem, st); break;
     case kSumKindPlane16: launch_grouped_k<kSumKindPlane16>(d_groups, ngroups, total, smem, st); break;
+    case kSumKindFold8S: launch_grouped_k<kSumKindFold8S>(d_groups, ngroups, total, smem, st); break;
+    case kSumKindFold8WS: launch_grouped_k<kSumKindFold8WS>(d_groups, ngroups, total, smem, st); break;
+    case kSumKindFold16S: launch_grouped_k<kSumKindFold16S>(d_groups, ngroups, total, smem, st); break;
+    case kSumKindPlane16S: launch_grouped_k<kSumKindPlane16S>(d_groups, ngroups, total, smem, st); break;
+    case kSumKindPlane32S: launch_grouped_k<kSumKindPlane32S>(d_groups, ngroups, total, smem, st); break;
     default: launch_grouped_k<kSumKindPlane32>(d_groups, ngroups, total, smem, st); break;
   }
 }
