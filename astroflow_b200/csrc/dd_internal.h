@@ -397,6 +397,13 @@ constexpr int kErrWaitEmpty = 2;  // the producer gave up waiting for a free sta
 #define DD_SUM16T_NW 6
 #endif
 constexpr int kSum16TNW = DD_SUM16T_NW;
+#ifndef DD_PHASE8_NW
+#define DD_PHASE8_NW 7
+#endif
+// Downsampled brute force: slices of half a second are a few thousand columns, so a block
+// tile takes fewer words than the chunk-long sums (1000 channels, 61,441 samples, bins of
+// two, 501 trials: 5 / 7 / 9 words 1.31 / 1.19 / 1.46 ms).
+constexpr int kPhase8NW = DD_PHASE8_NW;
 // Folded sums: rows per thread, words per lane and blocks per SM.  Few rows of many
 // words: a row of a stage costs one load of its offsets and four addresses whatever its
 // words.  Measured (4096 channels, 2^17 samples, 6001 trials, stage 1 / stage 2, ms; and
@@ -478,7 +485,8 @@ int sum_kind(const SumLaunch& L);
 inline int sum_kind_tile(int kind) {
   const auto words = [](int rb, int nw) { return sum_tile_samples(4, nw) * rb / kSumRows; };
   switch (kind) {
-    case kSumKindU8Out16: case kSumKindU8Flush: case kSumKindU8Phase:
+    case kSumKindU8Phase: return sum_tile_samples(1, kPhase8NW) * kSumRowsPT8 / kSumRows;
+    case kSumKindU8Out16: case kSumKindU8Flush:
       return sum_tile_samples(1, DD_SUM8_NW) * kSumRowsPT8 / kSumRows;
     case kSumKindU16Wide: case kSumKindU16Phase: return sum_tile_samples(2, DD_SUM16W_NW) * kSumRowsPTW / kSumRows;
     case kSumKindU16Twin: return sum_tile_samples(2, kSum16TNW) * kSumRowsPTT / kSumRows;

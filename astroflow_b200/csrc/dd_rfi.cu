@@ -716,16 +716,23 @@ __global__ void __launch_bounds__(256) k_prep_fold(PrepArgs a) {
 // words are read from c0 & ~3.  Bound by issue (80 % busy) beside the memory: row
 // pointers and counts are set up once per thread, the tile comes from one 32-bit
 // division, and nothing is 64-bit per load.  4096 channels x 151,000 samples in time
-// order 257 us (4.8 TB/s; 480 us with four loads in flight per thread and 64-bit rows),
-// 131,072 samples folded 905 us (3.9 TB/s).
+// order 216 us (5.7 TB/s; 480 us with four loads in flight per thread and 64-bit rows),
+// 131,072 samples folded 690 us (5.1 TB/s; 905 us with every load and store predicated
+// and two-way bank conflicts).  The phase rows of downsampled brute force are laid out
+// by one launch per phase (t0 the phase, strides times ds, WS 0: taken from ws).
 struct PrepWords {
   int64_t fs, nwords, pitch;  // nwords: words to store per channel; pitch in words
+  int ws;
+  int64_t t0;
 };
 template <typename T, int WS>
-__global__ void __launch_bounds__(256, 6) k_prep_w(PrepArgs a, PrepWords q) {
+__global__ void __launch_bounds__(256, sizeof(T) == 1 && WS == 1 ? 5 : 6) k_prep_w(PrepArgs a, PrepWords q) {
   constexpr int F = 4 / sizeof(T);   // samples per word
+  const int ws = WS ? WS : q.ws;
   constexpr int V = sizeof(T);       // 32-bit words per four channels
-  __shared__ uint32_t tile[64][65];  // [channel][word]
+  // [16 * b + w][word] for channel 4w + b: with 66 words a row, the 16 channel groups and
+  // two words that a warp stores at a time fall into 32 banks
+  __shared__ uint32_t tile[64][66];
   int64_t group;
   const int64_t sb = prep_tile(a, a.c0 & ~int64_t(3), &group) * 64;
   const int64_t cb = (a.c0 & ~int64_t(3)) + group * 64;
@@ -756,15 +763,15 @@ __global__ void __launch_bounds__(256, 6) k_prep_w(PrepArgs a, PrepWords q) {
   bool mixed = false;
 #pragma unroll
   for (int f = 0; f < F; ++f) {
-    const int64_t t0 = WS * sb + q.fs * f;
-    src[f] = static_cast<const T*>(a.x) + (t0 + WS * r0) * a.nchans + c;
-    const int64_t left = a.nsamp - t0;  // words i with WS * i < left
-    have[f] = !cvalid || left <= 0 ? 0 : left >= WS * 64 ? 64 : (static_cast<int>(left) + WS - 1) / WS;
+    const int64_t t0 = q.t0 + ws * sb + q.fs * f;
+    src[f] = static_cast<const T*>(a.x) + (t0 + ws * r0) * a.nchans + c;
+    const int64_t left = a.nsamp - t0;  // words i with ws * i < left
+    have[f] = !cvalid || left <= 0 ? 0 : left >= ws * 64 ? 64 : (static_cast<int>(left) + ws - 1) / ws;
 #pragma unroll
     for (int v = 0; v < V; ++v) mask[f][v] = keep[v];
     if (a.segmask && have[f]) {
       const int sg = find_seg(a.seg_t0, a.nseg, t0);
-      mixed |= sg + 1 < a.nseg && static_cast<int64_t>(a.seg_t0[sg + 1]) <= t0 + WS * 63;
+      mixed |= sg + 1 < a.nseg && static_cast<int64_t>(a.seg_t0[sg + 1]) <= t0 + ws * 63;
       const uint32_t m4 = ~__vcmpne4(*reinterpret_cast<const uint32_t*>(
                                          a.segmask + static_cast<int64_t>(sg) * a.nchans + c), 0u);
       if constexpr (V == 1) {
@@ -775,30 +782,38 @@ __global__ void __launch_bounds__(256, 6) k_prep_w(PrepArgs a, PrepWords q) {
       }
     }
   }
-  const int64_t step = 16 * WS * a.nchans;
+  const int64_t step = static_cast<int64_t>(16 * ws) * a.nchans;
   uint32_t in[4][F][V];
 #pragma unroll
-  for (int k = 0; k < 4; ++k)
+  for (int f = 0; f < F; ++f) {
+    auto load = [&](int k) {
+      if constexpr (V == 1) {
+        in[k][f][0] = __ldg(reinterpret_cast<const uint32_t*>(src[f] + k * step));
+      } else {
+        const uint2 u = __ldg(reinterpret_cast<const uint2*>(src[f] + k * step));
+        in[k][f][0] = u.x;
+        in[k][f][V - 1] = u.y;
+      }
+    };
+    if (have[f] == 64) {  // (all tiles but a slot's last)
 #pragma unroll
-    for (int f = 0; f < F; ++f) {
+      for (int k = 0; k < 4; ++k) load(k);
+    } else {
 #pragma unroll
-      for (int v = 0; v < V; ++v) in[k][f][v] = 0;
-      if (r0 + 16 * k < have[f]) {
-        if constexpr (V == 1) {
-          in[k][f][0] = __ldg(reinterpret_cast<const uint32_t*>(src[f] + k * step));
-        } else {
-          const uint2 u = __ldg(reinterpret_cast<const uint2*>(src[f] + k * step));
-          in[k][f][0] = u.x;
-          in[k][f][V - 1] = u.y;
-        }
+      for (int k = 0; k < 4; ++k) {
+#pragma unroll
+        for (int v = 0; v < V; ++v) in[k][f][v] = 0;
+        if (r0 + 16 * k < have[f]) load(k);
       }
     }
+  }
+  if (a.segmask && mixed) {  // rows of several IQRM segments: one by one
 #pragma unroll
-  for (int k = 0; k < 4; ++k) {
+    for (int k = 0; k < 4; ++k)
 #pragma unroll
-    for (int f = 0; f < F; ++f) {
-      if (mixed && r0 + 16 * k < have[f]) {  // rows of several IQRM segments: one by one
-        const int64_t t = WS * (sb + r0 + 16 * k) + q.fs * f;
+      for (int f = 0; f < F; ++f) {
+        if (r0 + 16 * k >= have[f]) continue;
+        const int64_t t = q.t0 + ws * (sb + r0 + 16 * k) + q.fs * f;
         const uint32_t m4 = ~__vcmpne4(*reinterpret_cast<const uint32_t*>(
                                            a.segmask + static_cast<int64_t>(find_seg(a.seg_t0, a.nseg, t)) * a.nchans + c), 0u);
         if constexpr (V == 1) {
@@ -807,12 +822,22 @@ __global__ void __launch_bounds__(256, 6) k_prep_w(PrepArgs a, PrepWords q) {
           in[k][f][0] &= __byte_perm(m4, 0u, 0x1100) & keep[0];
           in[k][f][V - 1] &= __byte_perm(m4, 0u, 0x3322) & keep[V - 1];
         }
-      } else {
+      }
+  } else if (a.segmask || a.keep) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+#pragma unroll
+      for (int f = 0; f < F; ++f)
 #pragma unroll
         for (int v = 0; v < V; ++v) in[k][f][v] &= mask[f][v];
-      }
-      if (a.zdm_off && r0 + 16 * k < have[f]) {
-        const uint32_t off = a.zdm_off[WS * (sb + r0 + 16 * k) + q.fs * f];
+  }
+  if (a.zdm_off) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+#pragma unroll
+      for (int f = 0; f < F; ++f) {
+        if (r0 + 16 * k >= have[f]) continue;
+        const uint32_t off = a.zdm_off[q.t0 + ws * (sb + r0 + 16 * k) + q.fs * f];
 #pragma unroll
         for (int v = 0; v < V; ++v) {
           const uint32_t u = in[k][f][v];
@@ -821,7 +846,9 @@ __global__ void __launch_bounds__(256, 6) k_prep_w(PrepArgs a, PrepWords q) {
           in[k][f][v] = (d & inrange[v]) | (u & ~inrange[v]);
         }
       }
-    }
+  }
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
     uint32_t o[4];
     if constexpr (V == 1) {
       const uint32_t v0 = in[k][0][0], v1 = in[k][1][0], v2 = in[k][F - 2][0], v3 = in[k][F - 1][0];
@@ -838,19 +865,28 @@ __global__ void __launch_bounds__(256, 6) k_prep_w(PrepArgs a, PrepWords q) {
       o[3] = __byte_perm(in[k][0][V - 1], in[k][1][V - 1], 0x7632);
     }
 #pragma unroll
-    for (int b = 0; b < 4; ++b) tile[4 * w + b][r0 + 16 * k] = o[b];
+    for (int b = 0; b < 4; ++b) tile[16 * b + w][r0 + 16 * k] = o[b];
   }
   __syncthreads();
+  // a warp stores channels row, row + 8, ... of the tile, 64 words each
   const int lane = threadIdx.x & 31, row = threadIdx.x >> 5;
-  const int64_t words = q.nwords - sb;
-  const int64_t pitch = q.pitch;
-  uint32_t* dst = static_cast<uint32_t*>(a.out) + (cb + row - a.c0) * pitch + sb + lane;
+  const int words = static_cast<int>(min(q.nwords - sb, static_cast<int64_t>(64)));
+  const int ch0 = static_cast<int>(max(a.c0 - cb, static_cast<int64_t>(0)));
+  const int ch1 = static_cast<int>(min(a.c1 - cb, static_cast<int64_t>(64)));
+  uint32_t* dst = static_cast<uint32_t*>(a.out) + (cb + row - a.c0) * q.pitch + sb + lane;
+  const uint32_t* from = &tile[16 * (row & 3) + (row >> 2)][lane];
+  if (words == 64 && ch0 == 0 && ch1 == 64) {
 #pragma unroll
-  for (int r = 0; r < 64; r += 8, dst += 8 * pitch) {
-    const int64_t cc = cb + row + r;
-    if (cc < a.c0 || cc >= a.c1) continue;
-    if (lane < words) dst[0] = tile[row + r][lane];
-    if (lane + 32 < words) dst[32] = tile[row + r][lane + 32];
+    for (int r = 0; r < 8; ++r, dst += 8 * q.pitch) {
+      dst[0] = from[2 * r * 66];
+      dst[32] = from[2 * r * 66 + 32];
+    }
+    return;
+  }
+  for (int r = 0; r < 8; ++r, dst += 8 * q.pitch) {
+    if (row + 8 * r < ch0 || row + 8 * r >= ch1) continue;
+    if (lane < words) dst[0] = from[2 * r * 66];
+    if (lane + 32 < words) dst[32] = from[2 * r * 66 + 32];
   }
 }
 
@@ -1036,8 +1072,21 @@ void launch_prep(const PrepArgs& a, cudaStream_t st) {
   const int F = a.nbits == 8 ? 4 : 2;
   const bool wide = a.out && a.nbits <= 16 && !a.zdm_mean && a.nchans % 4 == 0 &&
                     reinterpret_cast<uintptr_t>(a.x) % (a.nbits / 2) == 0;
-  if (wide && (a.fold > 1 || (a.ds == 1 && a.pitch % F == 0 && reinterpret_cast<uintptr_t>(a.out) % 4 == 0))) {
-    const PrepWords q = a.fold > 1 ? PrepWords{a.seg, a.nwords, a.pitch} : PrepWords{1, (a.nsamp + F - 1) / F, a.pitch / F};
+  if (wide && a.ds > 1 && a.ds <= 16 && a.pitch % F == 0 && reinterpret_cast<uintptr_t>(a.out) % 4 == 0) {
+    for (int ph = 0; ph < a.ds; ++ph) {
+      PrepArgs p = a;
+      p.out = static_cast<char*>(a.out) + ph * a.pitch * (a.nbits / 8);
+      const int64_t rows = (a.nsamp - ph + a.ds - 1) / a.ds;
+      if (rows <= 0) continue;
+      const PrepWords q{a.ds, (rows + F - 1) / F, a.ds * (a.pitch / F), F * a.ds, ph};
+      const unsigned grid = blocks((q.nwords + 63) / 64, a.c0 & ~int64_t(3));
+      if (a.nbits == 8) k_prep_w<uint8_t, 0><<<grid, 256, 0, st>>>(p, q);
+      else k_prep_w<uint16_t, 0><<<grid, 256, 0, st>>>(p, q);
+      DD_LAUNCHED();
+    }
+  } else if (wide && (a.fold > 1 || (a.ds == 1 && a.pitch % F == 0 && reinterpret_cast<uintptr_t>(a.out) % 4 == 0))) {
+    const PrepWords q = a.fold > 1 ? PrepWords{a.seg, a.nwords, a.pitch, 1, 0}
+                                   : PrepWords{1, (a.nsamp + F - 1) / F, a.pitch / F, F, 0};
     const unsigned grid = blocks((q.nwords + 63) / 64, a.c0 & ~int64_t(3));
     if (a.nbits == 8 && a.fold > 1) k_prep_w<uint8_t, 1><<<grid, 256, 0, st>>>(a, q);
     else if (a.nbits == 8) k_prep_w<uint8_t, 4><<<grid, 256, 0, st>>>(a, q);

@@ -1241,7 +1241,7 @@ __device__ __forceinline__ void run_one(const SumLaunch& L, uint3 blk, uint32_t*
   else if constexpr (KIND == kSumKindU8Flush) sum_u8<kSumRowsPT8, DD_SUM8_NW, false>(L, blk, sw, P);
   else if constexpr (KIND == kSumKindU16Wide) sum_u16_wide<kSumRowsPTW, DD_SUM16W_NW>(L, blk, sw, P);
   else if constexpr (KIND == kSumKindU16Twin) sum_u16_twin<kSumRowsPTT, kSum16TNW>(L, blk, sw, P);
-  else if constexpr (KIND == kSumKindU8Phase) sum_u8<kSumRowsPT8, DD_SUM8_NW, false, kModePhase>(L, blk, sw, P);
+  else if constexpr (KIND == kSumKindU8Phase) sum_u8<kSumRowsPT8, kPhase8NW, false, kModePhase>(L, blk, sw, P);
   else if constexpr (KIND == kSumKindU16Phase) sum_u16_wide<kSumRowsPTW, DD_SUM16W_NW, kModePhase>(L, blk, sw, P);
   else if constexpr (KIND == kSumKindFold8) sum_fold8<kFold8RB, kFold8NW, true>(L, blk, sw, P);
   else if constexpr (KIND == kSumKindFold8W) sum_fold8<kFold8WRB, kFold8WNW, false>(L, blk, sw, P);
@@ -1372,7 +1372,8 @@ size_t sum_smem_bytes(int win_bytes, int stages, int qs) {
 size_t sum_kind_extra_smem(int kind) {
   // the flush staging of the 8-bit kernel with 32-bit outputs: one segment of
   // 32-bit sums per warp
-  return kind == kSumKindU8Flush || kind == kSumKindU8Phase ? static_cast<size_t>(kWarps) * 32 * DD_SUM8_NW * 4 * sizeof(uint32_t) : 0;
+  const int nw = kind == kSumKindU8Flush ? DD_SUM8_NW : kind == kSumKindU8Phase ? kPhase8NW : 0;
+  return static_cast<size_t>(kWarps) * 32 * nw * 4 * sizeof(uint32_t);
 }
 
 size_t sum_launch_smem(const SumLaunch& L) {
@@ -1443,7 +1444,7 @@ void launch_sum(const SumLaunch& L, cudaStream_t st) {
     case kSumKindU8Flush: launch_k(k_sum_u8<kSumRowsPT8, DD_SUM8_NW, false>, grid, smem, L, st); break;
     case kSumKindU16Wide: launch_k(k_sum_u16w<kSumRowsPTW, DD_SUM16W_NW>, grid, smem, L, st); break;
     case kSumKindU16Twin: launch_k(k_sum_u16t<kSumRowsPTT, kSum16TNW>, grid, smem, L, st); break;
-    case kSumKindU8Phase: launch_k(k_sum_u8<kSumRowsPT8, DD_SUM8_NW, false, kModePhase>, grid, smem, L, st); break;
+    case kSumKindU8Phase: launch_k(k_sum_u8<kSumRowsPT8, kPhase8NW, false, kModePhase>, grid, smem, L, st); break;
     case kSumKindU16Phase: launch_k(k_sum_u16w<kSumRowsPTW, DD_SUM16W_NW, kModePhase>, grid, smem, L, st); break;
     case kSumKindWord64: launch_k(k_sum_to64<kTo64RB, kTo64NW, false>, grid, smem, L, st); break;
     case kSumKindPlane64: launch_k(k_sum_to64<kTo64RB, kTo64NW, true>, grid, smem, L, st); break;
