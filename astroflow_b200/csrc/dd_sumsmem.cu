@@ -1408,6 +1408,7 @@ std::vector<SumDesc> build_sum_desc(const std::vector<int32_t>& tab, int64_t nro
   const int64_t nblk = (nrows + blk - 1) / blk;
   std::vector<SumDesc> d(static_cast<size_t>(nblk * per * ncols));
   int32_t most = 0;
+  std::vector<int32_t> lo(static_cast<size_t>(ncols)), hi(static_cast<size_t>(ncols));
   for (int64_t b = 0; b < nblk; ++b) {
     const int64_t b0 = b * blk, b1 = std::min(nrows, b0 + blk);
     for (int64_t gi = 0; gi < per; ++gi) {
@@ -1415,19 +1416,24 @@ std::vector<SumDesc> build_sum_desc(const std::vector<int32_t>& tab, int64_t nro
       const int64_t r1 = std::min(b1, r0 + kSumRows);
       SumDesc* row = d.data() + (b * per + gi) * ncols;
       if (r0 >= r1) continue;
-      for (int64_t c = 0; c < ncols; ++c) row[c].lo = row[c].span = tab[r0 * ncols + c];
-      for (int64_t r = r0 + 1; r < r1; ++r)  // span holds the largest offset for now
+      const int32_t* first = tab.data() + r0 * ncols;
+      std::copy(first, first + ncols, lo.begin());
+      std::copy(first, first + ncols, hi.begin());
+      for (int64_t r = r0 + 1; r < r1; ++r) {
+        const int32_t* v = tab.data() + r * ncols;
         for (int64_t c = 0; c < ncols; ++c) {
-          row[c].lo = std::min(row[c].lo, tab[r * ncols + c]);
-          row[c].span = std::max(row[c].span, tab[r * ncols + c]);
+          lo[c] = std::min(lo[c], v[c]);
+          hi[c] = std::max(hi[c], v[c]);
         }
+      }
       for (int64_t c = 0; c < ncols; ++c) {
-        row[c].span -= row[c].lo;
+        row[c].lo = lo[c];
+        row[c].span = hi[c] - lo[c];
         most = std::max(most, row[c].span);
       }
       for (int64_t r = r0; r < r1; ++r)
         for (int64_t c = 0; c < ncols; ++c)
-          row[c].rel[r - r0] = static_cast<uint16_t>(tab[r * ncols + c] - row[c].lo);
+          row[c].rel[r - r0] = static_cast<uint16_t>(tab[r * ncols + c] - lo[c]);
     }
   }
   *spread = most;
