@@ -325,13 +325,18 @@ std::vector<int32_t> skew_stage1(dd_plan& P, std::vector<int32_t>& skew) {
     for (int64_t sb = 0; sb < P.nsb; ++sb) {
       const int64_t c0 = sb * P.sbw, c1 = std::min<int64_t>(c0 + P.sbw, P.dch);
       int32_t* sk = skew.data() + (g * P.nsb + sb) * kSumRows;
-      int first = 0, last = 0, reach = 0;
-      for (int64_t r = g * kSumRows; r < std::min((g + 1) * kSumRows, P.ndm_nom); ++r) {
+      const int64_t r0 = g * kSumRows, r1 = std::min(r0 + kSumRows, P.ndm_nom);
+      int least[kSumRows], last = 0, reach = 0;
+      bool grows = true;  // delays grow with the DM (kernels rely on it for the skews)
+      for (int64_t r = r0; r < r1; ++r) {
+        const int32_t* row = tab.data() + r * P.dch;
+        least[r - r0] = *std::min_element(row + c0, row + c1);
+        grows = grows && (r == r0 || least[r - r0] >= least[r - r0 - 1]);
+      }
+      for (int64_t r = r0; r < r1; ++r) {
         int32_t* row = tab.data() + r * P.dch;
-        const int least = *std::min_element(row + c0, row + c1);
-        if (r == g * kSumRows) first = least;
-        last = std::max(last, (least - first) & ~15);  // delays grow with the DM
-        sk[r - g * kSumRows] = last;
+        last = grows ? (least[r - r0] - least[0]) & ~15 : 0;
+        sk[r - r0] = last;
         for (int64_t c = c0; c < c1; ++c) {
           row[c] -= last;
           reach = std::max(reach, row[c]);

@@ -528,9 +528,9 @@ constexpr uint64_t kPoolBytes = uint64_t(64) << 20;
 constexpr int kMaxDevices = 64;
 std::mutex g_pool_mutex;
 cudaMemPool_t g_pool[kMaxDevices] = {};
-cudaMemPool_t image_pool() {
+cudaMemPool_t image_pool(cudaStream_t st) {
   int dev = 0;
-  DD_CUDA_TRY(cudaGetDevice(&dev));
+  DD_CUDA_TRY(cudaStreamGetDevice(st, &dev));
   if (dev < 0 || dev >= kMaxDevices) return nullptr;
   std::lock_guard<std::mutex> lock(g_pool_mutex);
   if (!g_pool[dev]) {
@@ -548,7 +548,7 @@ cudaMemPool_t image_pool() {
 }
 void* scratch_alloc(size_t bytes, cudaStream_t st, std::vector<void*>& scratch) {
   void* p = nullptr;
-  const cudaMemPool_t pool = image_pool();
+  const cudaMemPool_t pool = image_pool(st);
   bytes = std::max<size_t>(bytes, 16);
   if (pool) DD_CUDA_TRY(cudaMallocFromPoolAsync(&p, bytes, pool, st));
   else DD_CUDA_TRY(cudaMallocAsync(&p, bytes, st));
@@ -594,6 +594,7 @@ extern "C" int dd_images(const void* dm_time, int32_t elem_bytes, int64_t nrows,
     if (nrows < 1 || nslices < 0 || target < 1 || target > 4 * kImgThreads)
       throw Error{DD_ERR_INVALID, "bad image geometry"};
     if (nslices == 0) return DD_OK;
+    scratch.reserve(16);  // (a block is noted as soon as it is allocated)
     for (int32_t i = 0; i < nslices; ++i)
       if (col_count[i] < 1 || col_start[i] < 0 || col_start[i] + col_count[i] > row_pitch)
         throw Error{DD_ERR_INVALID, "slice outside the rows"};
@@ -793,6 +794,9 @@ extern "C" int dd_images(const void* dm_time, int32_t elem_bytes, int64_t nrows,
   } catch (const Error& e) {
     set_error(e.msg);
     rc = e.code;
+  } catch (const std::exception& e) {
+    set_error(e.what());
+    rc = DD_ERR_RUNTIME;
   }
   for (void* p : scratch) cudaFreeAsync(p, st);
   return rc;
