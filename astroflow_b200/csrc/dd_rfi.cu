@@ -4,8 +4,8 @@
 //  * IQRM channel masks (src/core/iqrm.cu:21-185, 203-345), computed entirely on
 //    the device: per-channel sums are exact 64-bit integers (the reference's
 //    double sums of integer samples are exact, so the statistics agree), and
-//    the per-lag sort, percentiles, threshold and votes run in one block per
-//    window instead of the reference's two host round trips per lag;
+//    differences, quartiles, threshold and votes run in one block per (window,
+//    lag) instead of the reference's two host round trips per lag;
 //  * window-mask application (src/rfi/rfimarker.cu:309-390), zero-DM over a
 //    channel range with an exact integer mean, and the static channel mask
 //    (rfimarker.cu:469-488), fused into the pass that writes the channel-major
@@ -708,8 +708,8 @@ __global__ void __launch_bounds__(256) k_prep_fold(PrepArgs a) {
 
 // Both layouts without downsampling, with word loads: output word i of channel c holds
 // the samples t = WS * i + fs * f, f = 0 .. F-1, of the channel (F = 4 of 8 bits, 2 of
-// 16): WS 1 and fs seg fold the chunk, WS F and fs 1 keep its order.  A thread loads four
-// channels (4 or 8 bytes) of the F samples of four words, applies the masks and the
+// 16, 1 of 32): WS 1 and fs seg fold the chunk, WS F and fs 1 keep its order.  A thread
+// loads four channels (4, 8 or 16 bytes) of the F samples of four words, applies the masks and the
 // zero-DM offset to whole words, puts the samples of each channel together by byte
 // permutes, and the block stores 64 words of 64 channels through shared memory, which
 // each output word passes once.  Needs nchans % 4 == 0 and an aligned input; channel
@@ -725,6 +725,13 @@ struct PrepWords {
   int ws;
   int64_t t0;
 };
+// Byte masks of four channels as masks of their samples, word v of the four channels.
+template <typename T>
+__device__ __forceinline__ uint32_t expand_mask(uint32_t m4, int v) {
+  if constexpr (sizeof(T) == 1) return m4;
+  if constexpr (sizeof(T) == 2) return __byte_perm(m4, 0u, v ? 0x3322 : 0x1100);
+  return __byte_perm(m4, 0u, 0x1111 * v);
+}
 template <typename T, int WS>
 __global__ void __launch_bounds__(256, sizeof(T) == 1 && WS == 1 ? 5 : 6) k_prep_w(PrepArgs a, PrepWords q) {
   constexpr int F = 4 / sizeof(T);   // samples per word
@@ -749,9 +756,10 @@ __global__ void __launch_bounds__(256, sizeof(T) == 1 && WS == 1 ? 5 : 6) k_prep
 #pragma unroll
     for (int b = 0; b < 4; ++b) {
       const int64_t ch = c + b;
-      const uint32_t lane = V == 1 ? 0xffu << (8 * b) : 0xffffu << (16 * (b & 1));
-      if (a.keep && !a.keep[ch]) keep[V == 1 ? 0 : b >> 1] &= ~lane;
-      if (a.zdm_off && ch >= a.zdm_cs && ch < a.zdm_ce) inrange[V == 1 ? 0 : b >> 1] |= lane;
+      const int v = b * V / 4;  // the word and lane of channel b
+      const uint32_t lane = V == 1 ? 0xffu << (8 * b) : V == 2 ? 0xffffu << (16 * (b & 1)) : ~0u;
+      if (a.keep && !a.keep[ch]) keep[v] &= ~lane;
+      if (a.zdm_off && ch >= a.zdm_cs && ch < a.zdm_ce) inrange[v] |= lane;
     }
   }
   // this thread's words of the tile are r0 + 16k: of each sample slot f the first row,
@@ -774,12 +782,8 @@ __global__ void __launch_bounds__(256, sizeof(T) == 1 && WS == 1 ? 5 : 6) k_prep
       mixed |= sg + 1 < a.nseg && static_cast<int64_t>(a.seg_t0[sg + 1]) <= t0 + ws * 63;
       const uint32_t m4 = ~__vcmpne4(*reinterpret_cast<const uint32_t*>(
                                          a.segmask + static_cast<int64_t>(sg) * a.nchans + c), 0u);
-      if constexpr (V == 1) {
-        mask[f][0] &= m4;
-      } else {
-        mask[f][0] &= __byte_perm(m4, 0u, 0x1100);
-        mask[f][V - 1] &= __byte_perm(m4, 0u, 0x3322);
-      }
+#pragma unroll
+      for (int v = 0; v < V; ++v) mask[f][v] &= expand_mask<T>(m4, v);
     }
   }
   const int64_t step = static_cast<int64_t>(16 * ws) * a.nchans;
@@ -789,6 +793,12 @@ __global__ void __launch_bounds__(256, sizeof(T) == 1 && WS == 1 ? 5 : 6) k_prep
     auto load = [&](int k) {
       if constexpr (V == 1) {
         in[k][f][0] = __ldg(reinterpret_cast<const uint32_t*>(src[f] + k * step));
+      } else if constexpr (V == 4) {
+        const uint4 u = __ldg(reinterpret_cast<const uint4*>(src[f] + k * step));
+        in[k][f][0] = u.x;
+        in[k][f][1] = u.y;
+        in[k][f][2] = u.z;
+        in[k][f][3] = u.w;
       } else {
         const uint2 u = __ldg(reinterpret_cast<const uint2*>(src[f] + k * step));
         in[k][f][0] = u.x;
@@ -816,12 +826,8 @@ __global__ void __launch_bounds__(256, sizeof(T) == 1 && WS == 1 ? 5 : 6) k_prep
         const int64_t t = q.t0 + ws * (sb + r0 + 16 * k) + q.fs * f;
         const uint32_t m4 = ~__vcmpne4(*reinterpret_cast<const uint32_t*>(
                                            a.segmask + static_cast<int64_t>(find_seg(a.seg_t0, a.nseg, t)) * a.nchans + c), 0u);
-        if constexpr (V == 1) {
-          in[k][f][0] &= m4 & keep[0];
-        } else {
-          in[k][f][0] &= __byte_perm(m4, 0u, 0x1100) & keep[0];
-          in[k][f][V - 1] &= __byte_perm(m4, 0u, 0x3322) & keep[V - 1];
-        }
+#pragma unroll
+        for (int v = 0; v < V; ++v) in[k][f][v] &= expand_mask<T>(m4, v) & keep[v];
       }
   } else if (a.segmask || a.keep) {
 #pragma unroll
@@ -841,8 +847,9 @@ __global__ void __launch_bounds__(256, sizeof(T) == 1 && WS == 1 ? 5 : 6) k_prep
 #pragma unroll
         for (int v = 0; v < V; ++v) {
           const uint32_t u = in[k][f][v];
-          const uint32_t d = V == 1 ? __vsubus4(u, min(off, 255u) * 0x01010101u)
-                                    : __vsubus2(u, min(off, 65535u) * 0x00010001u);
+          const uint32_t d = V == 1   ? __vsubus4(u, min(off, 255u) * 0x01010101u)
+                             : V == 2 ? __vsubus2(u, min(off, 65535u) * 0x00010001u)
+                                      : u - min(u, off);
           in[k][f][v] = (d & inrange[v]) | (u & ~inrange[v]);
         }
       }
@@ -858,6 +865,9 @@ __global__ void __launch_bounds__(256, sizeof(T) == 1 && WS == 1 ? 5 : 6) k_prep
       o[1] = __byte_perm(lo01, lo23, 0x7632);
       o[2] = __byte_perm(hi01, hi23, 0x5410);
       o[3] = __byte_perm(hi01, hi23, 0x7632);
+    } else if constexpr (V == 4) {
+#pragma unroll
+      for (int b = 0; b < 4; ++b) o[b] = in[k][0][b];
     } else {
       o[0] = __byte_perm(in[k][0][0], in[k][1][0], 0x5410);
       o[1] = __byte_perm(in[k][0][0], in[k][1][0], 0x7632);
@@ -1069,10 +1079,9 @@ void launch_prep(const PrepArgs& a, cudaStream_t st) {
     return static_cast<unsigned>(n);
   };
   // the word-wise kernel applies integer zero-DM offsets only
-  const int F = a.nbits == 8 ? 4 : 2;
-  const bool wide = a.out && a.nbits <= 16 && !a.zdm_mean && a.nchans % 4 == 0 &&
-                    reinterpret_cast<uintptr_t>(a.x) % (a.nbits / 2) == 0;
-  if (wide && a.ds > 1 && a.ds <= 16 && a.pitch % F == 0 && reinterpret_cast<uintptr_t>(a.out) % 4 == 0) {
+  const int F = 32 / a.nbits;
+  const bool wide = a.out && !a.zdm_mean && a.nchans % 4 == 0 && reinterpret_cast<uintptr_t>(a.x) % (a.nbits / 2) == 0;
+  if (wide && a.nbits <= 16 && a.ds > 1 && a.ds <= 16 && a.pitch % F == 0 && reinterpret_cast<uintptr_t>(a.out) % 4 == 0) {
     for (int ph = 0; ph < a.ds; ++ph) {
       PrepArgs p = a;
       p.out = static_cast<char*>(a.out) + ph * a.pitch * (a.nbits / 8);
@@ -1088,7 +1097,8 @@ void launch_prep(const PrepArgs& a, cudaStream_t st) {
     const PrepWords q = a.fold > 1 ? PrepWords{a.seg, a.nwords, a.pitch, 1, 0}
                                    : PrepWords{1, (a.nsamp + F - 1) / F, a.pitch / F, F, 0};
     const unsigned grid = blocks((q.nwords + 63) / 64, a.c0 & ~int64_t(3));
-    if (a.nbits == 8 && a.fold > 1) k_prep_w<uint8_t, 1><<<grid, 256, 0, st>>>(a, q);
+    if (a.nbits == 32) k_prep_w<uint32_t, 1><<<grid, 256, 0, st>>>(a, q);
+    else if (a.nbits == 8 && a.fold > 1) k_prep_w<uint8_t, 1><<<grid, 256, 0, st>>>(a, q);
     else if (a.nbits == 8) k_prep_w<uint8_t, 4><<<grid, 256, 0, st>>>(a, q);
     else if (a.fold > 1) k_prep_w<uint16_t, 1><<<grid, 256, 0, st>>>(a, q);
     else k_prep_w<uint16_t, 2><<<grid, 256, 0, st>>>(a, q);

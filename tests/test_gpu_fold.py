@@ -169,3 +169,29 @@ def test_32bit_sums_equal_oracle(n, nchans, hi, step, ds, width):
     bw = np.concatenate(O.bruteforce_cpu(x, nchans, filfreq, 64e-6, 0.0, hi, bs, be, step, 1, ts,
                                          delay=bp.tables()[0]), axis=1)
     assert np.array_equal(bp.run(xd).view(torch.int64).cpu().numpy().view(np.uint64), bw)
+
+
+# 32-bit layout by words: masks that change inside a tile of 64 samples, zero-DM offsets and
+# zeroed channels, at tile remainders; 37 channels take the per-sample kernel.
+@pytest.mark.parametrize("n,nchans,width", [(511, 36, 16), (2049, 132, 64), (3001, 40, 8), (1027, 37, 9)])
+def test_32bit_layout_with_masks(n, nchans, width):
+    rng = np.random.default_rng(n + nchans)
+    x = rng.integers(0, 2 ** 32, size=(n, nchans), dtype=np.uint64).astype(np.uint32)
+    foff = float(F32(300.0 / nchans))
+    hdr = dict(tsamp=float(F32(64e-6)), fch1=1150.0, foff=foff, nbits=32, nchans=nchans, ndata=n)
+    freq = O.freq_table_header(hdr["fch1"], hdr["foff"], nchans)
+    fs, fe = float(F32(freq[0])), float(F32(freq[-1]))
+    iq = IqrmParams(mode=0, radius_frac=0.1, nsigma=3.0, win_sec=n * 64e-6 * 0.4, hop_sec=n * 64e-6 * 0.2)
+    plan = Plan(hdr, 0.0, 60.0, fs, fe, 0.5, 1, algorithm="subband", subband_width=width,
+                zero_dm_mode="range", rfi=RfiParams(use_zero_dm=True, use_iqrm=True, iqrm=iq, use_mask=True),
+                bad_channels=[2])
+    ref = x.copy()
+    cs, ce = plan.info["chan_start"], plan.info["chan_end"]
+    t0, t1, masks = O.iqrm_masks(ref, nchans, cs, ce, float(F32(F32(64e-6) * F32(1))), iq)
+    O.apply_window_masks(ref, nchans, t0, t1, masks)
+    O.zero_dm_range_exact(ref, nchans, cs, ce)
+    O.mark_channels(ref, nchans, [2])
+    op = O.subband_plan(freq, n, 0.0, 60.0, fs, fe, 0.5, 1, sb_width=width)
+    want = O.subband_sums(ref, nchans, op, *plan.tables())
+    got = plan.run(torch.from_numpy(x.view(np.int32)).cuda().view(torch.uint32))
+    assert np.array_equal(got.view(torch.int64).cpu().numpy().view(np.uint64), want)
