@@ -749,8 +749,6 @@ SumLaunch stage1_launch(const dd_plan& P, int64_t t0) {
   L.kind = stage1_kind(P);
   L.src = static_cast<const char*>(P.d_x.p);
   L.src_pitch = P.xpitch * x_elem(P);
-  L.off = P.d_delay.as<int32_t>();
-  L.off_pitch = P.dch;
   L.base = t0;
   L.valid = P.nbin;
   L.max_off = P.max_off1;
@@ -783,8 +781,6 @@ SumLaunch stage2_launch(const dd_plan& P, int64_t t0, void* output) {
   L.kind = stage2_kind(P);
   L.src = static_cast<const char*>(P.d_inter.p);
   L.src_pitch = P.tile_pitch * inter_elem(P);
-  L.off = P.d_res.as<int32_t>();
-  L.off_pitch = P.nsb;
   L.base = 0;
   L.valid = INT64_MAX;
   L.nsrc_total = P.nsb;
@@ -882,8 +878,6 @@ SumLaunch brute_launch(const dd_plan& P, void* output) {
   L.kind = brute_kind(P);
   L.src = static_cast<const char*>(P.d_x.p);
   L.src_pitch = P.xpitch * x_elem(P);
-  L.off = P.d_delay.as<int32_t>();
-  L.off_pitch = P.nc;
   L.base = 0;
   L.valid = (P.nin + P.p.time_downsample - 1) / P.p.time_downsample;
   L.max_off = P.max_delay / P.p.time_downsample + 1;

@@ -186,8 +186,8 @@ void launch_iqrm_stats(const void* x, int nbits, int64_t nsamp, int64_t nchans, 
                        int64_t csub, const uint32_t* d_win, int nwin,
                        unsigned long long* d_sums, cudaStream_t st);
 size_t iqrm_scratch_bytes(int nwin, int64_t csub, int nlags);
-// Throws DD_ERR_INVALID when csub channels exceed what k_iqrm_lag's
-// shared-memory sort holds on the current device.
+// Throws DD_ERR_INVALID when csub channels exceed what the statistics and votes of
+// one window may hold in shared memory on the current device.
 void check_iqrm_channels(int64_t csub);
 void launch_iqrm_decide(const unsigned long long* d_sums, int nwin, const uint32_t* d_win,
                         int64_t nchans, int64_t cs, int64_t csub, int mode, float nsigma,
@@ -308,8 +308,6 @@ struct SumLaunch {
   int kind;                // SumKind
   const char* src;         // byte address of source row 0
   int64_t src_pitch;       // bytes between source rows
-  const int32_t* off;      // per-row, per-source offsets (elements)
-  int64_t off_pitch;       // entries between consecutive rows of `off`
   int64_t base;            // element index added to every offset
   int64_t valid;           // source elements from here on are zero: windows starting there are skipped
   int64_t max_off;         // largest offset of any row and source
@@ -341,7 +339,7 @@ struct SumLaunch {
   // every first sample of a slice modulo ds.
   int ds, sub_bytes;
   int64_t sps, nin, phase_pitch, desc_pattern;
-  int stages;              // staged source pairs in flight (2..4)
+  int stages;              // groups of sources in flight (2..kSumMaxStages)
   int* err;                // device error word: set when a bounded wait gives up
   // 16-bit subband sums with a one-sample-shifted twin (0: none): the twin of the
   // element at byte address a sits at a + twin_off and holds the element before
@@ -356,7 +354,7 @@ struct SumLaunch {
 #ifndef DD_SUM_SMEM_KB
 #define DD_SUM_SMEM_KB 100
 #endif
-constexpr int kSumMaxStages = DD_SUM_MAX_STAGES;  // staged source pairs in flight, at most
+constexpr int kSumMaxStages = DD_SUM_MAX_STAGES;  // groups of sources in flight, at most
 void launch_sum(const SumLaunch& L, cudaStream_t st);
 int sum_tile_samples(int src_bytes, int nw);
 // Shared memory of a staged sum with `stages` pairs in flight.

@@ -4,29 +4,33 @@
 //
 //   out[r][t] = sum_i src_i[base + off(r, i) + t],   t in [0, T) of the block's tile.
 //
-// A block owns RB output rows and T consecutive samples.  Sources are processed
-// two at a time.  The time window of each source that the block's rows need,
+// A block owns kSumRows output rows, dealt to its warp groups (RB rows each), and T
+// consecutive words of them.  Sources are processed in groups of two or four.  The time
+// window of each source that the block's rows need,
 // [base + min_r off, base + max_r off + T), is brought into shared memory by one
 // bulk asynchronous copy (cp.async.bulk, completion counted in bytes on an
-// mbarrier); up to `stages` source pairs are in flight in a ring of buffers.
+// mbarrier); up to `stages` groups are in flight in a ring of buffers.
 // The warps take turns as the producer (run_pipeline), each refilling a buffer once
 // every warp has released it (an "empty" mbarrier with one arrival per warp).  The
 // window bounds and each row's offset inside its window come from descriptors
 // precomputed on the host (SumDesc), which the producing warp has loaded ahead (one
 // lane per source and row).
 //
-// Summing: lanes own 32-bit output words (an odd number of consecutive words, or
-// interleaved words l, l+32, ...), so a warp's shared loads are free of bank
-// conflicts; a shift that is not a multiple of 4 bytes costs one funnel shift of
-// two words.  8-bit samples are added two at a time by two-way dot products with
-// the weights (1, 2^15) (see dot_lo); 16-bit stage-1 sums come with a twin shifted by one sample so that
-// stage 2 reads aligned words only (sum_u16_twin), four sources at a time in
-// packed 16-bit lanes; 16-bit samples are aligned pairwise and summed whole
-// beside their high halves (sum_u16_wide).  Outputs leave through shared memory
-// as 16-byte chunks where a lane's words are scattered (16-bit stage-1 sums and
-// their twin; the 32-bit flushes of 8-bit sums of more than 128 sources, which
-// read back the block's own partial sums).  A missing source (source count not
-// a multiple of the group) reads a zeroed window.
+// Layouts.  Folded chunks (the default where the delays are short against the chunk)
+// hold in one 32-bit word samples that lie a segment apart, so every delay is a whole
+// number of words and each source word is one aligned shared load; their lanes own
+// interleaved words (l, l + 32, ...).  Chunks in time order (short against their
+// delays: a beam's pushes) pay one funnel shift of two words per unaligned word; their
+// lanes own an odd number of consecutive words (8- and 16-bit samples) or read the
+// subband sums' one-sample-shifted twin (sum_u16_twin).  Downsampled brute force reads
+// one phase row per delay, 32-bit samples are whole words.  All of these keep a warp's
+// shared loads free of bank conflicts.
+// 8-bit samples are added two at a time by two-way dot products with the weights
+// (1, 2^15) (see dot_lo), 16-bit samples in packed lanes or whole beside their high
+// halves.  Outputs leave through shared memory as 16-byte chunks where a lane's words
+// are scattered (16-bit stage-1 sums in time order and their twin).  Sums of more
+// sources than a 15-bit field holds are added to the output in several flushes.
+// A missing source (source count not a multiple of the group) reads a zeroed window.
 //
 // Every wait on an mbarrier is bounded (about two seconds of SM clock); a wait
 // that gives up records an error code in L.err and the block stops summing, and
@@ -48,7 +52,7 @@ constexpr int kThreads = kWarps * 32;
 #ifndef DD_SUM_MAX_STAGES
 #define DD_SUM_MAX_STAGES 8
 #endif
-constexpr int kMaxStages = DD_SUM_MAX_STAGES;  // staged source pairs in flight, at most
+constexpr int kMaxStages = DD_SUM_MAX_STAGES;  // groups of sources in flight, at most
 constexpr long long kWaitCycles = 4000000000LL;
 
 // ------------------------------------------------------------------ mbarrier helpers
@@ -1096,13 +1100,13 @@ __device__ __forceinline__ void sum_to64(const SumLaunch& L, uint3 blk, uint32_t
 // its sums (SumLaunch::twin_off): a row whose offset for a source is odd reads
 // that source's twin, so every source word a row needs is one aligned shared
 // load, with no permute.  Four sources per stage are added in packed 16-bit
-// lanes (each <= 64 x 255, four <= 65280) and folded into two 32-bit sums as in
-// sum_u16_quad; lanes own interleaved words (lane l: l, l + 32, ...), so the
-// loads of a warp are 32 consecutive words for any words per lane.  With half
-// the instructions of the quad kernel it waits on its shared loads instead
+// lanes (each <= 64 x 255, four <= 65280) and folded into two 32-bit sums; lanes own
+// interleaved words (lane l: l, l + 32, ...), so the loads of a warp are 32
+// consecutive words for any words per lane.  It waits on its shared loads
 // (long-scoreboard stalls 3.3 per issue at two blocks per SM), so it is built for
-// three blocks per SM: 36.7 ms per headline step against 43.2 at two blocks and
-// 46.8 for the quad kernel.
+// three blocks per SM: 36.7 ms for 4096 channels, 2^20 samples, 6001 trials against
+// 43.2 at two blocks (with four rows per warp and turns 32.8).  Chunks that fold take
+// sum_plane16 instead.
 #ifndef DD_SUM16T_MINB
 #define DD_SUM16T_MINB 3
 #endif
@@ -1381,7 +1385,7 @@ size_t sum_launch_smem(const SumLaunch& L) {
   return sum_smem_bytes(L.win_bytes, L.stages, sum_kind_qs(kind)) + sum_kind_extra_smem(kind);
 }
 
-// Staged source pairs for a window size: as many as fit DD_SUM_SMEM_KB of shared
+// Stages (groups of sources) for a window size: as many as fit DD_SUM_SMEM_KB of shared
 // memory (two blocks per SM at the default), at least two.
 // The twin-window stage-2 kernel (eight windows per stage) is limited by the
 // latency of its shared loads rather than by issue: it takes at most
