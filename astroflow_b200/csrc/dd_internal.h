@@ -123,6 +123,7 @@ struct dd_plan {
   dd::DevBuf d_delay, d_res, d_lags, d_bad_keep, d_win, d_seg_t0;
   dd::DevBuf d_binned;   // binned / working copy of the input [nbin][nchans]
   dd::DevBuf d_x;        // prepared channel-major input
+  dd::DevBuf d_xlimit;   // PrepArgs::limit (empty: the sums read all of d_x)
   dd::DevBuf d_host_in, d_host_out;  // device side of dd_run_host (kept across calls)
   cudaStream_t copy_stream = nullptr; // dd_run_host: output copies overlapping the sums
   cudaEvent_t host_done = nullptr;    // the last host-path output copy enqueued
@@ -223,6 +224,9 @@ struct PrepArgs {
   // channel in one 32-bit word, words [0, nwords)
   int fold;
   int64_t seg, nwords;
+  // per 64 channels from c0 & ~3 on: positions from here on are read by no sum and may be
+  // left out (nullptr: write them all)
+  const int32_t* limit;
   void* full_out;          // optional [nsamp][nchans] copy after all stages
 };
 void launch_prep(const PrepArgs& a, cudaStream_t st);

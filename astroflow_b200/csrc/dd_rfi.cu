@@ -742,6 +742,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 1 && WS == 1 ? 5 : 6) k_prep
   __shared__ uint32_t tile[64][66];
   int64_t group;
   const int64_t sb = prep_tile(a, a.c0 & ~int64_t(3), &group) * 64;
+  if (a.limit && q.t0 + ws * sb >= a.limit[group]) return;
   const int64_t cb = (a.c0 & ~int64_t(3)) + group * 64;
   const int w = threadIdx.x & 15, r0 = threadIdx.x >> 4;
   const int64_t c = cb + 4 * w;

@@ -195,3 +195,16 @@ def test_32bit_layout_with_masks(n, nchans, width):
     want = O.subband_sums(ref, nchans, op, *plan.tables())
     got = plan.run(torch.from_numpy(x.view(np.int32)).cuda().view(torch.uint32))
     assert np.array_equal(got.view(torch.int64).cpu().numpy().view(np.uint64), want)
+
+
+# The layout leaves out the positions past each 64 channels' largest delay: several groups of
+# channels, a band that starts inside one and off the load words, two chunks in turn.
+@pytest.mark.parametrize("n,nchans,nbits,hi,band", [
+    (6001, 390, 8, 150.0, 0.13), (6001, 388, 8, 900.0, 0.13), (9000, 260, 16, 150.0, 0.31),
+    (4100, 516, 16, 900.0, 0.07),
+])
+def test_layout_up_to_the_largest_delays(n, nchans, nbits, hi, band):
+    plan, x, want = subband(n, nchans, nbits, hi, 1.0, 1, 64, band, True, False)
+    other = dev(np.ascontiguousarray(x[::-1]))
+    plan.run(other)
+    assert np.array_equal(to_np(plan.run(dev(x))), want)
