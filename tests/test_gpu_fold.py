@@ -208,3 +208,14 @@ def test_layout_up_to_the_largest_delays(n, nchans, nbits, hi, band):
     other = dev(np.ascontiguousarray(x[::-1]))
     plan.run(other)
     assert np.array_equal(to_np(plan.run(dev(x))), want)
+
+
+# Zero-DM offsets by words: more and fewer words than the loads in flight, a band that starts
+# and ends inside a word, masked segments.
+@pytest.mark.parametrize("n,nchans,nbits,band", [
+    (700, 1024, 8, 0.0), (701, 1028, 8, 0.13), (650, 2052, 8, 0.0007), (700, 36, 8, 0.1),
+    (650, 512, 16, 0.0), (651, 518, 16, 0.13), (640, 30, 16, 0.1),
+])
+def test_zero_dm_by_words(n, nchans, nbits, band):
+    plan, x, want = subband(n, nchans, nbits, 20.0, 1.0, 1, 64, band, True, True)
+    assert np.array_equal(to_np(plan.run(dev(x))), want)
