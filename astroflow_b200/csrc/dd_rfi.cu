@@ -80,15 +80,17 @@ __device__ __forceinline__ T binned_value(uint64_t sum, uint64_t cnt) {
   return static_cast<T>(v < static_cast<double>(vmax) ? v : static_cast<double>(vmax));
 }
 
-// DS: the bin width (2, 4, 8), or 0 for any.  A block covers 256 words of channels and
-// `rows` bins; with a fixed width the samples of several bins are loaded before the first
-// is summed (sixteen loads in flight per thread; 2,048 channels x 300,001 samples in bins
-// of four 242 us with one bin at a time).
-template <typename T, int DS>
+// DS: the bin width (2, 4, 8), or 0 for any.  W: the word of channels that a thread loads,
+// 32 bits, or less where rows do not start on one.  A block covers 256 words of channels
+// and `rows` bins; with a fixed width the samples of several bins are loaded before the
+// first is summed (sixteen loads in flight per thread; 2,048 channels x 300,001 samples in
+// bins of four 242 us with one bin at a time; 2,870 channels, whose rows are whole pairs,
+// 1380 us with the expression evaluated per bin, now 253).
+template <typename T, typename W, int DS>
 __global__ void __launch_bounds__(256) k_time_binning_lut(const T* __restrict__ in, T* __restrict__ out,
                                                           int64_t nchans, int64_t ndata, int ds, int64_t nout,
                                                           int rows, const T* __restrict__ lut) {
-  constexpr int V = 4 / sizeof(T);
+  constexpr int V = sizeof(W) / sizeof(T);
   constexpr int R = DS ? 16 / DS : 1;  // bins at a time
   const int64_t c = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) * V;
   if (c >= nchans) return;
@@ -103,7 +105,7 @@ __global__ void __launch_bounds__(256) k_time_binning_lut(const T* __restrict__ 
       const T b = cnt == ds ? __ldg(lut + sum[v]) : binned_value<T>(sum[v], static_cast<uint64_t>(cnt));
       o |= static_cast<uint32_t>(b) << (8 * sizeof(T) * v);
     }
-    *reinterpret_cast<uint32_t*>(out + k * nchans + c) = o;
+    *reinterpret_cast<W*>(out + k * nchans + c) = static_cast<W>(o);
   };
   const int64_t k1 = min(nout, (static_cast<int64_t>(blockIdx.y) + 1) * rows);
   int64_t k = static_cast<int64_t>(blockIdx.y) * rows;
@@ -113,7 +115,7 @@ __global__ void __launch_bounds__(256) k_time_binning_lut(const T* __restrict__ 
       const T* p = in + k * DS * nchans + c;
       uint32_t w[R * DS];
 #pragma unroll
-      for (int i = 0; i < R * DS; ++i) w[i] = __ldg(reinterpret_cast<const uint32_t*>(p + i * nchans));
+      for (int i = 0; i < R * DS; ++i) w[i] = __ldg(reinterpret_cast<const W*>(p + i * nchans));
 #pragma unroll
       for (int r = 0; r < R; ++r) {
         uint32_t sum[V];
@@ -130,14 +132,14 @@ __global__ void __launch_bounds__(256) k_time_binning_lut(const T* __restrict__ 
     uint32_t sum[V];
 #pragma unroll
     for (int v = 0; v < V; ++v) sum[v] = 0;
-    for (int64_t t = t0; t < t1; ++t) add(__ldg(reinterpret_cast<const uint32_t*>(in + t * nchans + c)), sum);
+    for (int64_t t = t0; t < t1; ++t) add(__ldg(reinterpret_cast<const W*>(in + t * nchans + c)), sum);
     store(k, sum, static_cast<int>(t1 - t0));
   }
 }
-template <typename T>
+template <typename T, typename W>
 void launch_time_binning_lut(const void* in, void* out, int64_t ndata, int64_t nchans, int ds,
                              int64_t nout, const void* lut, cudaStream_t st) {
-  const int64_t words = nchans / (4 / static_cast<int64_t>(sizeof(T)));
+  const int64_t words = nchans / static_cast<int64_t>(sizeof(W) / sizeof(T));
   const int64_t gx = (words + 255) / 256;
   int rows = 16;  // bins per block: more where the grid would pass its limit
   while ((nout + rows - 1) / rows > 65535) rows *= 2;
@@ -146,10 +148,10 @@ void launch_time_binning_lut(const void* in, void* out, int64_t ndata, int64_t n
   T* o = static_cast<T*>(out);
   const T* l = static_cast<const T*>(lut);
   switch (ds) {
-    case 2: k_time_binning_lut<T, 2><<<g, 256, 0, st>>>(i, o, nchans, ndata, ds, nout, rows, l); break;
-    case 4: k_time_binning_lut<T, 4><<<g, 256, 0, st>>>(i, o, nchans, ndata, ds, nout, rows, l); break;
-    case 8: k_time_binning_lut<T, 8><<<g, 256, 0, st>>>(i, o, nchans, ndata, ds, nout, rows, l); break;
-    default: k_time_binning_lut<T, 0><<<g, 256, 0, st>>>(i, o, nchans, ndata, ds, nout, rows, l); break;
+    case 2: k_time_binning_lut<T, W, 2><<<g, 256, 0, st>>>(i, o, nchans, ndata, ds, nout, rows, l); break;
+    case 4: k_time_binning_lut<T, W, 4><<<g, 256, 0, st>>>(i, o, nchans, ndata, ds, nout, rows, l); break;
+    case 8: k_time_binning_lut<T, W, 8><<<g, 256, 0, st>>>(i, o, nchans, ndata, ds, nout, rows, l); break;
+    default: k_time_binning_lut<T, W, 0><<<g, 256, 0, st>>>(i, o, nchans, ndata, ds, nout, rows, l); break;
   }
   DD_LAUNCHED();
 }
@@ -686,7 +688,7 @@ __global__ void k_prep(PrepArgs a) {
   }
 }
 
-// Folded layout, any channel count and alignment: word s of channel c holds the
+// Folded layout with a float mean per sample to subtract: word s of channel c holds the
 // samples s + f * seg, f = 0 .. F-1 (F = 4 of 8 bits, 2 of 16).  Tile: 64 words x 64
 // channels, 256 threads.
 template <typename T>
@@ -721,8 +723,10 @@ __global__ void __launch_bounds__(256) k_prep_fold(PrepArgs a) {
 // loads four channels (4, 8 or 16 bytes) of the F samples of four words, applies the masks and the
 // zero-DM offset to whole words, puts the samples of each channel together by byte
 // permutes, and the block stores 64 words of 64 channels through shared memory, which
-// each output word passes once.  Needs nchans % 4 == 0 and an aligned input; channel
-// words are read from c0 & ~3.  Bound by issue (80 % busy) beside the memory: row
+// each output word passes once.  Channel words are read from c0 & ~3; RAGGED: rows do not
+// start on a word of four channels (nchans % 4 or the input's address), channels are
+// loaded one by one (2,870 channels x 75,001 samples folded 263 us, 1152 us with the
+// segment search and offset per sample of k_prep_fold).  Bound by issue (80 % busy) beside the memory: row
 // pointers and counts are set up once per thread, the tile comes from one 32-bit
 // division, and nothing is 64-bit per load.  4096 channels x 151,000 samples in time
 // order 216 us (5.7 TB/s; 480 us with four loads in flight per thread and 64-bit rows),
@@ -741,8 +745,8 @@ __device__ __forceinline__ uint32_t expand_mask(uint32_t m4, int v) {
   if constexpr (sizeof(T) == 2) return __byte_perm(m4, 0u, v ? 0x3322 : 0x1100);
   return __byte_perm(m4, 0u, 0x1111 * v);
 }
-template <typename T, int WS>
-__global__ void __launch_bounds__(256, sizeof(T) == 1 && WS == 1 ? 5 : 6) k_prep_w(PrepArgs a, PrepWords q) {
+template <typename T, int WS, bool RAGGED>
+__global__ void __launch_bounds__(256, RAGGED ? 4 : sizeof(T) == 1 && WS == 1 ? 5 : 6) k_prep_w(PrepArgs a, PrepWords q) {
   constexpr int F = 4 / sizeof(T);   // samples per word
   const int ws = WS ? WS : q.ws;
   constexpr int V = sizeof(T);       // 32-bit words per four channels
@@ -766,6 +770,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 1 && WS == 1 ? 5 : 6) k_prep
 #pragma unroll
     for (int b = 0; b < 4; ++b) {
       const int64_t ch = c + b;
+      if (RAGGED && ch >= a.nchans) break;
       const int v = b * V / 4;  // the word and lane of channel b
       const uint32_t lane = V == 1 ? 0xffu << (8 * b) : V == 2 ? 0xffffu << (16 * (b & 1)) : ~0u;
       if (a.keep && !a.keep[ch]) keep[v] &= ~lane;
@@ -785,7 +790,17 @@ __global__ void __launch_bounds__(256, sizeof(T) == 1 && WS == 1 ? 5 : 6) k_prep
     const int64_t left = a.nsamp - t0;  // words i with ws * i < left
     have[f] = !cvalid || left <= 0 ? 0 : left >= ws * 64 ? 64 : (static_cast<int>(left) + ws - 1) / ws;
     auto load = [&](int k) {
-      if constexpr (V == 1) {
+      if constexpr (RAGGED) {
+        T e[4];
+#pragma unroll
+        for (int b = 0; b < 4; ++b) e[b] = c + b < a.nchans ? __ldg(src + k * step + b) : T(0);
+#pragma unroll
+        for (int v = 0; v < V; ++v) {
+          in[k][f][v] = 0;
+#pragma unroll
+          for (int b = 0; b < F; ++b) in[k][f][v] |= static_cast<uint32_t>(e[F * v + b]) << (8 * sizeof(T) * b);
+        }
+      } else if constexpr (V == 1) {
         in[k][f][0] = __ldg(reinterpret_cast<const uint32_t*>(src + k * step));
       } else if constexpr (V == 4) {
         const uint4 u = __ldg(reinterpret_cast<const uint4*>(src + k * step));
@@ -818,7 +833,15 @@ __global__ void __launch_bounds__(256, sizeof(T) == 1 && WS == 1 ? 5 : 6) k_prep
       // the mask of the IQRM segment that holds the tile's rows of this slot
       const int64_t t0 = q.t0 + ws * sb + q.fs * f;
       const auto seg_mask = [&](int sg) {
-        return ~__vcmpne4(*reinterpret_cast<const uint32_t*>(a.segmask + static_cast<int64_t>(sg) * a.nchans + c), 0u);
+        const uint8_t* p = a.segmask + static_cast<int64_t>(sg) * a.nchans + c;
+        if constexpr (RAGGED) {
+          uint32_t m = 0;
+#pragma unroll
+          for (int b = 0; b < 4; ++b)
+            if (c + b < a.nchans && p[b]) m |= 0xffu << (8 * b);
+          return ~m;
+        }
+        return ~__vcmpne4(*reinterpret_cast<const uint32_t*>(p), 0u);
       };
       const int sg = a.segmask ? find_seg(a.seg_t0, a.nseg, t0) : 0;
       if (a.segmask && sg + 1 < a.nseg && static_cast<int64_t>(a.seg_t0[sg + 1]) <= t0 + ws * 63) {
@@ -939,10 +962,17 @@ void launch_binning_lut(void* lut, int nbits, int ds, cudaStream_t st) {
 void launch_time_binning(const void* in, void* out, int nbits, int64_t ndata, int64_t nchans,
                          int ds, const void* lut, cudaStream_t st) {
   const int64_t nout = (ndata + ds - 1) / ds;
-  if (lut && (nbits == 8 || nbits == 16) && nchans % (32 / nbits) == 0 &&
-      reinterpret_cast<uintptr_t>(in) % 4 == 0 && reinterpret_cast<uintptr_t>(out) % 4 == 0) {
-    if (nbits == 8) launch_time_binning_lut<uint8_t>(in, out, ndata, nchans, ds, nout, lut, st);
-    else launch_time_binning_lut<uint16_t>(in, out, ndata, nchans, ds, nout, lut, st);
+  if (lut && (nbits == 8 || nbits == 16)) {
+    // the widest word that every row starts on
+    const auto starts = [&](int64_t bytes) {
+      return nchans * (nbits / 8) % bytes == 0 && reinterpret_cast<uintptr_t>(in) % bytes == 0 &&
+             reinterpret_cast<uintptr_t>(out) % bytes == 0;
+    };
+    if (nbits == 16 && starts(4)) launch_time_binning_lut<uint16_t, uint32_t>(in, out, ndata, nchans, ds, nout, lut, st);
+    else if (nbits == 16) launch_time_binning_lut<uint16_t, uint16_t>(in, out, ndata, nchans, ds, nout, lut, st);
+    else if (starts(4)) launch_time_binning_lut<uint8_t, uint32_t>(in, out, ndata, nchans, ds, nout, lut, st);
+    else if (starts(2)) launch_time_binning_lut<uint8_t, uint16_t>(in, out, ndata, nchans, ds, nout, lut, st);
+    else launch_time_binning_lut<uint8_t, uint8_t>(in, out, ndata, nchans, ds, nout, lut, st);
     return;
   }
   const dim3 grid(static_cast<unsigned>((nchans + 255) / 256),
@@ -1085,7 +1115,12 @@ void launch_prep(const PrepArgs& a, cudaStream_t st) {
   };
   // the word-wise kernel applies integer zero-DM offsets only
   const int F = 32 / a.nbits;
-  const bool wide = a.out && !a.zdm_mean && a.nchans % 4 == 0 && reinterpret_cast<uintptr_t>(a.x) % (a.nbits / 2) == 0;
+  const auto run = [&](auto kernel, auto kernel_ragged, unsigned grid, const PrepArgs& p, const PrepWords& q, bool r) {
+    if (r) kernel_ragged<<<grid, 256, 0, st>>>(p, q);
+    else kernel<<<grid, 256, 0, st>>>(p, q);
+  };
+  const bool wide = a.out && !a.zdm_mean;
+  const bool ragged = a.nchans % 4 != 0 || reinterpret_cast<uintptr_t>(a.x) % (a.nbits / 2) != 0;
   if (wide && a.nbits <= 16 && a.ds > 1 && a.ds <= 16 && a.pitch % F == 0 && reinterpret_cast<uintptr_t>(a.out) % 4 == 0) {
     for (int ph = 0; ph < a.ds; ++ph) {
       PrepArgs p = a;
@@ -1094,19 +1129,19 @@ void launch_prep(const PrepArgs& a, cudaStream_t st) {
       if (rows <= 0) continue;
       const PrepWords q{a.ds, (rows + F - 1) / F, a.ds * (a.pitch / F), F * a.ds, ph};
       const unsigned grid = blocks((q.nwords + 63) / 64, a.c0 & ~int64_t(3));
-      if (a.nbits == 8) k_prep_w<uint8_t, 0><<<grid, 256, 0, st>>>(p, q);
-      else k_prep_w<uint16_t, 0><<<grid, 256, 0, st>>>(p, q);
+      if (a.nbits == 8) run(k_prep_w<uint8_t, 0, false>, k_prep_w<uint8_t, 0, true>, grid, p, q, ragged);
+      else run(k_prep_w<uint16_t, 0, false>, k_prep_w<uint16_t, 0, true>, grid, p, q, ragged);
       DD_LAUNCHED();
     }
   } else if (wide && (a.fold > 1 || (a.ds == 1 && a.pitch % F == 0 && reinterpret_cast<uintptr_t>(a.out) % 4 == 0))) {
     const PrepWords q = a.fold > 1 ? PrepWords{a.seg, a.nwords, a.pitch, 1, 0}
                                    : PrepWords{1, (a.nsamp + F - 1) / F, a.pitch / F, F, 0};
     const unsigned grid = blocks((q.nwords + 63) / 64, a.c0 & ~int64_t(3));
-    if (a.nbits == 32) k_prep_w<uint32_t, 1><<<grid, 256, 0, st>>>(a, q);
-    else if (a.nbits == 8 && a.fold > 1) k_prep_w<uint8_t, 1><<<grid, 256, 0, st>>>(a, q);
-    else if (a.nbits == 8) k_prep_w<uint8_t, 4><<<grid, 256, 0, st>>>(a, q);
-    else if (a.fold > 1) k_prep_w<uint16_t, 1><<<grid, 256, 0, st>>>(a, q);
-    else k_prep_w<uint16_t, 2><<<grid, 256, 0, st>>>(a, q);
+    if (a.nbits == 32) run(k_prep_w<uint32_t, 1, false>, k_prep_w<uint32_t, 1, true>, grid, a, q, ragged);
+    else if (a.nbits == 8 && a.fold > 1) run(k_prep_w<uint8_t, 1, false>, k_prep_w<uint8_t, 1, true>, grid, a, q, ragged);
+    else if (a.nbits == 8) run(k_prep_w<uint8_t, 4, false>, k_prep_w<uint8_t, 4, true>, grid, a, q, ragged);
+    else if (a.fold > 1) run(k_prep_w<uint16_t, 1, false>, k_prep_w<uint16_t, 1, true>, grid, a, q, ragged);
+    else run(k_prep_w<uint16_t, 2, false>, k_prep_w<uint16_t, 2, true>, grid, a, q, ragged);
     DD_LAUNCHED();
   } else if (a.out && a.fold > 1) {
     const unsigned grid = blocks((a.nwords + 63) / 64, a.c0);

@@ -219,3 +219,19 @@ def test_layout_up_to_the_largest_delays(n, nchans, nbits, hi, band):
 def test_zero_dm_by_words(n, nchans, nbits, band):
     plan, x, want = subband(n, nchans, nbits, 20.0, 1.0, 1, 64, band, True, True)
     assert np.array_equal(to_np(plan.run(dev(x))), want)
+
+
+# Rows that start off a load word: binning by pairs and single channels, the layout's last
+# channels, masks and offsets beside them; a tile's remainders in time.
+@pytest.mark.parametrize("n,nchans,nbits,ds", [
+    (2561, 97, 8, 1), (4100, 98, 8, 2), (4099, 99, 8, 4), (1030, 66, 8, 3), (8200, 65, 8, 8),
+    (2050, 131, 16, 1), (2051, 130, 16, 2), (4103, 67, 16, 4),
+])
+def test_ragged_rows(n, nchans, nbits, ds):
+    plan, x, want = subband(n, nchans, nbits, 60.0, 0.5, ds, 16, 0.1, True, True)
+    assert np.array_equal(to_np(plan.run(dev(x))), want)
+
+
+@pytest.mark.parametrize("n,nchans,width", [(513, 37, 9), (2049, 131, 64)])
+def test_ragged_rows_of_32_bits(n, nchans, width):
+    test_32bit_layout_with_masks(n, nchans, width)
