@@ -754,7 +754,8 @@ extern "C" int dd_images(const void* dm_time, int32_t elem_bytes, int64_t nrows,
         }
         continue;
       }
-      const int64_t step = std::min<int64_t>(g.n, std::max<int64_t>(1, kHorizontalBytes / (npix * 4)));
+      // (a launch takes the slices as its grid's y: 65535 at most)
+      const int64_t step = std::min<int64_t>(std::min<int64_t>(g.n, 65535), std::max<int64_t>(1, kHorizontalBytes / (npix * 4)));
       for (int64_t g0 = 0; g0 < g.n; g0 += step) {
         ImgLaunch L{};
         float* img = float_images(step);
@@ -781,7 +782,7 @@ extern "C" int dd_images(const void* dm_time, int32_t elem_bytes, int64_t nrows,
         L.inv_area = inv_area;
         L.out = img;
         L.by_slot = resized ? 1 : 0;
-        const unsigned ns = static_cast<unsigned>(std::min<int64_t>(g.n - g0, std::min<int64_t>(step, 65535)));
+        const unsigned ns = static_cast<unsigned>(std::min(g.n - g0, step));
         k_resize<<<dim3(static_cast<unsigned>(target), ns), kImgThreads, 0, st>>>(L);
         DD_LAUNCHED();
         if (images) {
