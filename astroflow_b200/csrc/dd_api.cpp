@@ -374,17 +374,17 @@ void upload(DevBuf& b, const void* h, size_t bytes) {
 // 2^17 samples 8.67 -> 8.49 ms, a beam's push of 10,172 samples 1.10 -> 1.00 ms.
 void set_xlimit(dd_plan& P, int64_t first, int64_t nchan, int64_t cols) {
   const int64_t pad = first & 3, rows = static_cast<int64_t>(P.h_delay.size()) / nchan;
-  std::vector<int32_t> limit(static_cast<size_t>((pad + nchan + 63) / 64), 0);
+  std::vector<int64_t> limit(static_cast<size_t>((pad + nchan + 63) / 64), 0);
   for (int64_t r = 0; r < rows; ++r) {
     const int32_t* d = P.h_delay.data() + r * nchan;
     for (size_t g = 0; g < limit.size(); ++g) {
       const int64_t c0 = std::max<int64_t>(static_cast<int64_t>(g) * 64 - pad, 0);
       const int64_t c1 = std::min<int64_t>(static_cast<int64_t>(g + 1) * 64 - pad, nchan);
-      limit[g] = std::max(limit[g], *std::max_element(d + c0, d + c1));
+      limit[g] = std::max<int64_t>(limit[g], *std::max_element(d + c0, d + c1));
     }
   }
-  for (int32_t& v : limit) v = static_cast<int32_t>(std::min<int64_t>(v + cols, INT32_MAX));
-  upload(P.d_xlimit, limit.data(), sizeof(int32_t) * limit.size());
+  for (int64_t& v : limit) v += cols;  // (time order: up to 2^32 positions)
+  upload(P.d_xlimit, limit.data(), sizeof(int64_t) * limit.size());
 }
 
 // Time tiling of the subband path for a subband-sum budget (bytes per tile): the
@@ -759,7 +759,7 @@ void run_rfi_and_prep(dd_plan& P, const void* input, uint8_t* masks_out, uint32_
   a.fold = P.fold;
   a.seg = P.seg;
   a.nwords = std::min(P.nbin, P.xpitch);
-  a.limit = P.d_xlimit.as<int32_t>();
+  a.limit = P.d_xlimit.as<int64_t>();
   a.full_out = prepped;
   launch_prep(a, st);
 }
@@ -948,7 +948,7 @@ void run_brute_prep(dd_plan& P, const void* input, void* prepped, cudaStream_t s
   a.fold = P.fold;
   a.seg = P.seg;
   a.nwords = std::min(P.nin, P.xpitch);
-  a.limit = P.d_xlimit.as<int32_t>();
+  a.limit = P.d_xlimit.as<int64_t>();
   a.full_out = prepped;
   launch_prep(a, st);
 }

@@ -226,7 +226,7 @@ struct PrepArgs {
   int64_t seg, nwords;
   // per 64 channels from c0 & ~3 on: positions from here on are read by no sum and may be
   // left out (nullptr: write them all)
-  const int32_t* limit;
+  const int64_t* limit;
   void* full_out;          // optional [nsamp][nchans] copy after all stages
 };
 void launch_prep(const PrepArgs& a, cudaStream_t st);

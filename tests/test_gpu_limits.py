@@ -1,5 +1,5 @@
 """Calls at the limits of a launch, a row or the device: more slices than a grid dimension
-holds."""
+holds, rows of more than 2^31 samples."""
 import numpy as np
 import pytest
 
@@ -22,3 +22,21 @@ def test_more_slices_than_a_launch_takes():
     got = postprocess.device_images(d, starts, np.full(n, width), target=target).cpu().numpy()
     want = np.stack([CVI.image(raw[:, s:s + width], target) for s in range(7)])
     assert np.array_equal(got, want[starts])
+
+
+def test_rows_past_two_to_the_31():
+    """One trial (DM 0) over two channels of 32-bit samples longer than 2^31: the layout and
+    the sums reach the end of the rows (about 52 GB on the device)."""
+    from astroflow_b200.dedisp import Plan
+
+    n = 2 ** 31 + 4099
+    if torch.cuda.mem_get_info()[0] < 60e9:
+        pytest.skip("needs 60 GB of device memory")
+    x = torch.empty((n, 2), dtype=torch.int32, device="cuda").random_(0, 2 ** 31 - 1)
+    hdr = dict(tsamp=6.4e-5, fch1=1150.0, foff=1.0, nbits=32, nchans=2, ndata=n)
+    plan = Plan(hdr, 0.0, 0.0, 1150.0, 1151.0, 1.0, 1)
+    out = plan.run(x.view(torch.uint32)).view(torch.int64)
+    assert out.shape == (1, n)
+    for a in list(range(0, n, n // 5)) + [2 ** 31 - (1 << 20), 2 ** 31 - 70, n - 5000]:
+        b = min(n, a + (1 << 20))
+        assert torch.equal(out[0, a:b], x[a:b].to(torch.int64).sum(1)), a
