@@ -300,12 +300,16 @@ struct Prof {
   }
 };
 
-// Bytes of one staged window: the tile plus the rows' spread, 16-byte alignment
-// slack and the funnel shift's extra word; 0 when the four windows of a block
-// would not fit comfortably in shared memory.
-int window_bytes(int spread, int tile, int elem, int qs = 2) {
-  const int64_t w = round_up(static_cast<int64_t>(spread + tile) * elem + 40, 16);
-  return sum_smem_bytes(static_cast<int>(w), 2, qs) <= 200 * 1024 ? static_cast<int>(w) : 0;
+// Bytes of one staged window of a kernel variant: the tile plus the rows' spread, 16-byte
+// alignment slack and the funnel shift's extra word; 0 when the smallest ring (two stages
+// and the zeroed window) passes 200 KB, or a block's shared memory together with what the
+// variant stages past its ring and the kernels' own.
+int window_bytes(int spread, int kind) {
+  const int64_t w = round_up((static_cast<int64_t>(spread) + sum_kind_tile(kind)) * sum_kind_elem(kind) + 40, 16);
+  if (w > kSumBlockSmem) return 0;
+  const size_t ring = sum_smem_bytes(static_cast<int>(w), 2, sum_kind_qs(kind));
+  const bool fits = ring <= 200 * 1024 && ring + sum_kind_extra_smem(kind) + kSumStaticSmem <= kSumBlockSmem;
+  return fits ? static_cast<int>(w) : 0;
 }
 
 // Stage 1 adds the channels of a subband with the delays of kSumRows nominal DMs per
@@ -504,8 +508,8 @@ void create_subband(dd_plan& P) {
       P.small1 = blocks(stage1_kind(P), cols + P.max_res + P.max_skew1 / 2) * groups1 * P.nsb < kSumSmallBlocks;
       P.small2 = blocks(stage2_kind(P), cols) * groups2 * P.planes < kSumSmallBlocks;
       const int k1 = stage1_kind(P), k2 = stage2_kind(P);
-      P.win1 = window_bytes(spread1, sum_kind_tile(k1), sum_kind_elem(k1), sum_kind_qs(k1));
-      P.win2 = window_bytes(spread2, sum_kind_tile(k2), sum_kind_elem(k2), sum_kind_qs(k2));
+      P.win1 = window_bytes(spread1, k1);
+      P.win2 = window_bytes(spread2, k2);
     };
     set_windows(choose_fold(P, P.nout, P.dch, P.max_res + P.reach1, P.adds));
     if (P.fold > 1 && !(P.win1 && P.win2)) set_windows(1);  // the direct kernels read time order
@@ -586,8 +590,7 @@ void set_brute_window(dd_plan& P) {
       P.smallb = false;
       const int64_t cols = (P.out_cols + fold - 1) / fold, tile = sum_kind_tile(brute_kind(P));
       P.smallb = (cols + tile - 1) / tile * ((P.dm_steps + kSumRows - 1) / kSumRows) < kSumSmallBlocks;
-      const int k = brute_kind(P);
-      P.winb = window_bytes(spread, sum_kind_tile(k), sum_kind_elem(k), sum_kind_qs(k));
+      P.winb = window_bytes(spread, brute_kind(P));
     };
     set_window(choose_fold(P, P.out_cols, P.nc, P.max_delay, P.adds));
     if (P.fold > 1 && !P.winb) set_window(1);

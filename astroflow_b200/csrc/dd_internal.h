@@ -20,8 +20,10 @@ struct Error {
 #define DD_CUDA_TRY(call)                                                          \
   do {                                                                             \
     cudaError_t e_ = (call);                                                       \
-    if (e_ != cudaSuccess)                                                         \
+    if (e_ != cudaSuccess) {                                                       \
+      cudaGetLastError(); /* reported here: the thread's next check must not see it */ \
       throw ::dd::Error{DD_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_)}; \
+    }                                                                              \
   } while (0)
 
 // Kernel launches made by this library on the calling thread (monotonic).
@@ -359,6 +361,10 @@ struct SumLaunch {
 #define DD_SUM_SMEM_KB 100
 #endif
 constexpr int kSumMaxStages = DD_SUM_MAX_STAGES;  // groups of sources in flight, at most
+// Shared memory a block may have (227 KB on sm_100), and an upper bound of what the
+// staged-sum kernels declare statically (checked in dd_sumsmem.cu).
+constexpr size_t kSumBlockSmem = 227 * 1024;
+constexpr size_t kSumStaticSmem = 3072;
 void launch_sum(const SumLaunch& L, cudaStream_t st);
 int sum_tile_samples(int src_bytes, int nw);
 // Shared memory of a staged sum with `stages` pairs in flight.

@@ -1259,6 +1259,9 @@ __device__ __forceinline__ void run_one(const SumLaunch& L, uint3 blk, uint32_t*
   else sum_plane32<kPlane32RB, kPlane32NW>(L, blk, sw, P);
 }
 
+// Static shared memory of the largest staged-sum kernel (k_sum_batch).
+static_assert(sizeof(Pipe) + sizeof(SumLaunch) + 64 <= kSumStaticSmem, "window_bytes counts it");
+
 // Grouped launch: one grid over the blocks of several staged sums of the same
 // variant (the same stage of many plans), none of which reads another's output.
 template <int KIND>
