@@ -399,11 +399,11 @@ void set_tiling(dd_plan& P, int64_t budget) {
   const int copies = P.twin ? 2 : P.planes;
   P.seg = P.fold > 1 ? round_up((P.nout + P.fold - 1) / P.fold, 8) : P.nout;
   // The fewest tiles whose subband sums (tile and stage-2 halo) stay within the
-  // budget, all of the same length; chunks of 2^16 columns have two at least, so that
-  // the host path can copy one tile's columns out while the next is summed.
+  // budget, all of the same length: each costs stage 1 the halo and the skew of its rows
+  // once more (host_tile splits a single tile for the host path).
   const int64_t per_col = P.ndm_nom * P.nsb * inter_elem(P) * copies;
   const int64_t most = std::max<int64_t>(P.fold > 1 ? 1024 : kT, budget / per_col - P.max_res);
-  const int64_t ntiles = std::max<int64_t>((P.seg + most - 1) / most, P.nout >= 65536 ? 2 : 1);
+  const int64_t ntiles = (P.seg + most - 1) / most;
   const int64_t L = round_up((P.seg + ntiles - 1) / ntiles, 64);
   P.tile = L;
   P.inter_budget = budget;
@@ -502,7 +502,7 @@ void create_subband(dd_plan& P) {
       P.planes = fold == 1 ? 1 : P.inter16 ? 2 : fold;
       // blocks of one time tile with whole tiles of words
       P.small1 = P.small2 = false;
-      const int64_t cols = (P.nout + fold - 1) / fold / (P.nout >= 65536 ? 2 : 1);
+      const int64_t cols = (P.nout + fold - 1) / fold;
       const auto blocks = [&](int kind, int64_t c) { return (c + sum_kind_tile(kind) - 1) / sum_kind_tile(kind); };
       const int64_t groups1 = (P.ndm_nom + kSumRows - 1) / kSumRows, groups2 = P.ndm_nom * ((P.ndm0 + kSumRows - 1) / kSumRows);
       P.small1 = blocks(stage1_kind(P), cols + P.max_res + P.max_skew1 / 2) * groups1 * P.nsb < kSumSmallBlocks;
@@ -767,9 +767,16 @@ void run_rfi_and_prep(dd_plan& P, const void* input, uint8_t* masks_out, uint32_
   launch_prep(a, st);
 }
 
-// Staged-sum launches of one subband time tile starting at t0 (stage 1: the
+// Time tile of host-path runs: chunks of 2^16 columns take two at least, so that one
+// tile's columns are copied out while the next is summed (the copy takes longer than the
+// sums).
+int64_t host_tile(const dd_plan& P) {
+  return P.nout >= 65536 && P.tile >= P.seg ? round_up((P.seg + 1) / 2, 64) : P.tile;
+}
+
+// Staged-sum launches of the subband time tile [t0, t0 + tile) (stage 1: the
 // prepared input into the tile of subband sums; stage 2: the tile into the output).
-SumLaunch stage1_launch(const dd_plan& P, int64_t t0) {
+SumLaunch stage1_launch(const dd_plan& P, int64_t t0, int64_t tile) {
   SumLaunch L{};
   L.mode = SumLaunch::kStage1;
   L.kind = stage1_kind(P);
@@ -786,7 +793,7 @@ SumLaunch stage1_launch(const dd_plan& P, int64_t t0) {
   L.out_pitch = P.tile_pitch * inter_elem(P);
   L.out_col0 = 0;
   L.out_elem = static_cast<int>(inter_elem(P));
-  L.ncols = std::min<int64_t>(P.tile, P.seg - t0) + P.max_res;
+  L.ncols = std::min<int64_t>(tile, P.seg - t0) + P.max_res;
   L.seg_stride = plane_bytes(P);
   L.skew = P.d_skew1.as<int32_t>();
   L.max_skew = P.max_skew1;
@@ -801,7 +808,7 @@ SumLaunch stage1_launch(const dd_plan& P, int64_t t0) {
   return L;
 }
 
-SumLaunch stage2_launch(const dd_plan& P, int64_t t0, void* output) {
+SumLaunch stage2_launch(const dd_plan& P, int64_t t0, int64_t tile, void* output) {
   SumLaunch L{};
   L.mode = SumLaunch::kStage2;
   L.kind = stage2_kind(P);
@@ -816,7 +823,7 @@ SumLaunch stage2_launch(const dd_plan& P, int64_t t0, void* output) {
   L.out_pitch = P.nout * out_elem(P);
   L.out_col0 = t0;
   L.out_elem = out_elem(P);
-  L.ncols = std::min<int64_t>(P.tile, P.seg - t0);
+  L.ncols = std::min<int64_t>(tile, P.seg - t0);
   L.seg = P.seg;
   L.nout = P.nout;
   L.plane_bytes = plane_bytes(P);
@@ -839,19 +846,21 @@ using TileHook = std::function<void(int64_t, int64_t)>;
 // before_sums: called once the RFI stages and the layout are queued, before the
 // first sum that writes `output`.
 // before_out(t0, cols): called before the first launch that writes those columns.
+// tile: columns per time tile, at most the plan's (0: the plan's).
 void run_subband(dd_plan& P, const void* input, void* output, uint8_t* masks_out,
                  uint32_t* bounds_out, void* prepped, cudaStream_t st, Prof* pf = nullptr,
                  const TileHook& after_tile = TileHook(),
                  const std::function<void()>& before_sums = std::function<void()>(),
-                 const TileHook& before_out = TileHook()) {
+                 const TileHook& before_out = TileHook(), int64_t tile = 0) {
+  if (tile == 0) tile = P.tile;
   cudaEvent_t a = pf ? pf->mark() : nullptr;
   run_rfi_and_prep(P, input, masks_out, bounds_out, prepped, st);
   if (pf) pf->prep.emplace_back(a, pf->mark());
   if (before_sums) before_sums();
-  for (int64_t t0 = 0; t0 < P.seg; t0 += P.tile) {
+  for (int64_t t0 = 0; t0 < P.seg; t0 += tile) {
     cudaEvent_t b1 = pf ? pf->mark() : nullptr;
     if (P.win1) {
-      launch_sum(stage1_launch(P, t0), st);
+      launch_sum(stage1_launch(P, t0, tile), st);
     } else {
       Stage1Args s1{};
       s1.x = P.d_x.p;
@@ -863,17 +872,17 @@ void run_subband(dd_plan& P, const void* input, void* output, uint8_t* masks_out
       s1.ndm_nom = P.ndm_nom;
       s1.sbw = P.sbw;
       s1.t0 = t0;
-      s1.ncols = std::min<int64_t>(P.tile, P.seg - t0) + P.max_res;
+      s1.ncols = std::min<int64_t>(tile, P.seg - t0) + P.max_res;
       s1.inter = P.d_inter.p;
       s1.tile_pitch = P.tile_pitch;
       s1.inter16 = P.inter16;
       launch_stage1(s1, st);
     }
     if (pf) pf->s1.emplace_back(b1, pf->mark());
-    if (before_out) before_out(t0, std::min<int64_t>(P.tile, P.seg - t0));
+    if (before_out) before_out(t0, std::min<int64_t>(tile, P.seg - t0));
     cudaEvent_t b2 = pf ? pf->mark() : nullptr;
     if (P.win2) {
-      launch_sum(stage2_launch(P, t0, output), st);
+      launch_sum(stage2_launch(P, t0, tile, output), st);
     } else {
       Stage2Args s2{};
       s2.inter = P.d_inter.p;
@@ -883,7 +892,7 @@ void run_subband(dd_plan& P, const void* input, void* output, uint8_t* masks_out
       s2.nsb = P.nsb;
       s2.dm_steps = P.dm_steps;
       s2.ndm0 = P.ndm0;
-      s2.ncols = std::min<int64_t>(P.tile, P.nout - t0);
+      s2.ncols = std::min<int64_t>(tile, P.nout - t0);
       s2.out = output;
       s2.out_pitch = P.nout;
       s2.col0 = t0;
@@ -893,7 +902,7 @@ void run_subband(dd_plan& P, const void* input, void* output, uint8_t* masks_out
       launch_stage2(s2, st);
     }
     if (pf) pf->s2.emplace_back(b2, pf->mark());
-    if (after_tile) after_tile(t0, std::min<int64_t>(P.tile, P.seg - t0));
+    if (after_tile) after_tile(t0, std::min<int64_t>(tile, P.seg - t0));
   }
 }
 
@@ -1208,7 +1217,7 @@ int dd_plan_get_info(const dd_plan* P, dd_plan_info* info) {
     o.delay_rows = P->p.algorithm == DD_ALGO_BRUTE ? P->dm_steps : P->ndm_nom;
     o.delay_cols = P->p.algorithm == DD_ALGO_BRUTE ? P->nc : P->dch;
     o.table_mismatch_fp64 = P->table_mismatch_fp64;
-    o.tile_samples = P->tile * P->fold;
+    o.tile_samples = host_tile(*P) * P->fold;
     o.subband_sum_copies = P->p.algorithm == DD_ALGO_SUBBAND ? (P->twin ? 2 : 1) : 0;
     o.adds_per_run = P->adds;
     *info = o;
@@ -1305,7 +1314,7 @@ int dd_plan_autotune(dd_plan* P, const void* input, void* output, int32_t reps, 
     // stage counts that keep two blocks per SM for both stages
     auto fits = [&](int S) {
       if (S < 2 || S > kSumMaxStages) return false;
-      SumLaunch l1 = stage1_launch(*P, 0), l2 = stage2_launch(*P, 0, output);
+      SumLaunch l1 = stage1_launch(*P, 0, P->tile), l2 = stage2_launch(*P, 0, P->tile, output);
       l1.stages = l2.stages = S;
       return sum_launch_smem(l1) <= 113 * 1024 && sum_launch_smem(l2) <= 113 * 1024;
     };
@@ -1315,7 +1324,7 @@ int dd_plan_autotune(dd_plan* P, const void* input, void* output, int32_t reps, 
     rep.default_ms = time_shape();
     rep.best_ms = rep.default_ms;
     rep.best_budget_bytes = budget0;
-    rep.best_tile_samples = P->tile * P->fold;
+    rep.best_tile_samples = host_tile(*P) * P->fold;
     rep.best_stages = stages0;
     rep.candidates = 1;
     std::vector<int64_t> tiles_seen;
@@ -1337,7 +1346,7 @@ int dd_plan_autotune(dd_plan* P, const void* input, void* output, int32_t reps, 
         if (ms < rep.best_ms) {
           rep.best_ms = ms;
           rep.best_budget_bytes = budget;
-          rep.best_tile_samples = P->tile * P->fold;
+          rep.best_tile_samples = host_tile(*P) * P->fold;
           rep.best_stages = S;
         }
       }
@@ -1449,8 +1458,9 @@ void enqueue_host_run(dd_plan& P, const void* h_input, void* h_output, cudaStrea
       for (cudaEvent_t ev : evs) cudaEventDestroy(ev);
       for (cudaEvent_t ev : copied) cudaEventDestroy(ev);
     };
-    const bool same_tiling = P.host_pending && P.host_tile == P.tile &&
-                             P.host_tile_copied.size() == static_cast<size_t>((P.seg + P.tile - 1) / P.tile);
+    const int64_t tile = host_tile(P);
+    const bool same_tiling = P.host_pending && P.host_tile == tile &&
+                             P.host_tile_copied.size() == static_cast<size_t>((P.seg + tile - 1) / tile);
     try {
       run_subband(P, P.d_host_in.p, d_out, nullptr, nullptr, nullptr, st, nullptr,
                   [&](int64_t t0, int64_t n) {
@@ -1477,8 +1487,9 @@ void enqueue_host_run(dd_plan& P, const void* h_input, void* h_output, cudaStrea
                   },
                   [&](int64_t t0, int64_t) {
                     if (same_tiling)
-                      DD_CUDA_TRY(cudaStreamWaitEvent(st, P.host_tile_copied[t0 / P.tile], 0));
-                  });
+                      DD_CUDA_TRY(cudaStreamWaitEvent(st, P.host_tile_copied[t0 / tile], 0));
+                  },
+                  tile);
     } catch (...) {
       cudaStreamSynchronize(P.copy_stream);
       cleanup();
@@ -1488,7 +1499,7 @@ void enqueue_host_run(dd_plan& P, const void* h_input, void* h_output, cudaStrea
     for (cudaEvent_t ev : evs) cudaEventDestroy(ev);
     for (cudaEvent_t ev : P.host_tile_copied) cudaEventDestroy(ev);
     P.host_tile_copied.swap(copied);
-    P.host_tile = P.tile;
+    P.host_tile = tile;
   }
   DD_CUDA_TRY(cudaEventRecord(P.host_done, P.copy_stream));
   P.host_pending = true;
@@ -1601,8 +1612,8 @@ bool batched_plan(const dd_plan& P, bool persistent) {
   if (!persistent) return true;
   if (brute && P.p.time_downsample > 1) return false;  // no phase-row kernel in k_sum_batch
   return brute ? sum_launch_smem(brute_launch(P, nullptr)) <= kBatchSmemCap
-               : sum_launch_smem(stage1_launch(P, 0)) <= kBatchSmemCap &&
-                     sum_launch_smem(stage2_launch(P, 0, nullptr)) <= kBatchSmemCap;
+               : sum_launch_smem(stage1_launch(P, 0, P.tile)) <= kBatchSmemCap &&
+                     sum_launch_smem(stage2_launch(P, 0, P.tile, nullptr)) <= kBatchSmemCap;
 }
 
 long long group_blocks(const SumBatchGroup& g) {
@@ -1641,8 +1652,8 @@ void build_groups(dd_batch& B, void* const* outputs) {
         continue;
       }
       if (k * P.tile >= P.seg) continue;
-      stage[2 * k].emplace_back(p, stage1_launch(P, k * P.tile));
-      stage[2 * k + 1].emplace_back(p, stage2_launch(P, k * P.tile, outputs[p]));
+      stage[2 * k].emplace_back(p, stage1_launch(P, k * P.tile, P.tile));
+      stage[2 * k + 1].emplace_back(p, stage2_launch(P, k * P.tile, P.tile, outputs[p]));
     }
   int dev = 0, sms = 0;
   DD_CUDA_TRY(cudaGetDevice(&dev));

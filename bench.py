@@ -1042,7 +1042,7 @@ def main():
     bytes_per_unit = (wl["nsamp"] * wl["nchans"] * wl["nbits"] / 8 + units * 4) / units
     elem = wl["nbits"] // 8
     if wl["algorithm"] == "subband":
-        tile = min(int(info["nsamp_binned"]), int(info["tile_samples"]))
+        tile = -(-int(info["out_cols"]) // s1n)  # columns per launch
         dch = info["chan_end"] - info["chan_start"] + 1
         # bytes of one subband sum: 16-bit for 8-bit samples in subbands of <= 64
         # channels, else the reference's accumulator type

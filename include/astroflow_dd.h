@@ -170,7 +170,9 @@ typedef struct dd_plan_info {
   int64_t delay_rows;        /* rows of the delay table (ndm_nom or dm_steps) */
   int64_t delay_cols;        /* columns of the delay table (channels) */
   int64_t table_mismatch_fp64; /* delay entries where the table differs from the FP64 table */
-  int64_t tile_samples;      /* time samples per stage-1/stage-2 launch (subband) */
+  int64_t tile_samples;      /* time samples per tile of a host-buffer run (subband); runs on
+                                device buffers take the fewest tiles their subband sums' budget
+                                allows: one where these are its only two */
   double adds_per_run;       /* algorithmic integer additions per dd_run */
   int64_t subband_sum_copies; /* copies of each stage-1 sum in device memory: 2 when stage 1
                                  also writes the one-sample-shifted twin stage 2 reads, else 1 */

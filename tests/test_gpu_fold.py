@@ -235,3 +235,23 @@ def test_ragged_rows(n, nchans, nbits, ds):
 @pytest.mark.parametrize("n,nchans,width", [(513, 37, 9), (2049, 131, 64)])
 def test_ragged_rows_of_32_bits(n, nchans, width):
     test_32bit_layout_with_masks(n, nchans, width)
+
+
+# A chunk whose subband sums fit the budget is summed as one time tile (each tile costs stage
+# 1 the stage-2 halo and the skew of its rows again); the host path splits it to copy the
+# first half out meanwhile.
+@pytest.mark.parametrize("spec", [(70001, 64, 8, 400.0, 2.0, 1, 16, 0.0, False, False),
+                                  (66000, 48, 16, 3000.0, 100.0, 1, 16, 0.0, False, False)])
+def test_one_time_tile_where_the_sums_fit(spec):
+    plan, x, want = subband(*spec)
+    xd = dev(x)
+    assert plan.run_profiled(xd)["stage1_launches"] == 1
+    assert np.array_equal(to_np(plan.run(xd)), want)
+    outs = [np.empty(want.shape, np.uint32) for _ in range(3)]
+    for i in range(3):
+        plan.run_host_async(x, outs[i])
+        if i == 1:
+            assert np.array_equal(to_np(plan.run(xd)), want)
+    plan.run_host_join(sync=True)
+    for o in outs:
+        assert np.array_equal(o, want)
