@@ -65,12 +65,13 @@ int stage1_kind(const dd_plan& P) {
     const int k = P.nbits == 16 ? kSumKindFold16 : P.inter16 ? kSumKindFold8 : kSumKindFold8W;
     return P.small1 ? sum_kind_small(k) : k;
   }
-  return P.nbits == 16 ? kSumKindU16Wide : P.inter16 ? kSumKindU8Out16 : kSumKindU8Flush;
+  const int k = P.nbits == 16 ? kSumKindU16Wide : P.inter16 ? kSumKindU8Out16 : kSumKindU8Flush;
+  return P.few1 ? sum_kind_rows8(k) : k;
 }
 int stage2_kind(const dd_plan& P) {
   if (P.nbits == 32) return kSumKindPlane64;
   const int k = !P.inter16 ? kSumKindPlane32 : P.fold > 1 ? kSumKindPlane16 : kSumKindU16Twin;
-  return P.small2 ? sum_kind_small(k) : k;
+  return P.few2 ? sum_kind_rows8(k) : P.small2 ? sum_kind_small(k) : k;
 }
 int brute_kind(const dd_plan& P) {
   if (P.nbits == 32) return kSumKindWord64;
@@ -79,7 +80,8 @@ int brute_kind(const dd_plan& P) {
     const int k = P.nbits == 16 ? kSumKindFold16 : kSumKindFold8W;
     return P.smallb ? sum_kind_small(k) : k;
   }
-  return P.nbits == 16 ? kSumKindU16Wide : kSumKindU8Flush;
+  const int k = P.nbits == 16 ? kSumKindU16Wide : kSumKindU8Flush;
+  return P.fewb ? sum_kind_rows8(k) : k;
 }
 // Samples per folded word, or 1 where the fold does not pay.  A folded word holds the
 // samples of the segments at one position, so all positions up to a segment and the
@@ -312,24 +314,28 @@ int window_bytes(int spread, int kind) {
   return fits ? static_cast<int>(w) : 0;
 }
 
-// Stage 1 adds the channels of a subband with the delays of kSumRows nominal DMs per
+// Stage 1 adds the channels of a subband with the delays of `rows` nominal DMs per
 // block.  At one output column those delays lie far apart at the low end of the
 // band (5,250 samples for 8 rows of a 4096-channel chunk to DM 3000), so each row is
 // shifted by its smallest delay in the subband (rounded down to 16 samples, which
 // keeps its stores aligned): what is left, a delay's growth inside the subband, is
-// at most a few hundred samples.  Returns the shifted table and fills the skews
-// ([row group][subband][kSumRows], relative to the group's first row) and the reach
-// of the windows.
-std::vector<int32_t> skew_stage1(dd_plan& P, std::vector<int32_t>& skew) {
-  const int64_t ngrp = (P.ndm_nom + kSumRows - 1) / kSumRows;
-  skew.assign(static_cast<size_t>(ngrp * P.nsb * kSumRows), 0);
+// at most a few hundred samples.
+struct Stage1Tables {
+  std::vector<int32_t> skew;  // [row group][subband][kSumRows], relative to the group's first row
+  std::vector<SumDesc> desc;  // of the shifted delays
+  int spread = 0;
+  int64_t max_skew = 0, reach = 0, max_off = 0;  // as in dd_plan
+};
+Stage1Tables stage1_tables(const dd_plan& P, int rows) {
+  Stage1Tables t;
+  const int64_t ngrp = (P.ndm_nom + rows - 1) / rows;
+  t.skew.assign(static_cast<size_t>(ngrp * P.nsb * kSumRows), 0);
   std::vector<int32_t> tab(P.h_delay);
-  P.max_skew1 = P.reach1 = P.max_off1 = 0;
   for (int64_t g = 0; g < ngrp; ++g)
     for (int64_t sb = 0; sb < P.nsb; ++sb) {
       const int64_t c0 = sb * P.sbw, c1 = std::min<int64_t>(c0 + P.sbw, P.dch);
-      int32_t* sk = skew.data() + (g * P.nsb + sb) * kSumRows;
-      const int64_t r0 = g * kSumRows, r1 = std::min(r0 + kSumRows, P.ndm_nom);
+      int32_t* sk = t.skew.data() + (g * P.nsb + sb) * kSumRows;
+      const int64_t r0 = g * rows, r1 = std::min(r0 + rows, P.ndm_nom);
       int least[kSumRows], last = 0, reach = 0;
       bool grows = true;  // delays grow with the DM (kernels rely on it for the skews)
       for (int64_t r = r0; r < r1; ++r) {
@@ -346,11 +352,12 @@ std::vector<int32_t> skew_stage1(dd_plan& P, std::vector<int32_t>& skew) {
           reach = std::max(reach, row[c]);
         }
       }
-      P.max_skew1 = std::max<int64_t>(P.max_skew1, last);
-      P.reach1 = std::max<int64_t>(P.reach1, last + reach);
-      P.max_off1 = std::max<int64_t>(P.max_off1, reach);
+      t.max_skew = std::max<int64_t>(t.max_skew, last);
+      t.reach = std::max<int64_t>(t.reach, last + reach);
+      t.max_off = std::max<int64_t>(t.max_off, reach);
     }
-  return tab;
+  t.desc = build_sum_desc(tab, P.ndm_nom, P.dch, 0, &t.spread, rows);
+  return t;
 }
 
 void upload_desc(DevBuf& b, const std::vector<SumDesc>& d) {
@@ -491,12 +498,9 @@ void create_subband(dd_plan& P) {
   P.adds = static_cast<double>(P.ndm_nom) * P.dch * P.nout +
            static_cast<double>(P.dm_steps) * P.nsb * P.nout;
   {
-    std::vector<int32_t> skew;
-    const std::vector<int32_t> tab = skew_stage1(P, skew);
-    int spread1 = 0, spread2 = 0;
-    const std::vector<SumDesc> desc1 = build_sum_desc(tab, P.ndm_nom, P.dch, 0, &spread1);
-    const std::vector<SumDesc> desc2 = build_sum_desc(P.h_res, P.dm_steps, P.nsb, P.ndm0, &spread2);
-    P.spread1 = spread1;
+    Stage1Tables t1 = stage1_tables(P, kSumRows);
+    int spread2 = 0;
+    std::vector<SumDesc> desc2 = build_sum_desc(P.h_res, P.dm_steps, P.nsb, P.ndm0, &spread2);
     auto set_windows = [&](int fold) {
       P.fold = fold;
       P.planes = fold == 1 ? 1 : P.inter16 ? 2 : fold;
@@ -505,23 +509,48 @@ void create_subband(dd_plan& P) {
       const int64_t cols = (P.nout + fold - 1) / fold;
       const auto blocks = [&](int kind, int64_t c) { return (c + sum_kind_tile(kind) - 1) / sum_kind_tile(kind); };
       const int64_t groups1 = (P.ndm_nom + kSumRows - 1) / kSumRows, groups2 = P.ndm_nom * ((P.ndm0 + kSumRows - 1) / kSumRows);
-      P.small1 = blocks(stage1_kind(P), cols + P.max_res + P.max_skew1 / 2) * groups1 * P.nsb < kSumSmallBlocks;
+      P.small1 = blocks(stage1_kind(P), cols + P.max_res + t1.max_skew / 2) * groups1 * P.nsb < kSumSmallBlocks;
       P.small2 = blocks(stage2_kind(P), cols) * groups2 * P.planes < kSumSmallBlocks;
-      const int k1 = stage1_kind(P), k2 = stage2_kind(P);
-      P.win1 = window_bytes(spread1, k1);
-      P.win2 = window_bytes(spread2, k2);
+      P.win1 = window_bytes(t1.spread, stage1_kind(P));
+      P.win2 = window_bytes(spread2, stage2_kind(P));
     };
-    set_windows(choose_fold(P, P.nout, P.dch, P.max_res + P.reach1, P.adds));
+    set_windows(choose_fold(P, P.nout, P.dch, P.max_res + t1.reach, P.adds));
     if (P.fold > 1 && !(P.win1 && P.win2)) set_windows(1);  // the direct kernels read time order
+    if (P.fold == 1 && P.nbits <= 16) {
+      // coarse trial steps: eight rows a block (sum_kind_rows8)
+      if (!P.win1) {
+        Stage1Tables t = stage1_tables(P, 8);
+        P.few1 = true;
+        P.win1 = window_bytes(t.spread, stage1_kind(P));
+        if (P.win1) t1 = std::move(t);
+        else P.few1 = false;
+      }
+      if (!P.win2 || (!P.small2 && spread2 > 2 * sum_kind_tile(stage2_kind(P)))) {
+        int spread = 0;
+        std::vector<SumDesc> d = build_sum_desc(P.h_res, P.dm_steps, P.nsb, P.ndm0, &spread, 8);
+        P.few2 = true;
+        const int w = window_bytes(spread, stage2_kind(P));
+        if (w) {
+          P.win2 = w;
+          desc2 = std::move(d);
+        } else {
+          P.few2 = false;
+        }
+      }
+    }
     if (P.fold == 1 && P.inter16) {
       // 16-bit sums in time order: the staged stage 2 reads the twin that the staged
       // stage 1 writes
       P.twin = (P.win1 && P.win2) ? 1 : 0;
       if (!P.twin) P.win2 = 0;
     }
+    P.spread1 = t1.spread;
+    P.max_skew1 = t1.max_skew;
+    P.reach1 = t1.reach;
+    P.max_off1 = t1.max_off;
     if (P.win1) {
-      upload_desc(P.d_desc1, desc1);
-      upload(P.d_skew1, skew.data(), sizeof(int32_t) * skew.size());
+      upload_desc(P.d_desc1, t1.desc);
+      upload(P.d_skew1, t1.skew.data(), sizeof(int32_t) * t1.skew.size());
     }
     if (P.win2) upload_desc(P.d_desc2, desc2);
   }
@@ -584,7 +613,8 @@ void set_brute_window(dd_plan& P) {
   if (P.p.time_downsample > 1) {
     set_phase_window(P);
   } else {
-    const std::vector<SumDesc> desc = build_sum_desc(P.h_delay, P.dm_steps, P.nc, 0, &spread);
+    std::vector<SumDesc> desc = build_sum_desc(P.h_delay, P.dm_steps, P.nc, 0, &spread);
+    P.fewb = false;
     auto set_window = [&](int fold) {
       P.fold = fold;
       P.smallb = false;
@@ -594,6 +624,11 @@ void set_brute_window(dd_plan& P) {
     };
     set_window(choose_fold(P, P.out_cols, P.nc, P.max_delay, P.adds));
     if (P.fold > 1 && !P.winb) set_window(1);
+    if (P.fold == 1 && P.nbits <= 16 && !P.winb) {
+      P.fewb = true;  // coarse trial steps
+      desc = build_sum_desc(P.h_delay, P.dm_steps, P.nc, 0, &spread, sum_kind_rows(brute_kind(P)));
+      P.winb = window_bytes(spread, brute_kind(P));
+    }
     if (P.winb) upload_desc(P.d_descb, desc);
   }
   P.seg = P.fold > 1 ? round_up((P.out_cols + P.fold - 1) / P.fold, 8) : P.out_cols;
@@ -798,7 +833,7 @@ SumLaunch stage1_launch(const dd_plan& P, int64_t t0, int64_t tile) {
   L.skew = P.d_skew1.as<int32_t>();
   L.max_skew = P.max_skew1;
   L.win_bytes = P.win1;
-  L.grid_y = static_cast<unsigned>((P.ndm_nom + kSumRows - 1) / kSumRows);
+  L.grid_y = static_cast<unsigned>((P.ndm_nom + sum_kind_rows(L.kind) - 1) / sum_kind_rows(L.kind));
   L.grid_z = static_cast<unsigned>(P.nsb);
   L.desc = P.d_desc1.as<SumDesc>();
   L.desc_pitch = P.dch;
@@ -828,7 +863,7 @@ SumLaunch stage2_launch(const dd_plan& P, int64_t t0, int64_t tile, void* output
   L.nout = P.nout;
   L.plane_bytes = plane_bytes(P);
   L.win_bytes = P.win2;
-  L.grid_y = static_cast<unsigned>(P.ndm_nom * ((P.ndm0 + kSumRows - 1) / kSumRows));
+  L.grid_y = static_cast<unsigned>(P.ndm_nom * ((P.ndm0 + sum_kind_rows(L.kind) - 1) / sum_kind_rows(L.kind)));
   L.grid_z = static_cast<unsigned>(P.planes);
   L.desc = P.d_desc2.as<SumDesc>();
   L.desc_pitch = P.nsb;
@@ -937,7 +972,7 @@ SumLaunch brute_launch(const dd_plan& P, void* output) {
     L.desc_pattern = P.pattern_descs;
     if (!P.phases_merge) L.ncols = P.cols0;  // per slice; merged, the chunk is one slice
   }
-  L.grid_y = static_cast<unsigned>((P.dm_steps + kSumRows - 1) / kSumRows);
+  L.grid_y = static_cast<unsigned>((P.dm_steps + sum_kind_rows(L.kind) - 1) / sum_kind_rows(L.kind));
   L.grid_z = L.ds > 1 && !P.phases_merge ? static_cast<unsigned>(P.nslices) : 1;
   L.desc = P.d_descb.as<SumDesc>();
   L.desc_pitch = P.nc;
@@ -1611,6 +1646,7 @@ bool batched_plan(const dd_plan& P, bool persistent) {
   if (brute ? !P.winb : (!P.win1 || !P.win2)) return false;
   if (!persistent) return true;
   if (brute && P.p.time_downsample > 1) return false;  // no phase-row kernel in k_sum_batch
+  if (P.few1 || P.few2 || P.fewb) return false;        // nor the forms of eight rows
   return brute ? sum_launch_smem(brute_launch(P, nullptr)) <= kBatchSmemCap
                : sum_launch_smem(stage1_launch(P, 0, P.tile)) <= kBatchSmemCap &&
                      sum_launch_smem(stage2_launch(P, 0, P.tile, nullptr)) <= kBatchSmemCap;

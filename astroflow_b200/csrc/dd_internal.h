@@ -91,6 +91,7 @@ struct dd_plan {
   int64_t xpitch = 0;        // row pitch of the channel-major prepared input (elements)
   int win1 = 0, win2 = 0;    // staged window bytes of the shared-memory sums (0: not used)
   bool small1 = false, small2 = false, smallb = false;  // half tiles (sum_kind_small): stages, brute force
+  bool few1 = false, few2 = false, fewb = false;        // eight rows a block (sum_kind_rows8)
   int64_t max_skew1 = 0;     // largest row skew of stage 1
   int64_t reach1 = 0;        // largest offset a stage-1 window reads past its column
   int64_t spread1 = 0;       // largest spread of a stage-1 window
@@ -377,12 +378,12 @@ int sum_stages(int win_bytes, int qs = 2, size_t extra = 0, int cap_kb = 0);
 // Stages of a kernel variant for a window size (its windows per stage, staging
 // and shared-memory cap).
 int sum_kind_stages(int kind, int win_bytes);
-// Descriptors of a [nrows][ncols] offset table for row groups of kSumRows rows,
+// Descriptors of a [nrows][ncols] offset table for row groups of `rows` rows,
 // grouped within blocks of `group` rows (0: one block), in the launch's
 // blockIdx.y order, and the largest spread of a group's offsets (a window that holds
 // more than 65535 never fits shared memory, window_bytes).
 std::vector<SumDesc> build_sum_desc(const std::vector<int32_t>& tab, int64_t nrows,
-                                    int64_t ncols, int64_t group, int* spread);
+                                    int64_t ncols, int64_t group, int* spread, int rows = kSumRows);
 // Device error codes of the staged sums.
 constexpr int kErrWaitFull = 1;   // a consumer gave up waiting for a staged window
 constexpr int kErrWaitEmpty = 2;  // the producer gave up waiting for a free stage
@@ -412,6 +413,7 @@ constexpr int kSum16TNW = DD_SUM16T_NW;
 // tile takes fewer words than the chunk-long sums (1000 channels, 61,441 samples, bins of
 // two, 501 trials: 5 / 7 / 9 words 1.31 / 1.19 / 1.46 ms).
 constexpr int kPhase8NW = DD_PHASE8_NW;
+constexpr int kFlush8R8NW = 7;
 // Folded sums: rows per thread, words per lane and blocks per SM.  Few rows of many
 // words: a row of a stage costs one load of its offsets and four addresses whatever its
 // words.  Measured (4096 channels, 2^17 samples, 6001 trials, stage 1 / stage 2, ms; and
@@ -479,7 +481,9 @@ enum SumKind { kSumKindU8Out16, kSumKindU8Flush, kSumKindU16Wide, kSumKindU16Twi
                kSumKindU8Phase, kSumKindU16Phase, kSumKindFold8,
                kSumKindFold8W, kSumKindFold16, kSumKindPlane16, kSumKindPlane32,
                kSumKindFold8S, kSumKindFold8WS, kSumKindFold16S, kSumKindPlane16S, kSumKindPlane32S,
-               kSumKindWord64, kSumKindPlane64, kSumKinds };
+               kSumKindWord64, kSumKindPlane64,
+               kSumKindU8Out16R8, kSumKindU8FlushR8, kSumKindU16WideR8, kSumKindU16TwinR8,
+               kSumKindPlane32R8, kSumKinds };
 // The folded variants and Plane32 have a second form with tiles of half the words (S) for
 // launches that do not fill the GPU: a launch of fewer blocks than four per SM is bound by
 // the latency of one block.  336 channels, 5120 samples, 591 trials: 32.9 -> 24.8 us a
@@ -488,6 +492,28 @@ inline int sum_kind_small(int kind) {
   return kind >= kSumKindFold8 && kind <= kSumKindPlane32 ? kind + (kSumKindFold8S - kSumKindFold8) : kind;
 }
 constexpr long long kSumSmallBlocks = 4 * 148;
+// Time-order variants of eight rows a block (R8), on tiles twice as long (U8FlushR8: seven
+// words a lane, so that its staging past the ring leaves room for wider windows).  A
+// window holds the spread of its rows' delays, which grows with the trial step, and half the
+// rows spread half as far: where sixteen rows' windows pass shared memory these serve
+// instead of the direct kernels.  1024 channels, 2^17 samples, 96 brute-force trials:
+// 8 bits, 16-row spread 37,300 samples 10.4 -> 1.23 ms; 16 bits, 19,400 samples 11.9 -> 2.0
+// ms; stage 2 of 16-bit samples, 512 trials spreading over 4,900 samples per 16 2.10 -> 0.31
+// ms.  Stage 2 takes them already where 16 rows spread over more than two tiles: both
+// forms then stage as many bytes per addition, and wide windows leave fewer blocks per SM
+// (16 rows / 8 rows: twin, 2,820 samples 0.55 / 0.32 ms; 32-bit sums 0.38 / 0.30).
+inline int sum_kind_rows8(int kind) {
+  switch (kind) {
+    case kSumKindU8Out16: return kSumKindU8Out16R8;
+    case kSumKindU8Flush: return kSumKindU8FlushR8;
+    case kSumKindU16Wide: return kSumKindU16WideR8;
+    case kSumKindU16Twin: return kSumKindU16TwinR8;
+    case kSumKindPlane32: case kSumKindPlane32S: return kSumKindPlane32R8;
+    default: return kind;
+  }
+}
+// Output rows of a block.
+inline int sum_kind_rows(int kind) { return kind >= kSumKindU8Out16R8 ? 8 : kSumRows; }
 int sum_kind(const SumLaunch& L);
 // Tile of a kernel variant: samples per block, or words for the folded sums and Plane32.
 inline int sum_kind_tile(int kind) {
@@ -508,18 +534,29 @@ inline int sum_kind_tile(int kind) {
     case kSumKindPlane16S: return words(kPlane16RB, kPlane16NW / 2);
     case kSumKindPlane32S: return words(kPlane32RB, kPlane32NW / 2);
     case kSumKindWord64: case kSumKindPlane64: return words(kTo64RB, kTo64NW);
+    case kSumKindU8Out16R8: return sum_tile_samples(1, DD_SUM8_NW) * kSumRowsPT8 / 8;
+    case kSumKindU8FlushR8: return sum_tile_samples(1, kFlush8R8NW) * kSumRowsPT8 / 8;
+    case kSumKindU16WideR8: return sum_tile_samples(2, DD_SUM16W_NW) * kSumRowsPTW / 8;
+    case kSumKindU16TwinR8: return sum_tile_samples(2, kSum16TNW) * kSumRowsPTT / 8;
+    case kSumKindPlane32R8: return sum_tile_samples(4, kPlane32NW) * kPlane32RB / 8;
     default: return words(kPlane32RB, kPlane32NW);
   }
 }
 // Source windows per pipeline stage of a kernel variant.
 inline int sum_kind_qs(int kind) {
-  return kind == kSumKindU16Twin ? 8 : kind >= kSumKindFold8 ? 4 : 2;
+  if (kind == kSumKindU16Twin || kind == kSumKindU16TwinR8) return 8;
+  return kind >= kSumKindFold8 && kind < kSumKindU8Out16R8 ? 4 : 2;
 }
 // Bytes of a source element: samples, 16-bit sums or words.
 inline int sum_kind_elem(int kind) {
-  return kind == kSumKindU8Out16 || kind == kSumKindU8Flush || kind == kSumKindU8Phase ? 1
-         : kind == kSumKindPlane64                                                       ? 8
-         : kind >= kSumKindFold8                                                         ? 4 : 2;
+  switch (kind) {
+    case kSumKindU8Out16: case kSumKindU8Flush: case kSumKindU8Phase:
+    case kSumKindU8Out16R8: case kSumKindU8FlushR8: return 1;
+    case kSumKindU16Wide: case kSumKindU16Twin: case kSumKindU16Phase:
+    case kSumKindU16WideR8: case kSumKindU16TwinR8: return 2;
+    case kSumKindPlane64: return 8;
+    default: return 4;
+  }
 }
 // Shared memory of a launch (its variant's windows per stage, plus the variant's
 // staging past the ring, sum_kind_extra_smem).

@@ -4,7 +4,8 @@
 //
 //   out[r][t] = sum_i src_i[base + off(r, i) + t],   t in [0, T) of the block's tile.
 //
-// A block owns kSumRows output rows, dealt to its warp groups (RB rows each), and T
+// A block owns kSumRows output rows (eight where coarse trial steps spread them too far,
+// sum_kind_rows8), dealt to its warp groups (RB rows each), and T
 // consecutive words of them.  Sources are processed in groups of two or four.  The time
 // window of each source that the block's rows need,
 // [base + min_r off, base + max_r off + T), is brought into shared memory by one
@@ -150,7 +151,7 @@ __device__ __forceinline__ int64_t row_col(const Geo& g, int r) {
   return g.col - (g.skew ? __ldg(g.skew + r) : 0);
 }
 
-template <bool PHASES = false>
+template <bool PHASES = false, int ROWS = kSumRows>
 __device__ __forceinline__ Geo make_geo(const SumLaunch& L, int T, uint3 blk) {
   Geo g;
   const int64_t tile = blk.x;
@@ -162,13 +163,13 @@ __device__ __forceinline__ Geo make_geo(const SumLaunch& L, int T, uint3 blk) {
   switch (L.mode) {
     case SumLaunch::kStage1: {
       // rows: nominal DMs j0.. of subband sb; sources: the subband's channels
-      const int64_t j0 = static_cast<int64_t>(blk.y) * kSumRows;
+      const int64_t j0 = static_cast<int64_t>(blk.y) * ROWS;
       const int64_t sb = blk.z;
       const int64_t c0 = sb * L.group;
       g.src = L.src + c0 * L.src_pitch;
       g.desc = drow + c0;
       g.nsrc = static_cast<int>(min(static_cast<int64_t>(L.group), L.nsrc_total - c0));
-      g.nrows = static_cast<int>(min(static_cast<int64_t>(kSumRows), L.nrows_total - j0));
+      g.nrows = static_cast<int>(min(static_cast<int64_t>(ROWS), L.nrows_total - j0));
       g.out = L.out + (j0 * L.nsb_out + sb) * L.out_pitch + L.out_col0 * L.out_elem;
       g.out_pitch = L.nsb_out * L.out_pitch;
       g.skew = L.skew + (static_cast<int64_t>(blk.y) * L.nsb_out + sb) * kSumRows;
@@ -176,24 +177,24 @@ __device__ __forceinline__ Geo make_geo(const SumLaunch& L, int T, uint3 blk) {
     }
     case SumLaunch::kStage2: {
       // rows: fine DMs of nominal DM j; sources: the subband sums of j
-      const int per_nom = (L.group + kSumRows - 1) / kSumRows;
+      const int per_nom = (L.group + ROWS - 1) / ROWS;
       const int64_t j = blk.y / per_nom;
-      const int64_t m0 = j * L.group + static_cast<int64_t>(blk.y % per_nom) * kSumRows;
+      const int64_t m0 = j * L.group + static_cast<int64_t>(blk.y % per_nom) * ROWS;
       const int64_t mend = min((j + 1) * L.group, L.nrows_total);
       g.src = L.src + blk.z * L.plane_bytes + j * L.nsrc_total * L.src_pitch;
       g.desc = drow;
       g.nsrc = static_cast<int>(L.nsrc_total);
-      g.nrows = static_cast<int>(max(static_cast<int64_t>(0), min(static_cast<int64_t>(kSumRows), mend - m0)));
+      g.nrows = static_cast<int>(max(static_cast<int64_t>(0), min(static_cast<int64_t>(ROWS), mend - m0)));
       g.out = L.out + m0 * L.out_pitch + L.out_col0 * L.out_elem;
       g.out_pitch = L.out_pitch;
       break;
     }
     default: {  // brute force: rows = DMs, sources = channels
-      const int64_t m0 = static_cast<int64_t>(blk.y) * kSumRows;
+      const int64_t m0 = static_cast<int64_t>(blk.y) * ROWS;
       g.src = L.src;
       g.desc = drow;
       g.nsrc = static_cast<int>(L.nsrc_total);
-      g.nrows = static_cast<int>(min(static_cast<int64_t>(kSumRows), L.nrows_total - m0));
+      g.nrows = static_cast<int>(min(static_cast<int64_t>(ROWS), L.nrows_total - m0));
       g.out = L.out + m0 * L.out_pitch + L.out_col0 * L.out_elem;
       g.out_pitch = L.out_pitch;
       if constexpr (PHASES) {
@@ -372,25 +373,25 @@ __device__ __forceinline__ void produce_twin(const Geo& g, Pipe& P, uint32_t* sw
     }
 }
 
-// The same for sources of 32-bit words (folded samples and their sums), four per
+// The same for sources of 32-bit words (folded samples and their sums), QS per
 // stage: every offset is a whole word, so a row's offset needs no shift.  EW words per
 // element: 1, or 2 for 64-bit sums (offsets and tile in elements).
-template <int EW>
+template <int EW, int QS>
 __device__ __forceinline__ void produce_words(const Geo& g, Pipe& P, uint32_t* sw, int ww, int zero_q,
-                                              int tile, const GroupDesc<4>& d, int q, int s, int lane) {
+                                              int tile, const GroupDesc<QS>& d, int q, int s, int lane) {
   const int i = lane >> 4, r = lane & 15;
-  uint32_t nbytes[2] = {0, 0};
-  const char* gsrc[2] = {nullptr, nullptr};
+  uint32_t nbytes[QS / 2] = {};
+  const char* gsrc[QS / 2] = {};
 #pragma unroll
-  for (int h = 0; h < 2; ++h) {
+  for (int h = 0; h < QS / 2; ++h) {
     const int k = i + 2 * h;  // source of the stage
-    const int src = 4 * q + k;
+    const int src = QS * q + k;
     int idx = zero_q;
     const int64_t e0 = g.base + d.lo[h];
     if (src < g.nsrc && e0 < g.valid) {
       constexpr int kAlign = 4 / EW - 1;  // elements of a 16-byte unit, less one
       const int64_t a0 = e0 & ~int64_t(kAlign);
-      idx = (4 * s + k) * ww + EW * (static_cast<int>(e0 - a0) + d.rel[h]);
+      idx = (QS * s + k) * ww + EW * (static_cast<int>(e0 - a0) + d.rel[h]);
       if (r == 0) {
         nbytes[h] = static_cast<uint32_t>((e0 + d.span[h] + tile - a0 + kAlign) & ~int64_t(kAlign)) * 4u * EW;
         gsrc[h] = g.src + static_cast<int64_t>(src) * g.src_pitch + 4 * EW * a0;
@@ -398,14 +399,14 @@ __device__ __forceinline__ void produce_words(const Geo& g, Pipe& P, uint32_t* s
     }
     P.row[s][r][k] = idx;
   }
-  uint32_t total = nbytes[0] + nbytes[1];
+  uint32_t total = nbytes[0] + (QS == 4 ? nbytes[QS / 2 - 1] : 0u);
   total += __shfl_xor_sync(0xffffffffu, total, 16);
   __syncwarp();
   if (lane == 0) mbar_arrive_expect_tx(&P.full[s], total);
   __syncwarp();
 #pragma unroll
-  for (int h = 0; h < 2; ++h)
-    if (nbytes[h]) bulk_copy(sw + (4 * s + i + 2 * h) * ww, gsrc[h], nbytes[h], &P.full[s]);
+  for (int h = 0; h < QS / 2; ++h)
+    if (nbytes[h]) bulk_copy(sw + (QS * s + i + 2 * h) * ww, gsrc[h], nbytes[h], &P.full[s]);
 }
 
 // Delays past the chunk's end leave a block's first sources (the lowest frequencies)
@@ -446,7 +447,8 @@ constexpr int kModePlain = 0, kModeTwin = 1, kModeWords = 2, kModePhase = 3, kMo
 template <int SB, int QS, int MODE, bool SKIP, typename Setup, typename Body>
 __device__ __forceinline__ bool run_pipeline(const SumLaunch& L, Geo& g, Pipe& P,
                                              uint32_t* sw, int tile, Setup&& setup, Body&& body) {
-  static_assert(QS == (MODE == kModePlain || MODE == kModePhase ? 2 : 4), "sources per stage");
+  static_assert(MODE == kModePlain || MODE == kModePhase ? QS == 2 : QS == 4 || (QS == 2 && MODE == kModeWords),
+                "sources per stage");
   static_assert(kMaxStages <= kWarps, "each warp stages at most one group before the loop");
   constexpr int kWinPerSrc = MODE == kModeTwin ? 2 : 1;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -482,7 +484,7 @@ __device__ __forceinline__ bool run_pipeline(const SumLaunch& L, Geo& g, Pipe& P
     if constexpr (MODE == kModeTwin)
       produce_twin(g, P, sw, ww, zero_q, tile, L.twin_off, desc, next, s, lane);
     else if constexpr (MODE == kModeWords || MODE == kModeDwords)
-      produce_words<MODE == kModeDwords ? 2 : 1>(g, P, sw, ww, zero_q, tile, desc, next, s, lane);
+      produce_words<MODE == kModeDwords ? 2 : 1, QS>(g, P, sw, ww, zero_q, tile, desc, next, s, lane);
     else if constexpr (MODE == kModePhase)
       produce_phases<SB>(L, g, P, sw, ww, zero_q, tile, desc, phase, next, s, lane);
     else
@@ -545,9 +547,9 @@ __device__ __forceinline__ bool run_pipeline(const SumLaunch& L, Geo& g, Pipe& P
 // Rows of this thread's warp group that have columns in the block, as a bit mask: skews
 // move rows in and out of the first and last blocks of a launch, and the last row group
 // may hold fewer rows.
-template <int RB, int T>
+template <int RB, int T, int ROWS = kSumRows>
 __device__ __forceinline__ uint32_t active_rows(const Geo& g, int rbase) {
-  constexpr int kGroups = kSumRows / RB;
+  constexpr int kGroups = ROWS / RB;
   uint32_t act = 0;
 #pragma unroll
   for (int r = 0; r < RB; ++r)
@@ -572,15 +574,15 @@ __device__ __forceinline__ void for_rows(uint32_t act, F&& f) {
 }
 
 // ------------------------------------------------------------------ 8-bit samples
-template <int RB, int NW, bool OUT16, int MODE = kModePlain>
+template <int RB, int NW, bool OUT16, int MODE = kModePlain, int ROWS = kSumRows>
 __device__ __forceinline__ void sum_u8(const SumLaunch& L, uint3 blk, uint32_t* sw, Pipe& P) {
   static_assert(NW & 1, "an odd number of consecutive words per lane: conflict-free loads");
-  // RB rows per thread: the block's kSumRows rows are split over kSumRows/RB
+  // RB rows per thread: the block's ROWS rows are split over ROWS/RB
   // groups of warps, each group covering the whole tile for its RB rows
-  constexpr int kGroups = kSumRows / RB;
+  constexpr int kGroups = ROWS / RB;
   constexpr int kWarpsPerTile = kWarps / kGroups;
   constexpr int T = kWarpsPerTile * 32 * NW * 4;
-  Geo g = make_geo<MODE == kModePhase>(L, T, blk);
+  Geo g = make_geo<MODE == kModePhase, ROWS>(L, T, blk);
   if (g.nrows <= 0) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rbase = warp / kWarpsPerTile, wt = warp % kWarpsPerTile;
@@ -630,7 +632,7 @@ __device__ __forceinline__ void sum_u8(const SumLaunch& L, uint3 blk, uint32_t* 
   };
   int since = 0;       // sources summed in the fields since the last flush
   bool stored = false; // the output holds partial sums of an earlier flush
-  const bool ok = run_pipeline<1, 2, MODE, true>(L, g, P, sw, T, [&] { act = active_rows<RB, T>(g, rbase); }, [&](int s, const uint32_t* win) {
+  const bool ok = run_pipeline<1, 2, MODE, true>(L, g, P, sw, T, [&] { act = active_rows<RB, T, ROWS>(g, rbase); }, [&](int s, const uint32_t* win) {
     for_rows<RB>(act, [&](int r) {
       const int4 rw = row_info(P, s, rbase + kGroups * r);
       const uint32_t* w0 = win + rw.x + wbase;
@@ -717,14 +719,14 @@ __device__ __forceinline__ void sum_u8(const SumLaunch& L, uint3 blk, uint32_t* 
 // (two sources per three-input add); the low samples' sums come out at the end
 // as whole - (high << 16).  Three integer-pipe operations per word and source,
 // where taking the halves apart by masks and offset-dependent selects took five.
-template <int RB, int NW, int MODE = kModePlain>
+template <int RB, int NW, int MODE = kModePlain, int ROWS = kSumRows>
 __device__ __forceinline__ void sum_u16_wide(const SumLaunch& L, uint3 blk, uint32_t* sw, Pipe& P) {
-  // RB rows per thread: the block's rows are split over kSumRows/RB warp groups,
+  // RB rows per thread: the block's rows are split over ROWS/RB warp groups,
   // each covering the whole tile for its RB rows (as in sum_u8)
-  constexpr int kGroups = kSumRows / RB;
+  constexpr int kGroups = ROWS / RB;
   constexpr int kWarpsPerTile = kWarps / kGroups;
   constexpr int T = kWarpsPerTile * 32 * NW * 2;
-  Geo g = make_geo<MODE == kModePhase>(L, T, blk);
+  Geo g = make_geo<MODE == kModePhase, ROWS>(L, T, blk);
   if (g.nrows <= 0) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rbase = warp / kWarpsPerTile, wt = warp % kWarpsPerTile;
@@ -735,7 +737,7 @@ __device__ __forceinline__ void sum_u16_wide(const SumLaunch& L, uint3 blk, uint
   for (int r = 0; r < RB; ++r)
 #pragma unroll
     for (int k = 0; k < NW; ++k) lo32[r][k] = hi32[r][k] = 0;
-  const bool ok = run_pipeline<2, 2, MODE, true>(L, g, P, sw, 2 * T, [&] { act = active_rows<RB, T>(g, rbase); }, [&](int s, const uint32_t* win) {
+  const bool ok = run_pipeline<2, 2, MODE, true>(L, g, P, sw, 2 * T, [&] { act = active_rows<RB, T, ROWS>(g, rbase); }, [&](int s, const uint32_t* win) {
     for_rows<RB>(act, [&](int r) {
       const int4 rw = row_info(P, s, rbase + kGroups * r);
       const uint32_t* w0 = win + rw.x + wbase;
@@ -999,12 +1001,14 @@ __device__ __forceinline__ void sum_plane16(const SumLaunch& L, uint3 blk, uint3
 
 // Stage 2 of 32-bit subband sums (grid z = plane = segment; one plane when the sums
 // are not folded).  Sums wrap modulo 2^32 like the reference's uint32 accumulators.
-template <int RB, int NW>
+// Blocks of eight rows have two sources per stage, for windows twice as wide.
+template <int RB, int NW, int ROWS = kSumRows>
 __device__ __forceinline__ void sum_plane32(const SumLaunch& L, uint3 blk, uint32_t* sw, Pipe& P) {
-  constexpr int kGroups = kSumRows / RB;
+  constexpr int kGroups = ROWS / RB;
   constexpr int kWarpsPerTile = kWarps / kGroups;
   constexpr int T = kWarpsPerTile * 32 * NW;
-  Geo g = make_geo(L, T, blk);
+  constexpr int QS = ROWS == kSumRows ? 4 : 2;
+  Geo g = make_geo<false, ROWS>(L, T, blk);
   if (g.nrows <= 0) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rbase = warp / kWarpsPerTile;
@@ -1015,17 +1019,18 @@ __device__ __forceinline__ void sum_plane32(const SumLaunch& L, uint3 blk, uint3
   for (int r = 0; r < RB; ++r)
 #pragma unroll
     for (int k = 0; k < NW; ++k) acc[r][k] = 0;
-  const bool ok = run_pipeline<4, 4, kModeWords, false>(L, g, P, sw, T, [&] { act = active_rows<RB, T>(g, rbase); }, [&](int s, const uint32_t* win) {
+  const bool ok = run_pipeline<4, QS, kModeWords, false>(L, g, P, sw, T, [&] { act = active_rows<RB, T, ROWS>(g, rbase); }, [&](int s, const uint32_t* win) {
     for_rows<RB>(act, [&](int r) {
       const int4 a = row_info(P, s, rbase + kGroups * r);
       const uint32_t* w0 = win + a.x + wbase;
       const uint32_t* w1 = win + a.y + wbase;
-      const uint32_t* w2 = win + a.z + wbase;
-      const uint32_t* w3 = win + a.w + wbase;
 #pragma unroll
-      for (int k = 0; k < NW; ++k) {
-        acc[r][k] += w0[32 * k] + w1[32 * k];
-        acc[r][k] += w2[32 * k] + w3[32 * k];
+      for (int k = 0; k < NW; ++k) acc[r][k] += w0[32 * k] + w1[32 * k];
+      if constexpr (QS == 4) {
+        const uint32_t* w2 = win + a.z + wbase;
+        const uint32_t* w3 = win + a.w + wbase;
+#pragma unroll
+        for (int k = 0; k < NW; ++k) acc[r][k] += w2[32 * k] + w3[32 * k];
       }
     });
   });
@@ -1110,12 +1115,12 @@ __device__ __forceinline__ void sum_to64(const SumLaunch& L, uint3 blk, uint32_t
 #ifndef DD_SUM16T_MINB
 #define DD_SUM16T_MINB 3
 #endif
-template <int RB, int NW>
+template <int RB, int NW, int ROWS = kSumRows>
 __device__ __forceinline__ void sum_u16_twin(const SumLaunch& L, uint3 blk, uint32_t* sw, Pipe& P) {
-  constexpr int kGroups = kSumRows / RB;  // warp groups sharing the rows, as in sum_u8
+  constexpr int kGroups = ROWS / RB;  // warp groups sharing the rows, as in sum_u8
   constexpr int kWarpsPerTile = kWarps / kGroups;
   constexpr int T = kWarpsPerTile * 32 * NW * 2;
-  Geo g = make_geo(L, T, blk);
+  Geo g = make_geo<false, ROWS>(L, T, blk);
   if (g.nrows <= 0) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rbase = warp / kWarpsPerTile;
@@ -1126,7 +1131,7 @@ __device__ __forceinline__ void sum_u16_twin(const SumLaunch& L, uint3 blk, uint
   for (int r = 0; r < RB; ++r)
 #pragma unroll
     for (int k = 0; k < NW; ++k) lo[r][k] = hi[r][k] = 0;
-  const bool ok = run_pipeline<2, 4, kModeTwin, false>(L, g, P, sw, 2 * T, [&] { act = active_rows<RB, T>(g, rbase); }, [&](int s, const uint32_t* win) {
+  const bool ok = run_pipeline<2, 4, kModeTwin, false>(L, g, P, sw, 2 * T, [&] { act = active_rows<RB, T, ROWS>(g, rbase); }, [&](int s, const uint32_t* win) {
     for_rows<RB>(act, [&](int r) {
       const int4 a = row_info(P, s, rbase + kGroups * r);
       const uint32_t* w0 = win + a.x + wbase;
@@ -1162,23 +1167,23 @@ __device__ __forceinline__ void sum_u16_twin(const SumLaunch& L, uint3 blk, uint
   }
 }
 
-template <int RB, int NW, bool OUT16, int MODE = kModePlain>
+template <int RB, int NW, bool OUT16, int MODE = kModePlain, int ROWS = kSumRows>
 __global__ void __launch_bounds__(kThreads, DD_SUM8_MINB) k_sum_u8(SumLaunch L) {
   extern __shared__ __align__(128) uint32_t sw[];
   __shared__ Pipe P;
-  sum_u8<RB, NW, OUT16, MODE>(L, blockIdx, sw, P);
+  sum_u8<RB, NW, OUT16, MODE, ROWS>(L, blockIdx, sw, P);
 }
-template <int RB, int NW, int MODE = kModePlain>
+template <int RB, int NW, int MODE = kModePlain, int ROWS = kSumRows>
 __global__ void __launch_bounds__(kThreads, DD_SUM16W_MINB) k_sum_u16w(SumLaunch L) {
   extern __shared__ __align__(128) uint32_t sw[];
   __shared__ Pipe P;
-  sum_u16_wide<RB, NW, MODE>(L, blockIdx, sw, P);
+  sum_u16_wide<RB, NW, MODE, ROWS>(L, blockIdx, sw, P);
 }
-template <int RB, int NW>
+template <int RB, int NW, int ROWS = kSumRows>
 __global__ void __launch_bounds__(kThreads, DD_SUM16T_MINB) k_sum_u16t(SumLaunch L) {
   extern __shared__ __align__(128) uint32_t sw[];
   __shared__ Pipe P;
-  sum_u16_twin<RB, NW>(L, blockIdx, sw, P);
+  sum_u16_twin<RB, NW, ROWS>(L, blockIdx, sw, P);
 }
 template <int RB, int NW, bool PACK>
 __global__ void __launch_bounds__(kThreads, DD_FOLD8_MINB) k_sum_fold8(SumLaunch L) {
@@ -1204,11 +1209,11 @@ __global__ void __launch_bounds__(kThreads, 2) k_sum_to64(SumLaunch L) {
   __shared__ Pipe P;
   sum_to64<RB, NW, WIDE>(L, blockIdx, sw, P);
 }
-template <int RB, int NW>
+template <int RB, int NW, int ROWS = kSumRows>
 __global__ void __launch_bounds__(kThreads, DD_PLANE32_MINB) k_sum_plane32(SumLaunch L) {
   extern __shared__ __align__(128) uint32_t sw[];
   __shared__ Pipe P;
-  sum_plane32<RB, NW>(L, blockIdx, sw, P);
+  sum_plane32<RB, NW, ROWS>(L, blockIdx, sw, P);
 }
 
 // ------------------------------------------------------------------ batched launches
@@ -1256,6 +1261,11 @@ __device__ __forceinline__ void run_one(const SumLaunch& L, uint3 blk, uint32_t*
   else if constexpr (KIND == kSumKindFold16S) sum_fold16<kFold16RB, kFold16NW / 2>(L, blk, sw, P);
   else if constexpr (KIND == kSumKindPlane16S) sum_plane16<kPlane16RB, kPlane16NW / 2>(L, blk, sw, P);
   else if constexpr (KIND == kSumKindPlane32S) sum_plane32<kPlane32RB, kPlane32NW / 2>(L, blk, sw, P);
+  else if constexpr (KIND == kSumKindU8Out16R8) sum_u8<kSumRowsPT8, DD_SUM8_NW, true, kModePlain, 8>(L, blk, sw, P);
+  else if constexpr (KIND == kSumKindU8FlushR8) sum_u8<kSumRowsPT8, kFlush8R8NW, false, kModePlain, 8>(L, blk, sw, P);
+  else if constexpr (KIND == kSumKindU16WideR8) sum_u16_wide<kSumRowsPTW, DD_SUM16W_NW, kModePlain, 8>(L, blk, sw, P);
+  else if constexpr (KIND == kSumKindU16TwinR8) sum_u16_twin<kSumRowsPTT, kSum16TNW, 8>(L, blk, sw, P);
+  else if constexpr (KIND == kSumKindPlane32R8) sum_plane32<kPlane32RB, kPlane32NW, 8>(L, blk, sw, P);
   else sum_plane32<kPlane32RB, kPlane32NW>(L, blk, sw, P);
 }
 
@@ -1379,7 +1389,8 @@ size_t sum_smem_bytes(int win_bytes, int stages, int qs) {
 size_t sum_kind_extra_smem(int kind) {
   // the flush staging of the 8-bit kernel with 32-bit outputs: one segment of
   // 32-bit sums per warp
-  const int nw = kind == kSumKindU8Flush ? DD_SUM8_NW : kind == kSumKindU8Phase ? kPhase8NW : 0;
+  const int nw = kind == kSumKindU8Flush ? DD_SUM8_NW : kind == kSumKindU8Phase ? kPhase8NW
+                 : kind == kSumKindU8FlushR8 ? kFlush8R8NW : 0;
   return static_cast<size_t>(kWarps) * 32 * nw * 4 * sizeof(uint32_t);
 }
 
@@ -1405,13 +1416,13 @@ int sum_stages(int win_bytes, int qs, size_t extra, int cap_kb) {
 
 int sum_kind_stages(int kind, int win_bytes) {
   return sum_stages(win_bytes, sum_kind_qs(kind), sum_kind_extra_smem(kind),
-                    kind == kSumKindU16Twin ? DD_SUM16T_SMEM_KB : DD_SUM_SMEM_KB);
+                    kind == kSumKindU16Twin || kind == kSumKindU16TwinR8 ? DD_SUM16T_SMEM_KB : DD_SUM_SMEM_KB);
 }
 
 std::vector<SumDesc> build_sum_desc(const std::vector<int32_t>& tab, int64_t nrows,
-                                    int64_t ncols, int64_t group, int* spread) {
+                                    int64_t ncols, int64_t group, int* spread, int rows) {
   const int64_t blk = group > 0 ? group : nrows;
-  const int64_t per = (blk + kSumRows - 1) / kSumRows;  // row groups per block of rows
+  const int64_t per = (blk + rows - 1) / rows;  // row groups per block of rows
   const int64_t nblk = (nrows + blk - 1) / blk;
   std::vector<SumDesc> d(static_cast<size_t>(nblk * per * ncols));
   int32_t most = 0;
@@ -1419,8 +1430,8 @@ std::vector<SumDesc> build_sum_desc(const std::vector<int32_t>& tab, int64_t nro
   for (int64_t b = 0; b < nblk; ++b) {
     const int64_t b0 = b * blk, b1 = std::min(nrows, b0 + blk);
     for (int64_t gi = 0; gi < per; ++gi) {
-      const int64_t r0 = b0 + gi * kSumRows;
-      const int64_t r1 = std::min(b1, r0 + kSumRows);
+      const int64_t r0 = b0 + gi * rows;
+      const int64_t r1 = std::min(b1, r0 + rows);
       SumDesc* row = d.data() + (b * per + gi) * ncols;
       if (r0 >= r1) continue;
       const int32_t* first = tab.data() + r0 * ncols;
@@ -1470,6 +1481,11 @@ void launch_sum(const SumLaunch& L, cudaStream_t st) {
     case kSumKindFold16S: launch_k(k_sum_fold16<kFold16RB, kFold16NW / 2>, grid, smem, L, st); break;
     case kSumKindPlane16S: launch_k(k_sum_plane16<kPlane16RB, kPlane16NW / 2>, grid, smem, L, st); break;
     case kSumKindPlane32S: launch_k(k_sum_plane32<kPlane32RB, kPlane32NW / 2>, grid, smem, L, st); break;
+    case kSumKindU8Out16R8: launch_k(k_sum_u8<kSumRowsPT8, DD_SUM8_NW, true, kModePlain, 8>, grid, smem, L, st); break;
+    case kSumKindU8FlushR8: launch_k(k_sum_u8<kSumRowsPT8, kFlush8R8NW, false, kModePlain, 8>, grid, smem, L, st); break;
+    case kSumKindU16WideR8: launch_k(k_sum_u16w<kSumRowsPTW, DD_SUM16W_NW, kModePlain, 8>, grid, smem, L, st); break;
+    case kSumKindU16TwinR8: launch_k(k_sum_u16t<kSumRowsPTT, kSum16TNW, 8>, grid, smem, L, st); break;
+    case kSumKindPlane32R8: launch_k(k_sum_plane32<kPlane32RB, kPlane32NW, 8>, grid, smem, L, st); break;
     default: launch_k(k_sum_plane32<kPlane32RB, kPlane32NW>, grid, smem, L, st); break;
   }
 }
@@ -1522,6 +1538,11 @@ void launch_sum_grouped(const SumBatchGroup* d_groups, int ngroups, long long to
     case kSumKindFold16S: launch_grouped_k<kSumKindFold16S>(d_groups, ngroups, total, smem, st); break;
     case kSumKindPlane16S: launch_grouped_k<kSumKindPlane16S>(d_groups, ngroups, total, smem, st); break;
     case kSumKindPlane32S: launch_grouped_k<kSumKindPlane32S>(d_groups, ngroups, total, smem, st); break;
+    case kSumKindU8Out16R8: launch_grouped_k<kSumKindU8Out16R8>(d_groups, ngroups, total, smem, st); break;
+    case kSumKindU8FlushR8: launch_grouped_k<kSumKindU8FlushR8>(d_groups, ngroups, total, smem, st); break;
+    case kSumKindU16WideR8: launch_grouped_k<kSumKindU16WideR8>(d_groups, ngroups, total, smem, st); break;
+    case kSumKindU16TwinR8: launch_grouped_k<kSumKindU16TwinR8>(d_groups, ngroups, total, smem, st); break;
+    case kSumKindPlane32R8: launch_grouped_k<kSumKindPlane32R8>(d_groups, ngroups, total, smem, st); break;
     default: launch_grouped_k<kSumKindPlane32>(d_groups, ngroups, total, smem, st); break;
   }
 }

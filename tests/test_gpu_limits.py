@@ -1,11 +1,13 @@
 """Calls at the limits of a launch, a row or the device: more slices than a grid dimension
-holds, rows of more than 2^31 samples, staged windows as wide as shared memory."""
+holds, rows of more than 2^31 samples, staged windows as wide as shared memory, trial steps so
+coarse that rows are staged by eight or not at all."""
 import numpy as np
 import pytest
 
 pytestmark = pytest.mark.gpu
 
 torch = pytest.importorskip("torch")
+from test_gpu_fold import dev, subband, to_np  # noqa: E402
 
 
 def test_more_slices_than_a_launch_takes():
@@ -63,3 +65,51 @@ def test_brute_force_windows_at_the_shared_memory_limit(step, spread):
                                            delay=delay), axis=1)
     got = plan.run(torch.from_numpy(x).cuda()).view(torch.int32).cpu().numpy().view(np.uint32)
     assert np.array_equal(got, want)
+
+
+# Trial steps around the limits of sixteen and eight rows a block, and past both: 8 bits about
+# 10.4 and 22.5, 16 bits 5.5 and 11.  Batches launch the staged sums together; plans on the
+# direct kernels run on their own.
+@pytest.mark.parametrize("nbits,step,staged", [(8, 13.0, True), (8, 22.0, True), (8, 22.6, False),
+                                               (16, 5.7, True), (16, 10.9, True), (16, 11.3, False)])
+def test_brute_force_with_coarse_steps(nbits, step, staged):
+    from astroflow_b200.dedisp import Batch, Plan
+    from oracle import oracle as O
+
+    n, nc, tsamp = 100003, 16, 82e-6
+    x = np.random.default_rng(4).integers(0, 2 ** nbits, (n, nc)).astype(np.uint8 if nbits == 8 else np.uint16)
+    freq = O.freq_table_fil(400.0, 25.0, nc)
+    fs, fe = float(np.float32(freq[0])), float(np.float32(freq[-1]))
+    hdr = dict(tsamp=tsamp, fch1=400.0, foff=25.0, nbits=nbits, nchans=nc, ndata=n)
+    ts = n * tsamp * 0.49
+    plan = Plan(hdr, 0.0, 26.5 * step, fs, fe, step, 1, ts, algorithm="brute", freq_mode="fil")
+    want = np.concatenate(O.bruteforce_cpu(x, nc, freq, tsamp, 0.0, 26.5 * step, fs, fe, step, 1, ts,
+                                           delay=plan.tables()[0]), axis=1)
+    assert np.array_equal(to_np(plan.run(dev(x))), want)
+    for persistent in (False, True):
+        batch = Batch([plan], persistent=persistent)
+        assert np.array_equal(to_np(batch.run([dev(x)])[0]), want)
+        batch.status()
+        assert persistent or batch.info["own_plans"] == (0 if staged else 1)
+
+
+# The same for the two stages: wide rows of stage 2 (the twin's, 32-bit sums') and, with one
+# subband, of stage 1 (16-bit and 32-bit sums), up to steps that no staged form takes.
+@pytest.mark.parametrize("n,nchans,nbits,trials,step,width,staged", [
+    (30011, 64, 8, 99, 10.0, 16, True), (50001, 64, 8, 70, 30.0, 16, True), (50001, 64, 8, 70, 40.0, 16, True),
+    (30011, 64, 16, 99, 10.0, 16, True), (90001, 32, 16, 70, 40.0, 16, False), (90001, 32, 16, 70, 75.0, 16, False),
+    (40003, 64, 16, 99, 20.0, 16, True),
+    (30011, 256, 8, 99, 10.0, 128, True), (60002, 48, 8, 331, 8.0, 64, True), (60002, 48, 8, 331, 9.5, 64, False),
+    (60002, 70, 8, 331, 8.0, 70, True), (60002, 48, 16, 331, 4.0, 48, True), (60002, 48, 16, 331, 5.0, 48, False),
+])
+def test_subbands_with_coarse_steps(n, nchans, nbits, trials, step, width, staged):
+    from astroflow_b200.dedisp import Batch
+
+    plan, x, want = subband(n, nchans, nbits, step * (trials - 0.5), step, 1, width, 0.0, False, False, full=True)
+    assert np.array_equal(to_np(plan.run(dev(x))), want)
+    assert np.array_equal(plan.run_host(x), want)
+    for persistent in (False, True):
+        batch = Batch([plan], persistent=persistent)
+        assert np.array_equal(to_np(batch.run([dev(x)])[0]), want)
+        batch.status()
+        assert persistent or batch.info["own_plans"] == (0 if staged else 1)
