@@ -92,11 +92,34 @@ int brute_kind(const dd_plan& P) {
 // trials) 3.85 / 4.03, 95 (6001 trials) 9.10 / 12.0; 8192 channels of 16 bits, 2001
 // trials 20.0 / 29.5; brute force over 1024 channels 5.60 / 8.69.
 int choose_fold(const dd_plan& P, int64_t ncols, int64_t nchan, int64_t reach, double adds) {
-  if (P.nbits > 16) return 1;
+  if (P.nbits > 16 || !P.may_fold) return 1;
   const int fold = P.nbits == 8 ? 4 : 2;
   const int64_t words = std::min<int64_t>(P.nbin, (ncols + fold - 1) / fold + reach);
   const double extra = static_cast<double>(nchan) * (4.0 * words - static_cast<double>(P.nbin) * P.elem);
   return adds > 16.0 * extra ? fold : 1;
+}
+// f(true), and f(false) where that runs out of device memory: a folded chunk takes up to four
+// times the bytes of one in time order.
+template <typename F>
+void fold_if_it_fits(int device, F&& f) {
+  try {
+    f(true);
+    return;
+  } catch (const Error& e) {
+    if (e.code != DD_ERR_NOMEM) throw;
+  }
+  DeviceGuard g(device);
+  // the pool still maps what the failed attempt took, in pieces that need not fit the next
+  DD_CUDA_TRY(cudaStreamSynchronize(cudaStreamLegacy));
+  cudaMemPool_t pool = nullptr;
+  DD_CUDA_TRY(cudaDeviceGetDefaultMemPool(&pool, device));
+  DD_CUDA_TRY(cudaMemPoolTrimTo(pool, 0));
+  f(false);
+}
+// Refuses runs of a plan that a failed call (a delay table, autotuning) left without buffers.
+void check_buffers(const dd_plan& P) {
+  if (!P.d_x.p || (P.p.algorithm == DD_ALGO_SUBBAND && !P.d_inter.p))
+    throw Error{DD_ERR_NOMEM, "the plan's device buffers could not be allocated"};
 }
 // Byte offset from a subband-sum buffer to its twin (0: no twin).
 int64_t twin_offset(const dd_plan& P) { return P.twin ? P.inter_bytes : 0; }
@@ -554,7 +577,14 @@ void create_subband(dd_plan& P) {
     }
     if (P.win2) upload_desc(P.d_desc2, desc2);
   }
-  set_tiling(P, int64_t(DD_INTER_MB) << 20);
+  for (int64_t budget = int64_t(DD_INTER_MB) << 20;; budget /= 2) {
+    try {
+      set_tiling(P, budget);
+      break;
+    } catch (const Error& e) {
+      if (e.code != DD_ERR_NOMEM || budget < (int64_t(128) << 20)) throw;  // else: shorter tiles
+    }
+  }
   if (ds > 1 || callsite_zdm_active(P))
     P.d_binned.alloc(static_cast<size_t>(P.nbin * P.hdr.nchans) * P.elem);
   if (ds > 1 && binning_lut_entries(P.nbits, ds)) {
@@ -718,6 +748,7 @@ void create_rfi(dd_plan& P) {
 
 void run_rfi_and_prep(dd_plan& P, const void* input, uint8_t* masks_out, uint32_t* bounds_out,
                       void* prepped, cudaStream_t st) {
+  check_buffers(P);
   const int64_t n = P.hdr.nchans;
   const void* src = input;
   const int ds = P.p.time_downsample;
@@ -982,6 +1013,7 @@ SumLaunch brute_launch(const dd_plan& P, void* output) {
 }
 
 void run_brute_prep(dd_plan& P, const void* input, void* prepped, cudaStream_t st) {
+  check_buffers(P);
   PrepArgs a{};
   a.x = input;
   a.nbits = P.nbits;
@@ -1139,9 +1171,11 @@ const char* dd_last_error(void) { return g_last_error.c_str(); }
 namespace dd {
 namespace {
 // Builds a plan (throws on error).  nout > 0 limits a subband plan's output to
-// the first nout binned columns (the plan of a stream).
+// the first nout binned columns (the plan of a stream).  may_fold: false keeps the chunk
+// in time order.
 dd_plan* make_plan(const dd_header* header, const dd_plan_params* params, const dd_rfi_config* rfi,
-                   const int32_t* bad_channels, int32_t n_bad, int32_t device, int64_t nout) {
+                   const int32_t* bad_channels, int32_t n_bad, int32_t device, int64_t nout,
+                   bool may_fold) {
   if (!header || !params) throw Error{DD_ERR_INVALID, "header and params are required"};
   if (header->nbits != 8 && header->nbits != 16 && header->nbits != 32)
     throw Error{DD_ERR_INVALID, "nbits must be 8, 16 or 32"};
@@ -1168,6 +1202,7 @@ dd_plan* make_plan(const dd_header* header, const dd_plan_params* params, const 
   }
   if (bad_channels && n_bad > 0) P->bad.assign(bad_channels, bad_channels + n_bad);
   P->device = device;
+  P->may_fold = may_fold;
   P->nbits = header->nbits;
   P->elem = header->nbits / 8;
   P->nin = header->ndata;
@@ -1208,7 +1243,11 @@ int dd_plan_create(const dd_header* header, const dd_plan_params* params,
                    int32_t device, dd_plan** plan) {
   if (!plan) { set_error("plan pointer is NULL"); return DD_ERR_INVALID; }
   *plan = nullptr;
-  return guarded([&] { *plan = make_plan(header, params, rfi, bad_channels, n_bad, device, 0); });
+  return guarded([&] {
+    fold_if_it_fits(device, [&](bool fold) {
+      *plan = make_plan(header, params, rfi, bad_channels, n_bad, device, 0, fold);
+    });
+  });
 }
 
 int dd_plan_destroy(dd_plan* plan) {
@@ -1302,8 +1341,16 @@ int dd_plan_set_delay_table(dd_plan* P, const int32_t* delay) {
     std::memcpy(P->h_delay.data(), delay, sizeof(int32_t) * P->h_delay.size());
     P->max_delay = mx;
     ++P->generation;
-    set_brute_window(*P);
-    DD_CUDA_TRY(cudaMemcpy(P->d_delay.p, delay, sizeof(int32_t) * P->h_delay.size(), cudaMemcpyHostToDevice));
+    try {
+      fold_if_it_fits(P->device, [&](bool fold) {
+        P->may_fold = P->may_fold && fold;
+        set_brute_window(*P);
+      });
+      DD_CUDA_TRY(cudaMemcpy(P->d_delay.p, delay, sizeof(int32_t) * P->h_delay.size(), cudaMemcpyHostToDevice));
+    } catch (...) {
+      P->d_x.release();  // half set: runs are refused (check_buffers)
+      throw;
+    }
   });
 }
 
@@ -1964,7 +2011,10 @@ int dd_stream_open(const dd_header* header, const dd_plan_params* params, const 
                                   "of time_downsample"};
     DeviceGuard g(device);
     // the delays set the tail: learn them from a plan over one chunk
-    std::unique_ptr<dd_plan> probe(make_plan(header, params, rfi, bad_channels, n_bad, device, 0));
+    std::unique_ptr<dd_plan> probe;
+    fold_if_it_fits(device, [&](bool fold) {
+      probe.reset(make_plan(header, params, rfi, bad_channels, n_bad, device, 0, fold));
+    });
     const int64_t tail_bin = static_cast<int64_t>(probe->max_delay) + probe->max_res;
     probe.reset();
     S = new dd_stream();
@@ -1975,8 +2025,12 @@ int dd_stream_open(const dd_header* header, const dd_plan_params* params, const 
     S->row_bytes = static_cast<int64_t>(header->nchans) * (header->nbits / 8);
     dd_header h = *header;
     h.ndata = S->buf_len;
-    S->plan = make_plan(&h, params, rfi, bad_channels, n_bad, device, S->chunk / ds);
-    S->buf.alloc(static_cast<size_t>(2 * S->buf_len * S->row_bytes));
+    fold_if_it_fits(device, [&](bool fold) {
+      delete S->plan;
+      S->plan = nullptr;
+      S->plan = make_plan(&h, params, rfi, bad_channels, n_bad, device, S->chunk / ds, fold);
+      S->buf.alloc(static_cast<size_t>(2 * S->buf_len * S->row_bytes));
+    });
     DD_CUDA_TRY(cudaMemsetAsync(S->buf.p, 0, S->buf.bytes, cudaStreamLegacy));
     DD_CUDA_TRY(cudaStreamSynchronize(cudaStreamLegacy));
   });

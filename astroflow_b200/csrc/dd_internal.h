@@ -83,6 +83,7 @@ struct dd_plan {
   // columns per segment (all of them when not folded), planes of subband sums.  The
   // time tiles, and x and subband-sum pitches of a folded plan count words.
   int fold = 1;
+  bool may_fold = true;      // false: the folded layout's buffers did not fit the device
   int64_t seg = 0;
   int planes = 1;
   int twin = 0;              // stage 1 also writes the one-sample-shifted twin of its uint16 sums

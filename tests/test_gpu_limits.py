@@ -1,6 +1,6 @@
 """Calls at the limits of a launch, a row or the device: more slices than a grid dimension
 holds, rows of more than 2^31 samples, staged windows as wide as shared memory, trial steps so
-coarse that rows are staged by eight or not at all."""
+coarse that rows are staged by eight or not at all, plans whose folded layout does not fit."""
 import numpy as np
 import pytest
 
@@ -113,3 +113,53 @@ def test_subbands_with_coarse_steps(n, nchans, nbits, trials, step, width, stage
         assert np.array_equal(to_np(batch.run([dev(x)])[0]), want)
         batch.status()
         assert persistent or batch.info["own_plans"] == (0 if staged else 1)
+
+
+def fill_device(leave):
+    """All of the device's free memory but `leave` bytes."""
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    return torch.empty(torch.cuda.mem_get_info()[0] - leave, dtype=torch.uint8, device="cuda")
+
+
+# A folded chunk takes up to four times its bytes: with less memory left than that, the plan
+# keeps the chunk in time order (subband sums: shorter time tiles come first).  MiB: left for the plan or the stream (time order / folded take
+# 480 / 1045, 1143 / 1452 and, with the stream's own buffer, 2191 / 2409).
+@pytest.mark.parametrize("kind,nbits,leave_mb", [("brute", 8, 760), ("subband", 16, 1300), ("subband", 16, 800), ("stream", 16, 2310)])
+def test_plans_whose_folded_layout_does_not_fit(kind, nbits, leave_mb):
+    from astroflow_b200.dedisp import Plan, Stream
+
+    n, nc = 1 << 18, 1024
+    if kind == "stream":
+        n = 1 << 17
+    x = torch.randint(0, 127, (n, nc * nbits // 8), dtype=torch.uint8, device="cuda").view(
+        torch.uint8 if nbits == 8 else torch.uint16)
+    f32 = np.float32
+    hdr = dict(tsamp=float(f32(1.6e-4)), fch1=400.0, foff=float(f32(400.0 / nc)), nbits=nbits, nchans=nc, ndata=n)
+    fe = float(f32(400.0) + f32(nc - 1) * f32(400.0 / nc))
+
+    def make():
+        if kind == "brute":
+            return Plan(hdr, 0.0, 800.0, 400.0, fe, 2.5, 1, n * 1.6e-4 * 0.49, algorithm="brute", freq_mode="fil")
+        if kind == "subband":
+            return Plan(hdr, 0.0, 600.0, 400.0, fe, 1.0, 1)
+        return Stream(hdr, 0.0, 800.0, 400.0, fe, 0.5, 1)
+
+    def run(p, out):
+        return p.push(x, out) if kind == "stream" else p.run(x, out)
+
+    p = make()
+    out = p.empty_output()
+    want = run(p, out).view(torch.int32).cpu()
+    folded = p.info["workspace_bytes"]
+    p.close()
+    hog = fill_device(leave_mb << 20)
+    try:
+        p = make()
+        assert p.info["workspace_bytes"] < folded
+        out.view(torch.int32).zero_()
+        assert torch.equal(run(p, out).view(torch.int32).cpu(), want)
+        p.close()
+    finally:
+        del hog
+        torch.cuda.empty_cache()
