@@ -438,9 +438,10 @@ void set_tiling(dd_plan& P, int64_t budget) {
   P.tile = L;
   P.inter_budget = budget;
   // Stage-2 blocks past the tile's last column read up to one block tile beyond it
-  // (their columns are not stored).
+  // (their columns are not stored); the direct kernels (never folded) end on whole tiles of
+  // their own.
   const int64_t T2 = P.win2 ? sum_kind_tile(stage2_kind(P)) : kT;
-  P.tile_pitch = round_up(round_up(L + P.max_res, kT) + T2 + 64, 64);
+  P.tile_pitch = round_up((P.fold > 1 ? L + P.max_res : round_up(L + P.max_res, kT)) + T2 + 64, 64);
   // Stage-1 windows start before the chunk's end (later ones are skipped) and end a
   // block tile and their spread past their first element; the direct kernels read up to
   // the largest delay past a tile's last column.
