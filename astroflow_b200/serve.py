@@ -73,6 +73,51 @@ class Beam:
     slot: int = 0
 
 
+def workspace_bound(n: int, c: int, bits: int, tsamp: float, fch1: float, foff: float, ndm: int,
+                    kw: dict) -> int:
+    """Upper bound on a plan's workspace bytes, from its header and arguments.
+
+    The prepared input holds per channel either the samples in time order with the
+    largest delay after them, or, folded, a 32-bit word for every position up to a
+    segment (a quarter of 8-bit chunks, half of 16-bit ones) and the largest delay: up
+    to four times the samples.  Both end in a block tile and the spread of the delays a
+    block's rows share."""
+    ds, elem, fold = int(kw.get("time_downsample", 1)), bits // 8, 32 // bits
+    step, ndm0 = kw.get("dm_step", 1.0), int(kw.get("ndm0", 32))
+    brute = kw.get("algorithm", "subband") == "brute"
+    nb = -(-n // ds)
+    f0, f1 = sorted((fch1, fch1 + (c - 1) * foff))
+    per_dm = 4148.808 * (1.0 / f0 ** 2 - 1.0 / f1 ** 2) / (tsamp if brute else tsamp * ds)
+    block = 16 * step * (1 if brute else ndm0) * per_dm  # spread of sixteen rows
+    if brute:
+        reach = int(per_dm * kw["dm_high"]) + 2
+        # phase rows: the samples, the delay, a slice (at most the chunk), whole tiles
+        linear = elem * (2 * n + reach + ds * 16384)
+        folded = 4 * (n + 16384)
+        inter = 0
+        tables = 8 * ndm * c
+    else:
+        reach = int(per_dm * (kw["dm_high"] + ndm0 * step)) + 64
+        linear = elem * (nb + reach + int(min(block, 40960)) + 16384)
+        folded = 4 * (min(nb, nb // fold + reach) + int(min(block, 8192)) + 8192)
+        # a time tile of subband sums: the budget, or a least tile, or all columns
+        nom, width = -(-ndm // ndm0), int(kw.get("subband_width", 32))
+        rows = nom * -(-c // width)
+        packed = bits == 8 and width <= 64
+        res = int(per_dm * ndm0 * step) + 2
+        inter = max(per_col * (min(max((2 << 30) // per_col, least + res), cols + res) + pad)
+                    for per_col, cols, least, pad in
+                    ((rows * 4, nb, 4096, 10240),  # time order: 32-bit sums, or 16-bit ones twice
+                     (rows * (8 if packed else 4 * fold), nb // fold + 8, 1024, 1280)))
+        tables = 8 * (nom * c + ndm * -(-c // width))
+    rfi, windows = kw.get("rfi"), 0
+    binned = nb * c * elem if ds > 1 or (rfi is not None and rfi.use_zero_dm) else 0
+    if rfi is not None and rfi.use_iqrm:  # sums, statistics, votes and flags per window
+        q = rfi.iqrm
+        windows = 2 + int(n * tsamp / (q.hop_sec or q.win_sec)) if q.win_sec > 0 else 1
+    return c * (max(linear, folded) + 80 * windows) + binned + inter + tables + (64 << 20)
+
+
 class Server:
     """Continuous-batching dedispersion server on one GPU.
 
@@ -193,11 +238,11 @@ class Server:
         host, header, kw = t.payload[:3]
         g = (lambda k: header[k]) if isinstance(header, dict) else (lambda k: getattr(header, k))
         n, c, bits = int(g("ndata")), int(g("nchans")), int(g("nbits"))
-        # input, prepared copy, output rows (an upper bound on DM trials), one
-        # time tile of subband sums (the library's default budget: 2 GiB)
+        # input, output rows (an upper bound on DM trials), what the plan holds
         lo, hi, step = kw["dm_low"], kw["dm_high"], kw.get("dm_step", 1.0)
         ndm = int((hi - lo) / step) + 1
-        return 2 * n * c * bits // 8 + ndm * n * 4 + (2 << 30)
+        return n * c * bits // 8 + ndm * n * 4 + workspace_bound(
+            n, c, bits, float(g("tsamp")), float(g("fch1")), float(g("foff")), ndm, kw)
 
     def step(self) -> bool:
         """One pass: finish completed work, launch ready beam chunks, admit files.

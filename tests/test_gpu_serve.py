@@ -84,3 +84,30 @@ def test_requests_in_the_mix_equal_requests_alone():
         assert np.array_equal(t.result.view(torch.int32).cpu().numpy(), want)
         assert t.latency is not None and t.latency > 0
     srv.close()
+
+
+# What admission reserves for a file covers what its plan, input and output take, for folded
+# chunks (up to four times their bytes) and chunks in time order, with and without binning.
+@pytest.mark.parametrize("bits,nchans,n,f0,bw,tsamp,dm_high,step,kw", [
+    (8, 4096, 1 << 17, 1000.0, 500.0, 4.9e-5, 3000.0, 0.5, {}),
+    (8, 4096, 1 << 17, 1000.0, 500.0, 4.9e-5, 1500.0, 0.25, {}),
+    (16, 4096, 1 << 17, 1000.0, 500.0, 4.9e-5, 1500.0, 0.25, dict(subband_width=64)),
+    (8, 4096, 1 << 17, 1000.0, 500.0, 4.9e-5, 600.0, 8.0, dict(subband_width=128)),
+    (8, 2048, 1 << 17, 1000.0, 500.0, 4.9e-5, 3000.0, 1.0, dict(time_downsample=2)),
+    (8, 4096, 1 << 17, 1000.0, 500.0, 4.9e-5, 3000.0, 1.0, dict(algorithm="brute", freq_mode="fil", t_sample=3.0)),
+    (16, 1024, 1 << 17, 400.0, 400.0, 1.6e-4, 600.0, 4.0, dict(algorithm="brute", freq_mode="fil", t_sample=3.0,
+                                                              time_downsample=4)),
+    (8, 300, 5000, 1000.0, 500.0, 4.9e-5, 100.0, 1.0, dict(time_downsample=4)),
+])
+def test_admission_covers_what_a_file_takes(bits, nchans, n, f0, bw, tsamp, dm_high, step, kw):
+    from astroflow_b200.serve import Ticket
+
+    foff = float(F32(bw / nchans))
+    hdr = dict(tsamp=float(F32(tsamp)), fch1=f0, foff=foff, nbits=bits, nchans=nchans, ndata=n)
+    args = dict(dm_low=0.0, dm_high=dm_high, freq_start=f0, freq_end=float(F32(f0) + F32(nchans - 1) * F32(foff)),
+                dm_step=step, rfi=RfiParams(use_iqrm=True, iqrm=IqrmParams(win_sec=1.0, hop_sec=0.5)), **kw)
+    plan = Plan(hdr, **args)
+    takes = n * nchans * bits // 8 + plan.out_shape[0] * plan.out_shape[1] * 4 + plan.info["workspace_bytes"]
+    need = Server._file_need(None, Ticket(1, "file", 0.0, payload=(None, hdr, args)))
+    assert takes <= need <= 2 * takes + (512 << 20)
+    plan.close()
