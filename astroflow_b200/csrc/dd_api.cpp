@@ -1990,7 +1990,7 @@ struct dd_stream {
   int64_t chunk = 0, tail = 0, buf_len = 0;  // input samples
   int64_t row_bytes = 0;                     // bytes per input sample (all channels)
   // [samples][channels], 2 * buf_len samples: the tail of the next push starts at sample
-  // pos and its chunk follows; at the end of the buffer the tail is copied to the front.
+  // pos <= buf_len and its chunk follows; past that the tail is copied to the front.
   dd::DevBuf buf;
   int64_t pos = 0;
   int64_t pushed = 0;
@@ -2052,22 +2052,30 @@ int dd_stream_push(dd_stream* S, const void* chunk, void* output, void* stream) 
   return guarded([&] {
     DeviceGuard g(S->device);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    // a captured push is replayed with the addresses of its capture: it leaves the tail
+    // where it found it
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (st && st != cudaStreamLegacy) DD_CUDA_TRY(cudaStreamIsCapturing(st, &capture));
+    const auto copy = [&](char* to, const char* from, int64_t samples) {
+      DD_CUDA_TRY(cudaMemcpyAsync(to, from, static_cast<size_t>(samples * S->row_bytes),
+                                  cudaMemcpyDeviceToDevice, st));
+    };
     char* buf = static_cast<char*>(S->buf.p);
-    if (S->pos + S->buf_len > 2 * S->buf_len) {
-      // the tail moves to the front once in tail/chunk + 2 pushes (pos > buf_len: the two
-      // places do not overlap); copied on every push it took a tenth of a 0.5 s chunk's time
-      if (S->tail)
-        DD_CUDA_TRY(cudaMemcpyAsync(buf, buf + S->pos * S->row_bytes,
-                                    static_cast<size_t>(S->tail * S->row_bytes),
-                                    cudaMemcpyDeviceToDevice, st));
-      S->pos = 0;
-    }
     char* cur = buf + S->pos * S->row_bytes;
-    DD_CUDA_TRY(cudaMemcpyAsync(cur + S->tail * S->row_bytes, chunk,
-                                static_cast<size_t>(S->chunk * S->row_bytes),
-                                cudaMemcpyDeviceToDevice, st));
+    copy(cur + S->tail * S->row_bytes, static_cast<const char*>(chunk), S->chunk);
     run_subband(*S->plan, cur, output, nullptr, nullptr, nullptr, st);
-    S->pos += S->chunk;
+    if (capture == cudaStreamCaptureStatusActive) {
+      // one chunk's length at a time, so that no copy overlaps itself
+      for (int64_t t = 0; t < S->tail; t += S->chunk)
+        copy(cur + t * S->row_bytes, cur + (t + S->chunk) * S->row_bytes, std::min(S->chunk, S->tail - t));
+    } else if (S->pos + S->chunk > S->buf_len) {
+      // the tail moves to the front once in tail/chunk + 2 pushes (the two places do not
+      // overlap); copied on every push it took a tenth of a 0.5 s chunk's time
+      if (S->tail) copy(buf, cur + S->chunk * S->row_bytes, S->tail);
+      S->pos = 0;
+    } else {
+      S->pos += S->chunk;
+    }
     S->pushed += S->chunk;
   });
 }

@@ -492,7 +492,10 @@ typedef struct dd_stream_info {
 int dd_stream_open(const dd_header* header, const dd_plan_params* params,
                    const dd_rfi_config* rfi, const int32_t* bad_channels, int32_t n_bad,
                    int32_t device, dd_stream** stream_out);
-/* chunk: device [chunk_samples][nchans]; output: device [dm_steps][out_cols]. */
+/* chunk: device [chunk_samples][nchans]; output: device [dm_steps][out_cols].  A push
+ * captured into a CUDA graph leaves the tail where it found it, so that every replay
+ * continues the beam (after an uncaptured push of the process: the kernels load on their
+ * first launch); pushed_samples counts calls, not replays. */
 int dd_stream_push(dd_stream* s, const void* chunk, void* output, void* stream);
 int dd_stream_get_info(const dd_stream* s, dd_stream_info* info);
 /* The plan a stream runs (owned by the stream): its info and tables. */
