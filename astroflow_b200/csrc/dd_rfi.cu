@@ -364,15 +364,16 @@ __global__ void k_iqrm_stat(const unsigned long long* __restrict__ sums,
 // below each of the three candidates (warp sums by one reduction instruction, one
 // barrier).  Bound by the latency of those 32 rounds (30 us for 4,096 channels, the
 // whole decision 42 us); one block per window that sorted every lag's differences in
-// turn took 364 us for 8 lags of 4,096 channels and 597 us for 26 lags of 2,048.
+// turn took 364 us for 8 lags of 4,096 channels and 597 us for 26 lags of 2,048.  Few
+// channels take few warps, so that a round's barrier is short.
 // Dynamic shared memory: the csub keys.
-constexpr int kLagThreads = 512;
-__global__ void __launch_bounds__(kLagThreads) k_iqrm_lag(
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS) k_iqrm_lag(
     const uint32_t* __restrict__ win, int csub, float nsigma, const int32_t* __restrict__ lags,
     int nlags, int variant, const float* __restrict__ xs, int* __restrict__ recv,
     int* __restrict__ cast_, uint8_t* __restrict__ flags) {
   extern __shared__ uint32_t keys[];
-  constexpr int kWarpsL = kLagThreads / 32;
+  constexpr int kWarpsL = THREADS / 32;
   __shared__ uint32_t part[2][3][kWarpsL];
   const int l = blockIdx.y, w = blockIdx.x;
   if (win[2 * w + 1] == win[2 * w]) return;
@@ -383,7 +384,7 @@ __global__ void __launch_bounds__(kLagThreads) k_iqrm_lag(
   int* cc = cast_ + static_cast<int64_t>(w) * csub;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   // Lagged difference with edge clipping, make_diff_with_clipping (iqrm.cu:94-117).
-  for (int k = threadIdx.x; k < csub; k += kLagThreads) {
+  for (int k = threadIdx.x; k < csub; k += THREADS) {
     float v;
     if (lag < 0) {
       const int cut = csub + lag;
@@ -416,7 +417,7 @@ __global__ void __launch_bounds__(kLagThreads) k_iqrm_lag(
     // the largest t with at most rank keys below it is the key of that rank
     uint32_t c[3] = {0u, 0u, 0u};
     const uint32_t t0 = key[0] | (1u << bit), t1 = key[1] | (1u << bit), t2 = key[2] | (1u << bit);
-    for (int k = threadIdx.x; k < csub; k += kLagThreads) {
+    for (int k = threadIdx.x; k < csub; k += THREADS) {
       const uint32_t v = keys[k];
       c[0] += v < t0;
       c[1] += v < t1;
@@ -429,7 +430,7 @@ __global__ void __launch_bounds__(kLagThreads) k_iqrm_lag(
   }
   // the next order statistic: the same key again, or the least one above it
   uint32_t c[3] = {0u, 0u, 0u}, up[3] = {~0u, ~0u, ~0u};
-  for (int k = threadIdx.x; k < csub; k += kLagThreads) {
+  for (int k = threadIdx.x; k < csub; k += THREADS) {
     const uint32_t v = keys[k];
 #pragma unroll
     for (int j = 0; j < 3; ++j) {
@@ -457,7 +458,7 @@ __global__ void __launch_bounds__(kLagThreads) k_iqrm_lag(
   const bool skip = !(s > 0.f) || !isfinite(s);
   // flag_and_count_kernel (iqrm.cu:120-151).
   const float med = pct[1], thr = __fmul_rn(nsigma, s);
-  for (int i = threadIdx.x; i < csub; i += kLagThreads) {
+  for (int i = threadIdx.x; i < csub; i += THREADS) {
     const bool hit = !skip && __fsub_rn(key_value(keys[i]), med) > thr;
     fl[i] = hit ? 1 : 0;
     if (hit) {
@@ -1056,11 +1057,16 @@ void launch_iqrm_decide(const unsigned long long* d_sums, int nwin, const uint32
   const dim3 all(static_cast<unsigned>(nwin), static_cast<unsigned>((nchans + 255) / 256));
   k_iqrm_stat<<<all, 256, 0, st>>>(d_sums, d_win, nchans, csub, mode, variant, xs, recv, cast_, d_masks);
   DD_LAUNCHED();
-  const size_t smem = sizeof(uint32_t) * csub;
-  allow_dynamic_smem(k_iqrm_lag, smem);
-  k_iqrm_lag<<<dim3(static_cast<unsigned>(nwin), static_cast<unsigned>(nlags)), kLagThreads, smem, st>>>(
-      d_win, n, nsigma, d_lags, nlags, variant, xs, recv, cast_, flags);
-  DD_LAUNCHED();
+  const auto lag = [&](auto kernel, int threads) {
+    const size_t smem = sizeof(uint32_t) * csub;
+    allow_dynamic_smem(kernel, smem);
+    kernel<<<dim3(static_cast<unsigned>(nwin), static_cast<unsigned>(nlags)), threads, smem, st>>>(
+        d_win, n, nsigma, d_lags, nlags, variant, xs, recv, cast_, flags);
+    DD_LAUNCHED();
+  };
+  if (csub <= 32) lag(k_iqrm_lag<32>, 32);
+  else if (csub <= 128) lag(k_iqrm_lag<128>, 128);
+  else lag(k_iqrm_lag<512>, 512);
   const dim3 band(static_cast<unsigned>(nwin), static_cast<unsigned>((csub + 255) / 256));
   k_iqrm_merge<<<band, 256, 0, st>>>(d_win, nchans, cs, n, d_lags, nlags, recv, cast_, flags, d_masks);
   DD_LAUNCHED();

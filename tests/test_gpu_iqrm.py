@@ -52,3 +52,9 @@ def test_masks_equal_oracle(nbits, nchans, cs, ce, nsamp, win, flat, mode):
     assert n == len(t0)
     assert np.array_equal(masks[:n].cpu().numpy(), want)
     assert np.array_equal(bounds[:n].cpu().numpy(), np.stack([t0, t1], 1).astype(np.int32))
+
+
+# Bands around the block sizes of the order statistics (one warp, four, sixteen).
+@pytest.mark.parametrize("csub", [1, 2, 31, 32, 33, 127, 128, 129])
+def test_masks_of_few_channels(csub):
+    test_masks_equal_oracle(8, csub + 6, 3, 3 + csub, 700, 0.2, False, 1)
