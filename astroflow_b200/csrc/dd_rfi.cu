@@ -141,7 +141,12 @@ void launch_time_binning_lut(const void* in, void* out, int64_t ndata, int64_t n
                              int64_t nout, const void* lut, cudaStream_t st) {
   const int64_t words = nchans / static_cast<int64_t>(sizeof(W) / sizeof(T));
   const int64_t gx = (words + 255) / 256;
-  int rows = 16;  // bins per block: more where the grid would pass its limit
+  // bins per block: at least those loaded together; fewer than sixteen where the threads
+  // would not fill the GPU (1024 channels, 5,000 samples in bins of sixteen 30 -> 12 us), more
+  // where the grid would pass its limit
+  const int least = ds == 2 || ds == 4 || ds == 8 ? 16 / ds : 1;
+  int rows = 16;
+  while (rows > least && (nout + rows - 1) / rows * words < 148 * 2048) rows /= 2;
   while ((nout + rows - 1) / rows > 65535) rows *= 2;
   const dim3 g(static_cast<unsigned>(gx), static_cast<unsigned>((nout + rows - 1) / rows));
   const T* i = static_cast<const T*>(in);

@@ -255,3 +255,12 @@ def test_one_time_tile_where_the_sums_fit(spec):
     plan.run_host_join(sync=True)
     for o in outs:
         assert np.array_equal(o, want)
+
+
+# Bins per block: chunks of few bins and channels take fewer, down to those loaded together.
+@pytest.mark.parametrize("n,nchans,nbits,ds", [
+    (400, 16, 8, 2), (415, 17, 8, 16), (9000, 41, 8, 16), (2600, 64, 8, 5), (333, 16, 16, 8), (40000, 33, 16, 3),
+])
+def test_binning_of_small_chunks(n, nchans, nbits, ds):
+    plan, x, want = subband(n, nchans, nbits, 20.0, 0.5, ds, 16, 0.0, False, False)
+    assert np.array_equal(to_np(plan.run(dev(x))), want)
