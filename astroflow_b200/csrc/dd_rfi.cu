@@ -737,12 +737,13 @@ __global__ void __launch_bounds__(256) k_prep_fold(PrepArgs a) {
 // division, and nothing is 64-bit per load.  4096 channels x 151,000 samples in time
 // order 216 us (5.7 TB/s; 480 us with four loads in flight per thread and 64-bit rows),
 // 131,072 samples folded 690 us (5.1 TB/s; 905 us with every load and store predicated
-// and two-way bank conflicts).  The phase rows of downsampled brute force are laid out
-// by one launch per phase (t0 the phase, strides times ds, WS 0: taken from ws).
+// and two-way bank conflicts).  The phase rows of downsampled brute force
+// are laid out by one launch, grid y = phase (WS 0: strides times ds, ws taken from the
+// arguments).
 struct PrepWords {
   int64_t fs, nwords, pitch;  // nwords: words to store per channel; pitch in words
   int ws;
-  int64_t t0;
+  int64_t phase_pitch;  // WS 0: output words between phases
 };
 // Byte masks of four channels as masks of their samples, word v of the four channels.
 template <typename T>
@@ -754,6 +755,7 @@ __device__ __forceinline__ uint32_t expand_mask(uint32_t m4, int v) {
 template <typename T, int WS, bool RAGGED>
 __global__ void __launch_bounds__(256, RAGGED ? 4 : sizeof(T) == 1 && WS == 1 ? 5 : 6) k_prep_w(PrepArgs a, PrepWords q) {
   constexpr int F = 4 / sizeof(T);   // samples per word
+  const int ph = WS == 0 ? static_cast<int>(blockIdx.y) : 0;  // phase: its first sample
   const int ws = WS ? WS : q.ws;
   constexpr int V = sizeof(T);       // 32-bit words per four channels
   // [16 * b + w][word] for channel 4w + b: with 66 words a row, the 16 channel groups and
@@ -761,7 +763,7 @@ __global__ void __launch_bounds__(256, RAGGED ? 4 : sizeof(T) == 1 && WS == 1 ? 
   __shared__ uint32_t tile[64][66];
   int64_t group;
   const int64_t sb = prep_tile(a, a.c0 & ~int64_t(3), &group) * 64;
-  if (a.limit && q.t0 + ws * sb >= a.limit[group]) return;
+  if (a.limit && ph + ws * sb >= a.limit[group]) return;
   const int64_t cb = (a.c0 & ~int64_t(3)) + group * 64;
   const int w = threadIdx.x & 15, r0 = threadIdx.x >> 4;
   const int64_t c = cb + 4 * w;
@@ -791,7 +793,7 @@ __global__ void __launch_bounds__(256, RAGGED ? 4 : sizeof(T) == 1 && WS == 1 ? 
   uint32_t in[4][F][V];
 #pragma unroll
   for (int f = 0; f < F; ++f) {
-    const int64_t t0 = q.t0 + ws * sb + q.fs * f;
+    const int64_t t0 = ph + ws * sb + q.fs * f;
     const T* src = static_cast<const T*>(a.x) + (t0 + ws * r0) * a.nchans + c;
     const int64_t left = a.nsamp - t0;  // words i with ws * i < left
     have[f] = !cvalid || left <= 0 ? 0 : left >= ws * 64 ? 64 : (static_cast<int>(left) + ws - 1) / ws;
@@ -837,7 +839,7 @@ __global__ void __launch_bounds__(256, RAGGED ? 4 : sizeof(T) == 1 && WS == 1 ? 
     for (int f = 0; f < F; ++f) {
       if (!have[f]) continue;
       // the mask of the IQRM segment that holds the tile's rows of this slot
-      const int64_t t0 = q.t0 + ws * sb + q.fs * f;
+      const int64_t t0 = ph + ws * sb + q.fs * f;
       const auto seg_mask = [&](int sg) {
         const uint8_t* p = a.segmask + static_cast<int64_t>(sg) * a.nchans + c;
         if constexpr (RAGGED) {
@@ -873,7 +875,7 @@ __global__ void __launch_bounds__(256, RAGGED ? 4 : sizeof(T) == 1 && WS == 1 ? 
   if (a.zdm_off) {
 #pragma unroll
     for (int f = 0; f < F; ++f) {
-      const uint32_t* offs = a.zdm_off + (q.t0 + ws * (sb + r0) + q.fs * f);
+      const uint32_t* offs = a.zdm_off + (ph + ws * (sb + r0) + q.fs * f);
       uint32_t off[4];
 #pragma unroll
       for (int k = 0; k < 4; ++k) off[k] = r0 + 16 * k < have[f] ? __ldg(offs + 16 * k * ws) : 0u;
@@ -918,6 +920,7 @@ __global__ void __launch_bounds__(256, RAGGED ? 4 : sizeof(T) == 1 && WS == 1 ? 
   const int ch0 = static_cast<int>(max(a.c0 - cb, static_cast<int64_t>(0)));
   const int ch1 = static_cast<int>(min(a.c1 - cb, static_cast<int64_t>(64)));
   uint32_t* dst = static_cast<uint32_t*>(a.out) + (cb + row - a.c0) * q.pitch + sb + lane;
+  if constexpr (WS == 0) dst += ph * q.phase_pitch;
   const uint32_t* from = &tile[16 * (row & 3) + (row >> 2)][lane];
   if (words == 64 && ch0 == 0 && ch1 == 64) {
 #pragma unroll
@@ -1126,34 +1129,29 @@ void launch_prep(const PrepArgs& a, cudaStream_t st) {
   };
   // the word-wise kernel applies integer zero-DM offsets only
   const int F = 32 / a.nbits;
-  const auto run = [&](auto kernel, auto kernel_ragged, unsigned grid, const PrepArgs& p, const PrepWords& q, bool r) {
-    if (r) kernel_ragged<<<grid, 256, 0, st>>>(p, q);
-    else kernel<<<grid, 256, 0, st>>>(p, q);
+  const auto run = [&](auto kernel, auto kernel_ragged, dim3 grid, const PrepWords& q, bool r) {
+    if (r) kernel_ragged<<<grid, 256, 0, st>>>(a, q);
+    else kernel<<<grid, 256, 0, st>>>(a, q);
+    DD_LAUNCHED();
   };
   const bool wide = a.out && !a.zdm_mean;
   const bool ragged = a.nchans % 4 != 0 || reinterpret_cast<uintptr_t>(a.x) % (a.nbits / 2) != 0;
   if (wide && a.nbits <= 16 && a.ds > 1 && a.ds <= 16 && a.pitch % F == 0 && reinterpret_cast<uintptr_t>(a.out) % 4 == 0) {
-    for (int ph = 0; ph < a.ds; ++ph) {
-      PrepArgs p = a;
-      p.out = static_cast<char*>(a.out) + ph * a.pitch * (a.nbits / 8);
-      const int64_t rows = (a.nsamp - ph + a.ds - 1) / a.ds;
-      if (rows <= 0) continue;
-      const PrepWords q{a.ds, (rows + F - 1) / F, a.ds * (a.pitch / F), F * a.ds, ph};
-      const unsigned grid = blocks((q.nwords + 63) / 64, a.c0 & ~int64_t(3));
-      if (a.nbits == 8) run(k_prep_w<uint8_t, 0, false>, k_prep_w<uint8_t, 0, true>, grid, p, q, ragged);
-      else run(k_prep_w<uint16_t, 0, false>, k_prep_w<uint16_t, 0, true>, grid, p, q, ragged);
-      DD_LAUNCHED();
-    }
+    // (of phase 0; where a later one has a word less, its last one is zero)
+    const int64_t words = ((a.nsamp + a.ds - 1) / a.ds + F - 1) / F;
+    const PrepWords q{a.ds, words, a.ds * (a.pitch / F), F * a.ds, a.pitch / F};
+    const dim3 grid(blocks((words + 63) / 64, a.c0 & ~int64_t(3)), static_cast<unsigned>(a.ds));
+    if (a.nbits == 8) run(k_prep_w<uint8_t, 0, false>, k_prep_w<uint8_t, 0, true>, grid, q, ragged);
+    else run(k_prep_w<uint16_t, 0, false>, k_prep_w<uint16_t, 0, true>, grid, q, ragged);
   } else if (wide && (a.fold > 1 || (a.ds == 1 && a.pitch % F == 0 && reinterpret_cast<uintptr_t>(a.out) % 4 == 0))) {
     const PrepWords q = a.fold > 1 ? PrepWords{a.seg, a.nwords, a.pitch, 1, 0}
                                    : PrepWords{1, (a.nsamp + F - 1) / F, a.pitch / F, F, 0};
-    const unsigned grid = blocks((q.nwords + 63) / 64, a.c0 & ~int64_t(3));
-    if (a.nbits == 32) run(k_prep_w<uint32_t, 1, false>, k_prep_w<uint32_t, 1, true>, grid, a, q, ragged);
-    else if (a.nbits == 8 && a.fold > 1) run(k_prep_w<uint8_t, 1, false>, k_prep_w<uint8_t, 1, true>, grid, a, q, ragged);
-    else if (a.nbits == 8) run(k_prep_w<uint8_t, 4, false>, k_prep_w<uint8_t, 4, true>, grid, a, q, ragged);
-    else if (a.fold > 1) run(k_prep_w<uint16_t, 1, false>, k_prep_w<uint16_t, 1, true>, grid, a, q, ragged);
-    else run(k_prep_w<uint16_t, 2, false>, k_prep_w<uint16_t, 2, true>, grid, a, q, ragged);
-    DD_LAUNCHED();
+    const dim3 grid(blocks((q.nwords + 63) / 64, a.c0 & ~int64_t(3)));
+    if (a.nbits == 32) run(k_prep_w<uint32_t, 1, false>, k_prep_w<uint32_t, 1, true>, grid, q, ragged);
+    else if (a.nbits == 8 && a.fold > 1) run(k_prep_w<uint8_t, 1, false>, k_prep_w<uint8_t, 1, true>, grid, q, ragged);
+    else if (a.nbits == 8) run(k_prep_w<uint8_t, 4, false>, k_prep_w<uint8_t, 4, true>, grid, q, ragged);
+    else if (a.fold > 1) run(k_prep_w<uint16_t, 1, false>, k_prep_w<uint16_t, 1, true>, grid, q, ragged);
+    else run(k_prep_w<uint16_t, 2, false>, k_prep_w<uint16_t, 2, true>, grid, q, ragged);
   } else if (a.out && a.fold > 1) {
     const unsigned grid = blocks((a.nwords + 63) / 64, a.c0);
     if (a.nbits == 8) k_prep_fold<uint8_t><<<grid, 256, 0, st>>>(a);

@@ -264,3 +264,24 @@ def test_one_time_tile_where_the_sums_fit(spec):
 def test_binning_of_small_chunks(n, nchans, nbits, ds):
     plan, x, want = subband(n, nchans, nbits, 20.0, 0.5, ds, 16, 0.0, False, False)
     assert np.array_equal(to_np(plan.run(dev(x))), want)
+
+
+# All phase rows of a downsampled brute-force chunk are laid out by one launch, also where the
+# last phases have a sample less or none.
+@pytest.mark.parametrize("n,nc,nbits,ds,frac", [
+    (494, 26, 16, 16, 0.49), (1000, 65, 8, 7, 0.5), (4099, 64, 8, 2, 0.49), (2050, 66, 16, 3, 0.3), (13, 12, 8, 16, 0.9),
+])
+def test_one_launch_lays_out_all_phases(n, nc, nbits, ds, frac):
+    x = data(n, nc, nbits)
+    tsamp, foff = 1e-4, 300.0 / nc
+    freq = O.freq_table_fil(1150.0, foff, nc)
+    fs, fe = float(F32(freq[0])), float(F32(freq[-1]))
+    hdr = dict(tsamp=tsamp, fch1=1150.0, foff=foff, nbits=nbits, nchans=nc, ndata=n)
+    ts = n * tsamp * frac
+    plan = Plan(hdr, 0.0, 8.0, fs, fe, 1.0, ds, ts, algorithm="brute", freq_mode="fil")
+    want = np.concatenate(O.bruteforce_cpu(x, nc, freq, tsamp, 0.0, 8.0, fs, fe, 1.0, ds, ts,
+                                           delay=plan.tables()[0]), axis=1)
+    xd = dev(x)
+    # the layout, and the sums of all slices or (windows too wide to stage) of each
+    assert plan.run_profiled(xd)["launches"] <= 1 + -(-n // max(1, int(ts / tsamp)))
+    assert np.array_equal(to_np(plan.run(xd)), want)
