@@ -180,7 +180,8 @@ struct HLaunch {
   const char* src;       // element 0 of the DM-time rows
   const char* end;       // past their last element
   int64_t pitch;         // elements between rows
-  int64_t rows;
+  int64_t rows;          // rows of the pass
+  const int32_t* row;    // Lanczos: their source rows (nullptr: all of them, in order)
   int target, rows_per_block, win_bytes;
   const int64_t* col0;   // per slice: first column
   const int32_t* seg0;   // per 32 output columns: first source column and their number
@@ -208,7 +209,10 @@ __global__ void __launch_bounds__(kImgThreads) k_hresize(HLaunch L) {
   const int64_t r1 = min(L.rows, static_cast<int64_t>(blockIdx.x + 1) * L.rows_per_block);
   const char* base = L.src + (L.col0[slice] + first) * static_cast<int64_t>(sizeof(E));
   const int64_t row_bytes = L.pitch * static_cast<int64_t>(sizeof(E));
-  auto piece = [&](int64_t r) { return base + r * row_bytes; };
+  auto piece = [&](int64_t r) {
+    if (METHOD == kLanczos && L.row) r = __ldg(L.row + r);
+    return base + r * row_bytes;
+  };
   // copies row r's piece into slot s: whole 16-byte units inside the rows' memory, its
   // first and last elements by plain loads where a unit would leave it
   auto fetch = [&](int64_t r, int s) {
@@ -610,7 +614,8 @@ extern "C" int dd_images(const void* dm_time, int32_t elem_bytes, int64_t nrows,
     struct Group {
       int64_t cols = 0, n = 0;
       int method = 0, win = 0;
-      size_t c0, slot, hoff, hidx, hw, voff, vidx, vw, i0, nn, w, seg0, segn;
+      bool taps = false;  // the horizontal pass makes the vertical taps' rows only, in their order
+      size_t c0, slot, hoff, hidx, hw, voff, vidx, vw, i0, nn, w, seg0, segn, vtap = 0;
     };
     std::vector<Group> groups;
     Tables tabs;
@@ -680,6 +685,15 @@ extern "C" int dd_images(const void* dm_time, int32_t elem_bytes, int64_t nrows,
       g.i0 = tabs.add(i0);
       g.nn = tabs.add(n);
       g.w = tabs.add(w);
+      // Lanczos reads eight source rows per output row: of many more only those pass (60,000
+      // rows to 64 in 20 slices: 667 us with all of them, 93 a row at a time in one pass, now
+      // 28; 16,000 rows to 512 in 8 slices 608, 494, 203)
+      g.taps = g.method == kLanczos && nrows > 12 * static_cast<int64_t>(target);
+      if (g.taps) {
+        std::vector<int32_t> order(v.idx.size());
+        for (size_t i = 0; i < order.size(); ++i) order[i] = static_cast<int32_t>(i);
+        g.vtap = tabs.add(order);
+      }
       g.seg0 = tabs.add(seg0);
       g.segn = tabs.add(segn);
       groups.push_back(g);
@@ -704,7 +718,6 @@ extern "C" int dd_images(const void* dm_time, int32_t elem_bytes, int64_t nrows,
           img, npix, resized ? 1 : 0, slots, ext, lut, images);
       DD_LAUNCHED();
     };
-    const int64_t hbytes = nrows * target * static_cast<int64_t>(sizeof(float));  // per slice
     float* hres = nullptr;
     int64_t hslices = 0;
     for (const Group& g : groups) {
@@ -712,6 +725,8 @@ extern "C" int dd_images(const void* dm_time, int32_t elem_bytes, int64_t nrows,
                                  ? static_cast<float>(1.0 / (static_cast<double>(g.cols / target) * (nrows / target)))
                                  : 1.0f;
       const int ky = static_cast<int>(nrows / target), kx = static_cast<int>(g.cols / target);
+      const int64_t hrows = g.taps ? 8 * target : nrows;
+      const int64_t hbytes = hrows * target * static_cast<int64_t>(sizeof(float));  // per slice
       if (g.win <= kRingMaxBytes && hbytes <= kHorizontalBytes && nseg <= 65535) {
         const int64_t per = std::min<int64_t>(std::min<int64_t>(g.n, kHorizontalBytes / hbytes), 65535);
         if (per > hslices) {
@@ -720,7 +735,7 @@ extern "C" int dd_images(const void* dm_time, int32_t elem_bytes, int64_t nrows,
         }
         // eight rows per warp and turn; fewer rows per block where the grid is small
         int rpb = 128;
-        while (rpb > 32 && (nrows + rpb - 1) / rpb * nseg * per < 148 * 4) rpb /= 2;
+        while (rpb > 32 && (hrows + rpb - 1) / rpb * nseg * per < 148 * 4) rpb /= 2;
         for (int64_t s0 = 0; s0 < g.n; s0 += per) {
           const int64_t ns = std::min(per, g.n - s0);
           float* img = float_images(per);
@@ -728,7 +743,8 @@ extern "C" int dd_images(const void* dm_time, int32_t elem_bytes, int64_t nrows,
           L.src = static_cast<const char*>(dm_time);
           L.end = L.src + nrows * row_pitch * elem_bytes;
           L.pitch = row_pitch;
-          L.rows = nrows;
+          L.rows = hrows;
+          L.row = g.taps ? tabs.at<int32_t>(g.vidx) : nullptr;
           L.target = target;
           L.rows_per_block = rpb;
           L.win_bytes = g.win;
@@ -742,12 +758,12 @@ extern "C" int dd_images(const void* dm_time, int32_t elem_bytes, int64_t nrows,
           L.ha_w = tabs.at<float4>(g.w);
           L.kx = kx;
           L.out = hres;
-          const dim3 hg(static_cast<unsigned>((nrows + rpb - 1) / rpb), static_cast<unsigned>(nseg), static_cast<unsigned>(ns));
+          const dim3 hg(static_cast<unsigned>((hrows + rpb - 1) / rpb), static_cast<unsigned>(nseg), static_cast<unsigned>(ns));
           if (g.method == kAreaGeneral) launch_hresize<kAreaGeneral>(L, elem_bytes, hg, st);
           else if (g.method == kAreaInteger) launch_hresize<kAreaInteger>(L, elem_bytes, hg, st);
           else launch_hresize<kLanczos>(L, elem_bytes, hg, st);
           k_vresize<<<dim3(static_cast<unsigned>(target), static_cast<unsigned>(ns)), kImgThreads, 0, st>>>(
-              hres, nrows, target, g.method, tabs.at<int32_t>(g.voff), tabs.at<int32_t>(g.vidx),
+              hres, hrows, target, g.method, tabs.at<int32_t>(g.voff), tabs.at<int32_t>(g.taps ? g.vtap : g.vidx),
               tabs.at<float>(g.vw), ky, inv_area, tabs.at<int>(g.slot) + s0, resized ? 1 : 0, img, ext);
           DD_LAUNCHED();
           colorize(img, tabs.at<int>(g.slot) + s0, ns);

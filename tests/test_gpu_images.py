@@ -96,3 +96,17 @@ def test_bad_arguments_raise():
         postprocess.device_images(raw, [90], [20])
     with pytest.raises(ValueError):
         postprocess.device_images(raw, [0], [0])
+
+
+# Lanczos from more rows than its taps read: only the taps' rows are resampled.
+@pytest.mark.parametrize("rows,cols,target", [(513, 60, 64), (512, 60, 64), (20001, 64, 64), (5000, 100, 128), (4097, 300, 512)])
+@pytest.mark.parametrize("dt", [np.uint32, np.uint64])
+def test_lanczos_from_many_rows(rows, cols, target, dt):
+    raw = np.random.default_rng(rows).integers(0, 1 << 20, (rows, 3 * cols)).astype(dt)
+    starts = [0, cols // 2, 2 * cols]
+    got = postprocess.device_images(_dev(raw), starts, [cols] * 3, target=target, resized=True).cpu().numpy()
+    imgs = postprocess.device_images(_dev(raw), starts, [cols] * 3, target=target).cpu().numpy()
+    for i, s in enumerate(starts):
+        f = np.ascontiguousarray(raw[:, s:s + cols], dtype=np.float32)
+        np.testing.assert_array_equal(got[i], cv2.resize(f, (target, target), interpolation=cv2.INTER_LANCZOS4))
+        np.testing.assert_array_equal(imgs[i], CVI.image(raw[:, s:s + cols], target))
