@@ -202,14 +202,25 @@ __device__ __forceinline__ void add_window_sums(const uint32_t* __restrict__ win
   }
 }
 
+// Many short windows: a grid z each (their runs would hold a few samples, and a run costs
+// its windows' bounds and sums).
+__device__ __forceinline__ void take_window(const uint32_t*& win, int& nwin, int64_t csub,
+                                            unsigned long long*& sums) {
+  if (gridDim.z == 1) return;
+  win += 2 * static_cast<int64_t>(blockIdx.z);
+  sums += 2 * csub * blockIdx.z;
+  nwin = 1;
+}
+
 // One channel per thread; grid.y: chunks of samples.
 template <typename T>
 __global__ void k_iqrm_stats(const T* __restrict__ x, int64_t nsamp, int64_t nchans, int64_t cs,
-                             int64_t csub, const uint32_t* __restrict__ win, int nwin,
-                             int64_t chunk, unsigned long long* __restrict__ sums) {
+                             int64_t csub, const uint32_t* win, int nwin,
+                             int64_t chunk, unsigned long long* sums) {
   int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= csub) return;
   const int64_t c = cs + i;
+  take_window(win, nwin, csub, sums);
   const int64_t lo = static_cast<int64_t>(blockIdx.y) * chunk;
   const int64_t hi = lo + chunk < nsamp ? lo + chunk : nsamp;
   for_window_runs(win, nwin, lo, hi, [&](int64_t a, int64_t b, int w) {
@@ -233,9 +244,10 @@ __global__ void k_iqrm_stats(const T* __restrict__ x, int64_t nsamp, int64_t nch
 // with one read per window, byte-wise sums and 1024-row chunks only).
 __global__ void __launch_bounds__(128) k_iqrm_stats_u8w(
     const uint8_t* __restrict__ x, int64_t nsamp, int64_t nchans, int64_t cs, int64_t csub,
-    const uint32_t* __restrict__ win, int nwin, int64_t chunk, unsigned long long* __restrict__ sums) {
+    const uint32_t* win, int nwin, int64_t chunk, unsigned long long* sums) {
   const int64_t c4 = (cs & ~int64_t(3)) + 4 * (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x);
   if (c4 >= cs + csub) return;
+  take_window(win, nwin, csub, sums);
   const int64_t lo = static_cast<int64_t>(blockIdx.y) * chunk;
   const int64_t hi = lo + chunk < nsamp ? lo + chunk : nsamp;
   for_window_runs(win, nwin, lo, hi, [&](int64_t a, int64_t b, int w) {
@@ -275,9 +287,10 @@ __global__ void __launch_bounds__(128) k_iqrm_stats_u8w(
 // 64-bit sums of squares per chunk.  Needs nchans % 2 == 0 and an aligned input.
 __global__ void __launch_bounds__(128) k_iqrm_stats_u16w(
     const uint16_t* __restrict__ x, int64_t nsamp, int64_t nchans, int64_t cs, int64_t csub,
-    const uint32_t* __restrict__ win, int nwin, int64_t chunk, unsigned long long* __restrict__ sums) {
+    const uint32_t* win, int nwin, int64_t chunk, unsigned long long* sums) {
   const int64_t c2 = (cs & ~int64_t(1)) + 2 * (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x);
   if (c2 >= cs + csub) return;
+  take_window(win, nwin, csub, sums);
   const int64_t lo = static_cast<int64_t>(blockIdx.y) * chunk;
   const int64_t hi = lo + chunk < nsamp ? lo + chunk : nsamp;
   for_window_runs(win, nwin, lo, hi, [&](int64_t a, int64_t b, int w) {
@@ -1011,7 +1024,12 @@ void launch_iqrm_stats(const void* x, int nbits, int64_t nsamp, int64_t nchans, 
   const int64_t gx = (cols + threads - 1) / threads;
   int64_t chunk = 1024;
   while (chunk > 64 && gx * ((nsamp + chunk - 1) / chunk) < 148 * 8) chunk /= 2;
-  const dim3 grid(static_cast<unsigned>(gx), static_cast<unsigned>((nsamp + chunk - 1) / chunk));
+  // windows that start less than 64 samples apart are read one by one (240 channels, 100
+  // samples, windows of 32 every 2: 184 us with runs of two samples, 82 by one block per
+  // window before that, now 38; windows of 400 every 200 are better read together, 114 us
+  // against 172 apart)
+  const bool apart = nsamp < 64 * static_cast<int64_t>(nwin) && nwin <= 65535;
+  const dim3 grid(static_cast<unsigned>(gx), static_cast<unsigned>((nsamp + chunk - 1) / chunk), apart ? nwin : 1);
   if (u8w)
     k_iqrm_stats_u8w<<<grid, threads, 0, st>>>(static_cast<const uint8_t*>(x), nsamp, nchans, cs, csub, d_win, nwin, chunk, d_sums);
   else if (u16w)

@@ -58,3 +58,22 @@ def test_masks_equal_oracle(nbits, nchans, cs, ce, nsamp, win, flat, mode):
 @pytest.mark.parametrize("csub", [1, 2, 31, 32, 33, 127, 128, 129])
 def test_masks_of_few_channels(csub):
     test_masks_equal_oracle(8, csub + 6, 3, 3 + csub, 700, 0.2, False, 1)
+
+
+# Windows that start a few samples apart are summed one by one, the rest in shared runs.
+@pytest.mark.parametrize("nbits,nchans,nsamp,win,hop", [
+    (8, 240, 100, 32, 2), (8, 97, 100, 32, 3), (16, 60, 300, 7, 1), (16, 61, 128, 100, 9), (32, 30, 90, 30, 2),
+    (8, 64, 2000, 200, 70), (16, 64, 2000, 200, 63),
+])
+def test_masks_of_many_short_windows(nbits, nchans, nsamp, win, hop):
+    rng = np.random.default_rng(nsamp + nchans)
+    x = rng.integers(0, 200, (nsamp, nchans)).astype({8: np.uint8, 16: np.uint16, 32: np.uint32}[nbits])
+    x[:, 5] //= 9
+    x[nsamp // 2:, 17] = 3
+    iq = IqrmParams(mode=1, radius_frac=0.1, nsigma=3.0, geofactor=1.5, win_sec=win * TSAMP + 1e-7,
+                    hop_sec=hop * TSAMP + 1e-7, include_tail=True)
+    t0, t1, want = O.iqrm_masks(x.copy(), nchans, 2, nchans - 1, TSAMP, iq)
+    masks = torch.full((len(t0), nchans), 9, dtype=torch.uint8, device="cuda")
+    bounds = torch.zeros((len(t0), 2), dtype=torch.int32, device="cuda")
+    assert iqrm_masks_noalloc(to_dev(x), nchans, 2, nchans - 1, TSAMP, iq, masks, bounds) == len(t0)
+    assert t0[1] == hop and np.array_equal(masks.cpu().numpy(), want)
