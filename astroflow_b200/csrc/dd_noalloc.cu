@@ -167,13 +167,14 @@ extern "C" int dd_iqrm_masks_noalloc(const void* input, int32_t nbits, int64_t n
       if (lag < csub) nlags += 2;
       lag = std::max(static_cast<int>(g * lag), lag + 1);
     }
-    if (nlags) check_iqrm_channels(csub);  // the per-window sort fits shared memory
+    if (nlags) check_iqrm_channels(csub);  // a window's differences fit shared memory
 
     // Scratch layout inside g_iqrm_scratch.
     const size_t b_win = align256(sizeof(uint32_t) * 2 * nwin);
     const size_t b_lags = align256(sizeof(int32_t) * std::max(1, nlags));
     const size_t b_sums = align256(sizeof(unsigned long long) * 2 * csub * nwin);
-    const size_t b_work = align256(iqrm_scratch_bytes(nwin, csub, nlags));
+    // (a row of words more than the kernels use: the size that requests are accepted by)
+    const size_t b_work = align256(iqrm_scratch_bytes(nwin, csub, nlags) + sizeof(float) * nwin * csub);
     const size_t need = b_win + b_lags + b_sums + b_work;
     if (need > kScratchBytes) {
       char msg[256];

@@ -1044,26 +1044,24 @@ void launch_iqrm_stats(const void* x, int nbits, int64_t nsamp, int64_t nchans, 
 }
 
 size_t iqrm_scratch_bytes(int nwin, int64_t csub, int nlags) {
-  return static_cast<size_t>(nwin) * csub * (4 + 4 + 4 + 4 + nlags) + 256;
+  return static_cast<size_t>(nwin) * csub * (4 + 4 + 4 + nlags) + 256;
 }
 
-// k_iqrm_lag holds one window's csub differences in shared memory; band widths are
-// limited to those whose next power of two of floats fits the current device's opt-in
-// shared memory per block.
+// k_iqrm_lag holds one window's csub differences in shared memory.  Bands are limited to
+// the largest power of two of words that a block's opt-in shared memory holds (32,768
+// channels on sm_100), with room for the kernel's own.
 void check_iqrm_channels(int64_t csub) {
-  int64_t sort_n = 1;
-  while (sort_n < csub) sort_n <<= 1;
   int dev = 0, optin = 0;
   DD_CUDA_TRY(cudaGetDevice(&dev));
   DD_CUDA_TRY(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-  const int64_t need = static_cast<int64_t>(sizeof(float)) * sort_n;
-  if (need > optin) {
+  int64_t most = 1;
+  while (2 * most * static_cast<int64_t>(sizeof(uint32_t)) <= optin) most *= 2;
+  if (csub > most) {
     char msg[200];
     std::snprintf(msg, sizeof(msg),
-                  "IQRM over %lld channels needs a %lld-byte sort buffer, more than the %d bytes "
-                  "of shared memory a block can have (at most %d channels)",
-                  static_cast<long long>(csub), static_cast<long long>(need), optin,
-                  optin / static_cast<int>(sizeof(float)));
+                  "IQRM over %lld channels: a window's differences are held in a block's shared memory "
+                  "(%d bytes), at most %lld channels",
+                  static_cast<long long>(csub), optin, static_cast<long long>(most));
     throw Error{DD_ERR_INVALID, msg};
   }
 }
@@ -1072,9 +1070,9 @@ void launch_iqrm_decide(const unsigned long long* d_sums, int nwin, const uint32
                         int64_t nchans, int64_t cs, int64_t csub, int mode, float nsigma,
                         const int32_t* d_lags, int nlags, int variant, void* scratch,
                         uint8_t* d_masks, cudaStream_t st) {
-  // scratch (iqrm_scratch_bytes): statistics, an unused row, vote counters, flags
+  // scratch (iqrm_scratch_bytes): statistics, vote counters, flags
   char* p = static_cast<char*>(scratch);
-  float* xs = reinterpret_cast<float*>(p); p += 2 * sizeof(float) * nwin * csub;
+  float* xs = reinterpret_cast<float*>(p); p += sizeof(float) * nwin * csub;
   int* recv = reinterpret_cast<int*>(p); p += sizeof(int) * nwin * csub;
   int* cast_ = reinterpret_cast<int*>(p); p += sizeof(int) * nwin * csub;
   uint8_t* flags = reinterpret_cast<uint8_t*>(p);

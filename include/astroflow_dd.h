@@ -320,8 +320,8 @@ int dd_measure_int_add_rate(int32_t device, double* adds_per_second);
  *
  * All working memory comes from an 8 MiB array that the library keeps in a
  * GPU's memory from the first call on that GPU until the process exits;
- * requests whose working set exceeds it, and bands wider than the per-window
- * sort's shared memory holds, fail with DD_ERR_INVALID.  The first call on a
+ * requests whose working set exceeds it, and bands wider than a block's shared
+ * memory holds (32,768 channels), fail with DD_ERR_INVALID.  The first call on a
  * device resolves the array's address with that device current: make it before
  * any stream capture.  The library's device code loads lazily, so that first
  * call is also when the array takes its 8 MiB: a host that reserves most of the

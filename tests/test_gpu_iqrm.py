@@ -77,3 +77,13 @@ def test_masks_of_many_short_windows(nbits, nchans, nsamp, win, hop):
     bounds = torch.zeros((len(t0), 2), dtype=torch.int32, device="cuda")
     assert iqrm_masks_noalloc(to_dev(x), nchans, 2, nchans - 1, TSAMP, iq, masks, bounds) == len(t0)
     assert t0[1] == hop and np.array_equal(masks.cpu().numpy(), want)
+
+
+def test_widest_band():
+    """The widest band whose differences a block holds, and one channel more."""
+    test_masks_equal_oracle(8, 32769, 0, 32768, 20, 0.0, False, 1)
+    x = torch.zeros((8, 32770), dtype=torch.uint8, device="cuda")
+    masks = torch.zeros((1, 32770), dtype=torch.uint8, device="cuda")
+    bounds = torch.zeros((1, 2), dtype=torch.int32, device="cuda")
+    with pytest.raises(ValueError, match="at most 32768 channels"):
+        iqrm_masks_noalloc(x, 32770, 0, 32769, TSAMP, IqrmParams(radius_frac=1e-4, win_sec=0.0), masks, bounds)
