@@ -172,7 +172,7 @@ def test_32bit_sums_equal_oracle(n, nchans, hi, step, ds, width):
 
 
 # 32-bit layout by words: masks that change inside a tile of 64 samples, zero-DM offsets and
-# zeroed channels, at tile remainders; 37 channels take the per-sample kernel.
+# zeroed channels, at tile remainders; rows of 37 channels do not start on a word.
 @pytest.mark.parametrize("n,nchans,width", [(511, 36, 16), (2049, 132, 64), (3001, 40, 8), (1027, 37, 9)])
 def test_32bit_layout_with_masks(n, nchans, width):
     rng = np.random.default_rng(n + nchans)
@@ -235,6 +235,36 @@ def test_ragged_rows(n, nchans, nbits, ds):
 @pytest.mark.parametrize("n,nchans,width", [(513, 37, 9), (2049, 131, 64)])
 def test_ragged_rows_of_32_bits(n, nchans, width):
     test_32bit_layout_with_masks(n, nchans, width)
+
+
+# The same on whole tiles (launches of at least four blocks per SM; the cases above take half
+# tiles): one tile of every segment, a sample less and more, a last segment of a few columns,
+# odd channel counts, subbands wider than the packing holds, full-scale samples.
+@pytest.mark.parametrize("n,nchans,nbits,hi,step,width", [
+    (2560, 64, 8, 60.0, 0.01, 2), (2561, 64, 8, 60.0, 0.01, 2), (2559, 67, 8, 60.0, 0.01, 2),
+    (5125, 33, 8, 60.0, 0.01, 2), (17921, 260, 8, 60.0, 0.005, 65), (17923, 129, 8, 60.0, 0.005, 129),
+    (1280, 64, 16, 60.0, 0.01, 2), (1281, 67, 16, 60.0, 0.01, 2), (2561, 64, 16, 60.0, 0.01, 2),
+])
+def test_subband_on_whole_tiles(n, nchans, nbits, hi, step, width):
+    plan, x, want = subband(n, nchans, nbits, hi, step, 1, width, 0.0, False, False, full=True)
+    assert np.array_equal(to_np(plan.run(dev(x))), want)
+
+
+@pytest.mark.parametrize("n,nc,nbits,trials", [
+    (2560, 65, 8, 9490), (2561, 33, 8, 4800), (5119, 130, 8, 4790), (1280, 64, 16, 9490), (1281, 65, 16, 4800),
+])
+def test_brute_force_on_whole_tiles(n, nc, nbits, trials):
+    x = data(n, nc, nbits, full=True)
+    tsamp, foff, step = 1e-4, 300.0 / nc, 0.005
+    freq = O.freq_table_fil(1150.0, foff, nc)
+    fs, fe = float(F32(freq[0])), float(F32(freq[-1]))
+    hdr = dict(tsamp=tsamp, fch1=1150.0, foff=foff, nbits=nbits, nchans=nc, ndata=n)
+    hi, ts = (trials - 0.5) * step, n * tsamp * 0.49
+    plan = Plan(hdr, 0.0, hi, fs, fe, step, 1, ts, algorithm="brute", freq_mode="fil")
+    assert plan.out_shape[0] == trials
+    want = np.concatenate(O.bruteforce_cpu(x, nc, freq, tsamp, 0.0, hi, fs, fe, step, 1, ts,
+                                           delay=plan.tables()[0]), axis=1)
+    assert np.array_equal(to_np(plan.run(dev(x))), want)
 
 
 # A chunk whose subband sums fit the budget is summed as one time tile (each tile costs stage
