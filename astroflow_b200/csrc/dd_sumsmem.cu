@@ -50,10 +50,6 @@ namespace {
 
 constexpr int kWarps = 8;
 constexpr int kThreads = kWarps * 32;
-#ifndef DD_SUM_MAX_STAGES
-#define DD_SUM_MAX_STAGES 8
-#endif
-constexpr int kMaxStages = DD_SUM_MAX_STAGES;  // groups of sources in flight, at most
 constexpr long long kWaitCycles = 4000000000LL;
 
 // ------------------------------------------------------------------ mbarrier helpers
@@ -218,11 +214,11 @@ __device__ __forceinline__ Geo make_geo(const SumLaunch& L, int T, uint3 blk) {
 // Shared state of the pipeline.  A stage holds QS sources: two, or four with their
 // twins.
 struct __align__(16) Pipe {
-  uint64_t full[kMaxStages];   // completes when a stage's windows have landed
-  uint64_t empty[kMaxStages];  // completes when all warps released a stage
+  uint64_t full[kSumMaxStages];   // completes when a stage's windows have landed
+  uint64_t empty[kSumMaxStages];  // completes when all warps released a stage
   // per row: word index and shift (bits) of sample 0 in the window of source i of
   // the stage at [2i], [2i+1]; twin windows (four sources): word indices only
-  int row[kMaxStages][kSumRows][4];
+  int row[kSumMaxStages][kSumRows][4];
   uint32_t first[kWarps];      // first source with samples of the chunk, by warp
   int failed;
 };
@@ -449,7 +445,7 @@ __device__ __forceinline__ bool run_pipeline(const SumLaunch& L, Geo& g, Pipe& P
                                              uint32_t* sw, int tile, Setup&& setup, Body&& body) {
   static_assert(MODE == kModePlain || MODE == kModePhase ? QS == 2 : QS == 4 || (QS == 2 && MODE == kModeWords),
                 "sources per stage");
-  static_assert(kMaxStages <= kWarps, "each warp stages at most one group before the loop");
+  static_assert(kSumMaxStages <= kWarps, "each warp stages at most one group before the loop");
   constexpr int kWinPerSrc = MODE == kModeTwin ? 2 : 1;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int ww = L.win_bytes >> 2;
@@ -1409,7 +1405,7 @@ size_t sum_launch_smem(const SumLaunch& L) {
 #endif
 int sum_stages(int win_bytes, int qs, size_t extra, int cap_kb) {
   const size_t cap = static_cast<size_t>(cap_kb > 0 ? cap_kb : DD_SUM_SMEM_KB) * 1024;
-  int s = kMaxStages;
+  int s = kSumMaxStages;
   while (s > 2 && sum_smem_bytes(win_bytes, s, qs) + extra > cap) --s;
   return s;
 }
@@ -1460,7 +1456,7 @@ std::vector<SumDesc> build_sum_desc(const std::vector<int32_t>& tab, int64_t nro
 
 void launch_sum(const SumLaunch& L, cudaStream_t st) {
   dim3 grid(sum_grid_x(L), L.grid_y, L.grid_z);
-  if (L.stages < 2 || L.stages > kMaxStages) throw Error{DD_ERR_RUNTIME, "bad stage count"};
+  if (L.stages < 2 || L.stages > kSumMaxStages) throw Error{DD_ERR_RUNTIME, "bad stage count"};
   if (!L.desc || !L.err) throw Error{DD_ERR_RUNTIME, "staged sum without descriptors"};
   const size_t smem = sum_launch_smem(L);
   switch (sum_kind(L)) {
