@@ -663,10 +663,10 @@ void set_brute_window(dd_plan& P) {
     if (P.winb) upload_desc(P.d_descb, desc);
   }
   P.seg = P.fold > 1 ? round_up((P.out_cols + P.fold - 1) / P.fold, 8) : P.out_cols;
-  // folded windows start before the chunk's end and inside a segment and the padding of
-  // phase_len, and end a block tile and their spread later
+  // folded windows start before the chunk's end, at most the largest delay past a segment,
+  // and end a block tile and their spread later
   const int64_t pitch =
-      P.fold > 1 ? round_up(std::min(P.nin, P.seg + P.phase_len - P.nin) + sum_kind_tile(brute_kind(P)) + spread + 64, 64)
+      P.fold > 1 ? round_up(std::min<int64_t>(P.nin, P.seg + P.max_delay) + sum_kind_tile(brute_kind(P)) + spread + 64, 64)
                  : P.phase_len;
   if (P.p.time_downsample == 1) set_xlimit(P, P.cs, P.nc, P.seg);
   if (had && P.fold == fold0 && pitch == P.xpitch) return;

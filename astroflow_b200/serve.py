@@ -93,7 +93,7 @@ def workspace_bound(n: int, c: int, bits: int, tsamp: float, fch1: float, foff: 
         reach = int(per_dm * kw["dm_high"]) + 2
         # phase rows: the samples, the delay, a slice (at most the chunk), whole tiles
         linear = elem * (2 * n + reach + ds * 16384)
-        folded = 4 * (n + 16384)
+        folded = 4 * (min(n, n // fold + reach) + 16384)
         inter = 0
         tables = 8 * ndm * c
     else:

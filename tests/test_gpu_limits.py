@@ -129,6 +129,31 @@ def test_folded_subband_sums_stay_near_their_budget():
     plan.close()
 
 
+def test_folded_brute_force_holds_a_segment_and_the_largest_delay():
+    """Words of the folded layout end at the largest delay past a segment: a quarter of the
+    chunk and 34,000 samples of delay per channel, where the rows in time order need the
+    chunk, the delay and a slice."""
+    from astroflow_b200.dedisp import Plan
+    from oracle import oracle as O
+
+    n, nc, tsamp = 1 << 17, 64, 6.4e-5
+    freq = O.freq_table_fil(1000.0, 500.0 / nc, nc)
+    fs, fe = float(np.float32(freq[0])), float(np.float32(freq[-1]))
+    hdr = dict(tsamp=tsamp, fch1=1000.0, foff=500.0 / nc, nbits=8, nchans=nc, ndata=n)
+    plan = Plan(hdr, 0.0, 950.0, fs, fe, 1.0, 1, n * tsamp * 0.49, algorithm="brute", freq_mode="fil")
+    most = int(plan.tables()[0].max())
+    assert 30000 < most < 40000
+    assert plan.info["workspace_bytes"] < nc * 4 * (n // 4 + most + 4096) + plan.out_shape[0] * nc * 8 + (1 << 16)
+    # delays twice as long as the plan's own: the rows grow with them
+    x = np.random.default_rng(8).integers(0, 256, (n, nc)).astype(np.uint8)
+    table = np.minimum(plan.tables()[0] * 2, most + 15000).astype(np.int32)
+    plan.set_delay_table(table)
+    want = np.concatenate(O.bruteforce_cpu(x, nc, freq, tsamp, 0.0, 950.0, fs, fe, 1.0, 1, n * tsamp * 0.49,
+                                           delay=table), axis=1)
+    assert np.array_equal(to_np(plan.run(dev(x))), want)
+    plan.close()
+
+
 def fill_device(leave):
     """All of the device's free memory but `leave` bytes."""
     torch.cuda.synchronize()
@@ -138,8 +163,8 @@ def fill_device(leave):
 
 # A folded chunk takes up to four times its bytes: with less memory left than that, the plan
 # keeps the chunk in time order (subband sums: shorter time tiles come first).  MiB: left for the plan or the stream (time order / folded take
-# 480 / 1045, 1143 / 1452 and, with the stream's own buffer, 2191 / 2409).
-@pytest.mark.parametrize("kind,nbits,leave_mb", [("brute", 8, 760), ("subband", 16, 1300), ("subband", 16, 800), ("stream", 16, 2310)])
+# 480 / 658, 1143 / 1452 and, with the stream's own buffer, 2191 / 2409).
+@pytest.mark.parametrize("kind,nbits,leave_mb", [("brute", 8, 630), ("subband", 16, 1300), ("subband", 16, 800), ("stream", 16, 2310)])
 def test_plans_whose_folded_layout_does_not_fit(kind, nbits, leave_mb):
     from astroflow_b200.dedisp import Plan, Stream
 
@@ -167,11 +192,11 @@ def test_plans_whose_folded_layout_does_not_fit(kind, nbits, leave_mb):
     want = run(p, out).view(torch.int32).cpu()
     folded = p.info["workspace_bytes"]
     p.close()
+    out.view(torch.int32).zero_()
     hog = fill_device(leave_mb << 20)
     try:
         p = make()
         assert p.info["workspace_bytes"] < folded
-        out.view(torch.int32).zero_()
         assert torch.equal(run(p, out).view(torch.int32).cpu(), want)
         p.close()
     finally:
