@@ -1,6 +1,10 @@
 """Calls at the limits of a launch, a row or the device: more slices than a grid dimension
 holds, rows of more than 2^31 samples, staged windows as wide as shared memory, trial steps so
 coarse that rows are staged by eight or not at all, plans whose folded layout does not fit."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
@@ -154,51 +158,54 @@ def test_folded_brute_force_holds_a_segment_and_the_largest_delay():
     plan.close()
 
 
-def fill_device(leave):
-    """All of the device's free memory but `leave` bytes."""
-    torch.cuda.synchronize()
-    torch.cuda.empty_cache()
-    return torch.empty(torch.cuda.mem_get_info()[0] - leave, dtype=torch.uint8, device="cuda")
-
-
 # A folded chunk takes up to four times its bytes: with less memory left than that, the plan
-# keeps the chunk in time order (subband sums: shorter time tiles come first).  MiB: left for the plan or the stream (time order / folded take
-# 480 / 658, 1143 / 1452 and, with the stream's own buffer, 2191 / 2409).
-@pytest.mark.parametrize("kind,nbits,leave_mb", [("brute", 8, 630), ("subband", 16, 1300), ("subband", 16, 800), ("stream", 16, 2310)])
+# keeps the chunk in time order (subband sums: shorter time tiles come first).  In a process
+# of its own, whose memory holds nothing else; MiB left for the plan or the stream (time order /
+# folded take 480 / 658, 1143 / 1452 and, with the stream's own buffer, 2191 / 2409).
+SHORT_OF_MEMORY = """
+import sys
+import numpy as np
+import torch
+from astroflow_b200.dedisp import Plan, Stream
+
+kind, nbits, leave = sys.argv[1], int(sys.argv[2]), int(sys.argv[3]) << 20
+n, nc, f32 = 1 << (17 if kind == "stream" else 18), 1024, np.float32
+x = torch.randint(0, 127, (n, nc * nbits // 8), dtype=torch.uint8, device="cuda").view(
+    torch.uint8 if nbits == 8 else torch.uint16)
+hdr = dict(tsamp=float(f32(1.6e-4)), fch1=400.0, foff=float(f32(400.0 / nc)), nbits=nbits, nchans=nc, ndata=n)
+fe = float(f32(400.0) + f32(nc - 1) * f32(400.0 / nc))
+
+def make():
+    if kind == "brute":
+        return Plan(hdr, 0.0, 800.0, 400.0, fe, 2.5, 1, n * 1.6e-4 * 0.49, algorithm="brute", freq_mode="fil")
+    if kind == "subband":
+        return Plan(hdr, 0.0, 600.0, 400.0, fe, 1.0, 1)
+    return Stream(hdr, 0.0, 800.0, 400.0, fe, 0.5, 1)
+
+def run(p):
+    p.push(x, out) if kind == "stream" else p.run(x, out)
+    return out.view(torch.int32).cpu()
+
+p = make()
+out = p.empty_output()
+want = run(p)
+folded = p.info["workspace_bytes"]
+p.close()
+out.view(torch.int32).zero_()
+torch.cuda.synchronize()
+torch.cuda.empty_cache()
+hog = torch.empty(torch.cuda.mem_get_info()[0] - leave, dtype=torch.uint8, device="cuda")
+p = make()
+assert p.info["workspace_bytes"] < folded, (p.info["workspace_bytes"], folded)
+assert torch.equal(run(p), want)
+"""
+
+
+@pytest.mark.parametrize("kind,nbits,leave_mb", [("brute", 8, 630), ("subband", 16, 1300), ("subband", 16, 800),
+                                                 ("stream", 16, 2310)])
 def test_plans_whose_folded_layout_does_not_fit(kind, nbits, leave_mb):
-    from astroflow_b200.dedisp import Plan, Stream
-
-    n, nc = 1 << 18, 1024
-    if kind == "stream":
-        n = 1 << 17
-    x = torch.randint(0, 127, (n, nc * nbits // 8), dtype=torch.uint8, device="cuda").view(
-        torch.uint8 if nbits == 8 else torch.uint16)
-    f32 = np.float32
-    hdr = dict(tsamp=float(f32(1.6e-4)), fch1=400.0, foff=float(f32(400.0 / nc)), nbits=nbits, nchans=nc, ndata=n)
-    fe = float(f32(400.0) + f32(nc - 1) * f32(400.0 / nc))
-
-    def make():
-        if kind == "brute":
-            return Plan(hdr, 0.0, 800.0, 400.0, fe, 2.5, 1, n * 1.6e-4 * 0.49, algorithm="brute", freq_mode="fil")
-        if kind == "subband":
-            return Plan(hdr, 0.0, 600.0, 400.0, fe, 1.0, 1)
-        return Stream(hdr, 0.0, 800.0, 400.0, fe, 0.5, 1)
-
-    def run(p, out):
-        return p.push(x, out) if kind == "stream" else p.run(x, out)
-
-    p = make()
-    out = p.empty_output()
-    want = run(p, out).view(torch.int32).cpu()
-    folded = p.info["workspace_bytes"]
-    p.close()
-    out.view(torch.int32).zero_()
-    hog = fill_device(leave_mb << 20)
-    try:
-        p = make()
-        assert p.info["workspace_bytes"] < folded
-        assert torch.equal(run(p, out).view(torch.int32).cpu(), want)
-        p.close()
-    finally:
-        del hog
-        torch.cuda.empty_cache()
+    torch.cuda.empty_cache()
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", SHORT_OF_MEMORY, kind, str(nbits), str(leave_mb)], cwd=root,
+                       capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
