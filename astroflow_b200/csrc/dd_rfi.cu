@@ -745,14 +745,15 @@ __global__ void __launch_bounds__(256) k_prep_fold(PrepArgs a) {
 // each output word passes once.  Channel words are read from c0 & ~3; RAGGED: rows do not
 // start on a word of four channels (nchans % 4 or the input's address), channels are
 // loaded one by one (2,870 channels x 75,001 samples folded 263 us, 1152 us with the
-// segment search and offset per sample of k_prep_fold).  Bound by issue (80 % busy) beside the memory: row
-// pointers and counts are set up once per thread, the tile comes from one 32-bit
+// segment search and offset per sample of k_prep_fold).  Bound by its loads beside the
+// memory (warps wait on them 4.4 cycles per issue, issue is 65 % busy, DRAM moves 4.9
+// TB/s): row pointers and counts are set up once per thread, the tile comes from one 32-bit
 // division, and nothing is 64-bit per load.  4096 channels x 151,000 samples in time
-// order 216 us (5.7 TB/s; 480 us with four loads in flight per thread and 64-bit rows),
-// 131,072 samples folded 690 us (5.1 TB/s; 905 us with every load and store predicated
-// and two-way bank conflicts).  The phase rows of downsampled brute force
-// are laid out by one launch, grid y = phase (WS 0: strides times ds, ws taken from the
-// arguments).
+// order 216 us (5.7 TB/s; 480 us with four loads in flight per thread and 64-bit rows);
+// 131,072 samples folded, delays to DM 3000, 480 us (2.4 GB; 690 us with all channels
+// written up to the plan's largest delay, 905 with every load and store predicated and
+// two-way bank conflicts).  The phase rows of downsampled brute force are laid out by one
+// launch, grid y = phase (WS 0: strides times ds, ws taken from the arguments).
 struct PrepWords {
   int64_t fs, nwords, pitch;  // nwords: words to store per channel; pitch in words
   int ws;
