@@ -86,8 +86,9 @@ def workspace_bound(n: int, c: int, bits: int, tsamp: float, fch1: float, foff: 
     step, ndm0 = kw.get("dm_step", 1.0), int(kw.get("ndm0", 32))
     brute = kw.get("algorithm", "subband") == "brute"
     nb = -(-n // ds)
-    f0, f1 = sorted((fch1, fch1 + (c - 1) * foff))
-    per_dm = 4148.808 * (1.0 / f0 ** 2 - 1.0 / f1 ** 2) / (tsamp if brute else tsamp * ds)
+    table = kw.get("freq_table")  # (files with one may leave fch1 at zero)
+    f0, f1 = sorted((fch1, fch1 + (c - 1) * foff)) if table is None else (float(min(table)), float(max(table)))
+    per_dm = 4148.808 * (1.0 / f0 ** 2 - 1.0 / f1 ** 2) / (tsamp if brute else tsamp * ds) if f0 > 0 else 0.0
     block = 16 * step * (1 if brute else ndm0) * per_dm  # spread of sixteen rows
     if brute:
         reach = int(per_dm * kw["dm_high"]) + 2
@@ -107,7 +108,7 @@ def workspace_bound(n: int, c: int, bits: int, tsamp: float, fch1: float, foff: 
         res = int(per_dm * ndm0 * step) + 2
         inter = max(per_col * (min(max((2 << 30) // per_col, least + res), cols + res) + pad)
                     for per_col, cols, least, pad in
-                    ((rows * 4, nb, 4096, 10240),  # time order: 32-bit sums, or 16-bit ones twice
+                    ((rows * 4, nb, 2048, 4352),  # time order: 32-bit sums, or 16-bit ones twice
                      (rows * (8 if packed else 4 * fold), nb // fold + 8, 1024, 1280)))
         tables = 8 * (nom * c + ndm * -(-c // width))
     rfi, windows = kw.get("rfi"), 0
