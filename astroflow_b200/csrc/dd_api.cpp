@@ -1348,6 +1348,9 @@ int dd_plan_set_delay_table(dd_plan* P, const int32_t* delay) {
         set_brute_window(*P);
       });
       DD_CUDA_TRY(cudaMemcpy(P->d_delay.p, delay, sizeof(int32_t) * P->h_delay.size(), cudaMemcpyHostToDevice));
+      // buffers, their zeros and the tables were queued on the legacy stream: runs may be on
+      // streams that do not wait for it
+      DD_CUDA_TRY(cudaStreamSynchronize(cudaStreamLegacy));
     } catch (...) {
       P->d_x.release();  // half set: runs are refused (check_buffers)
       throw;

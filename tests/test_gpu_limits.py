@@ -158,6 +158,31 @@ def test_folded_brute_force_holds_a_segment_and_the_largest_delay():
     plan.close()
 
 
+def test_runs_beside_the_legacy_stream_after_a_new_delay_table():
+    """A table whose delays change the layout's size takes new buffers; a run on a stream that
+    does not wait for the legacy one follows at once."""
+    from astroflow_b200.dedisp import Plan
+    from oracle import oracle as O
+
+    n, nc, tsamp = 20000, 300, 6.4e-5
+    freq = O.freq_table_fil(1000.0, 500.0 / nc, nc)
+    fs, fe = float(np.float32(freq[0])), float(np.float32(freq[-1]))
+    hdr = dict(tsamp=tsamp, fch1=1000.0, foff=500.0 / nc, nbits=8, nchans=nc, ndata=n)
+    plan = Plan(hdr, 0.0, 99.5, fs, fe, 1.0, 1, n * tsamp * 0.49, algorithm="brute", freq_mode="fil")
+    x = np.random.default_rng(9).integers(0, 256, (n, nc)).astype(np.uint8)
+    xd, out, own = dev(x), plan.empty_output(), plan.tables()[0]
+    side = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    for k in (3, 0, 2, 1):
+        table = (own * k // 3).astype(np.int32)
+        plan.set_delay_table(table)
+        plan.run(xd, out, side)
+        side.synchronize()
+        want = np.concatenate(O.bruteforce_cpu(x, nc, freq, tsamp, 0.0, 99.5, fs, fe, 1.0, 1, n * tsamp * 0.49,
+                                               delay=table), axis=1)
+        assert np.array_equal(to_np(out), want)
+
+
 # A folded chunk takes up to four times its bytes: with less memory left than that, the plan
 # keeps the chunk in time order (subband sums: shorter time tiles come first).  In a process
 # of its own, whose memory holds nothing else; MiB left for the plan or the stream (time order /
