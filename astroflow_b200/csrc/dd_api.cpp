@@ -98,6 +98,14 @@ int choose_fold(const dd_plan& P, int64_t ncols, int64_t nchan, int64_t reach, d
   const double extra = static_cast<double>(nchan) * (4.0 * words - static_cast<double>(P.nbin) * P.elem);
   return adds > 16.0 * extra ? fold : 1;
 }
+// Gives back what the pool still maps of released buffers, in pieces that need not fit the
+// next ones.
+void trim_pool(int device) {
+  DD_CUDA_TRY(cudaStreamSynchronize(cudaStreamLegacy));
+  cudaMemPool_t pool = nullptr;
+  DD_CUDA_TRY(cudaDeviceGetDefaultMemPool(&pool, device));
+  DD_CUDA_TRY(cudaMemPoolTrimTo(pool, 0));
+}
 // f(true), and f(false) where that runs out of device memory: a folded chunk takes up to four
 // times the bytes of one in time order.
 template <typename F>
@@ -109,11 +117,7 @@ void fold_if_it_fits(int device, F&& f) {
     if (e.code != DD_ERR_NOMEM) throw;
   }
   DeviceGuard g(device);
-  // the pool still maps what the failed attempt took, in pieces that need not fit the next
-  DD_CUDA_TRY(cudaStreamSynchronize(cudaStreamLegacy));
-  cudaMemPool_t pool = nullptr;
-  DD_CUDA_TRY(cudaDeviceGetDefaultMemPool(&pool, device));
-  DD_CUDA_TRY(cudaMemPoolTrimTo(pool, 0));
+  trim_pool(device);
   f(false);
 }
 // Refuses runs of a plan that a failed call (a delay table, autotuning) left without buffers.
@@ -458,69 +462,11 @@ void set_tiling(dd_plan& P, int64_t budget) {
   DD_CUDA_TRY(cudaStreamSynchronize(cudaStreamLegacy));
 }
 
-void create_subband(dd_plan& P) {
-  P.sbw = P.p.subband_width > 0 ? P.p.subband_width : 32;
-  P.ndm0 = P.p.ndm0 > 0 ? P.p.ndm0 : 32;
-  const int ds = P.p.time_downsample;
-  P.nbin = (P.nin + ds - 1) / ds;
-  if (P.nout <= 0 || P.nout > P.nbin) P.nout = P.nbin;
-  P.dch = P.ce - P.cs + 1;
-  P.nsb = (P.dch + P.sbw - 1) / P.sbw;
-  P.ndm_nom = (P.dm_steps + P.ndm0 - 1) / P.ndm0;
-  P.h_delay.assign(static_cast<size_t>(P.ndm_nom * P.dch), 0);
-  P.h_res.assign(static_cast<size_t>(P.dm_steps * P.nsb), 0);
-  DevBuf d_freq;
-  upload(d_freq, P.freq.data(), sizeof(double) * P.freq.size());
-  P.d_delay.alloc(sizeof(int32_t) * P.h_delay.size());
-  P.d_res.alloc(sizeof(int32_t) * P.h_res.size());
-  launch_subband_tables(d_freq.as<double>(), P.cs, P.ce, P.p.dm_low, P.p.dm_step, P.dm_steps,
-                        P.sbw, P.ndm0, P.ref_freq, P.tsamp, ds,
-                        P.d_delay.as<int32_t>(), P.d_res.as<int32_t>(), 0);
-  DD_CUDA_TRY(cudaMemcpy(P.h_delay.data(), P.d_delay.p, sizeof(int32_t) * P.h_delay.size(),
-                         cudaMemcpyDeviceToHost));
-  DD_CUDA_TRY(cudaMemcpy(P.h_res.data(), P.d_res.p, sizeof(int32_t) * P.h_res.size(),
-                         cudaMemcpyDeviceToHost));
-  // FP64 comparison table for the coarse delays (and replacement in FP64 mode).
-  int64_t mism = 0;
-  const double tsamp = P.tsamp, r = P.freq[P.ce];
-  std::vector<double> disp(static_cast<size_t>(P.dch));
-  for (int64_t c = 0; c < P.dch; ++c) {
-    const double f = P.freq[P.cs + c];
-    disp[c] = 1.0 / (f * f) - 1.0 / (r * r);
-  }
-  for (int64_t j = 0; j < P.ndm_nom; ++j) {
-    const double dm = static_cast<double>(P.p.dm_low) + static_cast<double>(j) * P.ndm0 * P.p.dm_step;
-    for (int64_t c = 0; c < P.dch; ++c) {
-      const int v = static_cast<int>(std::floor(4148.808 * dm * disp[c] / tsamp + 0.5)) / ds;
-      mism += (v != P.h_delay[j * P.dch + c]);
-      if (P.p.table_mode == DD_TABLE_FP64) P.h_delay[j * P.dch + c] = v;
-    }
-  }
-  if (P.p.table_mode == DD_TABLE_FP64) {
-    for (int64_t m = 0; m < P.dm_steps; ++m) {
-      const int64_t j = m / P.ndm0;
-      const double dd = (static_cast<double>(m) - static_cast<double>(j * P.ndm0)) * P.p.dm_step;
-      for (int64_t sb = 0; sb < P.nsb; ++sb) {
-        const int64_t ch0 = P.cs + sb * P.sbw;
-        const int64_t ch1 = std::min<int64_t>(ch0 + P.sbw, P.ce + 1);
-        const double f = P.freq[(ch0 + ch1 - 1) / 2];
-        P.h_res[m * P.nsb + sb] = static_cast<int>(std::floor(4148.808 * dd * (1.0 / (f * f) - 1.0 / (r * r)) / (tsamp * ds) + 0.5));
-      }
-    }
-    DD_CUDA_TRY(cudaMemcpy(P.d_delay.p, P.h_delay.data(), sizeof(int32_t) * P.h_delay.size(), cudaMemcpyHostToDevice));
-    DD_CUDA_TRY(cudaMemcpy(P.d_res.p, P.h_res.data(), sizeof(int32_t) * P.h_res.size(), cudaMemcpyHostToDevice));
-  }
-  P.table_mismatch_fp64 = mism;
-  int mind = 0, minr = 0;
-  P.max_delay = 0;
-  P.max_res = 0;
-  for (int v : P.h_delay) { P.max_delay = std::max(P.max_delay, v); mind = std::min(mind, v); }
-  for (int v : P.h_res) { P.max_res = std::max(P.max_res, v); minr = std::min(minr, v); }
-  if (mind < 0 || minr < 0)
-    throw invalid("negative dispersion delays (DM below zero or band order) are not supported");
-  P.inter16 = (P.nbits == 8 && P.sbw <= 64) ? 1 : 0;
-  P.adds = static_cast<double>(P.ndm_nom) * P.dch * P.nout +
-           static_cast<double>(P.dm_steps) * P.nsb * P.nout;
+// Layout, kernel variants and tiling of a subband plan whose tables are made, and the buffers
+// they take.
+void layout_subband(dd_plan& P) {
+  P.few1 = P.few2 = false;
+  P.twin = 0;
   {
     Stage1Tables t1 = stage1_tables(P, kSumRows);
     int spread2 = 0;
@@ -586,6 +532,72 @@ void create_subband(dd_plan& P) {
       if (e.code != DD_ERR_NOMEM || budget < (int64_t(128) << 20)) throw;  // else: shorter tiles
     }
   }
+}
+
+void create_subband(dd_plan& P) {
+  P.sbw = P.p.subband_width > 0 ? P.p.subband_width : 32;
+  P.ndm0 = P.p.ndm0 > 0 ? P.p.ndm0 : 32;
+  const int ds = P.p.time_downsample;
+  P.nbin = (P.nin + ds - 1) / ds;
+  if (P.nout <= 0 || P.nout > P.nbin) P.nout = P.nbin;
+  P.dch = P.ce - P.cs + 1;
+  P.nsb = (P.dch + P.sbw - 1) / P.sbw;
+  P.ndm_nom = (P.dm_steps + P.ndm0 - 1) / P.ndm0;
+  P.h_delay.assign(static_cast<size_t>(P.ndm_nom * P.dch), 0);
+  P.h_res.assign(static_cast<size_t>(P.dm_steps * P.nsb), 0);
+  DevBuf d_freq;
+  upload(d_freq, P.freq.data(), sizeof(double) * P.freq.size());
+  P.d_delay.alloc(sizeof(int32_t) * P.h_delay.size());
+  P.d_res.alloc(sizeof(int32_t) * P.h_res.size());
+  launch_subband_tables(d_freq.as<double>(), P.cs, P.ce, P.p.dm_low, P.p.dm_step, P.dm_steps,
+                        P.sbw, P.ndm0, P.ref_freq, P.tsamp, ds,
+                        P.d_delay.as<int32_t>(), P.d_res.as<int32_t>(), 0);
+  DD_CUDA_TRY(cudaMemcpy(P.h_delay.data(), P.d_delay.p, sizeof(int32_t) * P.h_delay.size(),
+                         cudaMemcpyDeviceToHost));
+  DD_CUDA_TRY(cudaMemcpy(P.h_res.data(), P.d_res.p, sizeof(int32_t) * P.h_res.size(),
+                         cudaMemcpyDeviceToHost));
+  // FP64 comparison table for the coarse delays (and replacement in FP64 mode).
+  int64_t mism = 0;
+  const double tsamp = P.tsamp, r = P.freq[P.ce];
+  std::vector<double> disp(static_cast<size_t>(P.dch));
+  for (int64_t c = 0; c < P.dch; ++c) {
+    const double f = P.freq[P.cs + c];
+    disp[c] = 1.0 / (f * f) - 1.0 / (r * r);
+  }
+  for (int64_t j = 0; j < P.ndm_nom; ++j) {
+    const double dm = static_cast<double>(P.p.dm_low) + static_cast<double>(j) * P.ndm0 * P.p.dm_step;
+    for (int64_t c = 0; c < P.dch; ++c) {
+      const int v = static_cast<int>(std::floor(4148.808 * dm * disp[c] / tsamp + 0.5)) / ds;
+      mism += (v != P.h_delay[j * P.dch + c]);
+      if (P.p.table_mode == DD_TABLE_FP64) P.h_delay[j * P.dch + c] = v;
+    }
+  }
+  if (P.p.table_mode == DD_TABLE_FP64) {
+    for (int64_t m = 0; m < P.dm_steps; ++m) {
+      const int64_t j = m / P.ndm0;
+      const double dd = (static_cast<double>(m) - static_cast<double>(j * P.ndm0)) * P.p.dm_step;
+      for (int64_t sb = 0; sb < P.nsb; ++sb) {
+        const int64_t ch0 = P.cs + sb * P.sbw;
+        const int64_t ch1 = std::min<int64_t>(ch0 + P.sbw, P.ce + 1);
+        const double f = P.freq[(ch0 + ch1 - 1) / 2];
+        P.h_res[m * P.nsb + sb] = static_cast<int>(std::floor(4148.808 * dd * (1.0 / (f * f) - 1.0 / (r * r)) / (tsamp * ds) + 0.5));
+      }
+    }
+    DD_CUDA_TRY(cudaMemcpy(P.d_delay.p, P.h_delay.data(), sizeof(int32_t) * P.h_delay.size(), cudaMemcpyHostToDevice));
+    DD_CUDA_TRY(cudaMemcpy(P.d_res.p, P.h_res.data(), sizeof(int32_t) * P.h_res.size(), cudaMemcpyHostToDevice));
+  }
+  P.table_mismatch_fp64 = mism;
+  int mind = 0, minr = 0;
+  P.max_delay = 0;
+  P.max_res = 0;
+  for (int v : P.h_delay) { P.max_delay = std::max(P.max_delay, v); mind = std::min(mind, v); }
+  for (int v : P.h_res) { P.max_res = std::max(P.max_res, v); minr = std::min(minr, v); }
+  if (mind < 0 || minr < 0)
+    throw invalid("negative dispersion delays (DM below zero or band order) are not supported");
+  P.inter16 = (P.nbits == 8 && P.sbw <= 64) ? 1 : 0;
+  P.adds = static_cast<double>(P.ndm_nom) * P.dch * P.nout +
+           static_cast<double>(P.dm_steps) * P.nsb * P.nout;
+  layout_subband(P);
   if (ds > 1 || callsite_zdm_active(P))
     P.d_binned.alloc(static_cast<size_t>(P.nbin * P.hdr.nchans) * P.elem);
   if (ds > 1 && binning_lut_entries(P.nbits, ds)) {
@@ -1490,6 +1502,18 @@ int dd_measure_int_add_rate(int32_t device, double* adds_per_second) {
 }
 
 namespace {
+// Lays the plan out again, folded or not, and waits for it.
+void relayout(dd_plan& P, bool may_fold) {
+  P.may_fold = may_fold;
+  ++P.generation;
+  P.d_x.release();
+  P.d_inter.release();
+  trim_pool(P.device);
+  if (P.p.algorithm == DD_ALGO_BRUTE) set_brute_window(P);
+  else layout_subband(P);
+  DD_CUDA_TRY(cudaStreamSynchronize(cudaStreamLegacy));
+}
+
 // Queues one host-path run on `st`: input copy, run, output copies (each time
 // tile's columns on the plan's copy stream while the next tile is summed).  Each
 // time tile's sums wait for the earlier queued run's copy of the same output
@@ -1509,13 +1533,30 @@ void enqueue_host_run(dd_plan& P, const void* h_input, void* h_output, cudaStrea
     DD_CUDA_TRY(cudaStreamSynchronize(st));
     P.host_pending = false;
   }
-  if (P.d_host_in.bytes < in_bytes) P.d_host_in.alloc(in_bytes);
-  if (P.d_host_out.bytes < out_bytes) {
-    P.d_host_out.release();
+  const auto buffers = [&] {
+    if (P.d_host_in.bytes < in_bytes) P.d_host_in.alloc(in_bytes);
+    if (P.d_host_out.bytes < out_bytes) {
+      P.d_host_out.release();
+      try {
+        P.d_host_out.alloc(out_bytes);
+      } catch (const Error& er) {
+        throw Error{DD_ERR_NOMEM, "output allocation failed: " + er.msg};
+      }
+    }
+  };
+  try {
+    buffers();
+  } catch (const Error& e) {
+    if (e.code != DD_ERR_NOMEM || P.fold == 1) throw;
+    // the chunk in time order may leave room for them
     try {
-      P.d_host_out.alloc(out_bytes);
-    } catch (const Error& er) {
-      throw Error{DD_ERR_NOMEM, "output allocation failed: " + er.msg};
+      P.d_host_in.release();
+      relayout(P, false);
+      buffers();
+    } catch (const Error&) {
+      P.d_host_in.release();
+      relayout(P, true);
+      throw;
     }
   }
   // buffers are allocated stream-ordered on the legacy stream: make them visible to `st`

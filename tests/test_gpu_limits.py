@@ -187,6 +187,7 @@ def test_runs_beside_the_legacy_stream_after_a_new_delay_table():
 # keeps the chunk in time order (subband sums: shorter time tiles come first).  In a process
 # of its own, whose memory holds nothing else; MiB left for the plan or the stream (time order /
 # folded take 480 / 658, 1143 / 1452 and, with the stream's own buffer, 2191 / 2409).
+# "host" has the plan and lacks memory for its host path's own buffers (577 MiB).
 SHORT_OF_MEMORY = """
 import sys
 import numpy as np
@@ -201,7 +202,7 @@ hdr = dict(tsamp=float(f32(1.6e-4)), fch1=400.0, foff=float(f32(400.0 / nc)), nb
 fe = float(f32(400.0) + f32(nc - 1) * f32(400.0 / nc))
 
 def make():
-    if kind == "brute":
+    if kind in ("brute", "host"):
         return Plan(hdr, 0.0, 800.0, 400.0, fe, 2.5, 1, n * 1.6e-4 * 0.49, algorithm="brute", freq_mode="fil")
     if kind == "subband":
         return Plan(hdr, 0.0, 600.0, 400.0, fe, 1.0, 1)
@@ -219,15 +220,24 @@ p.close()
 out.view(torch.int32).zero_()
 torch.cuda.synchronize()
 torch.cuda.empty_cache()
+if kind == "host":
+    p = make()
+    host = x.cpu().numpy()
+    del out
+    torch.cuda.empty_cache()
 hog = torch.empty(torch.cuda.mem_get_info()[0] - leave, dtype=torch.uint8, device="cuda")
-p = make()
-assert p.info["workspace_bytes"] < folded, (p.info["workspace_bytes"], folded)
-assert torch.equal(run(p), want)
+if kind == "host":
+    for _ in range(2):
+        assert np.array_equal(p.run_host(host).view(np.int32), want.numpy())
+else:
+    p = make()
+    assert p.info["workspace_bytes"] < folded, (p.info["workspace_bytes"], folded)
+    assert torch.equal(run(p), want)
 """
 
 
 @pytest.mark.parametrize("kind,nbits,leave_mb", [("brute", 8, 630), ("subband", 16, 1300), ("subband", 16, 800),
-                                                 ("stream", 16, 2310)])
+                                                 ("stream", 16, 2310), ("host", 8, 500)])
 def test_plans_whose_folded_layout_does_not_fit(kind, nbits, leave_mb):
     torch.cuda.empty_cache()
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
